@@ -427,6 +427,11 @@ __device__ void bconfig_adjoint(cgx::cluster_group& cl, const BatchArgs& a, cons
     Sw[i] = ldcg4(J.w + X.off + i);
   }
   __syncthreads();
+  blists(a, X, S, coul, (c.flags & BF_SR) != 0);
+  if (coul && polar) {
+    cl.sync();  // every CTA's partner lists
+    if (bcached(a, X)) bcache<false>(a, X, S);
+  }
   double g[kFitMax];
   for (int p = 0; p < kFitMax; ++p) g[p] = 0.0;
   int iters = 0;
@@ -438,16 +443,18 @@ __device__ void bconfig_adjoint(cgx::cluster_group& cl, const BatchArgs& a, cons
       double dm[3] = {0, 0, 0};
       if (a.ipol[gi]) {
         double4 si = S.s[i];
-        int ti = S.t[i];
+        int ti = btyp(S.t[i]);
         double4 mui = S.v[i], wi4 = Sw[i];
-        for (int j = lane; j < X.n; j += 32) {
-          if (j == i) continue;
+        const unsigned short* row = bnbl(a, X, 0, i);
+        const int nn = bnbn(a, X, 0)[i];
+        for (int k = lane; k < nn; k += 32) {
+          const int j = bnbr(row, k);
           double4 sj = S.s[j];
           double rxd, ryd, rzd;
           double r2d = min_image_exact(c.A, xsub(si.x, sj.x), xsub(si.y, sj.y), xsub(si.z, sj.z),
                                        rxd, ryd, rzd);
           if (r2d > c.rc2) continue;
-          int tj = S.t[j];
+          int tj = btyp(S.t[j]);
           double4 muj = S.v[j], wj4 = Sw[j];
           bool ia = half_mask(i, j);
           double sg = ia ? 1.0 : -1.0;
@@ -480,8 +487,8 @@ __device__ void bconfig_adjoint(cgx::cluster_group& cl, const BatchArgs& a, cons
       double4 o = make_double4(0, 0, 0, 0);
       if (a.ipol[gi]) {
         double4 rr = J.rhs[gi], rc = J.lam[gi];
-        double4 ax = bmat3(a.inv + 9 * (size_t)gi, a.x[gi]);
-        double4 E = a.E[gi];
+        double4 ax = bmat3(a.inv + 9 * (size_t)gi, ldcg4(a.x + gi));
+        double4 E = ldcg4(a.E + gi);
         double R[3] = {ax.x - E.x, ax.y - E.y, ax.z - E.z};
         double gm[3] = {0, 0, 0};
         if (J.gmu) {
@@ -523,51 +530,59 @@ __device__ void bconfig_adjoint(cgx::cluster_group& cl, const BatchArgs& a, cons
   for (int i = X.i0 + warp; i < X.i1; i += nwarp) {
     int gi = X.off + i;
     double4 si = S.s[i];
-    int ti = S.t[i];
+    int ti = btyp(S.t[i]);
     double4 mui = S.v[i], wi4 = Sw[i];
-    double4 li4 = J.lam[gi];
+    double4 li4 = ldcg4(J.lam + gi);
     double wi[3] = {wi4.x, wi4.y, wi4.z}, li[3] = {li4.x, li4.y, li4.z};
-    for (int j = lane; j < X.n; j += 32) {
-      if (j == i) continue;
+    if (any_sr) {
+      const unsigned short* row = bnbl(a, X, 1, i);
+      const int nn = bnbn(a, X, 1)[i];
+      for (int k = lane; k < nn; k += 32) {
+        const int j = bnbr(row, k);
+        double4 sj = S.s[j];
+        double r[3];
+        double r2d = min_image_exact(c.A, xsub(si.x, sj.x), xsub(si.y, sj.y), xsub(si.z, sj.z), r[0],
+                                     r[1], r[2]);
+        int tj = btyp(S.t[j]);
+        const NBPair& P = S.nb[ti * c.ntype + tj];
+        if (r2d < P.rcutsq) sr_pair_adjoint(PJ, P, lbmhftd, ti, tj, r2d, r, wi, g);
+      }
+    }
+    const unsigned short* row = bnbl(a, X, 0, i);
+    const int nn = any_es ? bnbn(a, X, 0)[i] : 0;
+    for (int k = lane; k < nn; k += 32) {
+      const int j = bnbr(row, k);
       double4 sj = S.s[j];
       double rxd, ryd, rzd;
       double r2d = min_image_exact(c.A, xsub(si.x, sj.x), xsub(si.y, sj.y), xsub(si.z, sj.z), rxd,
                                    ryd, rzd);
-      int tj = S.t[j];
-      if (any_sr) {
-        const NBPair& P = S.nb[ti * c.ntype + tj];
-        if (r2d < P.rcutsq) {
-          double r[3] = {rxd, ryd, rzd};
-          sr_pair_adjoint(PJ, P, lbmhftd, ti, tj, r2d, r, wi, g);
-        }
-      }
-      if (any_es && r2d <= c.rc2) {
-        double4 muj = S.v[j], wj4 = Sw[j];
-        bool ia = half_mask(i, j);
-        double sg = ia ? 1.0 : -1.0;
-        double r[3] = {sg * rxd, sg * ryd, sg * rzd};
-        double4 ma4 = ia ? mui : muj, mb4 = ia ? muj : mui, wa4 = ia ? wi4 : wj4, wb4 = ia ? wj4 : wi4;
-        double ma[3] = {ma4.x, ma4.y, ma4.z}, mb[3] = {mb4.x, mb4.y, mb4.z};
-        double wa[3] = {wa4.x, wa4.y, wa4.z}, wb[3] = {wb4.x, wb4.y, wb4.z};
-        double d3[3];
-        int ta = ia ? ti : tj, tb = ia ? tj : ti;
-        es_pair_adjoint(PJ, S.es[ta * c.ntype + tb], ta, tb, r2d, c.alpha, r, ia ? si.w : sj.w,
-                        ia ? sj.w : si.w, ma, mb, ma4.x != 0.0 || ma4.y != 0.0 || ma4.z != 0.0,
-                        mb4.x != 0.0 || mb4.y != 0.0 || mb4.z != 0.0, task_qq, task_qd, task_dd,
-                        wa, wb, li, ia, d3, g);
-      }
+      if (r2d > c.rc2) continue;
+      int tj = btyp(S.t[j]);
+      double4 muj = S.v[j], wj4 = Sw[j];
+      bool ia = half_mask(i, j);
+      double sg = ia ? 1.0 : -1.0;
+      double r[3] = {sg * rxd, sg * ryd, sg * rzd};
+      double4 ma4 = ia ? mui : muj, mb4 = ia ? muj : mui, wa4 = ia ? wi4 : wj4, wb4 = ia ? wj4 : wi4;
+      double ma[3] = {ma4.x, ma4.y, ma4.z}, mb[3] = {mb4.x, mb4.y, mb4.z};
+      double wa[3] = {wa4.x, wa4.y, wa4.z}, wb[3] = {wb4.x, wb4.y, wb4.z};
+      double d3[3];
+      int ta = ia ? ti : tj, tb = ia ? tj : ti;
+      es_pair_adjoint(PJ, S.es[ta * c.ntype + tb], ta, tb, r2d, c.alpha, r, ia ? si.w : sj.w,
+                      ia ? sj.w : si.w, ma, mb, ma4.x != 0.0 || ma4.y != 0.0 || ma4.z != 0.0,
+                      mb4.x != 0.0 || mb4.y != 0.0 || mb4.z != 0.0, task_qq, task_qd, task_dd,
+                      wa, wb, li, ia, d3, g);
     }
   }
   // per-ion terms: polarisability, self energy of the charges
   const double selfa = c.alpha / sqrt(kPi);
   for (int i = X.i0 + threadIdx.x; i < X.i1; i += blockDim.x) {
     int gi = X.off + i;
-    int ti = S.t[i];
+    int ti = btyp(S.t[i]);
     for (int p = 0; p < J.nparam; ++p) {
       const FitParam& fp = J.prm[p];
       if (fp.kind == FIT_POL && ti == fp.t1 && a.ipol[gi]) {
         double al = a.pol[9 * (size_t)gi];
-        double4 m = a.x[gi], l = J.lam[gi];
+        double4 m = ldcg4(a.x + gi), l = ldcg4(J.lam + gi);
         double mm = m.x * m.x + m.y * m.y + m.z * m.z, lm = l.x * m.x + l.y * m.y + l.z * m.z;
         g[p] += lm / (al * al) - 0.5 * gU * cu * mm / (al * al);
       }
@@ -636,15 +651,7 @@ __global__ void __launch_bounds__(512) k_batch_adjoint(BatchArgs a, AdjArgs J, i
     cl.sync();
     if (qpos >= a.nconf) break;
     int cfg = a.order[qpos];
-    const BConf* c = a.conf + cfg;
-    X.c = c;
-    X.cfg = cfg;
-    X.n = c->n;
-    X.off = c->off;
-    X.i0 = (int)((long long)X.n * X.rank / X.C);
-    X.i1 = (int)((long long)X.n * (X.rank + 1) / X.C);
-    X.part = a.part + (size_t)cfg * kBMaxC * 2 * kBPart;
-    X.parity = 0;
+    bctx_set(a, X, cfg);
     bconfig_adjoint(cl, a, J, X, S, Sw);
     __syncthreads();
   }

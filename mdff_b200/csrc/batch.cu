@@ -58,7 +58,19 @@ struct mdff_batch {
           *d_p = nullptr, *d_mu = nullptr, *d_E = nullptr;
   double2* d_tab64 = nullptr;
   float2* d_tab32 = nullptr;
-  double2* d_rho = nullptr;
+  // phase records and the workspaces of the resident CTAs (BatchArgs)
+  unsigned char* d_rec = nullptr;
+  unsigned char* d_ws = nullptr;  // the allocation that holds them
+  double4* d_rpart = nullptr;
+  double* d_gpart = nullptr;
+  unsigned short *d_nbl = nullptr, *d_cj = nullptr;
+  int *d_nbn = nullptr, *d_cn = nullptr;
+  double4* d_c64 = nullptr;
+  double* d_b64 = nullptr;
+  float4* d_c32 = nullptr;
+  float* d_b32 = nullptr;
+  size_t rpart_ld = 1, ccap = 0, npol_max = 0;
+  int ws_ctas = 0, ws_clusters = 0;  // CTAs and clusters the workspaces are sized for
   double *d_force = nullptr, *d_part = nullptr, *d_out = nullptr, *d_pack = nullptr;
   double* h_out = nullptr;
   // launch
@@ -155,7 +167,20 @@ BatchArgs make_args(mdff_batch* h, const double* d_pos, double* d_force) {
   a.s = h->d_s;
   a.tab64 = h->d_tab64;
   a.tab32 = h->d_tab32;
-  a.rho = h->d_rho;
+  a.rec = h->d_rec;
+  a.rpart = h->d_rpart;
+  a.rpart_ld = h->rpart_ld;
+  a.gpart = h->d_gpart;
+  a.wn = h->nmax;
+  a.nbl = h->d_nbl;
+  a.nbn = h->d_nbn;
+  a.ccap = h->ccap;
+  a.cj = h->d_cj;
+  a.cn = h->d_cn;
+  a.c64 = h->d_c64;
+  a.b64 = h->d_b64;
+  a.c32 = h->d_c32;
+  a.b32 = h->d_b32;
   a.Estat = h->d_Estat;
   a.x = h->d_x;
   a.r = h->d_r;
@@ -167,6 +192,73 @@ BatchArgs make_args(mdff_batch* h, const double* d_pos, double* d_force) {
   a.part = h->d_part;
   a.out = h->d_out;
   return a;
+}
+
+// Workspaces for `ncl` resident clusters of `cluster` CTAs: grown (never
+// shrunk) when a launch shape has more of them; the graph, which holds their
+// addresses, is rebuilt then.  The pair cache takes at most an eighth of the
+// device memory; boxes whose pairs do not fit recompute them.
+int ensure_workspace(mdff_batch* h, int ncl, int cluster) {
+  const int ctas = ncl * cluster;
+  if (ctas <= h->ws_ctas && ncl <= h->ws_clusters) return MDFF_OK;
+  BCK(cudaStreamSynchronize(h->st));
+  if (h->exec) {
+    cudaGraphExecDestroy(h->exec);
+    h->exec = nullptr;
+  }
+  if (h->d_ws) cudaFree(h->d_ws);
+  h->d_ws = nullptr;
+  const size_t nc = std::max(ctas, h->ws_ctas), nl = std::max(ncl, h->ws_clusters), wn = h->nmax;
+  h->ws_ctas = h->ws_clusters = 0;
+  // one allocation, carved up; nothing of it is read before it is written
+  const size_t entry = sizeof(double4) + sizeof(double) + sizeof(unsigned short) +
+                       (h->mixed ? sizeof(float4) + sizeof(float) : 0);
+  size_t mfree = 0, mtot = 0;
+  BCK(cudaMemGetInfo(&mfree, &mtot));
+  size_t cap = h->npol_max * h->npol_max;
+  cap = std::min(cap, std::min(mtot / 8, mfree / 2) / (entry * nl));
+  for (int pass = 0; pass < 2; ++pass) {
+    size_t o = 0;
+    auto take = [&](size_t bytes) {
+      const size_t at = o;
+      o += (bytes + 255) / 256 * 256;
+      return at;
+    };
+    const size_t o_rp = take(nc * 2 * h->rpart_ld * sizeof(double4));
+    const size_t o_gp = take(nc * kBSplit * 6 * wn * sizeof(double));
+    const size_t o_nl = take(nl * 2 * wn * wn * sizeof(unsigned short));
+    const size_t o_nn = take(nl * 2 * wn * sizeof(int));
+    const size_t o_cn = take(nl * wn * sizeof(int));
+    const size_t o_c64 = take(nl * cap * sizeof(double4)), o_b64 = take(nl * cap * sizeof(double));
+    const size_t o_cj = take(nl * cap * sizeof(unsigned short));
+    const size_t o_c32 = take(h->mixed ? nl * cap * sizeof(float4) : 0);
+    const size_t o_b32 = take(h->mixed ? nl * cap * sizeof(float) : 0);
+    if (cudaMalloc((void**)&h->d_ws, o) != cudaSuccess) {
+      cudaGetLastError();
+      h->d_ws = nullptr;
+      if (pass == 0 && cap > 0) {
+        cap = 0;  // no room for the pair cache: the boxes recompute their pairs
+        continue;
+      }
+      h->err = "cudaMalloc: workspace of the batched engine";
+      return MDFF_ERR_NOMEM;
+    }
+    h->d_rpart = (double4*)(h->d_ws + o_rp);
+    h->d_gpart = (double*)(h->d_ws + o_gp);
+    h->d_nbl = (unsigned short*)(h->d_ws + o_nl);
+    h->d_nbn = (int*)(h->d_ws + o_nn);
+    h->d_cn = (int*)(h->d_ws + o_cn);
+    h->d_c64 = (double4*)(h->d_ws + o_c64);
+    h->d_b64 = (double*)(h->d_ws + o_b64);
+    h->d_cj = (unsigned short*)(h->d_ws + o_cj);
+    h->d_c32 = (float4*)(h->d_ws + o_c32);
+    h->d_b32 = (float*)(h->d_ws + o_b32);
+    break;
+  }
+  h->ccap = cap;
+  h->ws_ctas = (int)nc;
+  h->ws_clusters = (int)nl;
+  return MDFF_OK;
 }
 
 // persistent grid: as many clusters as fit on the device at once (at most one
@@ -194,7 +286,7 @@ int prepare_shape(mdff_batch* h, Shape sh, int* nclusters) {
     return MDFF_ERR_CUDA;
   }
   *nclusters = std::min(ncl, h->nconf);
-  return MDFF_OK;
+  return ensure_workspace(h, *nclusters, sh.cluster);
 }
 
 int launch_batch(mdff_batch* h, const BatchArgs& a, Shape sh, int ncl, cudaStream_t st) {
@@ -338,7 +430,7 @@ int create_impl(mdff_batch* h, const mdff_params* psets, int npsets, const mdff_
   std::vector<ESPair> es;
   std::vector<int4> rows;
   std::vector<double> cost(h->nconf);
-  long long tab_total = 0;
+  long long tab_total = 0, rec_total = 0;
   long long ktot = 0;
   int ntot = 0;
   h->conf.resize(h->nconf);
@@ -425,12 +517,24 @@ int create_impl(mdff_batch* h, const mdff_params* psets, int npsets, const mdff_
     B.omega = S.L.omega;
     B.alpha = P.alphaES;
     B.rc2 = P.cutlongrange * P.cutlongrange;
+    B.rs2 = P.cutshortrange * P.cutshortrange;
     B.coul_unit = S.coul_unit;
     B.nb_off = (int)nb.size();
     B.es_off = (int)es.size();
     nb.insert(nb.end(), S.nb.begin(), S.nb.end());
     es.insert(es.end(), S.es.begin(), S.es.end());
-    typ.insert(typ.end(), S.itype.begin(), S.itype.end());
+    {
+      // packed words (batch_rec.cuh): type, polarisable flag, rank; the k-th
+      // polarisable ion in word k
+      std::vector<int> w(n);
+      int rk = 0;
+      for (int i = 0; i < (int)n; ++i) {
+        w[i] |= S.itype[i] | (S.ipol[i] ? 16 | (rk << 5) : 0);
+        if (S.ipol[i]) w[rk++] |= i << 16;
+      }
+      typ.insert(typ.end(), w.begin(), w.end());
+      h->npol_max = std::max(h->npol_max, (size_t)rk);
+    }
     ipol.insert(ipol.end(), S.ipol.begin(), S.ipol.end());
     q.insert(q.end(), S.q.begin(), S.q.end());
     pol.insert(pol.end(), S.pol.begin(), S.pol.end());
@@ -453,7 +557,22 @@ int create_impl(mdff_batch* h, const mdff_params* psets, int npsets, const mdff_
       B.ntab = P.kES[0] + 1 + P.kES[1] + 1 + std::max(P.kES[2], 4) + 1;
       B.tab_off = tab_total;
       B.tab_ld = (int)n;
-      tab_total += (long long)B.ntab * n;
+      // (boxes start on a 128-byte line: a line of one box is never read
+      // while another box's cluster writes it)
+      tab_total += ((long long)B.ntab * n + 15) / 16 * 16;
+      const int nz = B.kz + 1, nxy = B.kx + 1 + B.ky + 1;
+      B.t64 = brho_tile(nz, true);
+      B.t32 = brho_tile(nz, false);
+      B.kt = bfld_tile(nz);
+      B.zo64 = nxy * 16;
+      B.zo32 = (nxy * 8 + 15) / 16 * 16;
+      B.rs64 = (B.zo64 + (nz + B.t64 - 1) / B.t64 * B.t64 * 32 + 31) / 32 * 32;
+      B.rs32 = (B.zo32 + (nz + B.t32 - 1) / B.t32 * B.t32 * 16 + 31) / 32 * 32;
+      B.rec64 = rec_total;
+      rec_total += ((long long)B.rs64 * n + 127) / 128 * 128;
+      B.rec32 = rec_total;
+      if (h->mixed) rec_total += ((long long)B.rs32 * n + 127) / 128 * 128;
+      h->rpart_ld = std::max(h->rpart_ld, (size_t)B.nrows * nz);
       rows.insert(rows.end(), M.rows.begin(), M.rows.end());
       if (M.nk > 0) {
         Ak.insert(Ak.end(), M.Ak.begin(), M.Ak.begin() + M.nk);
@@ -506,7 +625,7 @@ int create_impl(mdff_batch* h, const mdff_params* psets, int npsets, const mdff_
   BALLOC(h->d_E, ntot);
   BALLOC(h->d_tab64, (size_t)std::max<long long>(tab_total, 1));
   if (h->mixed) BALLOC(h->d_tab32, (size_t)std::max<long long>(tab_total, 1));
-  BALLOC(h->d_rho, (size_t)std::max<long long>(ktot, 1));
+  BALLOC(h->d_rec, (size_t)std::max<long long>(rec_total, 1));
   BALLOC(h->d_force, 3 * (size_t)ntot);
   BALLOC(h->d_pack, 3 * (size_t)ntot);
   BALLOC(h->d_part, (size_t)h->nconf * kBMaxC * 2 * kBPart);
@@ -588,7 +707,7 @@ void destroy_impl(mdff_batch* h) {
   void* bufs[] = {h->d_conf, h->d_order, h->d_queue, h->d_typ, h->d_ipol, h->d_pos, h->d_q,
                   h->d_pol, h->d_inv, h->d_dip, h->d_nb, h->d_es, h->d_rows, h->d_Ak, h->d_kvec,
                   h->d_s, h->d_Estat, h->d_x, h->d_r, h->d_z, h->d_p, h->d_mu, h->d_E,
-                  h->d_tab64, h->d_tab32, h->d_rho, h->d_force, h->d_part, h->d_out, h->d_pack,
+                  h->d_tab64, h->d_tab32, h->d_rec, h->d_ws, h->d_force, h->d_part, h->d_out, h->d_pack,
                   h->d_w, h->d_rhs, h->d_lam, h->d_ch, h->d_grad, h->d_info, h->d_gin};
   for (void* b : bufs)
     if (b) cudaFree(b);
@@ -892,6 +1011,10 @@ int mdff_gpu_batch_adjoint(mdff_batch_handle h, const double* gE, const double* 
     return MDFF_ERR_CUDA;
   }
   ncl = std::min(ncl, h->nconf);
+  {
+    int s = ensure_workspace(h, ncl, sh.cluster);
+    if (s) return s;
+  }
   cfg.gridDim = dim3(sh.cluster * ncl);
   cfg.stream = h->st;
   BatchArgs a = make_args(h, h->graph_pos, h->graph_force);

@@ -28,6 +28,7 @@
 #include "common.cuh"
 #include "realspace.cuh"
 #include "recip.cuh"
+#include "batch_rec.cuh"
 
 namespace mdff {
 
@@ -35,8 +36,8 @@ namespace cgx = cooperative_groups;
 
 constexpr int kBMaxT = 4;          // types of a batched configuration
 constexpr int kBPart = 16;         // values per CTA partial slot
-constexpr int kBKChunk = 1024;     // k of rho' staged per shared-memory chunk
-constexpr int kBNZ = 8;            // nz per structure-factor work item
+constexpr int kBKChunk = 1024;     // double2 of the staging buffer (kBStage bytes)
+constexpr int kBNZ = 8;            // nz per work item of the adjoint's structure factors
 constexpr int kBMaxC = 8;          // largest cluster
 constexpr int kBSlots = 48;        // per-configuration scalar slots
 
@@ -73,6 +74,11 @@ struct BConf {
   int lwfc[kBMaxT];      // Wannier centres per type (BF_WFC): < 0 centre type
   int ldip_wfc, pad2;
   double rcut_wfc;
+  // phase records of the structure factor (batch_rec.cuh): byte offset of the
+  // box, bytes per ion, byte offset of Z in a record, n tile; FP64 and FP32
+  long long rec64, rec32;
+  int rs64, rs32, zo64, zo32, t64, t32, kt, pad3;
+  double rs2;            // largest squared short-range cutoff of the box
 };
 
 struct BatchArgs {
@@ -81,7 +87,7 @@ struct BatchArgs {
   const int* order;      // queue position -> configuration (descending cost)
   int* queue;            // zeroed before every launch
   const double* pos;     // [3][ntot] Cartesian
-  const int* typ;        // [ntot] type within its configuration
+  const int* typ;        // [ntot] packed type, polarisable flag and ranks (btyp, bpol, brank, bpl)
   const double* q;       // [ntot]
   const int* ipol;       // [ntot] polarisable flag (ldip_polar of the type)
   const double* pol;     // [ntot][9]
@@ -95,7 +101,23 @@ struct BatchArgs {
   double4* s;            // [ntot] direct coordinates, w = q
   double2* tab64;        // phase tables, [entry][ion] per configuration
   float2* tab32;
-  double2* rho;          // [sum nk] rho' = A_k rho
+  unsigned char* rec;    // phase records of every configuration
+  // workspace of the resident CTAs (blockIdx.x) and clusters (blockIdx.x / C)
+  double4* rpart;        // [CTA][2][rpart_ld] structure-factor partials
+  size_t rpart_ld;
+  double* gpart;         // [CTA][kBSplit][6][wn] field sums per row subset
+  int wn;                // ions per row of the workspaces (nmax)
+  unsigned short* nbl;   // [cluster][2][wn][wn] partners within the long / short cutoff
+  int* nbn;              // [cluster][2][wn]
+  // pair cache of the dipole operator, rows of the box's polarisable ions
+  // (npol entries each) when npol^2 <= ccap, else the pairs are recomputed
+  size_t ccap;           // entries per cluster
+  unsigned short* cj;
+  int* cn;               // [cluster][wn]
+  double4* c64;          // (rx, ry, rz, B2)
+  double* b64;           // B1
+  float4* c32;
+  float* b32;
   double4 *Estat, *x, *r, *z, *p, *mu;  // [ntot]
   double4* E;            // [ntot] final field
   double* force;         // [3][ntot]
@@ -155,8 +177,10 @@ __device__ inline BShared batch_smem(unsigned char* base, int nmax) {
 struct BCtx {
   const BConf* c;
   int cfg, rank, C, i0, i1, n, off;
+  int p0, p1, npol;  // this CTA's polarisable ions (ranks), of npol in the box
+  int slot;          // cluster index in the launch
   double* part;   // this configuration's partial slots
-  int parity;
+  int parity, rpar;
 };
 
 // Sum NV values over the cluster; every thread of every CTA receives the
@@ -195,10 +219,14 @@ __device__ __forceinline__ double4 ldcg4(const double4* p) {
 __device__ inline void gather_vec(const BCtx& X, const double4* __restrict__ g, double4* sh) {
   for (int i = threadIdx.x; i < X.n; i += blockDim.x) sh[i] = ldcg4(g + X.off + i);
 }
-__device__ inline void gather_vec32(const BCtx& X, const double4* __restrict__ g, float4* sh) {
-  for (int i = threadIdx.x; i < X.n; i += blockDim.x) {
-    double4 v = ldcg4(g + X.off + i);
-    sh[i] = make_float4((float)v.x, (float)v.y, (float)v.z, 0.f);
+// the polarisable ions' 4-vectors by rank (R = float: FP32 copies)
+__device__ inline void gather_pol(const BCtx& X, const int* t, const double4* __restrict__ g, double4* sh) {
+  for (int k = threadIdx.x; k < X.npol; k += blockDim.x) sh[k] = ldcg4(g + X.off + bpl(t[k]));
+}
+__device__ inline void gather_pol32(const BCtx& X, const int* t, const double4* __restrict__ g, float4* sh) {
+  for (int k = threadIdx.x; k < X.npol; k += blockDim.x) {
+    const double4 v = ldcg4(g + X.off + bpl(t[k]));
+    sh[k] = make_float4((float)v.x, (float)v.y, (float)v.z, 0.f);
   }
 }
 
@@ -245,248 +273,471 @@ __device__ __forceinline__ double3 bmvec(const BConf& c, double mx, double my, d
 }
 
 // ---------------------------------------------------------------------------
-// reciprocal space (multipole_ES_rec, ewald_rec.f90:38-365) of one
-// configuration.  Weights: q from S.s[].w (has_q), mu from S.v (FP64) or
-// S.v32 (FP32).  Adds the field into E[own] and, with forces, q E + F_mu into
-// force[own] * coul_unit.  With do_str, es[0..6] receives this CTA's share of
-// (u_rec, tau_rec) already scaled as k_rec_energy.
+// weights (q, 2 pi B^T mu) of list entry k for the structure factor: mode 0 all
+// ions (q and mu from S.s, S.v by ion), 1 / 2 the polarisable ions (no charge,
+// mu from S.v / S.v32 by rank)
 template <typename R>
-__device__ void brec(cgx::cluster_group& cl, const BatchArgs& a, BCtx& X, const BShared& S,
-                     bool has_q, bool has_mu, bool forces, bool do_str, double4* __restrict__ Eown,
-                     double* __restrict__ force, double (&es)[7]) {
-  typedef typename cplx<R>::T Cx;
+struct BWeights {
+  const BConf* c;
+  const double4* s;
+  const double4* v;
+  const float4* v32;
+  int n0, mode;
+  bool has_q, has_mu;
+  __device__ __forceinline__ void operator()(int k, R (&w)[4]) const {
+    double mx = 0.0, my = 0.0, mz = 0.0;
+    if (has_mu) {
+      if (mode == 2) {
+        const float4 m = v32[n0 + k];
+        mx = m.x;
+        my = m.y;
+        mz = m.z;
+      } else {
+        const double4 m = v[n0 + k];
+        mx = m.x;
+        my = m.y;
+        mz = m.z;
+      }
+    }
+    const double3 m = bmvec(*c, mx, my, mz);
+    w[0] = (mode == 0 && has_q) ? (R)s[n0 + k].w : R(0);
+    w[1] = (R)m.x;
+    w[2] = (R)m.y;
+    w[3] = (R)m.z;
+  }
+};
+
+template <typename R>
+struct BRhoArgs {
+  const BConf* c;
+  const int4* rows;
+  BList src;             // ions of the structure factor
+  const int* t;
+  unsigned char* stage;
+  const unsigned char* rec;
+  double4* out;          // this CTA's partials
+  BWeights<R> w;
+};
+template <typename R>
+struct BFldArgs {
+  const BConf* c;
+  const int4* rows;
+  BList dst;             // ions of the field
+  const int* t;
+  unsigned char* stage;
+  const typename cplx<R>::T* tab;
+  const double* Ak;
+  const double4* part;   // rank 0's partials
+  size_t pld;
+  int C;
+  double* gp;
+  int gld;
+  BWeights<R> w;
+};
+
+template <typename R, int T, bool HM>
+__device__ __noinline__ void brho_n(const BRhoArgs<R>& r) {
+  const BConf& c = *r.c;
+  brho_t<R, T, HM>(r.rec, sizeof(R) == 8 ? c.rs64 : c.rs32, sizeof(R) == 8 ? c.zo64 : c.zo32, c.kx, c.kz,
+                   r.rows, c.nrows, r.src, r.t, r.stage, r.out, r.w);
+}
+template <typename R, bool HM>
+__device__ __forceinline__ void brho(const BRhoArgs<R>& r) {
+  switch (sizeof(R) == 8 ? r.c->t64 : r.c->t32) {
+    case 5: if constexpr (sizeof(R) == 8) brho_n<R, 5, HM>(r); break;
+    case 6: brho_n<R, 6, HM>(r); break;
+    case 7: brho_n<R, 7, HM>(r); break;
+    case 8: brho_n<R, 8, HM>(r); break;
+    case 9: if constexpr (sizeof(R) == 4) brho_n<R, 9, HM>(r); break;
+    case 10: if constexpr (sizeof(R) == 4) brho_n<R, 10, HM>(r); break;
+    default: if constexpr (sizeof(R) == 4) brho_n<R, 13, HM>(r); break;
+  }
+}
+template <typename R, int KT, bool MUF>
+__device__ __noinline__ int bfld_n(const BFldArgs<R>& r) {
+  const BConf& c = *r.c;
+  return bfld_t<R, KT, MUF>(r.tab, c.tab_ld, c.kx, c.ky, c.kz, r.rows, c.nrows, r.Ak, r.part, r.pld, r.C,
+                            r.dst, r.t, r.stage, r.gp, r.gld, r.w);
+}
+template <typename R, bool MUF>
+__device__ __forceinline__ int bfld(const BFldArgs<R>& r) {
+  switch (r.c->kt) {
+    case 6: return bfld_n<R, 6, MUF>(r);
+    case 8: return bfld_n<R, 8, MUF>(r);
+    case 10: return bfld_n<R, 10, MUF>(r);
+    default: return bfld_n<R, 13, MUF>(r);
+  }
+}
+
+template <typename R>
+__device__ __forceinline__ const typename cplx<R>::T* btab_base(const BatchArgs& a, const BConf& c);
+template <>
+__device__ __forceinline__ const double2* btab_base<double>(const BatchArgs& a, const BConf& c) {
+  return a.tab64 + c.tab_off;
+}
+template <>
+__device__ __forceinline__ const float2* btab_base<float>(const BatchArgs& a, const BConf& c) {
+  return a.tab32 + c.tab_off;
+}
+
+// Reciprocal pass of one configuration.  src: the ions with weights (mode 0:
+// all of this CTA's ions with charges and / or the dipoles in S.v; 1 / 2: its
+// polarisable ions with the vector in S.v / S.v32 by rank).  The field sums are
+// left in this CTA's gpart for the ions of dst (all or polarisable);
+// bfld_get reads them.  With do_str, es[0..6] receives this CTA's share of
+// (u_rec, tau_rec) scaled as k_rec_energy.  Returns the number of row subsets.
+// RR: precision of the structure factor.  The mixed engine's static and force
+// passes form it in FP64 (its rounding is common to all ions of the box: with
+// FP32 the force error of 64-1000 ion MgO boxes was twice as large), the
+// operator of its inner iterations in FP32 (the FP64 residual removes it).
+template <typename R, typename RR>
+__device__ __noinline__ int brec(cgx::cluster_group& cl, const BatchArgs& a, BCtx& X, const BShared& S, int mode,
+                    bool has_q, bool has_mu, bool dst_pol, bool muf, bool do_str, double (&es)[7]) {
   const BConf& c = *X.c;
   for (int k = 0; k < 7; ++k) es[k] = 0.0;
-  if (c.nk == 0) return;
+  if (c.nk == 0) return 0;
+  const BList src = mode == 0 ? BList{X.i0, X.i1 - X.i0, false} : BList{X.p0, X.p1 - X.p0, true};
+  const BList dst = dst_pol ? BList{X.p0, X.p1 - X.p0, true} : BList{X.i0, X.i1 - X.i0, false};
   const int4* rows = a.rows + c.row_off;
-  const int kz = c.kz;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-  // readers of the previous rho' are done before it is overwritten
-  cl.sync();
-  // ---- rho over this CTA's rows, all ions; lanes split the ions -----------
-  int r0 = (int)((long long)c.nrows * X.rank / X.C), r1 = (int)((long long)c.nrows * (X.rank + 1) / X.C);
-  const int ntile = (2 * kz + 1 + kBNZ - 1) / kBNZ;
-  int nitems = (r1 - r0) * ntile;
-  for (int it = warp; it < nitems; it += nwarp) {
-    int row = r0 + it / ntile, tile = it % ntile;
-    int4 ri = rows[row];
-    int nx = ri.x, ny = ri.y;
-    int nz0 = ri.z + tile * kBNZ;
-    if (nz0 > kz) continue;  // warp-uniform
-    int nzn = min(kBNZ, kz - nz0 + 1);
-    R accR[kBNZ], accI[kBNZ];
-#pragma unroll
-    for (int t = 0; t < kBNZ; ++t) accR[t] = accI[t] = R(0);
-    for (int i = lane; i < X.n; i += 32) {
-      Cx XY = bphase<R>(a, c, i, nx, ny, 0);
-      Cx Z1 = btab<R>(a, c, c.kx + 1 + c.ky + 1 + 1, i);
-      R qv = has_q ? (R)S.s[i].w : R(0);
-      R km = R(0), m3 = R(0);
-      if (has_mu) {
-        double4 mu = S.v[i];
-        double3 m = bmvec(c, mu.x, mu.y, mu.z);
-        km = (R)(nx * m.x + ny * m.y + nz0 * m.z);
-        m3 = (R)m.z;
-      }
-      Cx P;
-#pragma unroll
-      for (int t = 0; t < kBNZ; ++t) {
-        if ((t & 3) == 0 && (t == 0 || sizeof(R) == 4)) {
-          int nz = min(nz0 + t, kz);
-          P = bphase_z<R>(a, c, i, XY, nz);
-        }
-        accR[t] += qv * P.x - km * P.y;
-        accI[t] += qv * P.y + km * P.x;
-        km += m3;
-        if (t + 1 < kBNZ && (((t + 1) & 3) != 0 || sizeof(R) == 8)) P = cmul(P, Z1);
-      }
-    }
-#pragma unroll
-    for (int t = 0; t < kBNZ; ++t) {
-      R vr = warp_sum(accR[t]);
-      R vi = warp_sum(accI[t]);
-      if (lane == 0 && t < nzn) {
-        int kl = ri.w + (nz0 - ri.z) + t;
-        double A = a.Ak[c.k_off + kl];
-        double rr = (double)vr, ii = (double)vi;
-        a.rho[c.k_off + kl] = make_double2(A * rr, A * ii);
-        if (do_str) {
-          double st = (rr * rr + ii * ii) * A;
-          double4 kv = a.kvec[c.k_off + kl];
-          es[0] += st;
-          es[1] += (1.0 - kv.w * kv.x * kv.x) * st;
-          es[2] += (1.0 - kv.w * kv.y * kv.y) * st;
-          es[3] += (1.0 - kv.w * kv.z * kv.z) * st;
-          es[4] -= kv.w * kv.x * kv.y * st;
-          es[5] -= kv.w * kv.x * kv.z * st;
-          es[6] -= kv.w * kv.y * kv.z * st;
-        }
-      }
-    }
+  unsigned char* stage = reinterpret_cast<unsigned char*>(S.rho);
+  const size_t pld = 2 * a.rpart_ld;  // CTA to CTA
+  const double4* part = a.rpart + ((size_t)(blockIdx.x - X.rank) * 2 + X.rpar) * a.rpart_ld;
+  {
+    BRhoArgs<RR> q;
+    q.c = X.c;
+    q.rows = rows;
+    q.src = src;
+    q.t = S.t;
+    q.stage = stage;
+    q.rec = a.rec + (sizeof(RR) == 8 ? c.rec64 : c.rec32);
+    q.out = a.rpart + ((size_t)blockIdx.x * 2 + X.rpar) * a.rpart_ld;
+    q.w = BWeights<RR>{X.c, S.s, S.v, S.v32, src.n0, mode, has_q, has_mu};
+    // (the partials are double-buffered: a reader of the previous pass's half
+    // has passed this pass's barrier before that half is written again)
+    X.rpar ^= 1;
+    if (has_mu) brho<RR, true>(q);
+    else brho<RR, false>(q);
   }
+  cl.sync();
+  BFldArgs<R> r;
+  r.c = X.c;
+  r.rows = rows;
+  r.dst = dst;
+  r.t = S.t;
+  r.stage = stage;
+  r.tab = btab_base<R>(a, c);
+  r.Ak = a.Ak + c.k_off;
+  r.part = part;
+  r.pld = pld;
+  r.C = X.C;
+  r.gp = a.gpart + (size_t)blockIdx.x * kBSplit * 6 * a.wn;
+  r.gld = a.wn;
+  r.w = BWeights<R>{X.c, S.s, S.v, S.v32, dst.n0, 0, false, true};
   if (do_str) {
-    double tpi_V = kTwoPi / c.omega;
+    // energy and stress of this CTA's share of the rows
+    const int nz = c.kz + 1;
+    const double4* kv0 = a.kvec + c.k_off;
+    const int r0 = (int)((long long)c.nrows * X.rank / X.C), r1 = (int)((long long)c.nrows * (X.rank + 1) / X.C);
+    for (int e = threadIdx.x; e < (r1 - r0) * nz; e += blockDim.x) {
+      const int row = r0 + e / nz, n = e % nz;
+      const int4 ri = rows[row];
+      double2 rp, rm;
+      brho_pm(part, pld, X.C, nz, ri, row, n, nullptr, rp, rm);
+      for (int sg = 0; sg < 2; ++sg) {
+        if (sg ? !(n > 0 && ri.z < 0) : n < ri.z) continue;
+        const int k = ri.w + (sg ? -n : n) - ri.z;
+        const double2 v = sg ? rm : rp;
+        const double st = (v.x * v.x + v.y * v.y) * r.Ak[k];
+        const double4 kv = kv0[k];
+        es[0] += st;
+        es[1] += (1.0 - kv.w * kv.x * kv.x) * st;
+        es[2] += (1.0 - kv.w * kv.y * kv.y) * st;
+        es[3] += (1.0 - kv.w * kv.z * kv.z) * st;
+        es[4] -= kv.w * kv.x * kv.y * st;
+        es[5] -= kv.w * kv.x * kv.z * st;
+        es[6] -= kv.w * kv.y * kv.z * st;
+      }
+    }
+    const double tpi_V = kTwoPi / c.omega;
     es[0] *= 2.0 * tpi_V;
     for (int k = 1; k < 7; ++k) es[k] *= 2.0 * tpi_V / c.omega;
   }
-  cl.sync();
-  // ---- field / force of this CTA's ions over all k -----------------------
-  const bool muf = forces && has_mu;
-  int mown = X.i1 - X.i0;
-  int sub = 1;
-  while (sub < 32 && mown * sub * 2 <= (int)blockDim.x) sub *= 2;
-  int slots = blockDim.x / sub;
-  int iters = (mown + slots - 1) / slots;
-  const double scale = 2.0 * (2.0 * (kTwoPi / c.omega));
-  for (int itn = 0; itn < iters; ++itn) {
-    int slot = itn * slots + (int)threadIdx.x / sub;
-    int me = threadIdx.x % sub;
-    bool act = slot < mown;
-    int i = X.i0 + (act ? slot : 0);
-    double G[3] = {0, 0, 0}, H[3] = {0, 0, 0};
-    R m1 = R(0), m2 = R(0), m3 = R(0);
-    if (muf) {
-      double4 mu = S.v[i];
-      double3 m = bmvec(c, mu.x, mu.y, mu.z);
-      m1 = (R)m.x;
-      m2 = (R)m.y;
-      m3 = (R)m.z;
-    }
-    Cx Z1 = btab<R>(a, c, c.kx + 1 + c.ky + 1 + 1, i);
-    int ra = 0;
-    while (ra < c.nrows) {
-      int kbase = rows[ra].w;
-      int rb = ra;
-      while (rb < c.nrows) {
-        int4 rr = rows[rb];
-        if (rr.w + (kz - rr.z + 1) - kbase > kBKChunk) break;
-        ++rb;
-      }
-      int kend = (rb < c.nrows) ? rows[rb].w : c.nk;
-      __syncthreads();
-      for (int k = threadIdx.x; k < kend - kbase; k += blockDim.x)
-        S.rho[k] = __ldcg(a.rho + c.k_off + kbase + k);
-      __syncthreads();
-      if (act) {
-        for (int r = ra + me; r < rb; r += sub) {
-          int4 ri = rows[r];
-          int nx = ri.x, ny = ri.y, nz_lo = ri.z;
-          Cx XY = bphase<R>(a, c, i, nx, ny, 0);
-          Cx P = bphase_z<R>(a, c, i, XY, nz_lo);
-          R S0 = R(0), Sz = R(0), T0 = R(0), Tz = R(0);
-          R km = muf ? (R)nx * m1 + (R)ny * m2 + (R)nz_lo * m3 : R(0);
-          int nn = kz - nz_lo + 1;
-          const double2* rr = S.rho + (ri.w - kbase);
-          R tf = R(0);
-          for (int t = 0; t < nn; ++t, tf += R(1)) {
-            if (sizeof(R) == 4 && t > 0 && (t & 3) == 0) P = bphase_z<R>(a, c, i, XY, nz_lo + t);
-            double2 rv = rr[t];
-            R rhoR = (R)rv.x, rhoI = (R)rv.y;
-            R recarg = rhoI * P.x - rhoR * P.y;
-            S0 += recarg;
-            Sz += tf * recarg;
-            if (muf) {
-              R tt = km * (rhoR * P.x + rhoI * P.y);
-              T0 += tt;
-              Tz += tf * tt;
-              km += m3;
-            }
-            P = cmul(P, Z1);
-          }
-          G[0] += (double)nx * (double)S0;
-          G[1] += (double)ny * (double)S0;
-          G[2] += (double)nz_lo * (double)S0 + (double)Sz;
-          if (muf) {
-            H[0] += (double)nx * (double)T0;
-            H[1] += (double)ny * (double)T0;
-            H[2] += (double)nz_lo * (double)T0 + (double)Tz;
-          }
-        }
-      }
-      ra = rb;
-    }
-    // sum the sub-threads of the ion (consecutive lanes)
-    for (int o = 1; o < sub; o <<= 1)
+  if (muf) return bfld<R, true>(r);
+  return bfld<R, false>(r);
+}
+
+// field e (and dipole force fm) of list entry k from the row subsets' sums
+__device__ __forceinline__ void bfld_get(const BatchArgs& a, const BConf& c, int RS, int k, bool muf,
+                                         double (&e)[3], double (&fm)[3]) {
+  const double* gp = a.gpart + (size_t)blockIdx.x * kBSplit * 6 * a.wn;
+  double G[3] = {0, 0, 0}, H[3] = {0, 0, 0};
+  for (int s = 0; s < RS; ++s)
 #pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        G[d] += __shfl_xor_sync(FULL_MASK, G[d], o);
-        H[d] += __shfl_xor_sync(FULL_MASK, H[d], o);
-      }
-    if (act && me == 0) {
-      double e[3], fm[3];
-      for (int d = 0; d < 3; ++d) {
-        e[d] = -kTwoPi * (c.B[3 * d] * G[0] + c.B[3 * d + 1] * G[1] + c.B[3 * d + 2] * G[2]) * scale;
-        fm[d] = kTwoPi * (c.B[3 * d] * H[0] + c.B[3 * d + 1] * H[1] + c.B[3 * d + 2] * H[2]) * scale;
-      }
-      int gi = X.off + i;
-      double4 o = Eown[gi];
-      Eown[gi] = make_double4(o.x + e[0], o.y + e[1], o.z + e[2], 0.0);
-      if (forces) {
-        double qi = S.s[i].w;
-        force[gi] += (qi * e[0] + (muf ? fm[0] : 0.0)) * c.coul_unit;
-        force[a.ntot + gi] += (qi * e[1] + (muf ? fm[1] : 0.0)) * c.coul_unit;
-        force[2 * (size_t)a.ntot + gi] += (qi * e[2] + (muf ? fm[2] : 0.0)) * c.coul_unit;
-      }
+    for (int d = 0; d < 3; ++d) {
+      G[d] += gp[(size_t)(s * 6 + d) * a.wn + k];
+      if (muf) H[d] += gp[(size_t)(s * 6 + 3 + d) * a.wn + k];
     }
+  const double scale = 2.0 * (2.0 * (kTwoPi / c.omega));
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    e[d] = -kTwoPi * (c.B[3 * d] * G[0] + c.B[3 * d + 1] * G[1] + c.B[3 * d + 2] * G[2]) * scale;
+    fm[d] = kTwoPi * (c.B[3 * d] * H[0] + c.B[3 * d + 1] * H[1] + c.B[3 * d + 2] * H[2]) * scale;
   }
 }
 
 // ---------------------------------------------------------------------------
-// real-space field of the vector in S.v / S.v32 on this CTA's ions (warp per
-// ion, lanes over all ions of the box).  QQ: damped charge field; DD: dipole
-// field with dd_mask as k_es_field.  Result added into E[own].
+// Partner lists of this CTA's ions, ascending, within the long-range (which =
+// 0) and the short-range (1) cutoff plus a margin: every later pair loop walks
+// these (and takes the exact inclusion decision itself) instead of all ions of
+// the box, half of which lie outside the half-box cutoff and nearly all
+// outside a 4-6 A short-range cutoff.  The test is FP32 on coordinates wrapped
+// to [-0.5, 0.5); the margin covers its rounding, and a pair whose image is
+// ambiguous at that precision is always kept.
+__device__ __forceinline__ unsigned short* bnbl(const BatchArgs& a, const BCtx& X, int which, int i) {
+  return a.nbl + (((size_t)X.slot * 2 + which) * a.wn + i) * a.wn;
+}
+__device__ __forceinline__ int* bnbn(const BatchArgs& a, const BCtx& X, int which) {
+  return a.nbn + ((size_t)X.slot * 2 + which) * a.wn;
+}
+__device__ __noinline__ void blists(const BatchArgs& a, const BCtx& X, const BShared& S, bool coul, bool sr) {
+  const BConf& c = *X.c;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+  for (int i = threadIdx.x; i < X.n; i += blockDim.x) {
+    const double4 s = S.s[i];
+    S.v32[i] = make_float4((float)(s.x - rint(s.x)), (float)(s.y - rint(s.y)), (float)(s.z - rint(s.z)), 0.f);
+  }
+  __syncthreads();
+  float A[9];
+  float amax = 0.f;
+#pragma unroll
+  for (int k = 0; k < 9; ++k) {
+    A[k] = (float)c.A[k];
+    amax += fabsf(A[k]);
+  }
+  // rounding of r: 3 coordinates of 2^-24 each times the cell, 4x margin
+  const float rl = sqrtf((float)c.rc2), rs = sqrtf((float)c.rs2);
+  const float l2 = coul ? (float)c.rc2 * 1.00001f + 2e-6f * amax * rl : -1.f;
+  const float s2 = sr ? (float)c.rs2 * 1.00001f + 2e-6f * amax * rs : -1.f;
+  for (int i = X.i0 + warp; i < X.i1; i += nwarp) {
+    const float4 si = S.v32[i];
+    unsigned short *ll = bnbl(a, X, 0, i), *ls = bnbl(a, X, 1, i);
+    int ml = 0, ms = 0;
+    for (int j0 = 0; j0 < X.n; j0 += 32) {
+      const int j = j0 + lane;
+      bool kl = false, ksr = false;
+      if (j < X.n && j != i) {
+        const float4 sj = S.v32[j];
+        float dx = si.x - sj.x, dy = si.y - sj.y, dz = si.z - sj.z;
+        // nearest integer by the 2^23 shift (|d| <= 1)
+        dx -= __fadd_rn(__fadd_rn(dx, 12582912.f), -12582912.f);
+        dy -= __fadd_rn(__fadd_rn(dy, 12582912.f), -12582912.f);
+        dz -= __fadd_rn(__fadd_rn(dz, 12582912.f), -12582912.f);
+        const float x = A[0] * dx + A[1] * dy + A[2] * dz;
+        const float y = A[3] * dx + A[4] * dy + A[5] * dz;
+        const float z = A[6] * dx + A[7] * dy + A[8] * dz;
+        const float r2 = x * x + y * y + z * z;
+        const bool edge = fmaxf(fabsf(dx), fmaxf(fabsf(dy), fabsf(dz))) > 0.49999f;
+        kl = coul && (r2 <= l2 || edge);
+        ksr = sr && (r2 <= s2 || edge);
+      }
+      const unsigned bl = __ballot_sync(FULL_MASK, kl), bs = __ballot_sync(FULL_MASK, ksr);
+      const unsigned lt = (1u << lane) - 1u;
+      if (kl) ll[ml + __popc(bl & lt)] = (unsigned short)j;
+      if (ksr) ls[ms + __popc(bs & lt)] = (unsigned short)j;
+      ml += __popc(bl);
+      ms += __popc(bs);
+    }
+    if (lane == 0) {
+      bnbn(a, X, 0)[i] = ml;
+      bnbn(a, X, 1)[i] = ms;
+    }
+  }
+  __syncthreads();
+}
+// the lists are rewritten for every box a cluster takes and may have been
+// written by another CTA: read through L2
+__device__ __forceinline__ int bnbr(const unsigned short* l, int k) { return (int)__ldcg(l + k); }
+
+// ---------------------------------------------------------------------------
+// real-space field of the vector in S.v / S.v32 on this CTA's polarisable ions
+// (warp per ion, lanes over its partner list), added into E.  QQ: damped charge field; DD:
+// dipole field.  pol = false: vectors by ion, the reference's condition (both
+// dipoles nonzero); true: vectors by rank, both ions polarisable.
 template <typename R, bool QQ, bool DD>
-__device__ void bfield(const BatchArgs& a, const BCtx& X, const BShared& S, int damp, int dd_mask,
+__device__ __noinline__ void bfield(const BatchArgs& a, const BCtx& X, const BShared& S, int damp, bool pol,
                        double4* __restrict__ E) {
   const BConf& c = *X.c;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
   const R rc2 = (R)c.rc2;
-  for (int i = X.i0 + warp; i < X.i1; i += nwarp) {
-    double4 si = S.s[i];
-    int ti = S.t[i];
-    bool dip_i = false;
-    if (DD) {
-      if (dd_mask) dip_i = a.ipol[X.off + i] != 0;
-      else {
-        double4 m = S.v[i];
-        dip_i = m.x != 0 || m.y != 0 || m.z != 0;
-      }
+  for (int p = X.p0 + warp; p < X.p1; p += nwarp) {
+    const int i = bpl(S.t[p]);
+    const double4 si = S.s[i];
+    const int ti = btyp(S.t[i]);
+    bool dip_i = pol;
+    if (DD && !pol) {
+      const double4 m = S.v[i];
+      dip_i = m.x != 0 || m.y != 0 || m.z != 0;
     }
     R ex = R(0), ey = R(0), ez = R(0);
-    if (QQ || dip_i) {
-      for (int j = lane; j < X.n; j += 32) {
-        if (j == i) continue;
-        double4 sj = S.s[j];
-        R rx, ry, rz;
-        R r2 = pair_vec<R>(c.A, si, sj, rx, ry, rz);
-        if (r2 > rc2) continue;  // ewald_dir.f90:202
-        R mx = R(0), my = R(0), mz = R(0);
-        bool dd = false;
-        if (DD && dip_i) {
-          if (sizeof(R) == 4) {
-            float4 m = S.v32[j];
-            mx = (R)m.x; my = (R)m.y; mz = (R)m.z;
-          } else {
-            double4 m = S.v[j];
-            mx = (R)m.x; my = (R)m.y; mz = (R)m.z;
+    const unsigned short* row = bnbl(a, X, 0, i);
+    const int nn = (QQ || dip_i) ? __ldcg(bnbn(a, X, 0) + i) : 0;
+    for (int k = lane; k < nn; k += 32) {
+      const int j = bnbr(row, k);
+      const double4 sj = S.s[j];
+      const int tj = S.t[j];
+      R rx, ry, rz;
+      const R r2 = pair_vec<R>(c.A, si, sj, rx, ry, rz);
+      if (r2 > rc2) continue;  // ewald_dir.f90:202
+      R mx = R(0), my = R(0), mz = R(0);
+      bool dd = false;
+      if (DD && dip_i) {
+        if (pol) {
+          dd = bpol(tj);
+          if (dd) {
+            if (sizeof(R) == 4) {
+              const float4 m = S.v32[brank(tj)];
+              mx = (R)m.x; my = (R)m.y; mz = (R)m.z;
+            } else {
+              const double4 m = S.v[brank(tj)];
+              mx = (R)m.x; my = (R)m.y; mz = (R)m.z;
+            }
           }
-          if (dd_mask) {
-            dd = a.ipol[X.off + j] != 0;
-          } else {
-            double4 m = S.v[j];
-            dd = m.x != 0 || m.y != 0 || m.z != 0;
+        } else {
+          const double4 m = S.v[j];
+          mx = (R)m.x; my = (R)m.y; mz = (R)m.z;
+          dd = m.x != 0 || m.y != 0 || m.z != 0;
+        }
+      }
+      const double qj = QQ ? sj.w : 0.0;
+      if (!dd && (!QQ || qj == 0.0)) continue;
+      es_field_pair<R, QQ, DD>(S.es, c.ntype, i, j, ti, btyp(tj), rx, ry, rz, r2, (R)c.alpha, damp,
+                               qj, dd, mx, my, mz, ex, ey, ez, (c.flags & BF_THOLE) ? 1 : 0);
+    }
+    const double dx = warp_sum((double)ex), dy = warp_sum((double)ey), dz = warp_sum((double)ez);
+    if (lane == 0) {
+      const int gi = X.off + i;
+      const double4 o = E[gi];
+      E[gi] = make_double4(o.x + dx, o.y + dy, o.z + dz, 0.0);
+    }
+  }
+}
+
+// Pair cache of the dipole operator: for every polarisable ion of this CTA the
+// terms of T2(r) mu = B2 r (r.mu) - B1 mu of its polarisable partners within
+// the cutoff, formed once per box in FP64 (the operator is applied a dozen
+// times); MIXED keeps an FP32 copy for the inner iterations.  Row p (rank)
+// starts at p * npol.
+__device__ __forceinline__ bool bcached(const BatchArgs& a, const BCtx& X) {
+  return (size_t)X.npol * X.npol <= a.ccap;
+}
+template <bool MIXED>
+__device__ __noinline__ void bcache(const BatchArgs& a, const BCtx& X, const BShared& S) {
+  const BConf& c = *X.c;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+  const int thole = (c.flags & BF_THOLE) ? 1 : 0;
+  for (int p = X.p0 + warp; p < X.p1; p += nwarp) {
+    const int i = bpl(S.t[p]);
+    const double4 si = S.s[i];
+    const int ti = btyp(S.t[i]);
+    const unsigned short* row = bnbl(a, X, 0, i);
+    const int nn = __ldcg(bnbn(a, X, 0) + i);
+    const size_t base = (size_t)X.slot * a.ccap + (size_t)p * X.npol;
+    int m = 0;
+    for (int k0 = 0; k0 < nn; k0 += 32) {
+      const int k = k0 + lane;
+      bool keep = false;
+      double rx = 0, ry = 0, rz = 0, B1 = 0, B2 = 0;
+      int rk = 0;
+      if (k < nn) {
+        const int j = bnbr(row, k);
+        const int tj = S.t[j];
+        if (bpol(tj)) {
+          const double r2 = pair_vec<double>(c.A, si, S.s[j], rx, ry, rz);
+          if (r2 <= c.rc2) {
+            keep = true;
+            rk = brank(tj);
+            Radial<double> g;
+            radial<double, false>(r2, c.alpha, g);
+            double F1 = g.F1, F2 = g.F2;
+            if (thole) {
+              const bool ia = half_mask(i, j);
+              const int tjt = btyp(tj);
+              const ESPair& P = S.es[(ia ? ti : tjt) * c.ntype + (ia ? tjt : ti)];
+              if (P.thole) thole_radial<double>(P, g.d, F1, F2);
+            }
+            B1 = F1 * g.dm3;
+            B2 = 3.0 * F2 * g.dm5;
           }
         }
-        double qj = QQ ? sj.w : 0.0;
-        if (!dd && (!QQ || qj == 0.0)) continue;
-        es_field_pair<R, QQ, DD>(S.es, c.ntype, i, j, ti, S.t[j], rx, ry, rz, r2, (R)c.alpha, damp,
-                                 qj, dd, mx, my, mz, ex, ey, ez, (c.flags & BF_THOLE) ? 1 : 0);
+      }
+      const unsigned bal = __ballot_sync(FULL_MASK, keep);
+      if (keep) {
+        const size_t o = base + m + __popc(bal & ((1u << lane) - 1u));
+        a.cj[o] = (unsigned short)rk;
+        a.c64[o] = make_double4(rx, ry, rz, B2);
+        a.b64[o] = B1;
+        if (MIXED) {
+          a.c32[o] = make_float4((float)rx, (float)ry, (float)rz, (float)B2);
+          a.b32[o] = (float)B1;
+        }
+      }
+      m += __popc(bal);
+    }
+    if (lane == 0) a.cn[(size_t)X.slot * a.wn + p] = m;
+  }
+  __syncthreads();
+}
+
+// T2 v of the cached pairs on this CTA's polarisable ions (vector in S.v / S.v32
+// by rank), added into E
+template <typename R>
+__device__ __noinline__ void bfield_cached(const BatchArgs& a, const BCtx& X, const BShared& S, double4* __restrict__ E) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+  for (int p = X.p0 + warp; p < X.p1; p += nwarp) {
+    const size_t base = (size_t)X.slot * a.ccap + (size_t)p * X.npol;
+    const int n = a.cn[(size_t)X.slot * a.wn + p];
+    R ex = R(0), ey = R(0), ez = R(0);
+    constexpr int U = 4;
+    for (int k0 = lane; k0 < n; k0 += 32 * U) {
+      R x[U], y[U], z[U], b2[U], b1[U];
+      int j[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int k = k0 + 32 * u;
+        const bool ok = k < n;
+        const size_t o = base + (ok ? k : k0);
+        j[u] = a.cj[o];
+        if (sizeof(R) == 4) {
+          const float4 r = a.c32[o];
+          x[u] = (R)r.x; y[u] = (R)r.y; z[u] = (R)r.z; b2[u] = (R)r.w;
+          b1[u] = (R)a.b32[o];
+        } else {
+          const double4 r = a.c64[o];
+          x[u] = (R)r.x; y[u] = (R)r.y; z[u] = (R)r.z; b2[u] = (R)r.w;
+          b1[u] = (R)a.b64[o];
+        }
+        if (!ok) b2[u] = b1[u] = R(0);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        R mx, my, mz;
+        if (sizeof(R) == 4) {
+          const float4 m = S.v32[j[u]];
+          mx = (R)m.x; my = (R)m.y; mz = (R)m.z;
+        } else {
+          const double4 m = S.v[j[u]];
+          mx = (R)m.x; my = (R)m.y; mz = (R)m.z;
+        }
+        const R rm = b2[u] * (x[u] * mx + y[u] * my + z[u] * mz);
+        ex += rm * x[u] - b1[u] * mx;
+        ey += rm * y[u] - b1[u] * my;
+        ez += rm * z[u] - b1[u] * mz;
       }
     }
-    double dx = warp_sum((double)ex), dy = warp_sum((double)ey), dz = warp_sum((double)ez);
+    const double dx = warp_sum((double)ex), dy = warp_sum((double)ey), dz = warp_sum((double)ez);
     if (lane == 0) {
-      int gi = X.off + i;
-      double4 o = E[gi];
+      const int gi = X.off + bpl(S.t[p]);
+      const double4 o = E[gi];
       E[gi] = make_double4(o.x + dx, o.y + dy, o.z + dz, 0.0);
     }
   }
@@ -495,7 +746,7 @@ __device__ void bfield(const BatchArgs& a, const BCtx& X, const BShared& S, int 
 // ---------------------------------------------------------------------------
 // short range (FP64) on this CTA's ions: forces overwrite force[own];
 // acc[16] as k_shortrange.
-__device__ void bshort(const BatchArgs& a, const BCtx& X, const BShared& S, double (&acc)[kSRPart]) {
+__device__ __noinline__ void bshort(const BatchArgs& a, const BCtx& X, const BShared& S, double (&acc)[kSRPart]) {
   const BConf& c = *X.c;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
   const int do_bmh = (c.flags & BF_BMH) ? 1 : 0, do_lj = (c.flags & BF_LJ) ? 1 : 0;
@@ -503,15 +754,17 @@ __device__ void bshort(const BatchArgs& a, const BCtx& X, const BShared& S, doub
   for (int k = 0; k < kSRPart; ++k) acc[k] = 0.0;
   for (int i = X.i0 + warp; i < X.i1; i += nwarp) {
     double4 si = S.s[i];
-    int ti = S.t[i];
+    int ti = btyp(S.t[i]);
     double fb[3] = {0, 0, 0}, fl[3] = {0, 0, 0};
-    for (int j = lane; j < X.n; j += 32) {
-      if (j == i) continue;
+    const unsigned short* row = bnbl(a, X, 1, i);
+    const int nn = bnbn(a, X, 1)[i];
+    for (int k = lane; k < nn; k += 32) {
+      const int j = bnbr(row, k);
       double4 sj = S.s[j];
       double rx, ry, rz;
       double r2 = min_image_exact(c.A, xsub(si.x, sj.x), xsub(si.y, sj.y), xsub(si.z, sj.z), rx,
                                   ry, rz);
-      const NBPair& P = S.nb[ti * c.ntype + S.t[j]];
+      const NBPair& P = S.nb[ti * c.ntype + btyp(S.t[j])];
       if (r2 >= P.rcutsq) continue;  // non_bonded.f90:1154 strict <
       if (do_bmh && (P.A != 0.0 || P.wall != 0.0)) {
         double u, wij;
@@ -563,7 +816,7 @@ __device__ void bshort(const BatchArgs& a, const BCtx& X, const BShared& S, doub
 
 // final real-space pass (k_es_force) on this CTA's ions; mu in S.v (FP64).
 template <typename R>
-__device__ void bforce(const BatchArgs& a, const BCtx& X, const BShared& S, double (&acc)[kESPart]) {
+__device__ __noinline__ void bforce(const BatchArgs& a, const BCtx& X, const BShared& S, double (&acc)[kESPart]) {
   const BConf& c = *X.c;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
   const int task_qq = (c.flags & BF_QQ) ? 1 : 0, task_qd = (c.flags & BF_QD) ? 1 : 0;
@@ -571,18 +824,20 @@ __device__ void bforce(const BatchArgs& a, const BCtx& X, const BShared& S, doub
   for (int k = 0; k < kESPart; ++k) acc[k] = 0.0;
   for (int i = X.i0 + warp; i < X.i1; i += nwarp) {
     double4 si = S.s[i];
-    int ti = S.t[i];
+    int ti = btyp(S.t[i]);
     double qi = si.w;
     double4 mui = S.v[i];
     double e[3] = {0, 0, 0}, f[3] = {0, 0, 0};
-    for (int j = lane; j < X.n; j += 32) {
-      if (j == i) continue;
+    const unsigned short* row = bnbl(a, X, 0, i);
+    const int nn = bnbn(a, X, 0)[i];
+    for (int k = lane; k < nn; k += 32) {
+      const int j = bnbr(row, k);
       double4 sj = S.s[j];
       double rxd, ryd, rzd;
       double r2d = min_image_exact(c.A, xsub(si.x, sj.x), xsub(si.y, sj.y), xsub(si.z, sj.z), rxd,
                                    ryd, rzd);
       if (r2d > c.rc2) continue;
-      int tj = S.t[j];
+      int tj = btyp(S.t[j]);
       double qj = sj.w;
       double4 muj = S.v[j];
       bool i_is_a = half_mask(i, j);
@@ -655,7 +910,7 @@ __device__ void bmoments(cgx::cluster_group& cl, const BatchArgs& a, BCtx& X, co
   for (int i = X.i0 + threadIdx.x; i < X.i1; i += blockDim.x) {
     int gi = X.off + i;
     double qi = has_q ? S.s[i].w : 0.0;
-    double4 u = v ? v[gi] : make_double4(0, 0, 0, 0);
+    double4 u = v ? ldcg4(v + gi) : make_double4(0, 0, 0, 0);
     m[0] += qi * a.pos[gi];
     m[1] += qi * a.pos[a.ntot + gi];
     m[2] += qi * a.pos[2 * (size_t)a.ntot + gi];
@@ -668,22 +923,44 @@ __device__ void bmoments(cgx::cluster_group& cl, const BatchArgs& a, BCtx& X, co
   cluster_sum<8>(cl, X, S, m);
 }
 
+// the same sums added to the field of the polarisable ions: reciprocal field of
+// entry k - p0 plus self (+ surface) field of v
+__device__ void bfinish_pol(const BatchArgs& a, const BCtx& X, const BShared& S, int RS,
+                            const double4* __restrict__ v, double selfa2, bool lsurf, double fpi_3V,
+                            const double* tot, double4* __restrict__ E) {
+  const BConf& c = *X.c;
+  for (int p = X.p0 + threadIdx.x; p < X.p1; p += blockDim.x) {
+    const int gi = X.off + bpl(S.t[p]);
+    double e[3], fm[3];
+    bfld_get(a, c, RS, p - X.p0, false, e, fm);
+    const double4 m = ldcg4(v + gi);
+    double s[3] = {0.0, 0.0, 0.0};
+    if (lsurf)
+      for (int d = 0; d < 3; ++d) s[d] = -(tot[d] + tot[3 + d]) * fpi_3V;
+    const double4 o = E[gi];
+    E[gi] = make_double4(o.x + e[0] + s[0] + 2.0 * selfa2 * m.x, o.y + e[1] + s[1] + 2.0 * selfa2 * m.y,
+                         o.z + e[2] + s[2] + 2.0 * selfa2 * m.z, 0.0);
+  }
+}
+
 // T v (field of a dipole set alone: dd undamped between polarisable ions,
-// reciprocal dipole part, self / surface) on own ions into Tv.  The vector
-// must be in global memory (vg) for all ions of the box; it is gathered here.
+// reciprocal dipole part, self / surface) on this CTA's polarisable ions into
+// Tv.  The vector must be in global memory (vg) for all polarisable ions of the
+// box; it is gathered here by rank.
 template <typename R>
 __device__ void bmatvec(cgx::cluster_group& cl, const BatchArgs& a, BCtx& X, const BShared& S,
                         const double4* __restrict__ vg, double4* __restrict__ Tv) {
   const BConf& c = *X.c;
   cl.sync();  // every CTA's slice of vg is written
-  gather_vec(X, vg, S.v);
-  if (sizeof(R) == 4) gather_vec32(X, vg, S.v32);
-  for (int i = X.i0 + threadIdx.x; i < X.i1; i += blockDim.x) Tv[X.off + i] = make_double4(0, 0, 0, 0);
+  if (sizeof(R) == 4) gather_pol32(X, S.t, vg, S.v32);
+  else gather_pol(X, S.t, vg, S.v);
+  for (int p = X.p0 + threadIdx.x; p < X.p1; p += blockDim.x)
+    Tv[X.off + bpl(S.t[p])] = make_double4(0, 0, 0, 0);
   __syncthreads();
   double es[7];
-  brec<R>(cl, a, X, S, false, true, false, false, Tv, nullptr, es);
-  __syncthreads();
-  bfield<R, false, true>(a, X, S, 0, 1, Tv);
+  const int RS = brec<R, R>(cl, a, X, S, sizeof(R) == 4 ? 2 : 1, false, true, true, false, false, es);
+  if (bcached(a, X)) bfield_cached<R>(a, X, S, Tv);
+  else bfield<R, false, true>(a, X, S, 0, true, Tv);
   double tot[6] = {0, 0, 0, 0, 0, 0};
   if (c.flags & BF_SURF) {
     double m[8];
@@ -693,12 +970,14 @@ __device__ void bmatvec(cgx::cluster_group& cl, const BatchArgs& a, BCtx& X, con
   __syncthreads();
   double al = c.alpha;
   double selfa2 = 2.0 * (al / sqrt(kPi)) * al * al / 3.0;
-  bself(a, X, vg, selfa2, (c.flags & BF_SURF) != 0, 2.0 * (kTwoPi / c.omega / 3.0), tot, Tv);
+  bfinish_pol(a, X, S, RS, vg, selfa2, (c.flags & BF_SURF) != 0, 2.0 * (kTwoPi / c.omega / 3.0), tot, Tv);
   __syncthreads();
 }
 
 // PCG on (alpha^-1 - T) x = b over the polarisable ions of the configuration,
-// x holding the first guess.  The true residual is formed with the FP64
+// x holding the first guess (zero on the other ions).  Each CTA owns the
+// polarisable ions of its rank range, so that a box whose polarisable ions
+// are one type block still splits evenly over the cluster.  The true residual is formed with the FP64
 // operator; with MIXED the inner iterations use the FP32 operator and stop
 // at 1e-4 of that residual (iterative refinement), else they run to tol.
 // Stops on the reference's rmsd measure (get_rmsd_mu, moment_from_pola.f90:
@@ -715,20 +994,18 @@ __device__ void bsolve(cgx::cluster_group& cl, const BatchArgs& a, BCtx& X, cons
   while (true) {
     // true residual with the FP64 operator
     bmatvec<double>(cl, a, X, S, x, a.p);
+    // (the gather of x read every CTA's slice before this one changes)
     double v2[2] = {0.0, 0.0};
-    for (int i = X.i0 + threadIdx.x; i < X.i1; i += blockDim.x) {
-      int gi = X.off + i;
-      double4 ri = make_double4(0, 0, 0, 0), zi = make_double4(0, 0, 0, 0);
-      if (a.ipol[gi]) {
-        double4 ax = bmat3(a.inv + 9 * (size_t)gi, x[gi]);
-        double4 bi = b[gi], tx = a.p[gi];
-        ri = make_double4(bi.x + tx.x - ax.x, bi.y + tx.y - ax.y, bi.z + tx.z - ax.z, 0.0);
-        zi = bmat3(a.pol + 9 * (size_t)gi, ri);
-        const double* pl = a.pol + 9 * (size_t)gi;
-        double rr[3] = {ri.x, ri.y, ri.z};
-        for (int d = 0; d < 3; ++d)
-          if (pl[4 * d] != 0.0) v2[1] += rr[d] * rr[d];
-      }
+    for (int p = X.p0 + threadIdx.x; p < X.p1; p += blockDim.x) {
+      const int gi = X.off + bpl(S.t[p]);
+      double4 ax = bmat3(a.inv + 9 * (size_t)gi, ldcg4(x + gi));
+      double4 bi = ldcg4(b + gi), tx = a.p[gi];
+      double4 ri = make_double4(bi.x + tx.x - ax.x, bi.y + tx.y - ax.y, bi.z + tx.z - ax.z, 0.0);
+      double4 zi = bmat3(a.pol + 9 * (size_t)gi, ri);
+      const double* pl = a.pol + 9 * (size_t)gi;
+      double rr[3] = {ri.x, ri.y, ri.z};
+      for (int d = 0; d < 3; ++d)
+        if (pl[4 * d] != 0.0) v2[1] += rr[d] * rr[d];
       a.r[gi] = ri;
       a.z[gi] = zi;
       a.p[gi] = zi;
@@ -748,28 +1025,24 @@ __device__ void bsolve(cgx::cluster_group& cl, const BatchArgs& a, BCtx& X, cons
     const double tol_in = !MIXED ? tol : (trust ? 0.5 * tol : fmax(tol, 1e-4 * rmsd));
     double rms_last = rmsd;
     while (true) {
-      // Tp into Estat-free scratch: a.E (own rows) holds T p
+      // T p into a.E (the field buffer is free until the final pass)
       bmatvec<RM>(cl, a, X, S, a.p, a.E);
       double pq[1] = {0.0};
-      for (int i = X.i0 + threadIdx.x; i < X.i1; i += blockDim.x) {
-        int gi = X.off + i;
-        double4 qi = make_double4(0, 0, 0, 0);
-        if (a.ipol[gi]) {
-          double4 ap = bmat3(a.inv + 9 * (size_t)gi, a.p[gi]);
-          double4 tp = a.E[gi];
-          qi = make_double4(ap.x - tp.x, ap.y - tp.y, ap.z - tp.z, 0.0);
-        }
+      for (int p = X.p0 + threadIdx.x; p < X.p1; p += blockDim.x) {
+        const int gi = X.off + bpl(S.t[p]);
+        const double4 pi = a.p[gi];
+        const double4 ap = bmat3(a.inv + 9 * (size_t)gi, pi);
+        const double4 tp = a.E[gi];
+        const double4 qi = make_double4(ap.x - tp.x, ap.y - tp.y, ap.z - tp.z, 0.0);
         a.E[gi] = qi;  // q = A p
-        double4 pi = a.p[gi];
         pq[0] += pi.x * qi.x + pi.y * qi.y + pi.z * qi.z;
       }
       cluster_sum<1>(cl, X, S, pq);
       double alp = (pq[0] != 0.0) ? rz / pq[0] : 0.0;
       double u2[2] = {0.0, 0.0};
-      for (int i = X.i0 + threadIdx.x; i < X.i1; i += blockDim.x) {
-        int gi = X.off + i;
-        if (!a.ipol[gi]) continue;
-        double4 xi = x[gi], ri = a.r[gi], pi = a.p[gi], qi = a.E[gi];
+      for (int p = X.p0 + threadIdx.x; p < X.p1; p += blockDim.x) {
+        const int gi = X.off + bpl(S.t[p]);
+        double4 xi = ldcg4(x + gi), ri = a.r[gi], pi = a.p[gi], qi = a.E[gi];
         xi.x += alp * pi.x;
         xi.y += alp * pi.y;
         xi.z += alp * pi.z;
@@ -793,8 +1066,8 @@ __device__ void bsolve(cgx::cluster_group& cl, const BatchArgs& a, BCtx& X, cons
       if (!(rms_in > tol_in && iters < maxit)) break;
       double be = (rz != 0.0) ? u2[0] / rz : 0.0;
       rz = u2[0];
-      for (int i = X.i0 + threadIdx.x; i < X.i1; i += blockDim.x) {
-        int gi = X.off + i;
+      for (int p = X.p0 + threadIdx.x; p < X.p1; p += blockDim.x) {
+        const int gi = X.off + bpl(S.t[p]);
         double4 pi = a.p[gi], zi = a.z[gi];
         a.p[gi] = make_double4(zi.x + be * pi.x, zi.y + be * pi.y, zi.z + be * pi.z, 0.0);
       }
@@ -803,6 +1076,25 @@ __device__ void bsolve(cgx::cluster_group& cl, const BatchArgs& a, BCtx& X, cons
       rmsd = rms_last;
       break;
     }
+  }
+}
+
+// entry m of axis d of an ion's phase record (entries of n > kz stay zero)
+template <typename R>
+__device__ __forceinline__ void brec_put(unsigned char* rec, int zo, int d, int e0, int m, int kz, double cs,
+                                         double sn) {
+  typedef typename cplx<R>::T C2;
+  if (d < 2) {
+    C2 v;
+    v.x = (R)cs;
+    v.y = (R)sn;
+    reinterpret_cast<C2*>(rec)[e0 + m] = v;
+  } else if (m <= kz) {
+    R* z = reinterpret_cast<R*>(rec + zo) + 4 * m;
+    z[0] = (R)cs;
+    z[1] = (R)sn;
+    z[2] = (R)(m * cs);
+    z[3] = (R)(m * sn);
   }
 }
 
@@ -833,6 +1125,8 @@ __device__ void bconfig(cgx::cluster_group& cl, const BatchArgs& a, BCtx& X, con
           long long o = c.tab_off + (long long)(e0 + m) * c.tab_ld + i;
           a.tab64[o] = make_double2(cs, sn);
           if (MIXED) a.tab32[o] = make_float2((float)cs, (float)sn);
+          brec_put<double>(a.rec + c.rec64 + (size_t)i * c.rs64, c.zo64, d, e0, m, c.kz, cs, sn);
+          if (MIXED) brec_put<float>(a.rec + c.rec32 + (size_t)i * c.rs32, c.zo32, d, e0, m, c.kz, cs, sn);
         }
         e0 += km[d] + 1;
       }
@@ -848,6 +1142,7 @@ __device__ void bconfig(cgx::cluster_group& cl, const BatchArgs& a, BCtx& X, con
     S.t[i] = a.typ[X.off + i];
   }
   __syncthreads();
+  blists(a, X, S, coul, (c.flags & BF_SR) != 0);
   // ---- short range -------------------------------------------------------
   {
     double acc[kSRPart];
@@ -881,18 +1176,21 @@ __device__ void bconfig(cgx::cluster_group& cl, const BatchArgs& a, BCtx& X, con
   double rmsd = 0.0;
   for (int i = X.i0 + threadIdx.x; i < X.i1; i += blockDim.x) a.x[X.off + i] = make_double4(0, 0, 0, 0);
   if (c.flags & BF_POLAR) {
-    // ---- static field: damped charges + static dipoles --------------------
-    for (int i = X.i0 + threadIdx.x; i < X.i1; i += blockDim.x)
-      a.Estat[X.off + i] = make_double4(0, 0, 0, 0);
+    // the partner lists and the zeroed dipoles of every ion are in place
+    cl.sync();
+    // ---- static field: damped charges + static dipoles, at the polarisable
+    // ions (the solver reads it there) ----------------------------------------
+    for (int p = X.p0 + threadIdx.x; p < X.p1; p += blockDim.x)
+      a.Estat[X.off + bpl(S.t[p])] = make_double4(0, 0, 0, 0);
     gather_vec(X, a.dip, S.v);
-    if (MIXED) gather_vec32(X, a.dip, S.v32);
     __syncthreads();
-    if (task_qq && dipst) bfield<RM, true, true>(a, X, S, 1, 0, a.Estat);
-    else if (task_qq) bfield<RM, true, false>(a, X, S, 1, 0, a.Estat);
-    else if (dipst) bfield<RM, false, true>(a, X, S, 1, 0, a.Estat);
+    if (task_qq && dipst) bfield<RM, true, true>(a, X, S, 1, false, a.Estat);
+    else if (task_qq) bfield<RM, true, false>(a, X, S, 1, false, a.Estat);
+    else if (dipst) bfield<RM, false, true>(a, X, S, 1, false, a.Estat);
+    if (bcached(a, X)) bcache<MIXED>(a, X, S);
     __syncthreads();
     double es[7];
-    brec<RM>(cl, a, X, S, task_qq, dipst, false, false, a.Estat, nullptr, es);
+    const int RS = brec<RM, double>(cl, a, X, S, 0, task_qq, dipst, true, false, false, es);
     double tot[6] = {0, 0, 0, 0, 0, 0};
     if (lsurf) {
       double m[8];
@@ -900,16 +1198,17 @@ __device__ void bconfig(cgx::cluster_group& cl, const BatchArgs& a, BCtx& X, con
       for (int k = 0; k < 6; ++k) tot[k] = m[k];
     }
     __syncthreads();
-    bself(a, X, a.dip, selfa2, lsurf, fpi_3V, tot, a.Estat);
+    bfinish_pol(a, X, S, RS, a.dip, selfa2, lsurf, fpi_3V, tot, a.Estat);
     __syncthreads();
     // ---- PCG: (alpha^-1 - T) x = E_stat, x0 = alpha E_stat ----------------
-    for (int i = X.i0 + threadIdx.x; i < X.i1; i += blockDim.x) {
-      int gi = X.off + i;
-      a.x[gi] = a.ipol[gi] ? bmat3(a.pol + 9 * (size_t)gi, a.Estat[gi]) : make_double4(0, 0, 0, 0);
+    for (int p = X.p0 + threadIdx.x; p < X.p1; p += blockDim.x) {
+      const int gi = X.off + bpl(S.t[p]);
+      a.x[gi] = bmat3(a.pol + 9 * (size_t)gi, a.Estat[gi]);
     }
     const double tol = c.tol;
     bsolve<MIXED>(cl, a, X, S, a.Estat, a.x, tol, c.maxit, iters, rmsd);
     conv = rmsd <= tol ? 1 : 0;
+    cl.sync();  // the converged dipoles of every CTA are in place
   }
   // ---- u_pol, total dipoles (+ Wannier centres), catastrophe -------------
   {
@@ -917,7 +1216,7 @@ __device__ void bconfig(cgx::cluster_group& cl, const BatchArgs& a, BCtx& X, con
     double v[3] = {0.0, 0.0, 0.0};
     for (int i = X.i0 + threadIdx.x; i < X.i1; i += blockDim.x) {
       int gi = X.off + i;
-      double4 m = a.x[gi];
+      double4 m = ldcg4(a.x + gi);
       if (a.ipol[gi]) {
         const double* iv = a.inv + 9 * (size_t)gi;
         double mm[3] = {m.x, m.y, m.z};
@@ -926,14 +1225,14 @@ __device__ void bconfig(cgx::cluster_group& cl, const BatchArgs& a, BCtx& X, con
       }
       double4 d = a.dip[gi];
       double4 t = make_double4(d.x + m.x, d.y + m.y, d.z + m.z, 0.0);
-      if (wfc && c.lwfc[S.t[i]] >= 0) {
+      if (wfc && c.lwfc[btyp(S.t[i])] >= 0) {
         // moment_from_WFc (moment_from_pola.f90:686-738): -2 sum (r_c - r_i)
         // over the centres c with |r|^2 < rcut_wfc, in ascending centre order
         const double4 si = S.s[i];
         double w[3] = {0.0, 0.0, 0.0};
         int cnt = 0;
         for (int j = 0; j < X.n; ++j) {
-          if (c.lwfc[S.t[j]] >= 0) continue;
+          if (c.lwfc[btyp(S.t[j])] >= 0) continue;
           const double4 sj = S.s[j];
           double rx, ry, rz;
           const double r2 = min_image_exact(c.A, xsub(sj.x, si.x), xsub(sj.y, si.y), xsub(sj.z, si.z),
@@ -945,7 +1244,7 @@ __device__ void bconfig(cgx::cluster_group& cl, const BatchArgs& a, BCtx& X, con
             w[2] += rz;
           }
         }
-        if (c.lwfc[S.t[i]] > 0 && cnt != c.lwfc[S.t[i]]) v[2] = 1.0;  // :731-737
+        if (c.lwfc[btyp(S.t[i])] > 0 && cnt != c.lwfc[btyp(S.t[i])]) v[2] = 1.0;  // :731-737
         if (c.ldip_wfc) {
           t.x = t.x + -2.0 * w[0];
           t.y = t.y + -2.0 * w[1];
@@ -980,10 +1279,21 @@ __device__ void bconfig(cgx::cluster_group& cl, const BatchArgs& a, BCtx& X, con
   {
     bool has_mu = (c.flags & (BF_QD | BF_DD)) != 0;
     double es[7];
-    brec<RM>(cl, a, X, S, task_qq, has_mu, true, true, a.E, a.force, es);
+    const int RS = brec<RM, double>(cl, a, X, S, 0, task_qq, has_mu, false, has_mu, true, es);
     cluster_sum<7>(cl, X, S, es);
     if (X.rank == 0 && threadIdx.x == 0)
       for (int k = 0; k < 7; ++k) out[BS_REC + k] = es[k];
+    for (int i = X.i0 + threadIdx.x; i < X.i1; i += blockDim.x) {
+      const int gi = X.off + i;
+      double e[3], fm[3];
+      bfld_get(a, c, RS, i - X.i0, has_mu, e, fm);
+      const double4 o = a.E[gi];
+      a.E[gi] = make_double4(o.x + e[0], o.y + e[1], o.z + e[2], 0.0);
+      const double qi = S.s[i].w;
+      a.force[gi] += (qi * e[0] + fm[0]) * c.coul_unit;
+      a.force[a.ntot + gi] += (qi * e[1] + fm[1]) * c.coul_unit;
+      a.force[2 * (size_t)a.ntot + gi] += (qi * e[2] + fm[2]) * c.coul_unit;
+    }
   }
   double m[8];
   bmoments(cl, a, X, S, a.mu, true, m);
@@ -991,6 +1301,24 @@ __device__ void bconfig(cgx::cluster_group& cl, const BatchArgs& a, BCtx& X, con
     for (int k = 0; k < 8; ++k) out[BS_MOM + k] = m[k];
   __syncthreads();
   bself(a, X, a.mu, selfa2, lsurf, fpi_3V, m, a.E);
+}
+
+// configuration cfg becomes the cluster's: ion and polarisable-ion ranges of this CTA
+__device__ __forceinline__ void bctx_set(const BatchArgs& a, BCtx& X, int cfg) {
+  const BConf* c = a.conf + cfg;
+  X.c = c;
+  X.cfg = cfg;
+  X.n = c->n;
+  X.off = c->off;
+  X.i0 = (int)((long long)X.n * X.rank / X.C);
+  X.i1 = (int)((long long)X.n * (X.rank + 1) / X.C);
+  X.npol = c->npol;
+  X.p0 = (int)((long long)X.npol * X.rank / X.C);
+  X.p1 = (int)((long long)X.npol * (X.rank + 1) / X.C);
+  X.slot = (int)(blockIdx.x / X.C);
+  X.part = a.part + (size_t)cfg * kBMaxC * 2 * kBPart;
+  X.parity = 0;
+  X.rpar = 0;
 }
 
 // Persistent kernel: one cluster per configuration at a time, configurations
@@ -1011,15 +1339,7 @@ __global__ void __launch_bounds__(512) k_batch(BatchArgs a, int nmax) {
     cl.sync();  // rank 0 may overwrite its slot only after every CTA read it
     if (qpos >= a.nconf) break;
     int cfg = a.order[qpos];
-    const BConf* c = a.conf + cfg;
-    X.c = c;
-    X.cfg = cfg;
-    X.n = c->n;
-    X.off = c->off;
-    X.i0 = (int)((long long)X.n * X.rank / X.C);
-    X.i1 = (int)((long long)X.n * (X.rank + 1) / X.C);
-    X.part = a.part + (size_t)cfg * kBMaxC * 2 * kBPart;
-    X.parity = 0;
+    bctx_set(a, X, cfg);
     bconfig<MIXED>(cl, a, X, S);
     __syncthreads();
   }
