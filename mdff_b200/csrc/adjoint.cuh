@@ -261,9 +261,9 @@ __device__ void bsf(cgx::cluster_group& cl, const BatchArgs& a, BCtx& X, const B
 #pragma unroll
     for (int t = 0; t < kBNZ; ++t) accR[t] = accI[t] = 0.0;
     for (int i = lane; i < X.n; i += 32) {
-      double2 XY = bphase<double>(a, c, i, nx, ny, 0);
-      double2 Z1 = btab<double>(a, c, c.kx + 1 + c.ky + 1 + 1, i);
-      double2 P = bphase_z<double>(a, c, i, XY, nz0);
+      double2 XY = bphase(a, c, i, nx, ny, 0);
+      double2 Z1 = btab(a, c, c.kx + 1 + c.ky + 1 + 1, i);
+      double2 P = bphase_z(a, c, i, XY, nz0);
       double qv = hasq ? S.s[i].w : 0.0;
       double kv = 0.0, v3 = 0.0, kw = 1.0, w3 = 0.0;
       if (hasv) {
@@ -323,7 +323,7 @@ __device__ void brecsum(const BatchArgs& a, const BCtx& X, const BShared& S,
     double H[3] = {0, 0, 0}, K[3] = {0, 0, 0};
     double4 u = Sw[i];
     double3 m = bmvec(c, u.x, u.y, u.z);
-    double2 Z1 = btab<double>(a, c, c.kx + 1 + c.ky + 1 + 1, i);
+    double2 Z1 = btab(a, c, c.kx + 1 + c.ky + 1 + 1, i);
     int ra = 0;
     while (ra < c.nrows) {
       int kbase = rows[ra].w;
@@ -347,8 +347,8 @@ __device__ void brecsum(const BatchArgs& a, const BCtx& X, const BShared& S,
         for (int r = ra + me; r < rb; r += sub) {
           int4 ri = rows[r];
           int nx = ri.x, ny = ri.y, nz_lo = ri.z;
-          double2 XY = bphase<double>(a, c, i, nx, ny, 0);
-          double2 P = bphase_z<double>(a, c, i, XY, nz_lo);
+          double2 XY = bphase(a, c, i, nx, ny, 0);
+          double2 P = bphase_z(a, c, i, XY, nz_lo);
           double kw = nx * m.x + ny * m.y + nz_lo * m.z;
           double T0 = 0, Tz = 0, U0 = 0, Uz = 0;
           int nn = kz - nz_lo + 1;

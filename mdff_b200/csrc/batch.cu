@@ -4,12 +4,14 @@
 // then concatenates the per-ion and per-k tables.  One evaluation is a CUDA
 // graph of three nodes: zero the work queue, zero the scalar slots, launch the
 // persistent cluster kernel.  The launch shape (cluster size x threads per
-// CTA) is chosen by an autotuner that times every candidate on the batch.
+// CTA) follows from the boxes' costs (default_shape) unless the caller sets it or
+// has an autotuner time every candidate on the batch.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <functional>
 #include <mutex>
 #include <numeric>
 #include <string>
@@ -57,7 +59,7 @@ struct mdff_batch {
   double4 *d_s = nullptr, *d_Estat = nullptr, *d_x = nullptr, *d_r = nullptr, *d_z = nullptr,
           *d_p = nullptr, *d_mu = nullptr, *d_E = nullptr;
   double2* d_tab64 = nullptr;
-  float2* d_tab32 = nullptr;
+  double2* d_apm = nullptr;
   // phase records and the workspaces of the resident CTAs (BatchArgs)
   unsigned char* d_rec = nullptr;
   unsigned char* d_ws = nullptr;  // the allocation that holds them
@@ -70,11 +72,12 @@ struct mdff_batch {
   float4* d_c32 = nullptr;
   float* d_b32 = nullptr;
   size_t rpart_ld = 1, ccap = 0, npol_max = 0;
+  int stage_extra = 0;               // BatchArgs of the launch being set up
   int ws_ctas = 0, ws_clusters = 0;  // CTAs and clusters the workspaces are sized for
   double *d_force = nullptr, *d_part = nullptr, *d_out = nullptr, *d_pack = nullptr;
   double* h_out = nullptr;
   // launch
-  Shape shape{2, 256};
+  Shape shape{2, 512};
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   const double* graph_pos = nullptr;
@@ -166,7 +169,8 @@ BatchArgs make_args(mdff_batch* h, const double* d_pos, double* d_force) {
   a.kvec = h->d_kvec;
   a.s = h->d_s;
   a.tab64 = h->d_tab64;
-  a.tab32 = h->d_tab32;
+  a.apm = h->d_apm;
+  a.stage_extra = h->stage_extra;
   a.rec = h->d_rec;
   a.rpart = h->d_rpart;
   a.rpart_ld = h->rpart_ld;
@@ -264,8 +268,20 @@ int ensure_workspace(mdff_batch* h, int ncl, int cluster) {
 // persistent grid: as many clusters as fit on the device at once (at most one
 // per configuration).  Attribute and occupancy queries happen here, outside
 // any stream capture.
+// Shared memory of one CTA: `base` bytes of layout plus a larger staging buffer
+// where it costs no resident CTA (512 threads of 128 registers fill an SM, 256
+// half of it).
+size_t smem_with_stage(mdff_batch* h, size_t base, int threads, int* extra) {
+  const size_t room = threads >= 512 ? 227 * 1024 : 113 * 1024;
+  const size_t o = (base + 15) & ~(size_t)15;
+  *extra = 0;
+  if (o + 20 * 1024 <= room) *extra = (int)(std::min<size_t>(room - o, 40 * 1024) & ~(size_t)127);
+  (void)h;
+  return *extra ? o + *extra : base;
+}
+
 int prepare_shape(mdff_batch* h, Shape sh, int* nclusters) {
-  size_t smem = batch_smem_bytes(h->nmax);
+  size_t smem = smem_with_stage(h, batch_smem_bytes(h->nmax), sh.threads, &h->stage_extra);
   void (*fn)(BatchArgs, int) = h->mixed ? k_batch<true> : k_batch<false>;
   BCK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   cudaLaunchConfig_t cfg = {};
@@ -300,7 +316,8 @@ int launch_batch(mdff_batch* h, const BatchArgs& a, Shape sh, int ncl, cudaStrea
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   cfg.blockDim = dim3(sh.threads);
-  cfg.dynamicSmemBytes = batch_smem_bytes(h->nmax);
+  int extra = 0;
+  cfg.dynamicSmemBytes = smem_with_stage(h, batch_smem_bytes(h->nmax), sh.threads, &extra);
   cfg.stream = st;
   cfg.gridDim = dim3(sh.cluster * ncl);
   BCK(cudaLaunchKernelEx(&cfg, fn, a, h->nmax));
@@ -311,6 +328,7 @@ int launch_batch(mdff_batch* h, const BatchArgs& a, Shape sh, int ncl, cudaStrea
 int enqueue(mdff_batch* h, const double* d_pos, double* d_force, Shape sh, int ncl, cudaStream_t st) {
   BCK(cudaMemsetAsync(h->d_queue, 0, sizeof(int), st));
   BCK(cudaMemsetAsync(h->d_out, 0, sizeof(double) * kBSlots * h->nconf, st));
+  smem_with_stage(h, batch_smem_bytes(h->nmax), sh.threads, &h->stage_extra);
   return launch_batch(h, make_args(h, d_pos, d_force), sh, ncl, st);
 }
 
@@ -411,6 +429,52 @@ int finish(mdff_batch* h, mdff_batch_conf* conf) {
   return status;
 }
 
+// Time of one box (ms) on a cluster of C CTAs of 512 threads: fixed + par / C.  The
+// fixed part is the chain of barriers and latencies of a dipole solve (it does not shrink
+// with the cluster), par the pair loops (~ n^2) and the reciprocal sums (~ n nk).
+// Constants from 200 boxes of 64-200 and 10 of 100-900 ions (MgO type) over
+// C = 1..8; boxes without polarisation make one pass instead of a solve.
+struct BoxCost {
+  double fixed, par;
+};
+BoxCost box_cost(int n, int nk, int npol) {
+  const double nn = (double)n * n, nnk = (double)n * nk;
+  return npol > 0 ? BoxCost{0.4, 2.1e-6 * nn + 1.1e-6 * nnk} : BoxCost{0.08, 1.2e-6 * nn + 0.25e-6 * nnk};
+}
+
+// The cluster size with the shortest schedule: the boxes in queue order on
+// nsm / C clusters (one CTA of 512 threads per SM).  Many boxes want C = 1 or 2
+// (256 boxes of 64-1000 ions, mixed: C = 1 8.0, 2 4.9, 4 6.7 ms; 200 of 64-200:
+// 1.3, 1.6, 2.7), few boxes large clusters (24 boxes of 64-300, FP64: C = 2
+// 1.04, 4 0.77, 8 0.69 ms).
+Shape default_shape(const std::vector<BoxCost>& cost, const std::vector<int>& order, int nsm) {
+  Shape best{2, 512};
+  double tbest = 1e300;
+  for (int C = 1; C <= kBMaxC; C *= 2) {
+    std::vector<double> busy(std::max(1, nsm / C), 0.0);  // a heap of the clusters' end times
+    double end = 0.0;
+    for (int i : order) {
+      std::pop_heap(busy.begin(), busy.end(), std::greater<double>());
+      busy.back() += cost[i].fixed + cost[i].par / C;
+      end = std::max(end, busy.back());
+      std::push_heap(busy.begin(), busy.end(), std::greater<double>());
+    }
+    if (end < 0.97 * tbest) {
+      tbest = end;
+      best = Shape{C, 512};
+    }
+  }
+  return best;
+}
+
+// Tang-Toennies order 4 wherever a role damps (c != 0; c = 0 damps nothing at any
+// order), as the single engine's compile-time order
+bool tt4_of(const std::vector<ESPair>& es) {
+  for (const ESPair& e : es)
+    if (e.ldamp && ((e.ca != 0.0 && e.ka != 4) || (e.cb != 0.0 && e.kb != 4))) return false;
+  return true;
+}
+
 int create_impl(mdff_batch* h, const mdff_params* psets, int npsets, const mdff_batch_desc* d) {
   if (!psets || npsets <= 0 || !d || d->nconf <= 0 || !d->pset || !d->natmi || !d->cell_A) {
     h->err = "bad batch description";
@@ -426,10 +490,11 @@ int create_impl(mdff_batch* h, const mdff_params* psets, int npsets, const mdff_
   std::vector<int> typ, ipol;
   std::vector<double> q, pol, inv, Ak;
   std::vector<double4> dip, kvec;
+  std::vector<double2> apm;
   std::vector<NBPair> nb;
   std::vector<ESPair> es;
   std::vector<int4> rows;
-  std::vector<double> cost(h->nconf);
+  std::vector<BoxCost> cost(h->nconf);
   long long tab_total = 0, rec_total = 0;
   long long ktot = 0;
   int ntot = 0;
@@ -500,6 +565,7 @@ int create_impl(mdff_batch* h, const mdff_params* psets, int npsets, const mdff_
     if (P.lsurf) fl |= BF_SURF;
     if (P.thole_type != MDFF_THOLE_NONE) fl |= BF_THOLE;
     if (S.ldip_static) fl |= BF_DIPST;
+    if (tt4_of(S.es)) fl |= BF_TT4;
     // Wannier centres (moment_from_pola.f90:130-147): a type with lwfc > 0
     for (int t = 0; t < P.ntype; ++t) {
       B.lwfc[t] = P.lwfc[t];
@@ -561,17 +627,15 @@ int create_impl(mdff_batch* h, const mdff_params* psets, int npsets, const mdff_
       // while another box's cluster writes it)
       tab_total += ((long long)B.ntab * n + 15) / 16 * 16;
       const int nz = B.kz + 1, nxy = B.kx + 1 + B.ky + 1;
-      B.t64 = brho_tile(nz, true);
-      B.t32 = brho_tile(nz, false);
-      B.kt = bfld_tile(nz);
-      B.zo64 = nxy * 16;
-      B.zo32 = (nxy * 8 + 15) / 16 * 16;
-      B.rs64 = (B.zo64 + (nz + B.t64 - 1) / B.t64 * B.t64 * 32 + 31) / 32 * 32;
-      B.rs32 = (B.zo32 + (nz + B.t32 - 1) / B.t32 * B.t32 * 16 + 31) / 32 * 32;
-      B.rec64 = rec_total;
-      rec_total += ((long long)B.rs64 * n + 127) / 128 * 128;
-      B.rec32 = rec_total;
-      if (h->mixed) rec_total += ((long long)B.rs32 * n + 127) / 128 * 128;
+      B.zo = nxy * 16;
+      B.rs = brec_bytes(B.kx, B.ky, B.kz);
+      B.rec = rec_total;
+      rec_total += ((long long)B.rs * n + 127) / 128 * 128;
+      B.apm_off = (int)apm.size();
+      for (const int4& r : M.rows)
+        for (int m = 0; m < nz; ++m)
+          apm.push_back(make_double2(m >= r.z ? M.Ak[r.w + m - r.z] : 0.0,
+                                     m > 0 && r.z < 0 ? M.Ak[r.w - m - r.z] : 0.0));
       h->rpart_ld = std::max(h->rpart_ld, (size_t)B.nrows * nz);
       rows.insert(rows.end(), M.rows.begin(), M.rows.end());
       if (M.nk > 0) {
@@ -580,8 +644,7 @@ int create_impl(mdff_batch* h, const mdff_params* psets, int npsets, const mdff_
       }
       ktot += M.nk;
     }
-    // cost model for the queue order: pair loops ~ n^2, k sums ~ n nk
-    cost[c] = (double)n * n + 2.0 * (double)n * B.nk;
+    cost[c] = box_cost((int)n, B.nk, S.npol);
     ntot += (int)n;
     h->nmax = std::max(h->nmax, (int)n);
   }
@@ -590,13 +653,18 @@ int create_impl(mdff_batch* h, const mdff_params* psets, int npsets, const mdff_
   h->order.resize(h->nconf);
   std::iota(h->order.begin(), h->order.end(), 0);
   std::stable_sort(h->order.begin(), h->order.end(),
-                   [&](int x, int y) { return cost[x] > cost[y]; });
+                   [&](int x, int y) { return cost[x].par > cost[y].par; });
   // device
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev <= h->device) {
     h->err = "no CUDA device";
     return MDFF_ERR_NO_DEVICE;
   }
   BCK(cudaSetDevice(h->device));
+  {
+    int nsm = 148;
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
+    h->shape = default_shape(cost, h->order, nsm);
+  }
   BCK(cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking));
   BCK(cudaEventCreate(&h->ev0));
   BCK(cudaEventCreate(&h->ev1));
@@ -613,6 +681,7 @@ int create_impl(mdff_batch* h, const mdff_params* psets, int npsets, const mdff_
   BUPLOAD(h->d_rows, rows);
   BUPLOAD(h->d_Ak, Ak);
   BUPLOAD(h->d_kvec, kvec);
+  BUPLOAD(h->d_apm, apm);
   BALLOC(h->d_queue, 1);
   BALLOC(h->d_pos, 3 * (size_t)ntot);
   BALLOC(h->d_s, ntot);
@@ -624,7 +693,6 @@ int create_impl(mdff_batch* h, const mdff_params* psets, int npsets, const mdff_
   BALLOC(h->d_mu, ntot);
   BALLOC(h->d_E, ntot);
   BALLOC(h->d_tab64, (size_t)std::max<long long>(tab_total, 1));
-  if (h->mixed) BALLOC(h->d_tab32, (size_t)std::max<long long>(tab_total, 1));
   BALLOC(h->d_rec, (size_t)std::max<long long>(rec_total, 1));
   BALLOC(h->d_force, 3 * (size_t)ntot);
   BALLOC(h->d_pack, 3 * (size_t)ntot);
@@ -670,6 +738,7 @@ int refit_tables(mdff_batch* h) {
   std::vector<double> q, pol, inv;
   std::vector<NBPair> nb;
   std::vector<ESPair> es;
+  bool flags_changed = false;
   for (int c = 0; c < h->nconf; ++c) {
     mdff_params p = fitted_pset(h, h->pset_of[c]);
     for (int t = 0; t < MDFF_NTYPEMAX; ++t) p.natmi[t] = h->pconf[c].natmi[t];
@@ -683,12 +752,20 @@ int refit_tables(mdff_batch* h) {
       return s;
     }
     h->pconf[c] = S.p;
+    // (a fitted c may leave or reach zero)
+    const int fl = (h->conf[c].flags & ~BF_TT4) | (tt4_of(S.es) ? BF_TT4 : 0);
+    if (fl != h->conf[c].flags) {
+      h->conf[c].flags = fl;
+      flags_changed = true;
+    }
     nb.insert(nb.end(), S.nb.begin(), S.nb.end());
     es.insert(es.end(), S.es.begin(), S.es.end());
     q.insert(q.end(), S.q.begin(), S.q.end());
     pol.insert(pol.end(), S.pol.begin(), S.pol.end());
     inv.insert(inv.end(), S.inv.begin(), S.inv.end());
   }
+  if (flags_changed)
+    BCK(cudaMemcpyAsync(h->d_conf, h->conf.data(), sizeof(BConf) * h->conf.size(), cudaMemcpyHostToDevice, h->st));
   BCK(cudaMemcpyAsync(h->d_nb, nb.data(), sizeof(NBPair) * nb.size(), cudaMemcpyHostToDevice, h->st));
   BCK(cudaMemcpyAsync(h->d_es, es.data(), sizeof(ESPair) * es.size(), cudaMemcpyHostToDevice, h->st));
   BCK(cudaMemcpyAsync(h->d_q, q.data(), sizeof(double) * q.size(), cudaMemcpyHostToDevice, h->st));
@@ -707,7 +784,7 @@ void destroy_impl(mdff_batch* h) {
   void* bufs[] = {h->d_conf, h->d_order, h->d_queue, h->d_typ, h->d_ipol, h->d_pos, h->d_q,
                   h->d_pol, h->d_inv, h->d_dip, h->d_nb, h->d_es, h->d_rows, h->d_Ak, h->d_kvec,
                   h->d_s, h->d_Estat, h->d_x, h->d_r, h->d_z, h->d_p, h->d_mu, h->d_E,
-                  h->d_tab64, h->d_tab32, h->d_rec, h->d_ws, h->d_force, h->d_part, h->d_out, h->d_pack,
+                  h->d_tab64, h->d_apm, h->d_rec, h->d_ws, h->d_force, h->d_part, h->d_out, h->d_pack,
                   h->d_w, h->d_rhs, h->d_lam, h->d_ch, h->d_grad, h->d_info, h->d_gin};
   for (void* b : bufs)
     if (b) cudaFree(b);
@@ -1017,6 +1094,7 @@ int mdff_gpu_batch_adjoint(mdff_batch_handle h, const double* gE, const double* 
   }
   cfg.gridDim = dim3(sh.cluster * ncl);
   cfg.stream = h->st;
+  h->stage_extra = 0;  // the adjoint stages in the layout's own buffer
   BatchArgs a = make_args(h, h->graph_pos, h->graph_force);
   BCK(cudaMemsetAsync(h->d_queue, 0, sizeof(int), h->st));
   BCK(cudaEventRecord(h->ev0, h->st));

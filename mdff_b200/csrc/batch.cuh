@@ -58,7 +58,7 @@ enum {
 enum {
   BF_COUL = 1, BF_SR = 2, BF_BMH = 4, BF_BMHFTD = 8, BF_LJ = 16, BF_POLAR = 32,
   BF_QQ = 64, BF_QD = 128, BF_DD = 256, BF_SURF = 512, BF_DIPST = 1024, BF_THOLE = 2048,
-  BF_WFC = 4096
+  BF_WFC = 4096, BF_TT4 = 8192  // BF_TT4: every damped ion pair uses order 4
 };
 
 struct BConf {
@@ -74,10 +74,10 @@ struct BConf {
   int lwfc[kBMaxT];      // Wannier centres per type (BF_WFC): < 0 centre type
   int ldip_wfc, pad2;
   double rcut_wfc;
-  // phase records of the structure factor (batch_rec.cuh): byte offset of the
-  // box, bytes per ion, byte offset of Z in a record, n tile; FP64 and FP32
-  long long rec64, rec32;
-  int rs64, rs32, zo64, zo32, t64, t32, kt, pad3;
+  // phase records of the reciprocal sums (batch_rec.cuh): byte offset of the
+  // box, bytes per ion, byte offset of Z in a record; offset of apm
+  long long rec;
+  int rs, zo, apm_off, pad3;
   double rs2;            // largest squared short-range cutoff of the box
 };
 
@@ -98,15 +98,16 @@ struct BatchArgs {
   const int4* rows;      // per configuration at row_off: (nx, ny, nz_lo, k)
   const double* Ak;      // per configuration at k_off
   const double4* kvec;
+  const double2* apm;    // (A(+n), A(-n)) by (row, n), per configuration at apm_off
   double4* s;            // [ntot] direct coordinates, w = q
   double2* tab64;        // phase tables, [entry][ion] per configuration
-  float2* tab32;
   unsigned char* rec;    // phase records of every configuration
   // workspace of the resident CTAs (blockIdx.x) and clusters (blockIdx.x / C)
   double4* rpart;        // [CTA][2][rpart_ld] structure-factor partials
   size_t rpart_ld;
   double* gpart;         // [CTA][kBSplit][6][wn] field sums per row subset
   int wn;                // ions per row of the workspaces (nmax)
+  int stage_extra;       // bytes of staging buffer after the shared layout (0: the 16 KB within it)
   unsigned short* nbl;   // [cluster][2][wn][wn] partners within the long / short cutoff
   int* nbn;              // [cluster][2][wn]
   // pair cache of the dipole operator, rows of the box's polarisable ions
@@ -137,6 +138,8 @@ struct BShared {
   double* red;     // [kBPart * 32]
   double* res;     // [kBPart]
   int* cfg;        // [1]
+  unsigned char* stage;  // staging buffer of the reciprocal sums
+  int stage_bytes;
 };
 
 __host__ __device__ inline size_t batch_smem_bytes(int nmax) {
@@ -170,6 +173,8 @@ __device__ inline BShared batch_smem(unsigned char* base, int nmax) {
   S.res = reinterpret_cast<double*>(base + o); o += sizeof(double) * kBPart;
   S.t = reinterpret_cast<int*>(base + o); o += sizeof(int) * nmax;
   S.cfg = reinterpret_cast<int*>(base + o);
+  S.stage = reinterpret_cast<unsigned char*>(S.rho);
+  S.stage_bytes = kBKChunk * (int)sizeof(double2);
   return S;
 }
 
@@ -230,39 +235,23 @@ __device__ inline void gather_pol32(const BCtx& X, const int* t, const double4* 
   }
 }
 
-template <typename R>
-__device__ __forceinline__ typename cplx<R>::T btab(const BatchArgs& a, const BConf& c, int e, int i);
-template <>
-__device__ __forceinline__ double2 btab<double>(const BatchArgs& a, const BConf& c, int e, int i) {
+// phase tables of the adjoint's sums
+__device__ __forceinline__ double2 btab(const BatchArgs& a, const BConf& c, int e, int i) {
   return a.tab64[c.tab_off + (long long)e * c.tab_ld + i];
 }
-template <>
-__device__ __forceinline__ float2 btab<float>(const BatchArgs& a, const BConf& c, int e, int i) {
-  return a.tab32[c.tab_off + (long long)e * c.tab_ld + i];
-}
-
 // X_nx Y_ny Z_nz of ion i (negative indices by conjugation)
-template <typename R>
-__device__ __forceinline__ typename cplx<R>::T bphase(const BatchArgs& a, const BConf& c, int i,
-                                                      int nx, int ny, int nz) {
-  typedef typename cplx<R>::T Cx;
-  Cx X = btab<R>(a, c, nx, i);
-  int ay = ny < 0 ? -ny : ny;
-  Cx Y = btab<R>(a, c, c.kx + 1 + ay, i);
-  if (ny < 0) Y = cconj(Y);
+__device__ __forceinline__ double2 bphase_z(const BatchArgs& a, const BConf& c, int i, double2 XY, int nz) {
   int az = nz < 0 ? -nz : nz;
-  Cx Z = btab<R>(a, c, c.kx + 1 + c.ky + 1 + az, i);
-  if (nz < 0) Z = cconj(Z);
-  return cmul(cmul(X, Y), Z);
-}
-template <typename R>
-__device__ __forceinline__ typename cplx<R>::T bphase_z(const BatchArgs& a, const BConf& c, int i,
-                                                        typename cplx<R>::T XY, int nz) {
-  typedef typename cplx<R>::T Cx;
-  int az = nz < 0 ? -nz : nz;
-  Cx Z = btab<R>(a, c, c.kx + 1 + c.ky + 1 + az, i);
+  double2 Z = btab(a, c, c.kx + 1 + c.ky + 1 + az, i);
   if (nz < 0) Z = cconj(Z);
   return cmul(XY, Z);
+}
+__device__ __forceinline__ double2 bphase(const BatchArgs& a, const BConf& c, int i, int nx, int ny, int nz) {
+  double2 X = btab(a, c, nx, i);
+  int ay = ny < 0 ? -ny : ny;
+  double2 Y = btab(a, c, c.kx + 1 + ay, i);
+  if (ny < 0) Y = cconj(Y);
+  return bphase_z(a, c, i, cmul(X, Y), nz);
 }
 
 // m = 2 pi B^T mu (so that k.mu = n.m)
@@ -273,10 +262,8 @@ __device__ __forceinline__ double3 bmvec(const BConf& c, double mx, double my, d
 }
 
 // ---------------------------------------------------------------------------
-// weights (q, 2 pi B^T mu) of list entry k for the structure factor: mode 0 all
-// ions (q and mu from S.s, S.v by ion), 1 / 2 the polarisable ions (no charge,
-// mu from S.v / S.v32 by rank)
-template <typename R>
+// weights (q, 2 pi B^T mu) of list entry k: mode 0 all ions (q and mu from S.s,
+// S.v by ion), 1 / 2 the polarisable ions (no charge, mu from S.v / S.v32 by rank)
 struct BWeights {
   const BConf* c;
   const double4* s;
@@ -284,7 +271,7 @@ struct BWeights {
   const float4* v32;
   int n0, mode;
   bool has_q, has_mu;
-  __device__ __forceinline__ void operator()(int k, R (&w)[4]) const {
+  __device__ __forceinline__ void operator()(int k, double (&w)[4]) const {
     double mx = 0.0, my = 0.0, mz = 0.0;
     if (has_mu) {
       if (mode == 2) {
@@ -300,154 +287,133 @@ struct BWeights {
       }
     }
     const double3 m = bmvec(*c, mx, my, mz);
-    w[0] = (mode == 0 && has_q) ? (R)s[n0 + k].w : R(0);
-    w[1] = (R)m.x;
-    w[2] = (R)m.y;
-    w[3] = (R)m.z;
+    w[0] = (mode == 0 && has_q) ? s[n0 + k].w : 0.0;
+    w[1] = m.x;
+    w[2] = m.y;
+    w[3] = m.z;
   }
 };
 
-template <typename R>
-struct BRhoArgs {
+struct BRecArgs {
   const BConf* c;
   const int4* rows;
-  BList src;             // ions of the structure factor
+  BList src, dst;        // ions of the structure factor / of the field
   const int* t;
-  unsigned char* stage;
   const unsigned char* rec;
+  const double2* apm;
+  const double4* w;      // weights of src
+  unsigned char* buf;    // two buffers of CH records
+  int CH;
   double4* out;          // this CTA's partials
-  BWeights<R> w;
-};
-template <typename R>
-struct BFldArgs {
-  const BConf* c;
-  const int4* rows;
-  BList dst;             // ions of the field
-  const int* t;
-  unsigned char* stage;
-  const typename cplx<R>::T* tab;
-  const double* Ak;
   const double4* part;   // rank 0's partials
   size_t pld;
   int C;
+  unsigned char* stage;
+  int stage_bytes;
   double* gp;
   int gld;
-  BWeights<R> w;
+  BWeights wd;           // dipole weights of dst
 };
 
-template <typename R, int T, bool HM>
-__device__ __noinline__ void brho_n(const BRhoArgs<R>& r) {
+template <int NT, bool HM>
+__device__ __noinline__ void brho_n(const BRecArgs& r) {
   const BConf& c = *r.c;
-  brho_t<R, T, HM>(r.rec, sizeof(R) == 8 ? c.rs64 : c.rs32, sizeof(R) == 8 ? c.zo64 : c.zo32, c.kx, c.kz,
-                   r.rows, c.nrows, r.src, r.t, r.stage, r.out, r.w);
+  brho_t<NT, HM>(r.rec, c.rs, c.zo, c.kx, c.kz, r.rows, c.nrows, r.src, r.t, r.w, r.buf, r.CH, r.out);
 }
-template <typename R, bool HM>
-__device__ __forceinline__ void brho(const BRhoArgs<R>& r) {
-  switch (sizeof(R) == 8 ? r.c->t64 : r.c->t32) {
-    case 5: if constexpr (sizeof(R) == 8) brho_n<R, 5, HM>(r); break;
-    case 6: brho_n<R, 6, HM>(r); break;
-    case 7: brho_n<R, 7, HM>(r); break;
-    case 8: brho_n<R, 8, HM>(r); break;
-    case 9: if constexpr (sizeof(R) == 4) brho_n<R, 9, HM>(r); break;
-    case 10: if constexpr (sizeof(R) == 4) brho_n<R, 10, HM>(r); break;
-    default: if constexpr (sizeof(R) == 4) brho_n<R, 13, HM>(r); break;
+template <bool HM>
+__device__ __forceinline__ void brho(const BRecArgs& r) {
+  switch (r.c->kz / 4) {
+    case 0: brho_n<1, HM>(r); break;
+    case 1: brho_n<2, HM>(r); break;
+    case 2: brho_n<3, HM>(r); break;
+    default: brho_n<4, HM>(r); break;
   }
 }
-template <typename R, int KT, bool MUF>
-__device__ __noinline__ int bfld_n(const BFldArgs<R>& r) {
+template <int KS, bool MUF>
+__device__ __noinline__ int bfld_n(const BRecArgs& r) {
   const BConf& c = *r.c;
-  return bfld_t<R, KT, MUF>(r.tab, c.tab_ld, c.kx, c.ky, c.kz, r.rows, c.nrows, r.Ak, r.part, r.pld, r.C,
-                            r.dst, r.t, r.stage, r.gp, r.gld, r.w);
+  return bfld_t<KS, MUF>(r.rec, c.rs, c.zo, c.kx, c.kz, r.rows, c.nrows, r.apm, r.part, r.pld, r.C, r.dst, r.t,
+                         r.stage, r.stage_bytes, r.gp, r.gld, r.wd);
 }
-template <typename R, bool MUF>
-__device__ __forceinline__ int bfld(const BFldArgs<R>& r) {
-  switch (r.c->kt) {
-    case 6: return bfld_n<R, 6, MUF>(r);
-    case 8: return bfld_n<R, 8, MUF>(r);
-    case 10: return bfld_n<R, 10, MUF>(r);
-    default: return bfld_n<R, 13, MUF>(r);
+template <bool MUF>
+__device__ __forceinline__ int bfld(const BRecArgs& r) {
+  switch (r.c->kz / 2) {
+    case 0: case 1: case 2: return bfld_n<3, MUF>(r);
+    case 3: return bfld_n<4, MUF>(r);
+    case 4: return bfld_n<5, MUF>(r);
+    case 5: return bfld_n<6, MUF>(r);
+    default: return bfld_n<7, MUF>(r);
   }
 }
 
-template <typename R>
-__device__ __forceinline__ const typename cplx<R>::T* btab_base(const BatchArgs& a, const BConf& c);
-template <>
-__device__ __forceinline__ const double2* btab_base<double>(const BatchArgs& a, const BConf& c) {
-  return a.tab64 + c.tab_off;
-}
-template <>
-__device__ __forceinline__ const float2* btab_base<float>(const BatchArgs& a, const BConf& c) {
-  return a.tab32 + c.tab_off;
-}
-
-// Reciprocal pass of one configuration.  src: the ions with weights (mode 0:
-// all of this CTA's ions with charges and / or the dipoles in S.v; 1 / 2: its
-// polarisable ions with the vector in S.v / S.v32 by rank).  The field sums are
-// left in this CTA's gpart for the ions of dst (all or polarisable);
+// Reciprocal pass of one configuration.  mode 0: the weights of all of this
+// CTA's ions with charges and / or the dipoles in S.v; 1 / 2: of its
+// polarisable ions with the vector in S.v / S.v32 by rank.  The field sums are
+// left in this CTA's gpart for all its ions or (dst_pol) its polarisable ones;
 // bfld_get reads them.  With do_str, es[0..6] receives this CTA's share of
 // (u_rec, tau_rec) scaled as k_rec_energy.  Returns the number of row subsets.
-// RR: precision of the structure factor.  The mixed engine's static and force
-// passes form it in FP64 (its rounding is common to all ions of the box: with
-// FP32 the force error of 64-1000 ion MgO boxes was twice as large), the
-// operator of its inner iterations in FP32 (the FP64 residual removes it).
-template <typename R, typename RR>
 __device__ __noinline__ int brec(cgx::cluster_group& cl, const BatchArgs& a, BCtx& X, const BShared& S, int mode,
-                    bool has_q, bool has_mu, bool dst_pol, bool muf, bool do_str, double (&es)[7]) {
+                                 bool has_q, bool has_mu, bool dst_pol, bool muf, bool do_str, double (&es)[7]) {
   const BConf& c = *X.c;
   for (int k = 0; k < 7; ++k) es[k] = 0.0;
   if (c.nk == 0) return 0;
-  const BList src = mode == 0 ? BList{X.i0, X.i1 - X.i0, false} : BList{X.p0, X.p1 - X.p0, true};
-  const BList dst = dst_pol ? BList{X.p0, X.p1 - X.p0, true} : BList{X.i0, X.i1 - X.i0, false};
-  const int4* rows = a.rows + c.row_off;
-  unsigned char* stage = reinterpret_cast<unsigned char*>(S.rho);
-  const size_t pld = 2 * a.rpart_ld;  // CTA to CTA
-  const double4* part = a.rpart + ((size_t)(blockIdx.x - X.rank) * 2 + X.rpar) * a.rpart_ld;
-  {
-    BRhoArgs<RR> q;
-    q.c = X.c;
-    q.rows = rows;
-    q.src = src;
-    q.t = S.t;
-    q.stage = stage;
-    q.rec = a.rec + (sizeof(RR) == 8 ? c.rec64 : c.rec32);
-    q.out = a.rpart + ((size_t)blockIdx.x * 2 + X.rpar) * a.rpart_ld;
-    q.w = BWeights<RR>{X.c, S.s, S.v, S.v32, src.n0, mode, has_q, has_mu};
-    // (the partials are double-buffered: a reader of the previous pass's half
-    // has passed this pass's barrier before that half is written again)
-    X.rpar ^= 1;
-    if (has_mu) brho<RR, true>(q);
-    else brho<RR, false>(q);
-  }
-  cl.sync();
-  BFldArgs<R> r;
+  BRecArgs r;
   r.c = X.c;
-  r.rows = rows;
-  r.dst = dst;
+  r.rows = a.rows + c.row_off;
+  r.src = mode == 0 ? BList{X.i0, X.i1 - X.i0, false} : BList{X.p0, X.p1 - X.p0, true};
+  r.dst = dst_pol ? BList{X.p0, X.p1 - X.p0, true} : BList{X.i0, X.i1 - X.i0, false};
   r.t = S.t;
-  r.stage = stage;
-  r.tab = btab_base<R>(a, c);
-  r.Ak = a.Ak + c.k_off;
-  r.part = part;
-  r.pld = pld;
+  r.rec = a.rec + c.rec;
+  r.apm = a.apm + c.apm_off;
+  r.pld = 2 * a.rpart_ld;  // CTA to CTA
+  // (the partials are double-buffered: a reader of the previous pass's half
+  // has passed this pass's barrier before that half is written again)
+  r.part = a.rpart + ((size_t)(blockIdx.x - X.rank) * 2 + X.rpar) * a.rpart_ld;
+  r.out = a.rpart + ((size_t)blockIdx.x * 2 + X.rpar) * a.rpart_ld;
+  X.rpar ^= 1;
   r.C = X.C;
+  r.stage = S.stage;
+  r.stage_bytes = S.stage_bytes;
   r.gp = a.gpart + (size_t)blockIdx.x * kBSplit * 6 * a.wn;
   r.gld = a.wn;
-  r.w = BWeights<R>{X.c, S.s, S.v, S.v32, dst.n0, 0, false, true};
+  r.wd = BWeights{X.c, S.s, S.v, S.v32, r.dst.n0, 0, false, true};
+  {
+    // weights once per ion: in the staging buffer, else in the field's scratch
+    const BWeights ws{X.c, S.s, S.v, S.v32, r.src.n0, mode, has_q, has_mu};
+    // (the rest of the buffer holds the records in passing)
+    const bool in_stage = r.src.cnt * 32 <= S.stage_bytes / 3;
+    double4* w = in_stage ? reinterpret_cast<double4*>(S.stage) : reinterpret_cast<double4*>(r.gp);
+    r.buf = S.stage + (in_stage ? (r.src.cnt * 32 + 127) / 128 * 128 : 0);
+    const int ch = (int)((S.stage + S.stage_bytes - r.buf) / (2 * c.rs)) & ~3;
+    r.CH = ch < 32 ? ch : 32;
+    __syncthreads();
+    for (int k = threadIdx.x; k < r.src.cnt; k += blockDim.x) {
+      double v[4];
+      ws(k, v);
+      w[k] = make_double4(v[0], v[1], v[2], v[3]);
+    }
+    __syncthreads();
+    r.w = w;
+  }
+  if (has_mu) brho<true>(r);
+  else brho<false>(r);
+  cl.sync();
   if (do_str) {
     // energy and stress of this CTA's share of the rows
     const int nz = c.kz + 1;
     const double4* kv0 = a.kvec + c.k_off;
+    const double* Ak = a.Ak + c.k_off;
     const int r0 = (int)((long long)c.nrows * X.rank / X.C), r1 = (int)((long long)c.nrows * (X.rank + 1) / X.C);
     for (int e = threadIdx.x; e < (r1 - r0) * nz; e += blockDim.x) {
       const int row = r0 + e / nz, n = e % nz;
-      const int4 ri = rows[row];
+      const int4 ri = r.rows[row];
       double2 rp, rm;
-      brho_pm(part, pld, X.C, nz, ri, row, n, nullptr, rp, rm);
+      brho_pm(r.part, r.pld, X.C, (size_t)row * nz + n, nullptr, rp, rm);
       for (int sg = 0; sg < 2; ++sg) {
         if (sg ? !(n > 0 && ri.z < 0) : n < ri.z) continue;
         const int k = ri.w + (sg ? -n : n) - ri.z;
         const double2 v = sg ? rm : rp;
-        const double st = (v.x * v.x + v.y * v.y) * r.Ak[k];
+        const double st = (v.x * v.x + v.y * v.y) * Ak[k];
         const double4 kv = kv0[k];
         es[0] += st;
         es[1] += (1.0 - kv.w * kv.x * kv.x) * st;
@@ -462,8 +428,8 @@ __device__ __noinline__ int brec(cgx::cluster_group& cl, const BatchArgs& a, BCt
     es[0] *= 2.0 * tpi_V;
     for (int k = 1; k < 7; ++k) es[k] *= 2.0 * tpi_V / c.omega;
   }
-  if (muf) return bfld<R, true>(r);
-  return bfld<R, false>(r);
+  if (muf) return bfld<true>(r);
+  return bfld<false>(r);
 }
 
 // field e (and dipole force fm) of list entry k from the row subsets' sums
@@ -555,7 +521,7 @@ __device__ __noinline__ void blists(const BatchArgs& a, const BCtx& X, const BSh
   __syncthreads();
 }
 // the lists are rewritten for every box a cluster takes and may have been
-// written by another CTA: read through L2
+// written by another CTA: read through L2, one visit ahead of their use
 __device__ __forceinline__ int bnbr(const unsigned short* l, int k) { return (int)__ldcg(l + k); }
 
 // ---------------------------------------------------------------------------
@@ -563,7 +529,7 @@ __device__ __forceinline__ int bnbr(const unsigned short* l, int k) { return (in
 // (warp per ion, lanes over its partner list), added into E.  QQ: damped charge field; DD:
 // dipole field.  pol = false: vectors by ion, the reference's condition (both
 // dipoles nonzero); true: vectors by rank, both ions polarisable.
-template <typename R, bool QQ, bool DD>
+template <typename R, bool QQ, bool DD, int K = 0>
 __device__ __noinline__ void bfield(const BatchArgs& a, const BCtx& X, const BShared& S, int damp, bool pol,
                        double4* __restrict__ E) {
   const BConf& c = *X.c;
@@ -581,8 +547,10 @@ __device__ __noinline__ void bfield(const BatchArgs& a, const BCtx& X, const BSh
     R ex = R(0), ey = R(0), ez = R(0);
     const unsigned short* row = bnbl(a, X, 0, i);
     const int nn = (QQ || dip_i) ? __ldcg(bnbn(a, X, 0) + i) : 0;
+    int jn = lane < nn ? bnbr(row, lane) : 0;
     for (int k = lane; k < nn; k += 32) {
-      const int j = bnbr(row, k);
+      const int j = jn;
+      if (k + 32 < nn) jn = bnbr(row, k + 32);
       const double4 sj = S.s[j];
       const int tj = S.t[j];
       R rx, ry, rz;
@@ -610,7 +578,7 @@ __device__ __noinline__ void bfield(const BatchArgs& a, const BCtx& X, const BSh
       }
       const double qj = QQ ? sj.w : 0.0;
       if (!dd && (!QQ || qj == 0.0)) continue;
-      es_field_pair<R, QQ, DD>(S.es, c.ntype, i, j, ti, btyp(tj), rx, ry, rz, r2, (R)c.alpha, damp,
+      es_field_pair<R, QQ, DD, K>(S.es, c.ntype, i, j, ti, btyp(tj), rx, ry, rz, r2, (R)c.alpha, damp,
                                qj, dd, mx, my, mz, ex, ey, ez, (c.flags & BF_THOLE) ? 1 : 0);
     }
     const double dx = warp_sum((double)ex), dy = warp_sum((double)ey), dz = warp_sum((double)ez);
@@ -643,13 +611,15 @@ __device__ __noinline__ void bcache(const BatchArgs& a, const BCtx& X, const BSh
     const int nn = __ldcg(bnbn(a, X, 0) + i);
     const size_t base = (size_t)X.slot * a.ccap + (size_t)p * X.npol;
     int m = 0;
+    int jn = lane < nn ? bnbr(row, lane) : 0;
     for (int k0 = 0; k0 < nn; k0 += 32) {
       const int k = k0 + lane;
       bool keep = false;
       double rx = 0, ry = 0, rz = 0, B1 = 0, B2 = 0;
       int rk = 0;
+      const int j = jn;
+      if (k + 32 < nn) jn = bnbr(row, k + 32);
       if (k < nn) {
-        const int j = bnbr(row, k);
         const int tj = S.t[j];
         if (bpol(tj)) {
           const double r2 = pair_vec<double>(c.A, si, S.s[j], rx, ry, rz);
@@ -689,56 +659,82 @@ __device__ __noinline__ void bcache(const BatchArgs& a, const BCtx& X, const BSh
 }
 
 // T2 v of the cached pairs on this CTA's polarisable ions (vector in S.v / S.v32
-// by rank), added into E
+// by rank), added into E.  Eight lanes per row, four rows per warp, and the
+// next four entries of a lane in flight while the current ones are used: the
+// cache streams from L2, so what counts is the bytes in flight (a warp per row
+// with four entries a lane left most lanes idle in every row's last round and
+// paid its reduction per row).
+template <typename R>
+struct BPairs {
+  R x[4], y[4], z[4], b2[4], b1[4];
+  int j[4];
+};
+template <typename R>
+__device__ __forceinline__ void bpairs_load(const BatchArgs& a, size_t base, int k0, int n, BPairs<R>& q) {
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int k = k0 + 8 * u;
+    const bool ok = k < n;
+    const size_t o = base + (ok ? k : 0);
+    q.j[u] = a.cj[o];
+    if (sizeof(R) == 4) {
+      const float4 r = a.c32[o];
+      q.x[u] = (R)r.x; q.y[u] = (R)r.y; q.z[u] = (R)r.z; q.b2[u] = (R)r.w;
+      q.b1[u] = (R)a.b32[o];
+    } else {
+      const double4 r = a.c64[o];
+      q.x[u] = (R)r.x; q.y[u] = (R)r.y; q.z[u] = (R)r.z; q.b2[u] = (R)r.w;
+      q.b1[u] = (R)a.b64[o];
+    }
+    if (!ok) q.b2[u] = q.b1[u] = R(0);
+  }
+}
 template <typename R>
 __device__ __noinline__ void bfield_cached(const BatchArgs& a, const BCtx& X, const BShared& S, double4* __restrict__ E) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-  for (int p = X.p0 + warp; p < X.p1; p += nwarp) {
-    const size_t base = (size_t)X.slot * a.ccap + (size_t)p * X.npol;
-    const int n = a.cn[(size_t)X.slot * a.wn + p];
+  const int sub = lane >> 3, l8 = lane & 7;
+  for (int pb = X.p0 + 4 * warp; pb < X.p1; pb += 4 * nwarp) {
+    const int p = pb + sub;
+    const bool ok = p < X.p1;
+    const size_t base = (size_t)X.slot * a.ccap + (size_t)(ok ? p : pb) * X.npol;
+    const int n = ok ? a.cn[(size_t)X.slot * a.wn + p] : 0;
+    // rounds of the longest of the four rows (entry 0 of an empty row is read
+    // but not used; a row of the workspace always exists)
+    const int nm = __reduce_max_sync(FULL_MASK, n);
     R ex = R(0), ey = R(0), ez = R(0);
-    constexpr int U = 4;
-    for (int k0 = lane; k0 < n; k0 += 32 * U) {
-      R x[U], y[U], z[U], b2[U], b1[U];
-      int j[U];
+    BPairs<R> q;
+    if (nm > 0) bpairs_load<R>(a, base, l8, n, q);
+    for (int k0 = 0; k0 < nm; k0 += 32) {
+      const BPairs<R> c = q;
+      if (k0 + 32 < nm) bpairs_load<R>(a, base, k0 + 32 + l8, n, q);
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int k = k0 + 32 * u;
-        const bool ok = k < n;
-        const size_t o = base + (ok ? k : k0);
-        j[u] = a.cj[o];
-        if (sizeof(R) == 4) {
-          const float4 r = a.c32[o];
-          x[u] = (R)r.x; y[u] = (R)r.y; z[u] = (R)r.z; b2[u] = (R)r.w;
-          b1[u] = (R)a.b32[o];
-        } else {
-          const double4 r = a.c64[o];
-          x[u] = (R)r.x; y[u] = (R)r.y; z[u] = (R)r.z; b2[u] = (R)r.w;
-          b1[u] = (R)a.b64[o];
-        }
-        if (!ok) b2[u] = b1[u] = R(0);
-      }
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
+      for (int u = 0; u < 4; ++u) {
         R mx, my, mz;
+        const int j = k0 + l8 + 8 * u < n ? c.j[u] : 0;
         if (sizeof(R) == 4) {
-          const float4 m = S.v32[j[u]];
+          const float4 m = S.v32[j];
           mx = (R)m.x; my = (R)m.y; mz = (R)m.z;
         } else {
-          const double4 m = S.v[j[u]];
+          const double4 m = S.v[j];
           mx = (R)m.x; my = (R)m.y; mz = (R)m.z;
         }
-        const R rm = b2[u] * (x[u] * mx + y[u] * my + z[u] * mz);
-        ex += rm * x[u] - b1[u] * mx;
-        ey += rm * y[u] - b1[u] * my;
-        ez += rm * z[u] - b1[u] * mz;
+        const R rm = c.b2[u] * (c.x[u] * mx + c.y[u] * my + c.z[u] * mz);
+        if (k0 + l8 + 8 * u < n) {
+          ex += rm * c.x[u] - c.b1[u] * mx;
+          ey += rm * c.y[u] - c.b1[u] * my;
+          ez += rm * c.z[u] - c.b1[u] * mz;
+        }
       }
     }
-    const double dx = warp_sum((double)ex), dy = warp_sum((double)ey), dz = warp_sum((double)ez);
-    if (lane == 0) {
+    double d[3] = {(double)ex, (double)ey, (double)ez};
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) d[c] += __shfl_xor_sync(FULL_MASK, d[c], o);
+    if (ok && l8 == 0) {
       const int gi = X.off + bpl(S.t[p]);
       const double4 o = E[gi];
-      E[gi] = make_double4(o.x + dx, o.y + dy, o.z + dz, 0.0);
+      E[gi] = make_double4(o.x + d[0], o.y + d[1], o.z + d[2], 0.0);
     }
   }
 }
@@ -758,8 +754,10 @@ __device__ __noinline__ void bshort(const BatchArgs& a, const BCtx& X, const BSh
     double fb[3] = {0, 0, 0}, fl[3] = {0, 0, 0};
     const unsigned short* row = bnbl(a, X, 1, i);
     const int nn = bnbn(a, X, 1)[i];
+    int jn = lane < nn ? bnbr(row, lane) : 0;
     for (int k = lane; k < nn; k += 32) {
-      const int j = bnbr(row, k);
+      const int j = jn;
+      if (k + 32 < nn) jn = bnbr(row, k + 32);
       double4 sj = S.s[j];
       double rx, ry, rz;
       double r2 = min_image_exact(c.A, xsub(si.x, sj.x), xsub(si.y, sj.y), xsub(si.z, sj.z), rx,
@@ -814,69 +812,80 @@ __device__ __noinline__ void bshort(const BatchArgs& a, const BCtx& X, const BSh
   }
 }
 
-// final real-space pass (k_es_force) on this CTA's ions; mu in S.v (FP64).
-template <typename R>
-__device__ __noinline__ void bforce(const BatchArgs& a, const BCtx& X, const BShared& S, double (&acc)[kESPart]) {
+// final real-space pass (k_es_force) on this CTA's ions; mu in S.v (FP64).  K,
+// THOLE as k_es_force; a lane sums its visits in R (about sixteen), as there.
+template <typename R, int K, bool THOLE>
+__device__ __noinline__ void bforce_n(const BatchArgs& a, const BCtx& X, const BShared& S, double (&acc)[kESPart]) {
   const BConf& c = *X.c;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
   const int task_qq = (c.flags & BF_QQ) ? 1 : 0, task_qd = (c.flags & BF_QD) ? 1 : 0;
   const int task_dd = (c.flags & BF_DD) ? 1 : 0;
   for (int k = 0; k < kESPart; ++k) acc[k] = 0.0;
   for (int i = X.i0 + warp; i < X.i1; i += nwarp) {
-    double4 si = S.s[i];
-    int ti = btyp(S.t[i]);
-    double qi = si.w;
-    double4 mui = S.v[i];
-    double e[3] = {0, 0, 0}, f[3] = {0, 0, 0};
+    const double4 si = S.s[i];
+    const int ti = btyp(S.t[i]);
+    const double4 mui = S.v[i];
+    const R qi = (R)si.w, mi[3] = {(R)mui.x, (R)mui.y, (R)mui.z};
+    const bool dip_i = mui.x != 0.0 || mui.y != 0.0 || mui.z != 0.0;
+    R e[3] = {0, 0, 0}, f[3] = {0, 0, 0}, la[kESPart];
+#pragma unroll
+    for (int k = 0; k < kESPart; ++k) la[k] = R(0);
     const unsigned short* row = bnbl(a, X, 0, i);
     const int nn = bnbn(a, X, 0)[i];
+    int jn = lane < nn ? bnbr(row, lane) : 0;
     for (int k = lane; k < nn; k += 32) {
-      const int j = bnbr(row, k);
-      double4 sj = S.s[j];
-      double rxd, ryd, rzd;
-      double r2d = min_image_exact(c.A, xsub(si.x, sj.x), xsub(si.y, sj.y), xsub(si.z, sj.z), rxd,
-                                   ryd, rzd);
-      if (r2d > c.rc2) continue;
-      int tj = btyp(S.t[j]);
-      double qj = sj.w;
-      double4 muj = S.v[j];
-      bool i_is_a = half_mask(i, j);
+      const int j = jn;
+      if (k + 32 < nn) jn = bnbr(row, k + 32);
+      const double4 sj = S.s[j];
+      R r[3];
+      const R r2 = pair_vec<R>(c.A, si, sj, r[0], r[1], r[2]);
+      if (r2 > (R)c.rc2) continue;
+      const int tj = btyp(S.t[j]);
+      const double4 muj = S.v[j];
+      const bool i_is_a = half_mask(i, j);
       const ESPair& P = S.es[(i_is_a ? ti : tj) * c.ntype + (i_is_a ? tj : ti)];
-      R r[3] = {(R)rxd, (R)ryd, (R)rzd};
-      R mi[3] = {(R)mui.x, (R)mui.y, (R)mui.z}, mj[3] = {(R)muj.x, (R)muj.y, (R)muj.z};
-      bool dip_i = (mui.x != 0.0 || mui.y != 0.0 || mui.z != 0.0);
-      bool dip_j = (muj.x != 0.0 || muj.y != 0.0 || muj.z != 0.0);
+      const R mj[3] = {(R)muj.x, (R)muj.y, (R)muj.z};
+      const bool dip_j = muj.x != 0.0 || muj.y != 0.0 || muj.z != 0.0;
       R u, fi[3], Ei[3];
-      // the single engine's pair (i's frame; Thole on the dd field and energy
-      // where the pair's table entry has it)
-      es_force_ipair<R, 0, true>(P, i_is_a, P.ldamp != 0, (R)r2d, (R)c.alpha, r, (R)qi, (R)qj, mi,
-                                 mj, dip_i, dip_j, task_qq, task_qd, task_dd, u, fi, Ei);
+      // the single engine's pair (i's frame)
+      es_force_ipair<R, K, THOLE>(P, i_is_a, P.ldamp != 0, r2, (R)c.alpha, r, qi, (R)sj.w, mi, mj, dip_i, dip_j,
+                                  task_qq, task_qd, task_dd, u, fi, Ei);
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
-        f[d] += (double)fi[d];
-        e[d] += (double)Ei[d];
+        f[d] += fi[d];
+        e[d] += Ei[d];
       }
-      acc[0] += 0.5 * (double)u;
-      acc[1] += (double)(r[0] * fi[0]);
-      acc[2] += (double)(r[1] * fi[1]);
-      acc[3] += (double)(r[2] * fi[2]);
-      acc[4] += 0.5 * (double)(r[0] * fi[1] + r[1] * fi[0]);
-      acc[5] += 0.5 * (double)(r[0] * fi[2] + r[2] * fi[0]);
-      acc[6] += 0.5 * (double)(r[1] * fi[2] + r[2] * fi[1]);
+      la[0] += u;
+      la[1] += r[0] * fi[0];
+      la[2] += r[1] * fi[1];
+      la[3] += r[2] * fi[2];
+      la[4] += r[0] * fi[1] + r[1] * fi[0];
+      la[5] += r[0] * fi[2] + r[2] * fi[0];
+      la[6] += r[1] * fi[2] + r[2] * fi[1];
     }
 #pragma unroll
+    for (int k = 0; k < kESPart; ++k) acc[k] += (k >= 1 && k < 4 ? 1.0 : 0.5) * (double)la[k];
+    double ed[3], fd[3];
+#pragma unroll
     for (int d = 0; d < 3; ++d) {
-      e[d] = warp_sum(e[d]);
-      f[d] = warp_sum(f[d]);
+      ed[d] = warp_sum((double)e[d]);
+      fd[d] = warp_sum((double)f[d]);
     }
     if (lane == 0) {
       int gi = X.off + i;
-      a.E[gi] = make_double4(e[0], e[1], e[2], 0.0);
-      a.force[gi] += f[0] * c.coul_unit;
-      a.force[a.ntot + gi] += f[1] * c.coul_unit;
-      a.force[2 * (size_t)a.ntot + gi] += f[2] * c.coul_unit;
+      a.E[gi] = make_double4(ed[0], ed[1], ed[2], 0.0);
+      a.force[gi] += fd[0] * c.coul_unit;
+      a.force[a.ntot + gi] += fd[1] * c.coul_unit;
+      a.force[2 * (size_t)a.ntot + gi] += fd[2] * c.coul_unit;
     }
   }
+}
+template <typename R>
+__device__ __forceinline__ void bforce(const BatchArgs& a, const BCtx& X, const BShared& S, double (&acc)[kESPart]) {
+  const int fl = X.c->flags;
+  if (fl & BF_THOLE) bforce_n<R, 0, true>(a, X, S, acc);
+  else if (fl & BF_TT4) bforce_n<R, 4, false>(a, X, S, acc);
+  else bforce_n<R, 0, false>(a, X, S, acc);
 }
 
 __device__ __forceinline__ double4 bmat3(const double* m, double4 v) {
@@ -958,7 +967,7 @@ __device__ void bmatvec(cgx::cluster_group& cl, const BatchArgs& a, BCtx& X, con
     Tv[X.off + bpl(S.t[p])] = make_double4(0, 0, 0, 0);
   __syncthreads();
   double es[7];
-  const int RS = brec<R, R>(cl, a, X, S, sizeof(R) == 4 ? 2 : 1, false, true, true, false, false, es);
+  const int RS = brec(cl, a, X, S, sizeof(R) == 4 ? 2 : 1, false, true, true, false, false, es);
   if (bcached(a, X)) bfield_cached<R>(a, X, S, Tv);
   else bfield<R, false, true>(a, X, S, 0, true, Tv);
   double tot[6] = {0, 0, 0, 0, 0, 0};
@@ -1079,25 +1088,6 @@ __device__ void bsolve(cgx::cluster_group& cl, const BatchArgs& a, BCtx& X, cons
   }
 }
 
-// entry m of axis d of an ion's phase record (entries of n > kz stay zero)
-template <typename R>
-__device__ __forceinline__ void brec_put(unsigned char* rec, int zo, int d, int e0, int m, int kz, double cs,
-                                         double sn) {
-  typedef typename cplx<R>::T C2;
-  if (d < 2) {
-    C2 v;
-    v.x = (R)cs;
-    v.y = (R)sn;
-    reinterpret_cast<C2*>(rec)[e0 + m] = v;
-  } else if (m <= kz) {
-    R* z = reinterpret_cast<R*>(rec + zo) + 4 * m;
-    z[0] = (R)cs;
-    z[1] = (R)sn;
-    z[2] = (R)(m * cs);
-    z[3] = (R)(m * sn);
-  }
-}
-
 // ---------------------------------------------------------------------------
 // one configuration, whole cluster
 template <bool MIXED>
@@ -1124,9 +1114,10 @@ __device__ void bconfig(cgx::cluster_group& cl, const BatchArgs& a, BCtx& X, con
           sincospi(2.0 * (double)m * w, &sn, &cs);
           long long o = c.tab_off + (long long)(e0 + m) * c.tab_ld + i;
           a.tab64[o] = make_double2(cs, sn);
-          if (MIXED) a.tab32[o] = make_float2((float)cs, (float)sn);
-          brec_put<double>(a.rec + c.rec64 + (size_t)i * c.rs64, c.zo64, d, e0, m, c.kz, cs, sn);
-          if (MIXED) brec_put<float>(a.rec + c.rec32 + (size_t)i * c.rs32, c.zo32, d, e0, m, c.kz, cs, sn);
+          // (entries of n > kz stay zero)
+          unsigned char* rp = a.rec + c.rec + (size_t)i * c.rs;
+          if (d < 2) reinterpret_cast<double2*>(rp)[e0 + m] = make_double2(cs, sn);
+          else if (m <= c.kz) reinterpret_cast<double2*>(rp + c.zo)[m] = make_double2(cs, sn);
         }
         e0 += km[d] + 1;
       }
@@ -1185,12 +1176,13 @@ __device__ void bconfig(cgx::cluster_group& cl, const BatchArgs& a, BCtx& X, con
     gather_vec(X, a.dip, S.v);
     __syncthreads();
     if (task_qq && dipst) bfield<RM, true, true>(a, X, S, 1, false, a.Estat);
+    else if (task_qq && (c.flags & BF_TT4)) bfield<RM, true, false, 4>(a, X, S, 1, false, a.Estat);
     else if (task_qq) bfield<RM, true, false>(a, X, S, 1, false, a.Estat);
     else if (dipst) bfield<RM, false, true>(a, X, S, 1, false, a.Estat);
     if (bcached(a, X)) bcache<MIXED>(a, X, S);
     __syncthreads();
     double es[7];
-    const int RS = brec<RM, double>(cl, a, X, S, 0, task_qq, dipst, true, false, false, es);
+    const int RS = brec(cl, a, X, S, 0, task_qq, dipst, true, false, false, es);
     double tot[6] = {0, 0, 0, 0, 0, 0};
     if (lsurf) {
       double m[8];
@@ -1279,7 +1271,7 @@ __device__ void bconfig(cgx::cluster_group& cl, const BatchArgs& a, BCtx& X, con
   {
     bool has_mu = (c.flags & (BF_QD | BF_DD)) != 0;
     double es[7];
-    const int RS = brec<RM, double>(cl, a, X, S, 0, task_qq, has_mu, false, has_mu, true, es);
+    const int RS = brec(cl, a, X, S, 0, task_qq, has_mu, false, has_mu, true, es);
     cluster_sum<7>(cl, X, S, es);
     if (X.rank == 0 && threadIdx.x == 0)
       for (int k = 0; k < 7; ++k) out[BS_REC + k] = es[k];
@@ -1327,6 +1319,10 @@ template <bool MIXED>
 __global__ void __launch_bounds__(512) k_batch(BatchArgs a, int nmax) {
   extern __shared__ __align__(16) unsigned char bsm[];
   BShared S = batch_smem(bsm, nmax);
+  if (a.stage_extra) {
+    S.stage = bsm + batch_smem_extra_offset(nmax);
+    S.stage_bytes = a.stage_extra;
+  }
   cgx::cluster_group cl = cgx::this_cluster();
   BCtx X;
   X.rank = (int)cl.block_rank();

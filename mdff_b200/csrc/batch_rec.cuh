@@ -1,36 +1,37 @@
 // batch_rec.cuh -- reciprocal space (multipole_ES_rec, ewald_rec.f90:38-365)
-// of one configuration of the batched engine, as register-tiled products.
+// of one configuration of the batched engine, as FP64 tensor-core products.
 //
 // The mesh is rows (nx, ny) of nz = -kz..kz, and Z_{-n} = conj Z_n, so both
-// signs of nz come from one pass over n = 0..kz: with P = X_nx Y_ny, the
+// signs of nz come from one product over n = 0..kz: with P = X_nx Y_ny, the
 // ion's row weight U = (q + i (nx m1 + ny m2)) P and V = i m3 P,
-//   S(+-n) = a1 +- a2,  a1 = sum_i [ U c_n + i V n s_n ],  a2 = sum_i [ i U s_n + V n c_n ],
-// (c_n, s_n) = Z_n: 8 multiply-adds per (row, n) for two k vectors, no phase
-// recurrence, and the weights are formed once per (row, ion) instead of once
-// per k.  The field is the transpose: with sigma = rho'(n) + rho'(-n) and
+//   S(+-n) = a1 +- a2,  a1 = sum_i [ U c_n + i n V s_n ],  a2 = sum_i [ i U s_n + n V c_n ],
+// (c_n, s_n) = Z_n: a product with M = (re, im) of U and V of the rows, N =
+// (c_n, s_n), K = ions, 8 multiply-adds per (row, n) for two k vectors and no phase
+// recurrence.  The field is the transpose: with sigma = rho'(n) + rho'(-n) and
 // delta = rho'(n) - rho'(-n),
-//   T  = sum_n rho' conj(Z) = sum_n (sigma c_n - i delta s_n),
+//   T  = sum_nz rho' conj(Z) = sum_n (sigma c_n - i delta s_n),
 //   T1 = sum_nz nz rho' conj(Z) = sum_n n (delta c_n - i sigma s_n),
-// then recarg sums are Im(conj(P) T), Im(conj(P) T1).
+// a product with M = ions, K = (c_n, s_n) (times n, n^2), N = (re, im) of the rows; the recarg
+// sums are Im(conj(P) T), Im(conj(P) T1).
 //
-// Bound: FMA issue of the structure factor (FP32 or FP64 pipe) and the
-// broadcast loads that feed it.  brho: one lane per mesh row, the ion's phase
-// record (X, Y, and (c, s, n c, n s) per n, contiguous) read as broadcasts
-// through L1; the warps of a CTA split (row block, ion subset), every CTA
-// of the cluster takes its own ions and all rows, so a record is read by one
-// CTA only; the ion subsets are summed through shared memory in FP64 in a fixed order.
-// bfld: one lane per ion, (c, s) in registers, the coefficients of a row
-// broadcast from shared memory; the warps split (ion block, row subset).
-// Against one thread per (k tile, ion) with a phase recurrence and FP64
-// weights formed per tile: see the batch kernel's figures in batch.cuh.
+// Bound: the FP64 pipe.  brho: a warp owns 8 mesh rows and all ions of its CTA (no sum
+// over warps), four ions a step; the operands come from the ions' phase records (X, Y, then
+// (c, s) per n, contiguous) through L1.  Every CTA of the cluster takes its own
+// ions and all rows; the CTAs' partial sums meet in the field's staging.  bfld:
+// a warp owns 16 ions, their (c, s) in registers, and a subset of the rows, four
+// rows a step, whose coefficients are staged in shared memory.  Measured inside
+// the batch kernel (256 boxes of 64-1000 ions, mixed, 2 CTAs x 512 threads), per CTA and
+// application of the operator, against register tiles of scalar FMAs (FP32 in the
+// mixed engine): see batch.cuh.
 #pragma once
 #include "common.cuh"
+#include "dmma.cuh"
 #include "realspace.cuh"
 #include "recip.cuh"
 
 namespace mdff {
 
-constexpr int kBStage = 16384;  // bytes of the shared staging buffer (BShared::rho)
+constexpr int kBStage = 16384;  // least bytes of the shared staging buffer
 constexpr int kBSplit = 8;      // most row subsets of the field's ion blocks
 
 // words of an ion: type (4 bits), polarisable flag (1), its rank among the
@@ -40,30 +41,8 @@ __host__ __device__ __forceinline__ bool bpol(int t) { return ((t >> 4) & 1) != 
 __host__ __device__ __forceinline__ int brank(int t) { return (t >> 5) & 2047; }
 __host__ __device__ __forceinline__ int bpl(int t) { return (t >> 16) & 2047; }
 
-// n tile of the structure factor for kz + 1 values of n (FP64: at most 8 in
-// registers, more in two tiles) and the field's padded n count
-inline int brho_tile(int nz, bool fp64) {
-  if (fp64) {
-    const int nt = (nz + 7) / 8, t = (nz + nt - 1) / nt;
-    return t < 5 ? 5 : t;
-  }
-  return nz <= 6 ? 6 : nz <= 10 ? nz : 13;
-}
-inline int bfld_tile(int nz) { return nz <= 6 ? 6 : nz <= 8 ? 8 : nz <= 10 ? 10 : 13; }
-
-// (x, y, z, w) of a record entry
-__device__ __forceinline__ void bld4(const float* p, float (&v)[4]) {
-  const float4 a = *reinterpret_cast<const float4*>(p);
-  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-}
-__device__ __forceinline__ void bld4(const double* p, double (&v)[4]) {
-  const double2 a = *reinterpret_cast<const double2*>(p), b = *reinterpret_cast<const double2*>(p + 2);
-  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-}
-
 // the ions of a reciprocal pass on one CTA: ions n0.. (all ions) or the
-// polarisable ions of rank n0.. (pol), cnt of them; the weights of entry k are
-// w(k) = (q, m1, m2, m3)
+// polarisable ions of rank n0.. (pol), cnt of them
 struct BList {
   int n0, cnt;
   bool pol;
@@ -72,145 +51,156 @@ __device__ __forceinline__ int blist_ion(const BList& L, const int* t, int k) {
   return L.pol ? bpl(t[L.n0 + k]) : L.n0 + k;
 }
 
-// Partial structure factor of this CTA's ions over all rows:
-// out[row * (kz + 1) + n] = (a1, a2).  stage: kBStage bytes.  W(k, w): weights
-// of list entry k.
-template <typename R, int T, bool HM, typename W>
-__device__ __forceinline__ void brho_t(const unsigned char* __restrict__ rec, int stride, int zoff, int kx,
-                                       int kz, const int4* __restrict__ rows, int nrows, const BList& L,
-                                       const int* t, unsigned char* stage, double4* __restrict__ out,
-                                       const W& wfun) {
-  typedef typename cplx<R>::T C2;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int nrb = (nrows + 31) / 32, NR = nrb < nw ? nrb : nw, ks = nw / NR;
-  const int rbw = warp / ks, kk = warp % ks;
-  const bool act = rbw < NR;
-  const int nz = kz + 1;
-  constexpr int CAP = kBStage / (4 * (int)sizeof(R));
-  R* sw = reinterpret_cast<R*>(stage);
-  for (int rb0 = 0; rb0 < nrb; rb0 += NR)
-    for (int t0 = 0; t0 < nz; t0 += T) {
-      const int row = (rb0 + rbw) * 32 + lane;
-      const int4 ri = rows[row < nrows ? row : nrows - 1];
-      const R fx = (R)ri.x, fy = (R)ri.y;
-      const int ye = kx + 1 + (ri.y < 0 ? -ri.y : ri.y);
-      const R ys = ri.y < 0 ? R(-1) : R(1);
-      R acc[T][4];
-#pragma unroll
-      for (int u = 0; u < T; ++u) acc[u][0] = acc[u][1] = acc[u][2] = acc[u][3] = R(0);
-      for (int c0 = 0; c0 < L.cnt; c0 += CAP) {
-        const int cc = L.cnt - c0 < CAP ? L.cnt - c0 : CAP;
-        __syncthreads();
-        for (int k = threadIdx.x; k < cc; k += blockDim.x) {
-          R w[4];
-          wfun(c0 + k, w);
-#pragma unroll
-          for (int d = 0; d < 4; ++d) sw[4 * k + d] = w[d];
-        }
-        __syncthreads();
-        if (act)
-          for (int k = kk; k < cc; k += ks) {
-            const unsigned char* rp = rec + (size_t)blist_ion(L, t, c0 + k) * stride;
-            const C2* xy = reinterpret_cast<const C2*>(rp);
-            const R* z = reinterpret_cast<const R*>(rp + zoff) + 4 * t0;
-            const C2 X = xy[ri.x];
-            C2 Y = xy[ye];
-            Y.y *= ys;
-            R w[4];
-            bld4(sw + 4 * k, w);
-            const C2 P = cmul(X, Y);
-            const R km = fx * w[1] + fy * w[2];
-            R Ur, Ui;
-            if (HM) {
-              Ur = w[0] * P.x - km * P.y;
-              Ui = w[0] * P.y + km * P.x;
-            } else {
-              Ur = w[0] * P.x;
-              Ui = w[0] * P.y;
-            }
-            const R Vr = -w[3] * P.y, Vi = w[3] * P.x;
-#pragma unroll
-            for (int u = 0; u < T; ++u) {
-              R v[4];
-              bld4(z + 4 * u, v);
-              acc[u][0] += Ur * v[0];
-              acc[u][1] += Ui * v[0];
-              acc[u][2] -= Ui * v[1];
-              acc[u][3] += Ur * v[1];
-              if (HM) {
-                acc[u][0] -= Vi * v[3];
-                acc[u][1] += Vr * v[3];
-                acc[u][2] += Vr * v[2];
-                acc[u][3] += Vi * v[2];
-              }
-            }
-          }
-      }
-      // sum the ion subsets (warps of one row block) in order, FP64
-      constexpr int NB = sizeof(R) == 4 ? 2 : 1;  // n per round of the buffer (16 warps x 32 lanes)
-#pragma unroll
-      for (int u0 = 0; u0 < T; u0 += NB) {
-        __syncthreads();
-#pragma unroll
-        for (int b = 0; b < NB; ++b)
-          if (u0 + b < T) {
-            R* o = sw + 4 * ((b * nw + warp) * 32 + lane);
-#pragma unroll
-            for (int d = 0; d < 4; ++d) o[d] = acc[u0 + b < T ? u0 + b : 0][d];
-          }
-        __syncthreads();
-        for (int e = threadIdx.x; e < NB * NR * 32; e += blockDim.x) {
-          const int b = e / (NR * 32), rr = e % (NR * 32), n = t0 + u0 + b;
-          const int orow = rb0 * 32 + rr;
-          if (u0 + b >= T || n >= nz || orow >= nrows) continue;
-          double s[4] = {0.0, 0.0, 0.0, 0.0};
-          for (int c = 0; c < ks; ++c) {
-            const R* o = sw + 4 * ((b * nw + (rr >> 5) * ks + c) * 32 + (rr & 31));
-#pragma unroll
-            for (int d = 0; d < 4; ++d) s[d] += (double)o[d];
-          }
-          out[(size_t)orow * nz + n] = make_double4(s[0], s[1], s[2], s[3]);
-        }
-      }
-    }
-  __syncthreads();
+__device__ __forceinline__ void cp_async16(void* smem, const void* g) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(g)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// rho'(+n), rho'(-n) of (row, n) from the CTAs' partials (summed in rank
-// order), A_k scaled; for n = 0 and the half row (0, 0) the missing partner is zero
-__device__ __forceinline__ void brho_pm(const double4* __restrict__ part, size_t ld, int C, int nz,
-                                        const int4& ri, int row, int n, const double* __restrict__ Ak,
-                                        double2& rp, double2& rm) {
+// bytes of an ion's phase record: X, Y, then (c, s) of n = 0..kz padded with
+// zeros to whole tiles of brho (4 n) and steps of bfld (2 n, at least 3 steps);
+// 32 mod 128, so that the lanes of a fragment load hit distinct banks
+__host__ __device__ inline int brec_bytes(int kx, int ky, int kz) {
+  const int z1 = (kz / 4 + 1) * 64, z2 = (kz / 2 < 2 ? 3 : kz / 2 + 1) * 32;
+  const int b = (kx + 1 + ky + 1) * 16 + (z1 > z2 ? z1 : z2);
+  return (b + 95) / 128 * 128 + 32;
+}
+
+// Partial structure factor of this CTA's ions over all rows: out[row * (kz + 1)
+// + n] = (a1, a2).  w: weights (q, m1, m2, m3) of the list entries.  NT: tiles of
+// four n, covering kz + 1.  The records pass through shared memory (buf, two
+// buffers of CH records), every warp reading all of them.
+template <int NT, bool HM>
+__device__ __forceinline__ void brho_t(const unsigned char* __restrict__ rec, int stride, int zoff, int kx,
+                                       int kz, const int4* __restrict__ rows, int nrows, const BList& L,
+                                       const int* t, const double4* w, unsigned char* buf, int CH,
+                                       double4* __restrict__ out) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int g = lane >> 2, tt = lane & 3;
+  const int ng = (nrows + 7) / 8, nz = kz + 1;
+  const int pieces = stride / 16, nch = (L.cnt + CH - 1) / CH;
+  auto fetch = [&](int c) {
+    const int k0 = c * CH, m = (L.cnt - k0 < CH ? L.cnt - k0 : CH) * pieces;
+    unsigned char* o = buf + (size_t)(c & 1) * CH * stride;
+    for (int e = threadIdx.x; e < m; e += blockDim.x) {
+      const int k = e / pieces, pc = e - k * pieces;
+      cp_async16(o + k * stride + pc * 16, rec + (size_t)blist_ion(L, t, k0 + k) * stride + pc * 16);
+    }
+    cp_async_commit();
+  };
+  for (int it0 = 0; it0 < ng; it0 += nw) {
+    const int it = it0 + warp;
+    const bool act = it < ng;
+    const int row = it * 8 + g;
+    const int4 ri = rows[row < nrows ? row : nrows - 1];
+    const double fx = (double)ri.x, fy = (double)ri.y;
+    const int xo = ri.x * 16, yo = (kx + 1 + (ri.y < 0 ? -ri.y : ri.y)) * 16;
+    const bool yn = ri.y < 0;
+    double u[NT][4], v[HM ? NT : 1][4];
+#pragma unroll
+    for (int q = 0; q < NT; ++q)
+#pragma unroll
+      for (int d = 0; d < 4; ++d) {
+        u[q][d] = 0.0;
+        if (HM) v[HM ? q : 0][d] = 0.0;
+      }
+    if (nch > 0) fetch(0);
+    for (int c = 0; c < nch; ++c) {
+      if (c + 1 < nch) {
+        fetch(c + 1);
+        cp_async_wait<1>();
+      } else {
+        cp_async_wait<0>();
+      }
+      __syncthreads();
+      if (act) {
+        const int kb = c * CH, m = L.cnt - kb < CH ? L.cnt - kb : CH;
+        const unsigned char* rb = buf + (size_t)(c & 1) * CH * stride;
+#pragma unroll 2
+        for (int k0 = 0; k0 < m; k0 += 4) {
+          const bool ok = k0 + tt < m;  // weights zero past the end
+          const int k = ok ? k0 + tt : k0;
+          const unsigned char* rp = rb + k * stride;
+          const double2 X = *reinterpret_cast<const double2*>(rp + xo);
+          double2 Y = *reinterpret_cast<const double2*>(rp + yo);
+          Y.y = flip_if(Y.y, yn);
+          const double2* wp = reinterpret_cast<const double2*>(w + kb + k);
+          double2 wa = wp[0], wb = wp[1];
+          if (!ok) wa.x = wa.y = wb.x = wb.y = 0.0;
+          const double2 P = cmul(X, Y);
+          double Ur = wa.x * P.x, Ui = wa.x * P.y;
+          if (HM) {
+            const double km = fx * wa.y + fy * wb.x;
+            Ur -= km * P.y;
+            Ui += km * P.x;
+          }
+          const double Vr = -wb.y * P.y, Vi = wb.y * P.x;
+#pragma unroll
+          for (int s = 0; s < NT; ++s) {
+            const double b = reinterpret_cast<const double*>(rp + zoff)[8 * s + g];
+            dmma(u[s], Ur, Ui, b);
+            if (HM) dmma(v[HM ? s : 0], Vr, Vi, b);
+          }
+        }
+      }
+      __syncthreads();
+    }
+    if (act && row < nrows) {
+#pragma unroll
+      for (int s = 0; s < NT; ++s) {
+        // columns 2 tt, 2 tt + 1 = c_n, s_n of n
+        const int n = 4 * s + tt;
+        if (n >= nz) continue;
+        const double fn = (double)n;
+        const double* U = u[s];
+        const double* V = v[HM ? s : 0];
+        double4 o = make_double4(U[0], U[2], -U[3], U[1]);
+        if (HM) {
+          o.x -= fn * V[3];
+          o.y += fn * V[1];
+          o.z += fn * V[0];
+          o.w += fn * V[2];
+        }
+        out[(size_t)row * nz + n] = o;
+      }
+    }
+  }
+}
+
+// A_k rho(+n), A_k rho(-n) of (row, n) from the C CTAs' partials (summed in rank
+// order); apm: (A(+n), A(-n)) by (row, n), zero where the mesh has no such k
+__device__ __forceinline__ void brho_pm(const double4* __restrict__ part, size_t ld, int C, size_t e,
+                                        const double2* __restrict__ apm, double2& rp, double2& rm) {
+  const double2 A = apm ? apm[e] : make_double2(1.0, 1.0);
   double s[4] = {0.0, 0.0, 0.0, 0.0};
-  for (int c = 0; c < C; ++c) {
-    const double2* p = reinterpret_cast<const double2*>(part + (size_t)c * ld + (size_t)row * nz + n);
+  for (int c = 0; c < C; c += 2) {
+    const double2* p = reinterpret_cast<const double2*>(part + (size_t)c * ld + e);
+    const double2* p2 = reinterpret_cast<const double2*>(part + (size_t)(c + 1 < C ? c + 1 : c) * ld + e);
     const double2 u = __ldcg(p), v = __ldcg(p + 1);
-    s[0] += u.x;
-    s[1] += u.y;
-    s[2] += v.x;
-    s[3] += v.y;
+    double2 u2 = __ldcg(p2), v2 = __ldcg(p2 + 1);
+    if (c + 1 >= C) u2.x = u2.y = v2.x = v2.y = 0.0;
+    s[0] = s[0] + u.x + u2.x;
+    s[1] = s[1] + u.y + u2.y;
+    s[2] = s[2] + v.x + v2.x;
+    s[3] = s[3] + v.y + v2.y;
   }
-  // the row (0, 0) holds nz = 1..kz only (ri.z = 1), every other row -kz..kz
-  const bool hp = n >= ri.z, hm = n > 0 && ri.z < 0;
-  rp = hp ? make_double2(s[0] + s[2], s[1] + s[3]) : make_double2(0.0, 0.0);
-  rm = hm ? make_double2(s[0] - s[2], s[1] - s[3]) : make_double2(0.0, 0.0);
-  if (Ak) {
-    const double Ap = hp ? Ak[ri.w + n - ri.z] : 0.0, Am = hm ? Ak[ri.w - n - ri.z] : 0.0;
-    rp.x *= Ap;
-    rp.y *= Ap;
-    rm.x *= Am;
-    rm.y *= Am;
-  }
+  rp = make_double2(A.x * (s[0] + s[2]), A.x * (s[1] + s[3]));
+  rm = make_double2(A.y * (s[0] - s[2]), A.y * (s[1] - s[3]));
 }
 
 // row subsets per ion block: the count (up to kBSplit) that leaves the fewest
-// warps idle in the last round
+// warps idle in the last round, less 4 % per subset for an item's start-up
+// (loading the ions' phases, summing over lanes)
 __device__ __forceinline__ int bfld_split(int nib, int nw) {
   int best = 1;
   double eff = 0.0;
   for (int s = 1; s <= kBSplit; ++s) {
     const int items = nib * s, rounds = (items + nw - 1) / nw;
-    const double e = (double)items / (double)(rounds * nw) - 0.01 * s;
+    const double e = (double)items / (double)(rounds * nw) - 0.04 * s;
     if (e > eff) {
       eff = e;
       best = s;
@@ -222,138 +212,141 @@ __device__ __forceinline__ int bfld_split(int nib, int nw) {
 // Field (and dipole-force) sums of this CTA's ions over all k:
 // gp[(s * 6 + d) * gld + k], d = 0..2: sum_k n recarg, 3..5 (MUF): sum_k n
 // (k.m) recarg2, for row subset s = 0..split-1 of list entry k; returns split.
-// tab: phase tables [entry][ion] of leading dimension ld; part: the CTAs'
-// structure-factor partials.
-template <typename R, int KT, bool MUF, typename W>
-__device__ __forceinline__ int bfld_t(const typename cplx<R>::T* __restrict__ tab, int ld, int kx, int ky,
-                                      int kz, const int4* __restrict__ rows, int nrows,
-                                      const double* __restrict__ Ak, const double4* __restrict__ part,
-                                      size_t pld, int C, const BList& L, const int* t,
-                                      unsigned char* stage, double* __restrict__ gp, int gld, const W& wfun) {
-  typedef typename cplx<R>::T C2;
-  constexpr bool F32 = sizeof(R) == 4;
-  constexpr int RC = kBStage / (4 * (int)sizeof(R) * KT);  // rows per staged chunk
+// part: the CTAs' structure-factor partials.  KS: steps of two n, covering kz + 1.
+// W(k, w): dipole weights of list entry k (MUF).
+template <int KS, bool MUF, typename W>
+__device__ __forceinline__ int bfld_t(const unsigned char* __restrict__ rec, int stride, int zoff, int kx, int kz,
+                                      const int4* __restrict__ rows, int nrows, const double2* __restrict__ apm,
+                                      const double4* __restrict__ part, size_t pld, int C, const BList& L,
+                                      const int* t, unsigned char* stage, int stage_bytes, double* __restrict__ gp,
+                                      int gld, const W& wfun) {
+  constexpr int KN = 2 * KS;                             // padded n count
+  constexpr int RL = 4 * KN + (KS % 2 == 0 ? 8 : 0);     // doubles per staged row (bank spread)
+  const int RC = stage_bytes / (RL * 8) / 4 * 4;         // rows per staged chunk
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int nib = (L.cnt + 31) / 32, nz = kz + 1;
+  const int g = lane >> 2, tt = lane & 3;
+  const int nib = (L.cnt + 15) / 16, nz = kz + 1;
   const int RS = nib > 0 ? bfld_split(nib, nw) : 1;
-  R* sc = reinterpret_cast<R*>(stage);
+  double* sc = reinterpret_cast<double*>(stage);
+  // B[k][col]: k = (n, c or s) of lane tt, col = (row, re or im) of lane g; the
+  // values sigma, delta (re, im) of (row, n) are staged once and picked by index and sign:
+  //   T:  re = sigma_r c + delta_i s,  im = sigma_i c - delta_r s
+  //   T1: re = delta_r (n c) + sigma_i (n s),  im = delta_i (n c) - sigma_r (n s)
+  const int isS = tt & 1, comp = g & 1;
+  const int i0 = isS ? 3 - comp : comp, i1 = isS ? 1 - comp : 2 + comp;
+  const bool neg = isS && comp;
+  const int boff = (g >> 1) * RL + (tt >> 1) * 4;
   for (int ra = 0; ra < nrows; ra += RC) {
-    const int nr = nrows - ra < RC ? nrows - ra : RC;
+    const int nr = nrows - ra < RC ? nrows - ra : RC, nr4 = (nr + 3) / 4;
     __syncthreads();
-    for (int e = threadIdx.x; e < nr * KT; e += blockDim.x) {
-      const int rr = e / KT, n = e % KT;
+    for (int e = threadIdx.x; e < nr4 * 4 * KN; e += blockDim.x) {
+      const int rr = e / KN, n = e % KN;
       double2 rp = make_double2(0.0, 0.0), rm = rp;
-      if (n < nz) {
-        brho_pm(part, pld, C, nz, rows[ra + rr], ra + rr, n, Ak, rp, rm);
-      }
-      R* o = sc + 4 * e;
-      o[0] = (R)(rp.x + rm.x);
-      o[1] = (R)(rp.y + rm.y);
-      o[2] = n ? (R)(rp.x - rm.x) : R(0);
-      o[3] = n ? (R)(rp.y - rm.y) : R(0);
+      if (n < nz && rr < nr) brho_pm(part, pld, C, (size_t)(ra + rr) * nz + n, apm, rp, rm);
+      double2* o = reinterpret_cast<double2*>(sc + (size_t)rr * RL + 4 * n);
+      o[0] = make_double2(rp.x + rm.x, rp.y + rm.y);
+      o[1] = n ? make_double2(rp.x - rm.x, rp.y - rm.y) : make_double2(0.0, 0.0);
     }
     __syncthreads();
     for (int it = warp; it < nib * RS; it += nw) {
       const int ib = it % nib, rs = it / nib;
-      const int k = ib * 32 + lane;
-      const int kc = k < L.cnt ? k : L.cnt - 1;
-      const C2* tb = tab + blist_ion(L, t, kc);
-      // (FP64 keeps only (c, s) in registers and scales the products by n)
-      R c[KT], s[KT], nc[F32 ? KT : 1], ns[F32 ? KT : 1];
+      const unsigned char* rp[2];
+      double a[2][KS], an[2][KS], w[2][4];
 #pragma unroll
-      for (int n = 0; n < KT; ++n) {
-        C2 z;
-        z.x = z.y = R(0);
-        if (n < nz) z = tb[(size_t)(kx + 1 + ky + 1 + n) * ld];
-        c[n] = z.x;
-        s[n] = z.y;
-        if constexpr (F32) {
-          nc[n] = R(n) * z.x;
-          ns[n] = R(n) * z.y;
-        }
-      }
-      R w[4] = {R(0), R(0), R(0), R(0)};
-      if (MUF) wfun(kc, w);
-      double G[3] = {0.0, 0.0, 0.0}, H[3] = {0.0, 0.0, 0.0};
-      R g0 = R(0), g1 = R(0), g2 = R(0), h0 = R(0), h1 = R(0), h2 = R(0);
-      const int q0 = (int)((long long)nr * rs / RS), q1 = (int)((long long)nr * (rs + 1) / RS);
-      int nxc = q0 < q1 ? rows[ra + q0].x : 0;
-      C2 X = tb[(size_t)nxc * ld];
-      for (int r = q0; r < q1; ++r) {
-        const int4 ri = rows[ra + r];
-        if (ri.x != nxc) {
-          // the sums of one nx in R, the nx sums in FP64
-          G[0] += (double)nxc * (double)g0;
-          G[1] += (double)g1;
-          G[2] += (double)g2;
-          if (MUF) {
-            H[0] += (double)nxc * (double)h0;
-            H[1] += (double)h1;
-            H[2] += (double)h2;
-          }
-          g0 = g1 = g2 = h0 = h1 = h2 = R(0);
-          nxc = ri.x;
-          X = tb[(size_t)nxc * ld];
-        }
-        C2 Y = tb[(size_t)(kx + 1 + (ri.y < 0 ? -ri.y : ri.y)) * ld];
-        if (ri.y < 0) Y.y = -Y.y;
-        const C2 P = cmul(X, Y);
-        R tr = R(0), ti = R(0), t1r = R(0), t1i = R(0), t2r = R(0), t2i = R(0);
-        const R* q = sc + 4 * r * KT;
+      for (int q = 0; q < 2; ++q) {
+        const int k = ib * 16 + 8 * q + g;
+        const int kc = k < L.cnt ? k : L.cnt - 1;
+        rp[q] = rec + (size_t)blist_ion(L, t, kc) * stride;
+        const double* z = reinterpret_cast<const double*>(rp[q] + zoff);
 #pragma unroll
-        for (int n = 0; n < KT; ++n) {
-          R v[4];  // sigma, delta
-          bld4(q + 4 * n, v);
-          tr += v[0] * c[n];
-          tr += v[3] * s[n];
-          ti += v[1] * c[n];
-          ti -= v[2] * s[n];
-          if constexpr (F32) {
-            t1r += v[2] * nc[n];
-            t1r += v[1] * ns[n];
-            t1i += v[3] * nc[n];
-            t1i -= v[0] * ns[n];
-          } else {
-            t1r += R(n) * (v[2] * c[n] + v[1] * s[n]);
-            t1i += R(n) * (v[3] * c[n] - v[0] * s[n]);
-          }
+        for (int s = 0; s < KS; ++s) {
+          a[q][s] = z[4 * s + tt];
+          an[q][s] = (double)(2 * s + (tt >> 1)) * a[q][s];
+        }
+        if (MUF) wfun(kc, w[q]);
+      }
+      double G[2][3], H[2][3];
+#pragma unroll
+      for (int q = 0; q < 2; ++q)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) G[q][d] = H[q][d] = 0.0;
+      const int q0 = nr4 * rs / RS, q1 = nr4 * (rs + 1) / RS;
+      // this lane's row of the four, its X and Y one step ahead
+      int4 rn = make_int4(0, 0, 0, 0);
+      double2 Xn[2], Yn[2];
+      auto next = [&](int r4) {
+        const int r = ra + r4 * 4 + tt;
+        rn = rows[r < nrows ? r : nrows - 1];
+        const int ye = kx + 1 + (rn.y < 0 ? -rn.y : rn.y);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          Xn[q] = reinterpret_cast<const double2*>(rp[q])[rn.x];
+          Yn[q] = reinterpret_cast<const double2*>(rp[q])[ye];
+        }
+      };
+      if (q0 < q1) next(q0);
+      for (int r4 = q0; r4 < q1; ++r4) {
+        const int4 ri = rn;
+        const double2 X[2] = {Xn[0], Xn[1]}, Y[2] = {Yn[0], Yn[1]};
+        if (r4 + 1 < q1) next(r4 + 1);
+        double d0[4] = {0, 0, 0, 0}, d1[4] = {0, 0, 0, 0}, d2[4] = {0, 0, 0, 0};
+        const double* b = sc + (size_t)r4 * 4 * RL + boff;
+#pragma unroll
+        for (int s = 0; s < KS; ++s) {
+          const double b0 = flip_if(b[8 * s + i0], neg), b1 = flip_if(b[8 * s + i1], neg);
+          dmma(d0, a[0][s], a[1][s], b0);
+          dmma(d1, an[0][s], an[1][s], b1);
           if (MUF) {
-            t2r += R(n * n) * (v[0] * c[n] + v[3] * s[n]);
-            t2i += R(n * n) * (v[1] * c[n] - v[2] * s[n]);
+            const double fn = (double)(2 * s + (tt >> 1));
+            dmma(d2, fn * an[0][s], fn * an[1][s], b0);
           }
         }
-        const R S0 = P.x * ti - P.y * tr, S1 = P.x * t1i - P.y * t1r;
-        const R fy = (R)ri.y;
-        g0 += S0;
-        g1 += fy * S0;
-        g2 += S1;
-        if (MUF) {
-          const R R0 = P.x * tr + P.y * ti, R1 = P.x * t1r + P.y * t1i, R2 = P.x * t2r + P.y * t2i;
-          const R am = (R)ri.x * w[1] + fy * w[2];
-          const R y0 = am * R0 + w[3] * R1;
-          h0 += y0;
-          h1 += fy * y0;
-          h2 += am * R1 + w[3] * R2;
+        const double fx = (double)ri.x, fy = (double)ri.y;
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const double2 P = cmul(X[q], make_double2(Y[q].x, flip_if(Y[q].y, ri.y < 0)));
+          const double tr = d0[2 * q], ti = d0[2 * q + 1], ur = d1[2 * q], ui = d1[2 * q + 1];
+          const double S0 = P.x * ti - P.y * tr, S1 = P.x * ui - P.y * ur;
+          G[q][0] += fx * S0;
+          G[q][1] += fy * S0;
+          G[q][2] += S1;
+          if (MUF) {
+            const double vr = d2[2 * q], vi = d2[2 * q + 1];
+            const double R0 = P.x * tr + P.y * ti, R1 = P.x * ur + P.y * ui, R2 = P.x * vr + P.y * vi;
+            const double am = fx * w[q][1] + fy * w[q][2];
+            const double y0 = am * R0 + w[q][3] * R1;
+            H[q][0] += fx * y0;
+            H[q][1] += fy * y0;
+            H[q][2] += am * R1 + w[q][3] * R2;
+          }
         }
       }
-      G[0] += (double)nxc * (double)g0;
-      G[1] += (double)g1;
-      G[2] += (double)g2;
-      if (MUF) {
-        H[0] += (double)nxc * (double)h0;
-        H[1] += (double)h1;
-        H[2] += (double)h2;
-      }
-      if (k < L.cnt)
+      // (a row past the end has zero coefficients)
+#pragma unroll
+      for (int q = 0; q < 2; ++q)
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-          double* o = gp + (size_t)(rs * 6 + d) * gld + k;
-          o[0] = (ra ? o[0] : 0.0) + G[d];
+          G[q][d] += __shfl_xor_sync(FULL_MASK, G[q][d], 1);
+          G[q][d] += __shfl_xor_sync(FULL_MASK, G[q][d], 2);
           if (MUF) {
-            double* oh = o + 3 * (size_t)gld;
-            oh[0] = (ra ? oh[0] : 0.0) + H[d];
+            H[q][d] += __shfl_xor_sync(FULL_MASK, H[q][d], 1);
+            H[q][d] += __shfl_xor_sync(FULL_MASK, H[q][d], 2);
           }
         }
+      // lane tt writes component tt of its two ions
+      if (tt < 3) {
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const int k = ib * 16 + 8 * q + g;
+          if (k >= L.cnt) continue;
+          double* o = gp + (size_t)(rs * 6 + tt) * gld + k;
+          o[0] = (ra ? o[0] : 0.0) + (tt == 0 ? G[q][0] : tt == 1 ? G[q][1] : G[q][2]);
+          if (MUF) {
+            double* oh = o + 3 * (size_t)gld;
+            oh[0] = (ra ? oh[0] : 0.0) + (tt == 0 ? H[q][0] : tt == 1 ? H[q][1] : H[q][2]);
+          }
+        }
+      }
     }
   }
   __syncthreads();
