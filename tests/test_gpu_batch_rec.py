@@ -1,13 +1,13 @@
 """Reciprocal tiles, partner lists and pair cache of the batched engine at the
 edges of their ranges, against the CPU oracle.
 
-The structure factor runs in tiles of 32 mesh rows by 5-8 (FP64) or 6-13
-(FP32) values of nz, the field in padded nz counts 6 / 8 / 10 / 13, both from
-a 16 KB staging buffer (512 FP64 weights): meshes from one k vector per row to
-more row blocks than warps, nz counts on both sides of every tile width, a box
-with more ions on one CTA than the buffer holds, and a short-range cutoff
-beyond half the box.  FP64 tolerance: two dipole solves at 1e-12, 1e-9 as the
-other batch tests; mixed: the 1e-5 force bar."""
+The structure factor runs on groups of 8 mesh rows by tiles of 4 values of nz
+and steps of 4 ions, the field on 16 ions, steps of 2 nz and 4 rows, both from
+a staging buffer: meshes from one k vector per row to more row groups than
+warps, nz counts on both sides of every tile, ion counts that are not
+multiples of a step, a box whose weights do not fit the buffer on one CTA, and
+a short-range cutoff beyond half the box.  FP64 tolerance: two dipole solves at
+1e-12, 1e-9 as the other batch tests; mixed: the 1e-5 force bar."""
 import numpy as np
 import pytest
 
