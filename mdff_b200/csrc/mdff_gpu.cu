@@ -24,6 +24,7 @@
 #include "ko.cuh"
 #include "realspace.cuh"
 #include "recip.cuh"
+#include "recip_dm.cuh"
 #include "setup.h"
 
 using namespace mdff;
@@ -32,7 +33,8 @@ namespace {
 
 constexpr int NT = MDFF_NTYPEMAX;
 constexpr int kRhoThreads = 128;
-constexpr int kRhoChunk = 3072;    // ions per structure-factor block (4 chunks at 12k ions: fuller waves)
+constexpr int kRhoChunk = 3072;    // ions per block of k_rec_rho (meshes that do not fit k_rho_dm)
+constexpr int kRhoNzt = 16;        // its nz tile
 constexpr int kFieldThreads = 128;
 constexpr int kKoHist = 100;       // F_h, mu_h depth of scf_kO_v4 (moment_from_pola.f90:2050)
 
@@ -131,6 +133,9 @@ struct mdff_ctx {
   int rec_mode = 0;
   double* d_str = nullptr;
   int n_rho_chunks = 0;
+  // FP64 structure factor on the tensor cores (k_rho_dm): ions a staged buffer
+  // holds (0: the mesh does not fit), n tiles per pass and passes; most ion chunks
+  int dm_ci = 0, dm_nt = 0, dm_groups = 0;
   int nsm = 0;  // SMs of the device
   // FP32 structure factor of the CG operator on the tensor cores
   // (k_rec_rho_tc): ion chunk size and count; off when the mesh does not
@@ -422,6 +427,52 @@ static void lattice(mdff_ctx* h, const double* Ain) {
   h->omega = L.omega;
 }
 
+// ions per chunk of k_rho_dm over nion ions, and the chunks: one block per SM
+// over (row blocks x chunks x n passes), at least 16 ions a chunk
+static void rho_dm_shape(const mdff_ctx* h, int nion, int* chunk, int* nchunk) {
+  const int per = cdiv((int)h->rows.size(), kDmRows) * std::max(h->dm_groups, 1);
+  const int want = std::max(1, (h->nsm > 0 ? h->nsm : 148) / std::max(per, 1));
+  *chunk = std::max(16, cdiv(cdiv(nion, want), 8) * 8);
+  *nchunk = cdiv(nion, *chunk);
+}
+template <int NT>
+static int rho_dm_attr(int smem) {
+  if (cudaFuncSetAttribute(k_rho_dm<NT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+    return 1;
+  return cudaFuncSetAttribute(k_rho_dm<NT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess;
+}
+// most staged rows of k_field_dm (two blocks per SM up to 9 steps)
+static int field_dm_rc(int ks) { return (ks <= 9 ? 100 : 200) * 1024 / (field_dm_rl(ks) * 8) / 4 * 4; }
+template <int KS>
+static int field_dm_attr_k() {
+  const int smem = field_dm_rc(KS) * field_dm_rl(KS) * 8;
+  if (cudaFuncSetAttribute(k_field_dm<KS, DM_FIELD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+      cudaFuncSetAttribute(k_field_dm<KS, DM_FORCE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+      cudaFuncSetAttribute(k_field_dm<KS, DM_EFG>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+    return 1;
+  return 0;
+}
+#define FIELD_DM_SWITCH(KSV, CALL)  \
+  switch (KSV) {                    \
+    case 3: CALL(3); break;         \
+    case 4: CALL(4); break;         \
+    case 5: CALL(5); break;         \
+    case 6: CALL(6); break;         \
+    case 7: CALL(7); break;         \
+    case 8: CALL(8); break;         \
+    case 9: CALL(9); break;         \
+    case 11: CALL(11); break;       \
+    case 13: CALL(13); break;       \
+    default: CALL(16); break;       \
+  }
+static int field_dm_attr(int ks) {
+  int e = 0;
+#define FDA(K) e = field_dm_attr_k<K>()
+  FIELD_DM_SWITCH(ks, FDA)
+#undef FDA
+  return e;
+}
+
 // k mesh as rows (nx, ny) of consecutive nz (kspace.f90:143-207, same
 // half-space; the reference's |k|^2 order only changes summation order)
 static int build_mesh(mdff_ctx* h) {
@@ -469,6 +520,9 @@ static int build_mesh(mdff_ctx* h) {
   DALLOC(h->d_kvec, std::max(nk, 1));
   DALLOC(h->d_rchunk, h->rchunk.size());
   h->n_rho_chunks = cdiv(h->natm, kRhoChunk);
+  h->dm_ci = nrows > 0 ? rho_dm_ci(h->p.kES[0], h->p.kES[1], h->p.kES[2]) : 0;
+  h->dm_nt = rho_dm_nt(h->p.kES[2]);
+  h->dm_groups = rho_dm_groups(h->p.kES[2]);
   {
     // tensor-core structure factor: one CTA per SM over (row tiles x ion chunks)
     const char* env = std::getenv("MDFF_REC_TC");
@@ -498,7 +552,30 @@ static int build_mesh(mdff_ctx* h) {
       CK(cudaMemcpy(h->d_polslot, slot.data(), sizeof(int) * h->natm, cudaMemcpyHostToDevice));
     }
   }
-  DALLOC(h->d_rho_part, (size_t)std::max(h->n_rho_chunks, h->n_tc_chunks) * std::max(nk, 1));
+  int dm_chunks = 0, dm_len = 0;
+  rho_dm_shape(h, h->natm, &dm_len, &dm_chunks);
+  DALLOC(h->d_rho_part, (size_t)std::max({h->n_rho_chunks, h->n_tc_chunks, dm_chunks}) * std::max(nk, 1));
+  if (h->dm_ci) {
+    const int smem = (int)rho_dm_smem(h->p.kES[0], h->p.kES[1], h->p.kES[2], h->dm_ci);
+    int e = 0;
+    switch (h->dm_nt) {
+      case 1: e = rho_dm_attr<1>(smem); break;
+      case 2: e = rho_dm_attr<2>(smem); break;
+      case 3: e = rho_dm_attr<3>(smem); break;
+      case 4: e = rho_dm_attr<4>(smem); break;
+      default: e = rho_dm_attr<5>(smem); break;
+    }
+    if (e) {
+      h->err = "shared memory of k_rho_dm";
+      return MDFF_ERR_CUDA;
+    }
+  }
+  if (int ks = field_dm_ks(h->p.kES[2])) {
+    if (field_dm_attr(ks)) {
+      h->err = "shared memory of k_field_dm";
+      return MDFF_ERR_CUDA;
+    }
+  }
   if (h->rho_tc)
     CK(cudaFuncSetAttribute(k_rec_rho_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
                             (int)rho_tc_smem(h->p.kES[0], h->p.kES[1], h->p.kES[2])));
@@ -696,44 +773,90 @@ static SlotW slotw(const mdff_ctx* h) {
   return sw;
 }
 
-// nz tile of the structure factor: the width (8, 11, 13 or 16) that wastes
-// the fewest accumulator slots on rows of nzmax consecutive nz
-static int pick_nzt(int nzmax) {
-  // a whole row in one tile when it fits in 25 accumulators (per-ion set-up
-  // of the phases is then shared by all nz of the row)
-  if (nzmax == 25) return 25;
-  if (nzmax == 21) return 21;
-  const int cand[4] = {16, 13, 11, 8};
-  int best = 16, waste = 1 << 30;
-  for (int c : cand) {
-    int w = cdiv(nzmax, c) * c - nzmax;
-    if (w < waste) {
-      waste = w;
-      best = c;
+// FP64 structure factor of the weights d_w over the ions of imap (nion of them;
+// nullptr: all) into d_rho_part; returns the number of partial chunks.  Launch
+// errors surface at the caller's LAUNCH_CHECK.
+template <int NT>
+static void launch_rho_dm_n(mdff_ctx* h, dim3 g, size_t smem, const RecMesh& M, int n, const int* imap, int nion,
+                            int chunk, int has_mu) {
+  const double2* tab = h->d_tab64;
+  const double4* w = h->d_w;
+  if (has_mu)
+    (void)pdl_launch(k_rho_dm<NT, true>, g, dim3(kDmThreads), smem, h->st, tab, w, n, imap, nion, chunk, h->dm_ci, M,
+                     h->d_rho_part);
+  else
+    (void)pdl_launch(k_rho_dm<NT, false>, g, dim3(kDmThreads), smem, h->st, tab, w, n, imap, nion, chunk, h->dm_ci, M,
+                     h->d_rho_part);
+}
+static int launch_rho64(mdff_ctx* h, const RecMesh& M, int n, const int* imap, int nion, int has_q, int has_mu) {
+  if (h->dm_ci) {
+    int chunk, nchunk;
+    rho_dm_shape(h, nion, &chunk, &nchunk);
+    const dim3 g((unsigned)cdiv(M.nrows, kDmRows), (unsigned)nchunk, (unsigned)h->dm_groups);
+    const size_t smem = rho_dm_smem(M.kmax[0], M.kmax[1], M.kmax[2], h->dm_ci);
+    switch (h->dm_nt) {
+      case 1: launch_rho_dm_n<1>(h, g, smem, M, n, imap, nion, chunk, has_mu); break;
+      case 2: launch_rho_dm_n<2>(h, g, smem, M, n, imap, nion, chunk, has_mu); break;
+      case 3: launch_rho_dm_n<3>(h, g, smem, M, n, imap, nion, chunk, has_mu); break;
+      case 4: launch_rho_dm_n<4>(h, g, smem, M, n, imap, nion, chunk, has_mu); break;
+      default: launch_rho_dm_n<5>(h, g, smem, M, n, imap, nion, chunk, has_mu); break;
     }
+    return nchunk;
   }
-  return best;
+  // a mesh too large for the staging buffers: the phase recurrence over all ions
+  const int ntiles = cdiv(2 * M.kmax[2] + 1, kRhoNzt);
+  const dim3 g((unsigned)(M.nrows * ntiles), (unsigned)h->n_rho_chunks);
+  const double2* tab = h->d_tab64;
+  if (has_q && has_mu)
+    (void)pdl_launch(k_rec_rho<double, true, true, kRhoNzt>, g, dim3(kRhoThreads), 0, h->st, tab, h->d_w, n, kRhoChunk, M, ntiles, h->d_rho_part);
+  else if (has_q)
+    (void)pdl_launch(k_rec_rho<double, true, false, kRhoNzt>, g, dim3(kRhoThreads), 0, h->st, tab, h->d_w, n, kRhoChunk, M, ntiles, h->d_rho_part);
+  else
+    (void)pdl_launch(k_rec_rho<double, false, true, kRhoNzt>, g, dim3(kRhoThreads), 0, h->st, tab, h->d_w, n, kRhoChunk, M, ntiles, h->d_rho_part);
+  return h->n_rho_chunks;
 }
 
-template <typename R, int NZT>
-static void launch_rho(mdff_ctx* h, dim3 g, const typename cplx<R>::T* tab, int n, int chunk,
-                       const RecMesh& M, int ntiles, int has_q, int has_mu) {
-  if constexpr (std::is_same<R, float>::value) {
-    // FP32: two ions per thread in packed FP32x2 lanes
-    if (has_q && has_mu)
-      (void)pdl_launch(k_rec_rho_x2<true, true, NZT>, dim3(g), dim3(kRhoThreads), 0, h->st, tab, h->d_w32, n, chunk, M, ntiles, h->d_rho_part);
-    else if (has_q)
-      (void)pdl_launch(k_rec_rho_x2<true, false, NZT>, dim3(g), dim3(kRhoThreads), 0, h->st, tab, h->d_w32, n, chunk, M, ntiles, h->d_rho_part);
-    else
-      (void)pdl_launch(k_rec_rho_x2<false, true, NZT>, dim3(g), dim3(kRhoThreads), 0, h->st, tab, h->d_w32, n, chunk, M, ntiles, h->d_rho_part);
-    return;
-  }
-  if (has_q && has_mu)
-    (void)pdl_launch(k_rec_rho<R, true, true, NZT>, dim3(g), dim3(kRhoThreads), 0, h->st, tab, h->d_w, n, chunk, M, ntiles, h->d_rho_part);
-  else if (has_q)
-    (void)pdl_launch(k_rec_rho<R, true, false, NZT>, dim3(g), dim3(kRhoThreads), 0, h->st, tab, h->d_w, n, chunk, M, ntiles, h->d_rho_part);
+// FP64 field (mode DM_*) of rhoA at the ions of imap into d_G / d_H on the tensor
+// cores; returns the number of row groups
+template <int KS>
+static int launch_field_dm_k(mdff_ctx* h, const RecMesh& M, int n, const int* imap, int nion, int mode) {
+  const int tiles = cdiv(nion, kDmFldIons), nalloc = (int)h->rchunk.size() - 1;
+  const int nsm = h->nsm > 0 ? h->nsm : 148;
+  int ng = std::max(1, std::min({(KS <= 9 ? 2 : 1) * nsm / std::max(tiles, 1), cdiv(M.nrows, 4), nalloc}));
+  const int rpg = cdiv(cdiv(M.nrows, ng), 4) * 4;
+  ng = cdiv(M.nrows, rpg);
+  const int rc = std::min(rpg, field_dm_rc(KS));
+  const dim3 g((unsigned)tiles, (unsigned)ng);
+  const size_t smem = (size_t)rc * field_dm_rl(KS) * 8;
+  const double2* tab = h->d_tab64;
+  const double4* w = h->d_w;
+  const double2* rhoA = h->d_rhoA;
+#define FDL(MODE)                                                                                             \
+  (void)pdl_launch(k_field_dm<KS, MODE>, g, dim3(kDmFldThreads), smem, h->st, tab, w, n, imap, nion, M, rhoA, \
+                   rpg, rc, h->d_G, h->d_H)
+  if (mode == DM_FORCE) FDL(DM_FORCE);
+  else if (mode == DM_EFG) FDL(DM_EFG);
+  else FDL(DM_FIELD);
+#undef FDL
+  return ng;
+}
+static int launch_field_dm(mdff_ctx* h, const RecMesh& M, int n, const int* imap, int nion, int mode) {
+  int ng = 0;
+#define FDK(K) ng = launch_field_dm_k<K>(h, M, n, imap, nion, mode)
+  FIELD_DM_SWITCH(field_dm_ks(M.kmax[2]), FDK)
+#undef FDK
+  return ng;
+}
+
+// rho over the chunk partials (A_k scaled) into rhoA, A |rho|^2 into str
+static int rho_sum(mdff_ctx* h, const RecMesh& M, int nparts, double2* acc) {
+  if (nparts > 8)
+    PDL_CHECK(pdl_launch(k_rec_sum8, dim3(cdiv(h->nk, 32)), dim3(256), 0, h->st, (const double2*)h->d_rho_part, nparts,
+                         M, h->d_rhoA, h->d_str, acc));
   else
-    (void)pdl_launch(k_rec_rho<R, false, true, NZT>, dim3(g), dim3(kRhoThreads), 0, h->st, tab, h->d_w, n, chunk, M, ntiles, h->d_rho_part);
+    PDL_CHECK(pdl_launch(k_rec_sum, dim3(cdiv(h->nk, 256)), dim3(256), 0, h->st, (const double2*)h->d_rho_part, nparts,
+                         M, h->d_rhoA, h->d_str, acc));
+  return MDFF_OK;
 }
 
 // ion slots of the tensor-core structure factor: the polarisable ions
@@ -824,56 +947,46 @@ static int rec_pass_t(mdff_ctx* h, const typename cplx<R>::T* tab, const double4
     PDL_CHECK(pdl_launch(k_rec_weights, dim3(cdiv(n, 256)), dim3(256), 0, h->st, h->d_q, mu, n, h->d_cell, has_q, has_mu, h->d_w,
                          F32 ? h->d_w32 : nullptr, mu32, slotw(h)));
   }
-  int nzt = pick_nzt(2 * M.kmax[2] + 1);
-  int ntiles = cdiv(2 * M.kmax[2] + 1, nzt);
-  dim3 g((unsigned)(M.nrows * ntiles), (unsigned)h->n_rho_chunks);
-  int chunk = kRhoChunk;
   // algorithmic op counts per (k, ion) term (add = mul = 1, FMA = 2,
   // sin/cos/exp/sqrt = 1): structure factor k.r 5 + sin,cos 2 + q part 4 +
   // k.mu 5 + mu part 4; field/force pass: recarg/recarg2 8 + field 6 + F_q 6 + F_mu 12
   double ops_rho = (has_q && has_mu) ? 20.0 : (has_mu ? 16.0 : 11.0);
   double ops_fld = (forces && has_mu) ? 32.0 : (forces ? 17.0 : 20.0);
   int pr = prof_begin(h, KC_RHO, (double)h->nk * n * ops_rho);
-  int nparts = h->n_rho_chunks;
+  int nparts = 0;
   const int mode = h->rec_mode;
-  // the tensor-core structure factor serves the FP32 CG operator (dipoles
-  // alone, no forces), whose error the FP64 residual refinement removes; the
-  // static field and the force pass keep the CUDA-core kernels (FP32 sums
-  // with round-to-nearest).  The force pass after a CG solve takes the
+  // the tensor-core TF32 structure factor serves the FP32 CG operator (dipoles
+  // alone, no forces), whose error the FP64 residual refinement removes; every
+  // other pass forms it in FP64.  The force pass after a CG solve takes the
   // solve's accumulated rho' instead (REC_FROM_ACC).
   if (mode == REC_FROM_ACC) {
-    nparts = 0;
     PDL_CHECK(pdl_launch(k_rec_acc_finish, dim3(cdiv(h->nk, 256)), dim3(256), 0, h->st,
                          (const double2*)h->d_rho_acc, M, h->d_rhoA, h->d_str));
   } else if (F32 && h->rho_tc && pol_dipoles && !has_q && has_mu && !forces) {
     nparts = h->n_tc_chunks;
     launch_rho_tc(h, M, n);
   } else {
-    switch (nzt) {
-      case 8: launch_rho<R, 8>(h, g, tab, n, chunk, M, ntiles, has_q, has_mu); break;
-      case 11: launch_rho<R, 11>(h, g, tab, n, chunk, M, ntiles, has_q, has_mu); break;
-      case 13: launch_rho<R, 13>(h, g, tab, n, chunk, M, ntiles, has_q, has_mu); break;
-      case 21: launch_rho<R, 21>(h, g, tab, n, chunk, M, ntiles, has_q, has_mu); break;
-      case 25: launch_rho<R, 25>(h, g, tab, n, chunk, M, ntiles, has_q, has_mu); break;
-      default: launch_rho<R, 16>(h, g, tab, n, chunk, M, ntiles, has_q, has_mu); break;
-    }
+    const bool pol = pol_dipoles && !has_q && has_mu && h->d_polidx;
+    if (F32 && weights_ready)  // (the CG direction kernels write FP32 weights only)
+      PDL_CHECK(pdl_launch(k_rec_weights, dim3(cdiv(n, 256)), dim3(256), 0, h->st, h->d_q, mu, n, h->d_cell, has_q,
+                           has_mu, h->d_w, (float4*)nullptr, (float4*)nullptr, SlotW()));
+    nparts = launch_rho64(h, M, n, pol ? h->d_polidx : nullptr, pol ? (int)h->polidx.size() : n, has_q, has_mu);
   }
   LAUNCH_CHECK();
   prof_end(h, pr);
   double tpi_V = kTwoPi / h->omega;
-  // without energy the field pass sums the chunk partials while staging rho'
-  // (the CUDA-core field kernels when there are few chunks; the tensor-core
-  // B-tile builder always)
+  // without energy the tensor-core B-tile builder of the FP32 field sums the
+  // chunk partials itself
   int npart = 0;
   const bool field_tc = F32 && h->field_tc;
   if (mode == REC_FROM_ACC) {
     // rhoA and str are in place
-  } else if (e_out || (nparts > 4 && !field_tc) || mode == REC_SAVE_ACC || (mode == REC_NEED_RHOA && !field_tc)) {
+  } else if (e_out || !field_tc || mode == REC_SAVE_ACC) {
     // (REC_SAVE_ACC: this rho' starts the solve's accumulation; REC_NEED_RHOA:
     // the CG step after this operator adds it, which the tensor-core B-tile
     // builder writes while it sums the partials)
-    PDL_CHECK(pdl_launch(k_rec_sum, dim3(cdiv(h->nk, 256)), dim3(256), 0, h->st, (const double2*)h->d_rho_part, nparts,
-                         M, h->d_rhoA, h->d_str, mode == REC_SAVE_ACC ? h->d_rho_acc : (double2*)nullptr));
+    int e = rho_sum(h, M, nparts, mode == REC_SAVE_ACC ? h->d_rho_acc : (double2*)nullptr);
+    if (e) return e;
   } else {
     npart = nparts;
   }
@@ -891,7 +1004,9 @@ static int rec_pass_t(mdff_ctx* h, const typename cplx<R>::T* tab, const double4
   size_t smem = (size_t)h->max_chunk_k * sizeof(typename cplx<R>::T);
   bool muf = forces && has_mu;
   pr = prof_begin(h, KC_RECF, (double)h->nk * n * ops_fld);
-  if (field_tc) {
+  if (!F32 && field_dm_ks(M.kmax[2])) {
+    nch = launch_field_dm(h, M, n, imap, nion, muf ? DM_FORCE : DM_FIELD);
+  } else if (field_tc) {
     nch = launch_field_tc(h, M, n, muf, npart, imap, nion,
                           (mode == REC_NEED_RHOA && npart) ? h->d_rhoA : (double2*)nullptr);
   } else if constexpr (std::is_same<R, float>::value) {
@@ -929,7 +1044,7 @@ static int rec_pass(mdff_ctx* h, bool fp32, const double4* mu, int has_q, int ha
   if (fp32)
     return rec_pass_t<float>(h, h->d_tab32, mu, has_q, has_mu, forces, E, e_out, mu32, sf, defer_nch, weights_ready,
                              pol_dipoles);
-  return rec_pass_t<double>(h, h->d_tab64, mu, has_q, has_mu, forces, E, e_out, mu32, sf, defer_nch, false, false);
+  return rec_pass_t<double>(h, h->d_tab64, mu, has_q, has_mu, forces, E, e_out, mu32, sf, defer_nch, false, pol_dipoles);
 }
 
 // the self field 2 selfa2 mu (+ surface field of the reduced moments in mom
@@ -997,7 +1112,7 @@ static int field_of_mu(mdff_ctx* h, const double4* mu, int dd_mask, bool fp32, d
       k_es_field<double, false, true><<<nb, 256, 0, rs>>>(h->d_s, h->d_q, h->d_itype, h->d_ipolar, mu, h->L.nbr, h->L.nnb, h->L.cap, n, h->d_cell, h->d_estab, h->ntype, h->p.alphaES, cutsq, 0, dd_mask, E, h->p.thole_type);
     LAUNCH_CHECK();
     prof_end(h, pr);
-    return rec_pass(h, false, mu, 0, 1, 0, E, nullptr, sf);
+    return rec_pass(h, false, mu, 0, 1, 0, E, nullptr, sf, nullptr, nullptr, false, true);
   }
   // the CG operator with its FP32 operands ready (inside the CG graph too):
   // the cached real-space dipole field on the side stream beside the
@@ -2798,22 +2913,18 @@ int mdff_gpu_efg(mdff_handle h, double* efg) {
     int has_q = h->task_qq ? 1 : 0, has_mu = (h->task_qd || h->task_dd) ? 1 : 0;
     k_rec_weights<<<cdiv(n, 256), 256, 0, h->st>>>(h->d_q, h->d_mu_tot, n, h->d_cell, has_q, has_mu, h->d_w, nullptr, nullptr);
     LAUNCH_CHECK();
-    int nzt = pick_nzt(2 * M.kmax[2] + 1);
-    int ntiles = cdiv(2 * M.kmax[2] + 1, nzt);
-    dim3 gr((unsigned)(M.nrows * ntiles), (unsigned)h->n_rho_chunks);
-    switch (nzt) {
-      case 8: launch_rho<double, 8>(h, gr, h->d_tab64, n, kRhoChunk, M, ntiles, has_q, has_mu); break;
-      case 11: launch_rho<double, 11>(h, gr, h->d_tab64, n, kRhoChunk, M, ntiles, has_q, has_mu); break;
-      case 13: launch_rho<double, 13>(h, gr, h->d_tab64, n, kRhoChunk, M, ntiles, has_q, has_mu); break;
-      case 21: launch_rho<double, 21>(h, gr, h->d_tab64, n, kRhoChunk, M, ntiles, has_q, has_mu); break;
-      case 25: launch_rho<double, 25>(h, gr, h->d_tab64, n, kRhoChunk, M, ntiles, has_q, has_mu); break;
-      default: launch_rho<double, 16>(h, gr, h->d_tab64, n, kRhoChunk, M, ntiles, has_q, has_mu); break;
+    const int nparts = launch_rho64(h, M, n, nullptr, n, has_q, has_mu);
+    LAUNCH_CHECK();
+    int e = rho_sum(h, M, nparts, nullptr);
+    if (e) return e;
+    const double scale = 2.0 * (2.0 * (kTwoPi / h->omega));
+    if (field_dm_ks(M.kmax[2])) {
+      const int ng = launch_field_dm(h, M, n, nullptr, n, DM_EFG);
+      LAUNCH_CHECK();
+      k_efg_rec_sum<<<cdiv(n, 128), 128, 0, h->st>>>(h->d_G, h->d_H, ng, n, h->d_cell, scale, h->d_efg);
+    } else {
+      k_rec_efg<<<cdiv(n, 128), 128, 0, h->st>>>(h->d_tab64, n, M, h->d_rhoA, h->d_cell, scale, h->d_efg);
     }
-    LAUNCH_CHECK();
-    k_rec_sum<<<cdiv(h->nk, 256), 256, 0, h->st>>>(h->d_rho_part, h->n_rho_chunks, M, h->d_rhoA, h->d_str);
-    LAUNCH_CHECK();
-    double fpi_V = 2.0 * (kTwoPi / h->omega);
-    k_rec_efg<<<cdiv(n, 128), 128, 0, h->st>>>(h->d_tab64, n, M, h->d_rhoA, h->d_cell, 2.0 * fpi_V, h->d_efg);
     LAUNCH_CHECK();
   }
   double a = h->p.alphaES;

@@ -624,95 +624,6 @@ __device__ __forceinline__ float2 phase1(const float2* __restrict__ tab, int nat
   return phase_xyz<float>(tab, natm, i, nx, ny, nz, kx, ky);
 }
 
-// structure factor, FP32x2.  Thread t of the block handles ions a = i, b = i + 128
-// of each 256-ion step of its chunk (b absent -> weight 0).
-template <bool HAS_Q, bool HAS_MU, int NZT>
-static __global__ void __launch_bounds__(128) k_rec_rho_x2(const float2* __restrict__ tab,
-                                                    const float4* __restrict__ w, int natm,
-                                                    int chunk, RecMesh M, int ntiles,
-                                                    double2* __restrict__ part) {
-  pdl_wait();
-  pdl_trigger();
-  __shared__ double red[2 * NZT][4];
-  int row = blockIdx.x / ntiles, tile = blockIdx.x % ntiles;
-  int4 ri = M.rows[row];
-  int nx = ri.x, ny = ri.y, nz_lo = ri.z, koff = ri.w;
-  int kz = M.kmax[2];
-  int nz0 = nz_lo + tile * NZT;
-  if (nz0 > kz) return;
-  int nzn = kz - nz0 + 1;
-  if (nzn > NZT) nzn = NZT;
-  int a0 = blockIdx.y * chunk, a1 = a0 + chunk;
-  if (a1 > natm) a1 = natm;
-  float2 accR[NZT], accI[NZT];
-#pragma unroll
-  for (int t = 0; t < NZT; ++t) accR[t] = accI[t] = f2s(0.f);
-  const int kx = M.kmax[0], ky = M.kmax[1];
-  const size_t zoff = (size_t)(kx + 1 + ky + 1);
-  const float fnx = (float)nx, fny = (float)ny, fnz0 = (float)nz0;
-  for (int base = a0; base < a1; base += 256) {
-    int ia = base + threadIdx.x, ib = ia + 128;
-    if (ia >= a1) break;
-    bool vb = ib < a1;
-    int ibb = vb ? ib : ia;
-    float2 XYa = phase1(tab, natm, ia, nx, ny, 0, kx, ky);
-    float2 XYb = phase1(tab, natm, ibb, nx, ny, 0, kx, ky);
-    float2 Pa = phase_z<float>(tab, natm, ia, XYa, nz0, kx, ky);
-    float2 Pb = phase_z<float>(tab, natm, ibb, XYb, nz0, kx, ky);
-    float2 Z1a = tab[(zoff + 1) * natm + ia], Z1b = tab[(zoff + 1) * natm + ibb];
-    float2 Z4a = tab[(zoff + 4) * natm + ia], Z4b = tab[(zoff + 4) * natm + ibb];
-    float2 zr = f2(Z1a.x, Z1b.x), zi = f2(Z1a.y, Z1b.y);
-    float2 z4r = f2(Z4a.x, Z4b.x), z4i = f2(Z4a.y, Z4b.y);
-    float4 wa = w[ia], wb = w[ibb];
-    float2 q = f2(wa.x, vb ? wb.x : 0.f);
-    float2 m3 = f2(wa.w, vb ? wb.w : 0.f);
-    float2 km = f2(fnx * wa.y + fny * wa.z + fnz0 * wa.w,
-                   vb ? fnx * wb.y + fny * wb.z + fnz0 * wb.w : 0.f);
-    // phase at t = 4g + u: (P0 Z4^g) Z1^u
-    float2 gre = f2(Pa.x, Pb.x), gim = f2(Pa.y, Pb.y);
-    float2 pre = gre, pim = gim;
-#pragma unroll
-    for (int t = 0; t < NZT; ++t) {
-      if (t > 0) {
-        if ((t & 3) == 0) {
-          cmul2(gre, gim, z4r, z4i);
-          pre = gre;
-          pim = gim;
-        } else {
-          cmul2(pre, pim, zr, zi);
-        }
-      }
-      if (HAS_Q) {
-        accR[t] = __ffma2_rn(q, pre, accR[t]);
-        accI[t] = __ffma2_rn(q, pim, accI[t]);
-      }
-      if (HAS_MU) {
-        accR[t] = __ffma2_rn(f2(-km.x, -km.y), pim, accR[t]);
-        accI[t] = __ffma2_rn(km, pre, accI[t]);
-        km = __fadd2_rn(km, m3);
-      }
-    }
-  }
-  int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-#pragma unroll
-  for (int t = 0; t < NZT; ++t) {
-    float vr = warp_sum(accR[t].x + accR[t].y);
-    float vi = warp_sum(accI[t].x + accI[t].y);
-    if (lane == 0) {
-      red[2 * t][wp] = (double)vr;
-      red[2 * t + 1][wp] = (double)vi;
-    }
-  }
-  __syncthreads();
-  if ((int)threadIdx.x < nzn) {
-    int t = threadIdx.x;
-    double vr = red[2 * t][0] + red[2 * t][1] + red[2 * t][2] + red[2 * t][3];
-    double vi = red[2 * t + 1][0] + red[2 * t + 1][1] + red[2 * t + 1][2] + red[2 * t + 1][3];
-    int k = koff + (nz0 - nz_lo) + t;
-    part[(size_t)blockIdx.y * M.nk + k] = make_double2(vr, vi);
-  }
-}
-
 // field / force partials, FP32x2: ions a = blockIdx.x*256 + tid, b = a + 128.
 template <bool HAS_MU_FORCE>
 static __global__ void __launch_bounds__(128) k_rec_field_x2(const float2* __restrict__ tab,
