@@ -53,6 +53,7 @@ enum {
   S_DISP = 60,
   S_CGP = 64,    // CG plan of the graph: 64 rmsd of the FP64 residual, 65 stop,
                  // 66 outer iterations, 67 recurrence trusted
+  S_SCF = 68,    // 2: iterations and rmsd of the SCF loop on the device
   S_NSCAL = 72
 };
 
@@ -181,6 +182,12 @@ struct mdff_ctx {
   float* d_ddb1 = nullptr;
   int *d_ddj = nullptr, *d_ddn = nullptr;
   bool dd_cache_ok = false;
+  // FP64 dipole-field pair cache of the FP64 engine (k_dd64_build), rows by
+  // polarisable slot [npol][cap]; null when there was no room
+  double4* d_c64r = nullptr;
+  double* d_c64b = nullptr;
+  int *d_c64j = nullptr, *d_c64n = nullptr;
+  bool dd64_ok = false;          // holds the pairs of this call's positions
   double* d_efg = nullptr;       // [natm][9] electric field gradient (mdff_gpu_efg)
   // kO dipole algorithms (ko.cuh): residual f_ind, increment, find_min
   // point / previous residual (in place), previous dipoles, inner field;
@@ -660,6 +667,21 @@ static int alloc_list(mdff_ctx* h, int cap) {
     if (!h->d_ddn) DALLOC(h->d_ddn, h->natm);
     if (!h->d_Edd) DALLOC(h->d_Edd, h->natm);
   }
+  if (h->d_c64r) cudaFree(h->d_c64r);
+  h->d_c64r = nullptr;
+  h->dd64_ok = false;
+  if (h->p.precision == MDFF_PREC_FP64 && h->lpolar && !h->polidx.empty()) {
+    // one allocation, 44 bytes an entry; optional: without room the field
+    // kernels recompute the pairs
+    const size_t ent = h->polidx.size() * (size_t)cap;
+    if (!h->d_c64n) DALLOC(h->d_c64n, h->polidx.size());
+    if (ent <= ((size_t)1 << 30) && cudaMalloc((void**)&h->d_c64r, ent * 44) != cudaSuccess) {
+      cudaGetLastError();
+      h->d_c64r = nullptr;
+    }
+    h->d_c64b = (double*)(h->d_c64r + ent);
+    h->d_c64j = (int*)(h->d_c64b + ent);
+  }
   h->stats.list_capacity = cap * h->natm;
   return MDFF_OK;
 }
@@ -942,8 +964,8 @@ static int rec_pass_t(mdff_ctx* h, const typename cplx<R>::T* tab, const double4
   M.Ak = h->d_Ak;
   M.kvec = h->d_kvec;
   constexpr bool F32 = std::is_same<R, float>::value;
-  // (the FP32 CG direction kernels write the FP32 weights themselves)
-  if (!(F32 && weights_ready)) {
+  // (the FP32 CG direction kernels and the SCF step write their weights themselves)
+  if (!weights_ready) {
     PDL_CHECK(pdl_launch(k_rec_weights, dim3(cdiv(n, 256)), dim3(256), 0, h->st, h->d_q, mu, n, h->d_cell, has_q, has_mu, h->d_w,
                          F32 ? h->d_w32 : nullptr, mu32, slotw(h)));
   }
@@ -1044,7 +1066,8 @@ static int rec_pass(mdff_ctx* h, bool fp32, const double4* mu, int has_q, int ha
   if (fp32)
     return rec_pass_t<float>(h, h->d_tab32, mu, has_q, has_mu, forces, E, e_out, mu32, sf, defer_nch, weights_ready,
                              pol_dipoles);
-  return rec_pass_t<double>(h, h->d_tab64, mu, has_q, has_mu, forces, E, e_out, mu32, sf, defer_nch, false, pol_dipoles);
+  return rec_pass_t<double>(h, h->d_tab64, mu, has_q, has_mu, forces, E, e_out, mu32, sf, defer_nch, weights_ready,
+                            pol_dipoles);
 }
 
 // the self field 2 selfa2 mu (+ surface field of the reduced moments in mom
@@ -1078,6 +1101,30 @@ static int build_tables(mdff_ctx* h) {
   return MDFF_OK;
 }
 
+// E = T2 mu of the polarisable ions from the FP64 pair cache on stream st,
+// building it in the same sweep when this call has not yet (qq: + the damped
+// charge field)
+static int dd64_field(mdff_ctx* h, cudaStream_t st, const double4* mu, bool mask0, bool qq, double4* E) {
+  const int np = (int)h->polidx.size(), nb = cdiv((long)np * 32, 256);
+  const double cutsq = h->p.cutlongrange * h->p.cutlongrange;
+  if (!h->dd64_ok || qq) {
+#define DDB(QQ, K)                                                                                               \
+  k_dd64_build<QQ, K><<<nb, 256, 0, st>>>(h->d_s, h->d_q, h->d_polidx, np, h->L.nbr, h->L.nnb, h->L.cap,         \
+                                          h->d_cell, h->d_estab, h->ntype, h->p.alphaES, cutsq, h->p.thole_type, \
+                                          mask0 ? 1 : 0, mu, E, h->d_c64r, h->d_c64b, h->d_c64j, h->d_c64n)
+    if (qq && h->tt_k == 4) DDB(true, 4);
+    else if (qq) DDB(true, 0);
+    else DDB(false, 0);
+#undef DDB
+    h->dd64_ok = true;
+  } else {
+    k_dd64_apply<<<nb, 256, 0, st>>>(mu, h->d_polidx, np, h->d_c64r, h->d_c64b, h->d_c64j, h->d_c64n, h->L.cap,
+                                     mask0 ? 1 : 0, E);
+  }
+  LAUNCH_CHECK();
+  return MDFF_OK;
+}
+
 // field of a dipole set alone (charges zeroed, dd task, undamped): the SCF
 // induced pass / the CG operator.  E = T mu.
 // weights_ready: d_w32 / d_mu32 already hold the FP32 operands of mu (written
@@ -1088,7 +1135,9 @@ static int field_of_mu(mdff_ctx* h, const double4* mu, int dd_mask, bool fp32, d
   // FP32 CG operator with the pair cache: one kernel writes E (reciprocal +
   // self + cached real-space dipole field)
   const bool fused = fp32 && dd_mask == 1 && h->dd_cache_ok && h->nk > 0;
-  if (!fused) CK(cudaMemsetAsync(E, 0, sizeof(double4) * n, h->st));
+  // FP64 engine: the pair cache's kernels write E at the polarisable ions
+  const bool dd64 = !fp32 && !cached64 && h->d_c64r;
+  if (!fused && !dd64) CK(cudaMemsetAsync(E, 0, sizeof(double4) * n, h->st));
   double cutsq = h->p.cutlongrange * h->p.cutlongrange;
   int nb = cdiv((long)n * 32, 256);
   int s;
@@ -1106,7 +1155,10 @@ static int field_of_mu(mdff_ctx* h, const double4* mu, int dd_mask, bool fp32, d
     cudaStream_t rs;
     if ((s = rs_fork(h, &rs))) return s;
     int pr = prof_begin(h, KC_ESFIELD, 0);
-    if (cached64 && dd_mask == 1 && h->dd_cache_ok)
+    if (dd64) {
+      if ((s = dd64_field(h, rs, mu, dd_mask == 0, false, E))) return s;
+      h->launches--;  // (counted below)
+    } else if (cached64 && dd_mask == 1 && h->dd_cache_ok)
       k_dd_cached64<<<nb, 256, 0, rs>>>(mu, h->d_ddr, h->d_ddb1, h->d_ddj, h->d_ddn, h->L.cap, n, E);
     else
       k_es_field<double, false, true><<<nb, 256, 0, rs>>>(h->d_s, h->d_q, h->d_itype, h->d_ipolar, mu, h->L.nbr, h->L.nnb, h->L.cap, n, h->d_cell, h->d_estab, h->ntype, h->p.alphaES, cutsq, 0, dd_mask, E, h->p.thole_type);
@@ -1687,7 +1739,99 @@ static int cg_iteration(mdff_ctx* h, bool fp32, int in_graph, cudaGraphCondition
   return MDFF_OK;
 }
 
-// graph: while (cond) { cg_iteration }  -- built once per buffer generation
+// The SCF solve runs its iterations on the device when every piece of one is
+// fused for it: FP64, the plain algorithm, the pair cache, a reciprocal mesh that the
+// tensor-core kernels take, no surface term (a reduction of the dipoles per
+// iteration).  Otherwise solve_scf's host loop runs them.
+static bool scf_device_loop(const mdff_ctx* h) {
+  return h->p.lcoulomb && h->lpolar && h->p.solver == MDFF_SOLVER_SCF && h->p.precision == MDFF_PREC_FP64 &&
+         h->p.algo_moment_from_pola == MDFF_ALGO_SCF && !h->p.lsurf && h->nk > 0 && h->dm_ci &&
+         field_dm_ks(h->p.kES[2]) && h->d_c64r && !h->prof &&
+         (h->p.max_scf_pol_iter > 0 || h->p.min_scf_pol_iter > 0);
+}
+
+// one SCF iteration from the second on (pim.cuh); u_pol's partials go to the
+// upper half of d_part
+static double* upol_part(mdff_ctx* h) { return h->d_part + h->part_cap / 2; }
+static int scf_iteration(mdff_ctx* h, cudaGraphConditionalHandle hc) {
+  const int n = h->natm, np = (int)h->polidx.size(), nb = cdiv(n, 256);
+  int s;
+  PolDev P = poldev(h);
+  PDL_CHECK(pdl_launch(k_scf_step, dim3(nb), dim3(256), 0, h->st, (const double4*)h->d_Estat,
+                       (const double4*)h->d_Eind, P, n, (const CellC*)h->d_cell, h->d_mu_ind, h->d_w, upol_part(h)));
+  cudaStream_t rs;
+  if ((s = rs_fork(h, &rs))) return s;
+  if ((s = dd64_field(h, rs, h->d_mu_ind, true, false, h->d_Eind))) return s;
+  int nch = 0;
+  SelfField sf = self_field(h, h->d_mu_ind, h->d_scal + S_MOM2);
+  if ((s = rec_pass(h, false, h->d_mu_ind, 0, 1, 0, h->d_Eind, nullptr, sf, nullptr, &nch, true, true))) return s;
+  const int nbf = cdiv((long)np * 4, 256);
+  k_scf_field<<<nbf, 256, 0, h->st>>>(h->d_G, nch, n, h->d_polidx, np, h->d_cell,
+                                      2.0 * (2.0 * (kTwoPi / h->omega)), sf.selfa2, h->d_mu_ind, h->d_Estat, P,
+                                      h->d_Eind, h->d_part);
+  LAUNCH_CHECK();
+  PDL_CHECK(pdl_launch(k_scf_check, dim3(1), dim3(256), 0, h->st, (const double*)h->d_part, nbf,
+                       (const double*)nullptr, h->npol, h->p.conv_tol_ind, h->p.min_scf_pol_iter,
+                       h->p.max_scf_pol_iter, h->d_scal + S_SCF, hc));
+  return MDFF_OK;
+}
+
+// Adds the solver's loop to graph g after *dep: a head kernel that decides
+// whether to iterate (k_cg_plan from the FP64 residual, k_scf_check from the
+// first iteration's), then WHILE { one iteration }.  *last: the loop's node.
+static int add_solver_loop(mdff_ctx* h, cudaGraph_t g, const cudaGraphNode_t* dep, bool fp32, cudaGraphNode_t* last,
+                           int* body_launches) {
+  cudaGraphConditionalHandle hc;
+  CK(cudaGraphConditionalHandleCreate(&hc, g, 1, cudaGraphCondAssignDefault));
+  const bool cg = h->p.solver == MDFF_SOLVER_CG;
+  double* sc = h->d_scal + S_CG;
+  double* plan = h->d_scal + S_CGP;
+  int npol = h->npol;
+  double tol = h->p.cg_tol > 0 ? h->p.cg_tol : h->p.conv_tol_ind;
+  double maxit = (double)(h->p.cg_max_iter > 0 ? h->p.cg_max_iter : 200);
+  int f32 = fp32 ? 1 : 0;
+  void* cargs[] = {&sc, &plan, &npol, &tol, &maxit, &f32, &hc};
+  const double *nopart = nullptr, *r2 = h->d_scal + S_RMS;
+  int zero = 0, mn = h->p.min_scf_pol_iter, mx = h->p.max_scf_pol_iter;
+  double stol = h->p.conv_tol_ind;
+  double* ssc = h->d_scal + S_SCF;
+  void* sargs[] = {&nopart, &zero, &r2, &npol, &stol, &mn, &mx, &ssc, &hc};
+  cudaKernelNodeParams kp = {};
+  kp.func = cg ? (void*)k_cg_plan : (void*)k_scf_check;
+  kp.gridDim = dim3(1);
+  kp.blockDim = dim3(32);
+  kp.sharedMemBytes = 0;
+  kp.kernelParams = cg ? cargs : sargs;
+  cudaGraphNode_t head;
+  CK(cudaGraphAddKernelNode(&head, g, dep, dep ? 1 : 0, &kp));
+  cudaGraphNodeParams cp = {};
+  cp.type = cudaGraphNodeTypeConditional;
+  cp.conditional.handle = hc;
+  cp.conditional.type = cudaGraphCondTypeWhile;
+  cp.conditional.size = 1;
+  CK(cudaGraphAddNode(last, g, &head, 1, &cp));
+  bool prof = h->prof, ovl = h->call_overlap;
+  h->prof = false;
+  h->call_overlap = h->overlap;  // (the operator's real-space half beside its reciprocal half)
+  int launches0 = h->launches;
+  CK(cudaStreamBeginCaptureToGraph(h->st, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
+                                   cudaStreamCaptureModeThreadLocal));
+  int s = cg ? cg_iteration(h, fp32, 1, hc) : scf_iteration(h, hc);
+  cudaGraph_t captured;
+  cudaError_t e = cudaStreamEndCapture(h->st, &captured);
+  h->prof = prof;
+  h->call_overlap = ovl;
+  *body_launches = h->launches - launches0;
+  h->launches = launches0;
+  if (s) return s;
+  if (e != cudaSuccess) {
+    h->err = std::string("cudaStreamEndCapture: ") + cudaGetErrorString(e);
+    return MDFF_ERR_CUDA;
+  }
+  return MDFF_OK;
+}
+
+// graph of the solver's loop alone -- built once per buffer generation
 static int build_cg_graph(mdff_ctx* h, bool fp32) {
   if (h->cg_exec) cudaGraphExecDestroy(h->cg_exec);
   if (h->cg_graph) cudaGraphDestroy(h->cg_graph);
@@ -1696,52 +1840,61 @@ static int build_cg_graph(mdff_ctx* h, bool fp32) {
   cudaGraph_t g;
   CK(cudaGraphCreate(&g, 0));
   h->cg_graph = g;
-  cudaGraphConditionalHandle hc;
-  CK(cudaGraphConditionalHandleCreate(&hc, g, 1, cudaGraphCondAssignDefault));
-  // head: k_cg_plan decides from the FP64 residual and sets the condition
-  double* sc = h->d_scal + S_CG;
-  double* plan = h->d_scal + S_CGP;
-  int npol = h->npol;
-  double tol = h->p.cg_tol > 0 ? h->p.cg_tol : h->p.conv_tol_ind;
-  double maxit = (double)(h->p.cg_max_iter > 0 ? h->p.cg_max_iter : 200);
-  int f32 = fp32 ? 1 : 0;
-  void* kargs[] = {&sc, &plan, &npol, &tol, &maxit, &f32, &hc};
-  cudaKernelNodeParams kp = {};
-  kp.func = (void*)k_cg_plan;
-  kp.gridDim = dim3(1);
-  kp.blockDim = dim3(32);
-  kp.sharedMemBytes = 0;
-  kp.kernelParams = kargs;
-  cudaGraphNode_t head;
-  CK(cudaGraphAddKernelNode(&head, g, nullptr, 0, &kp));
-  cudaGraphNodeParams cp = {};
-  cp.type = cudaGraphNodeTypeConditional;
-  cp.conditional.handle = hc;
-  cp.conditional.type = cudaGraphCondTypeWhile;
-  cp.conditional.size = 1;
-  cudaGraphNode_t node;
-  CK(cudaGraphAddNode(&node, g, &head, 1, &cp));
-  cudaGraph_t body = cp.conditional.phGraph_out[0];
-  bool prof = h->prof, ovl = h->call_overlap;
-  h->prof = false;
-  h->call_overlap = false;
-  int launches0 = h->launches;
-  CK(cudaStreamBeginCaptureToGraph(h->st, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-  int s = cg_iteration(h, fp32, 1, hc);
-  cudaGraph_t captured;
-  cudaError_t e = cudaStreamEndCapture(h->st, &captured);
-  h->prof = prof;
-  h->call_overlap = ovl;
-  h->cg_body_launches = h->launches - launches0;
-  h->launches = launches0;
+  cudaGraphNode_t last;
+  int s = add_solver_loop(h, g, nullptr, fp32, &last, &h->cg_body_launches);
   if (s) return s;
-  if (e != cudaSuccess) {
-    h->err = std::string("cudaStreamEndCapture: ") + cudaGetErrorString(e);
-    return MDFF_ERR_CUDA;
-  }
   CK(cudaGraphInstantiate(&h->cg_exec, g, 0));
   h->cg_gen = h->gen;
   h->cg_fp32 = fp32 ? 1 : 0;
+  return MDFF_OK;
+}
+
+// the first SCF iteration (the predictor's dipoles, or alpha E_stat) up to its
+// residual sum in S_RMS
+static int scf_first(mdff_ctx* h, int itime, bool fp32) {
+  const int n = h->natm, nb = cdiv(n, 256);
+  int s;
+  PolDev P = poldev(h);
+  const bool ismd = h->p.calc == MDFF_CALC_MD, isopt = h->p.calc == MDFF_CALC_OPT;
+  if (!ismd && !isopt) {
+    k_induce<<<nb, 256, 0, h->st>>>(h->d_Estat, P, n, h->d_mu_ind);
+    LAUNCH_CHECK();
+  } else if ((s = aspc_predict(h, itime))) {
+    return s;
+  }
+  PDL_CHECK(pdl_launch(k_upol_part, dim3(nb), dim3(256), 0, h->st, (const double4*)h->d_mu_ind, P, n, upol_part(h)));
+  if ((s = field_of_mu(h, h->d_mu_ind, 0, fp32, h->d_Eind))) return s;
+  k_add4<<<nb, 256, 0, h->st>>>(h->d_Estat, h->d_Eind, n, h->d_Efield);
+  LAUNCH_CHECK();
+  if (ismd && (s = aspc_correct(h, itime))) return s;
+  k_rmsd_part<<<nb, 256, 0, h->st>>>(h->d_mu_ind, h->d_Efield, P, n, h->d_part);
+  LAUNCH_CHECK();
+  return reduce_into(h, nb, 1, h->d_scal + S_RMS);
+}
+// after the loop: u_pol of the last iteration's dipoles, the ASPC history
+static int scf_epilogue(mdff_ctx* h) {
+  PDL_CHECK(pdl_launch(k_reduce_partials, dim3(1), dim3(256), 0, h->st, (const double*)upol_part(h),
+                       cdiv(h->natm, 256), 1, h->d_scal + S_UPOL));
+  CK(cudaMemcpyAsync(h->d_hist, h->d_mu_ind, sizeof(double4) * h->natm, cudaMemcpyDeviceToDevice, h->st));
+  return MDFF_OK;
+}
+// iterations and residual of the loop from the host copies of the scalars
+static void scf_stats(mdff_ctx* h) {
+  h->stats.n_pol_iter = (int)h->h_scal[S_SCF];
+  h->stats.rmsd = h->h_scal[S_SCF + 1];
+  h->stats.converged = h->stats.rmsd <= h->p.conv_tol_ind;
+}
+static int solve_scf_device(mdff_ctx* h, int itime) {
+  int s;
+  if ((s = scf_first(h, itime, false))) return s;
+  if (h->cg_exec == nullptr || h->cg_gen != h->gen || h->cg_fp32 != 0)
+    if ((s = build_cg_graph(h, false))) return s;
+  CK(cudaGraphLaunch(h->cg_exec, h->st));
+  if ((s = scf_epilogue(h))) return s;
+  CK(cudaMemcpyAsync(h->h_scal + S_SCF, h->d_scal + S_SCF, sizeof(double) * 2, cudaMemcpyDeviceToHost, h->st));
+  CK(cudaStreamSynchronize(h->st));
+  scf_stats(h);
+  h->launches += h->cg_body_launches * (h->stats.n_pol_iter - 1) + 1;
   return MDFF_OK;
 }
 
@@ -1831,6 +1984,9 @@ static int merged_residual(mdff_ctx* h, bool fp32) {
     else SRC(0);
 #undef SRC
     h->dd_cache_ok = true;
+  } else if (!fp32 && h->d_c64r) {
+    if ((s = dd64_field(h, rs, h->d_mu_ind, false, true, E))) return s;
+    h->launches--;  // (counted below)
   } else {
 #define ESF2(K)                                                                                    \
   k_es_field<double, true, true, K><<<nbw, 256, 0, rs>>>(h->d_s, h->d_q, h->d_itype, h->d_ipolar,  \
@@ -2018,6 +2174,7 @@ static int solve_cg(mdff_ctx* h, int itime, bool fp32) {
 static int ef_front(mdff_ctx* h, bool fp32) {
   int n = h->natm, s;
   h->rho_acc_ok = false;
+  h->dd64_ok = false;
   PDL_CHECK(pdl_launch(k_kardir, dim3(cdiv(n, 256)), dim3(256), 0, h->st, h->d_pos, n, h->d_cell, h->d_itype,
                        h->d_ipolar, h->d_q, h->d_s));
   if ((s = list_update(h))) return s;
@@ -2070,6 +2227,7 @@ static int ef_solve(mdff_ctx* h, int itime, bool fp32) {
   if (h->p.solver == MDFF_SOLVER_CG) return solve_cg(h, itime, fp32);
   if (algo == MDFF_ALGO_KO_V1 || algo == MDFF_ALGO_KO_V2) return solve_ko_v12(h, itime, fp32, algo == MDFF_ALGO_KO_V2);
   if (algo == MDFF_ALGO_KO_V4_1) return solve_ko_v4(h, itime, fp32);
+  if (scf_device_loop(h)) return solve_scf_device(h, itime);
   return solve_scf(h, itime, fp32);
 }
 
@@ -2198,7 +2356,7 @@ static int run_engforce(mdff_ctx* h, int itime) {
 static bool step_graph_usable(const mdff_ctx* h, int itime) {
   if (h->prof || !h->have_list || h->lwannier) return false;
   if (!h->lpolar || !h->p.lcoulomb) return true;
-  if (h->p.solver != MDFF_SOLVER_CG) return false;
+  if (h->p.solver != MDFF_SOLVER_CG && !scf_device_loop(h)) return false;
   if (h->p.calc == MDFF_CALC_MD || h->p.calc == MDFF_CALC_OPT)
     return itime >= h->p.extrapolate_order + 1;  // constant ASPC coefficients
   return true;
@@ -2231,11 +2389,12 @@ static void step_graph_free(mdff_ctx* h) {
 
 static int build_step_graph(mdff_ctx* h, int itime, bool fp32) {
   step_graph_free(h);
-  const bool cg = h->p.lcoulomb && h->lpolar;
+  const bool solve = h->p.lcoulomb && h->lpolar, cg = solve && h->p.solver == MDFF_SOLVER_CG;
   int s;
-  // the operator reads the FP32 pair cache when the front fills it
+  // the operator reads the pair cache that the front fills
   if (cg && fp32 && h->d_ddr) h->dd_cache_ok = true;
-  if (cg && (h->cg_exec == nullptr || h->cg_gen != h->gen || h->cg_fp32 != (fp32 ? 1 : 0)))
+  if (solve && !fp32 && h->d_c64r) h->dd64_ok = true;
+  if (solve && (h->cg_exec == nullptr || h->cg_gen != h->gen || h->cg_fp32 != (fp32 ? 1 : 0)))
     if ((s = build_cg_graph(h, fp32))) return s;
   bool prof = h->prof;
   h->prof = false;
@@ -2248,6 +2407,7 @@ static int build_step_graph(mdff_ctx* h, int itime, bool fp32) {
   s = ef_front(h, fp32);
   if (!s && cg) s = cg_prologue(h, itime);
   if (!s && cg) s = cg_first_residual(h, fp32);
+  if (!s && solve && !cg) s = scf_first(h, itime, fp32);
   // a capture ends joined: the short-range pass (~100 us) joins at the end of
   // the front, which takes longer (static field + FP64 residual)
   if (!s) s = sr_join(h);
@@ -2257,7 +2417,7 @@ static int build_step_graph(mdff_ctx* h, int itime, bool fp32) {
     cudaGraphDestroy(gA);
     return s;
   }
-  s = cg ? cg_epilogue(h) : MDFF_OK;
+  s = cg ? cg_epilogue(h) : solve ? scf_epilogue(h) : MDFF_OK;
   if (!s) s = ef_back(h, fp32);
   if ((s = capture_end(h, s, &gB))) {
     cudaGraphDestroy(gA);
@@ -2272,47 +2432,9 @@ static int build_step_graph(mdff_ctx* h, int itime, bool fp32) {
   cudaGraphNode_t nA, nB, last;
   CK(cudaGraphAddChildGraphNode(&nA, g, nullptr, 0, gA));
   last = nA;
-  if (cg) {
-    // k_cg_plan + the inner WHILE node, as in the CG graph
-    cudaGraphConditionalHandle hc;
-    CK(cudaGraphConditionalHandleCreate(&hc, g, 1, cudaGraphCondAssignDefault));
-    double* sc = h->d_scal + S_CG;
-    double* plan = h->d_scal + S_CGP;
-    int npol = h->npol;
-    double tol = cg_tol_of(h);
-    double maxit = (double)cg_maxit_of(h);
-    int f32 = fp32 ? 1 : 0;
-    void* kargs[] = {&sc, &plan, &npol, &tol, &maxit, &f32, &hc};
-    cudaKernelNodeParams kp = {};
-    kp.func = (void*)k_cg_plan;
-    kp.gridDim = dim3(1);
-    kp.blockDim = dim3(32);
-    kp.kernelParams = kargs;
-    cudaGraphNode_t head;
-    CK(cudaGraphAddKernelNode(&head, g, &last, 1, &kp));
-    cudaGraphNodeParams cp = {};
-    cp.type = cudaGraphNodeTypeConditional;
-    cp.conditional.handle = hc;
-    cp.conditional.type = cudaGraphCondTypeWhile;
-    cp.conditional.size = 1;
-    cudaGraphNode_t wnode;
-    CK(cudaGraphAddNode(&wnode, g, &head, 1, &cp));
-    bool ovl = h->call_overlap;
-    h->call_overlap = false;
-    int l0 = h->launches;
-    CK(cudaStreamBeginCaptureToGraph(h->st, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
-                                     cudaStreamCaptureModeThreadLocal));
-    s = cg_iteration(h, fp32, 1, hc);
-    cudaGraph_t captured;
-    cudaError_t e = cudaStreamEndCapture(h->st, &captured);
-    h->call_overlap = ovl;
-    h->launches = l0;
-    if (s) return s;
-    if (e != cudaSuccess) {
-      h->err = std::string("cudaStreamEndCapture: ") + cudaGetErrorString(e);
-      return MDFF_ERR_CUDA;
-    }
-    last = wnode;
+  if (solve) {
+    int body = 0;
+    if ((s = add_solver_loop(h, g, &nA, fp32, &last, &body))) return s;
   }
   CK(cudaGraphAddChildGraphNode(&nB, g, &last, 1, gB));
   cudaGraphDestroy(gA);
@@ -2338,7 +2460,10 @@ static int run_engforce_graph(mdff_ctx* h, int itime, bool* used) {
   CK(cudaGraphLaunch(h->step_exec, h->st));
   CK(cudaStreamSynchronize(h->st));
   h->launches = h->step_launches;
-  if (h->p.lcoulomb && h->lpolar) {
+  if (h->p.lcoulomb && h->lpolar && h->p.solver != MDFF_SOLVER_CG) {
+    scf_stats(h);
+    h->launches += h->cg_body_launches * (h->stats.n_pol_iter - 1) + 1;
+  } else if (h->p.lcoulomb && h->lpolar) {
     double rmsd, rmsd0 = h->h_scal[S_CGP];
     int it, nres = 1;
     if (!cg_graph_outcome(h, &rmsd, &it)) {
@@ -3024,7 +3149,7 @@ void mdff_gpu_destroy(mdff_handle h) {
                   h->d_ko_g, h->d_ko_muprev, h->d_ko_fdir, h->d_Fh, h->d_muh, h->d_ko_x, h->d_part2,
                   h->d_lwfc, h->d_mu_wfc, h->d_qm32, h->d_Edd, h->d_fsr, h->d_hist_save,
                   h->d_rho_timg, h->d_polidx, h->d_rho_acc, h->d_w32s, h->d_polslot,
-                  h->d_rtpos};
+                  h->d_rtpos, h->d_c64r, h->d_c64n};
   for (void* q : ptrs)
     if (q) cudaFree(q);
   step_graph_free(h);

@@ -161,6 +161,107 @@ __global__ void k_self_surf_field(const double4* __restrict__ mu, int natm, doub
                       o.z + s2 + 2.0 * selfa2 * m.z, 0.0);
 }
 
+// ---- SCF iterations on the device -------------------------------------------
+// From the second on, an SCF iteration (moment_from_pola.f90:340-460) is
+//   k_scf_step: mu = alpha (E_stat + E_ind), the reciprocal weights of mu, u_pol
+//   the dipole field: cached real-space part (side stream), rho, field sums
+//   k_scf_field: E_ind = real + reciprocal + self, and the rmsd partials
+//   k_scf_check: rmsd, count, and the WHILE condition of the graph that runs
+// them, so that a solve needs no host round trip per iteration (14 launches, two
+// fills, a copy and a synchronisation before).
+
+__global__ void k_scf_step(const double4* __restrict__ Estat, const double4* __restrict__ Eind, PolDev P,
+                           int natm, const CellC* __restrict__ cell, double4* __restrict__ mu,
+                           double4* __restrict__ w, double* __restrict__ part) {
+  pdl_wait();
+  pdl_trigger();
+  __shared__ double red[32];
+  double v[1] = {0.0};
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < natm && P.ipolar[i]) {
+    const double4 a = Estat[i], b = Eind[i];
+    const double E[3] = {a.x + b.x, a.y + b.y, a.z + b.z};
+    const double* al = P.pol + 9 * (size_t)i;
+    const double* iv = P.invpol + 9 * (size_t)i;
+    double m[3];
+    for (int x = 0; x < 3; ++x) m[x] = ((al[3 * x] * E[0]) + al[3 * x + 1] * E[1]) + al[3 * x + 2] * E[2];
+    mu[i] = make_double4(m[0], m[1], m[2], 0.0);
+    const double* B = cell->B;
+    w[i] = make_double4(0.0, kTwoPi * (B[0] * m[0] + B[3] * m[1] + B[6] * m[2]),
+                        kTwoPi * (B[1] * m[0] + B[4] * m[1] + B[7] * m[2]),
+                        kTwoPi * (B[2] * m[0] + B[5] * m[1] + B[8] * m[2]));
+    for (int x = 0; x < 3; ++x)
+      for (int y = 0; y < 3; ++y) v[0] += m[x] * iv[3 * x + y] * m[y];
+  }
+  block_sum<1>(v, red);
+  if (threadIdx.x == 0) part[blockIdx.x] = v[0];
+}
+
+// four threads per polarisable ion split the field partials, as k_rec_field_sum
+__global__ void k_scf_field(const double4* __restrict__ Gpart, int nchunk, int natm, const int* __restrict__ polidx,
+                            int npol, const CellC* __restrict__ cell, double scale, double selfa2,
+                            const double4* __restrict__ mu, const double4* __restrict__ Estat, PolDev P,
+                            double4* __restrict__ Eind, double* __restrict__ part) {
+  __shared__ double red[32];
+  double v[1] = {0.0};
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, sl = t >> 2, sub = t & 3;
+  double g[3] = {0.0, 0.0, 0.0};
+  int i = 0;
+  if (sl < npol) {
+    i = polidx[sl];
+    for (int c = sub; c < nchunk; c += 4) {
+      const double4 u = Gpart[(size_t)c * natm + i];
+      g[0] += u.x;
+      g[1] += u.y;
+      g[2] += u.z;
+    }
+  }
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    g[a] += __shfl_xor_sync(FULL_MASK, g[a], 1);
+    g[a] += __shfl_xor_sync(FULL_MASK, g[a], 2);
+  }
+  if (sl < npol && sub == 0) {
+    const double* B = cell->B;
+    const double4 m = mu[i], o = Eind[i], st = Estat[i];
+    const double mm[3] = {m.x, m.y, m.z}, oo[3] = {o.x, o.y, o.z}, ss[3] = {st.x, st.y, st.z};
+    const double* al = P.pol + 9 * (size_t)i;
+    double e[3];
+    for (int a = 0; a < 3; ++a) {
+      const double er = -kTwoPi * (B[3 * a] * g[0] + B[3 * a + 1] * g[1] + B[3 * a + 2] * g[2]) * scale;
+      e[a] = oo[a] + er + 2.0 * selfa2 * mm[a];
+      if (al[4 * a] != 0.0) {  // get_rmsd_mu (:998-1027)
+        const double d = mm[a] / al[4 * a] - (ss[a] + e[a]);
+        v[0] += d * d;
+      }
+    }
+    Eind[i] = make_double4(e[0], e[1], e[2], 0.0);
+  }
+  block_sum<1>(v, red);
+  if (threadIdx.x == 0) part[blockIdx.x] = v[0];
+}
+
+// sc[0] = iterations, sc[1] = rmsd; r2 (head of the graph): the residual sum of
+// the first iteration, else the partials of k_scf_field.  The condition is the
+// host loop's.
+__global__ void k_scf_check(const double* __restrict__ part, int nblk, const double* __restrict__ r2, int npol,
+                            double tol, int miniter, int maxiter, double* __restrict__ sc,
+                            cudaGraphConditionalHandle hc) {
+  pdl_wait();
+  pdl_trigger();
+  __shared__ double red[32];
+  double v[1] = {0.0};
+  if (!r2)
+    for (int b = threadIdx.x; b < nblk; b += blockDim.x) v[0] += part[b];
+  block_sum<1>(v, red);
+  if (threadIdx.x != 0) return;
+  const double rmsd = sqrt((r2 ? *r2 : v[0]) / (double)npol);
+  const int it = r2 ? 1 : (int)sc[0] + 1;
+  sc[0] = (double)it;
+  sc[1] = rmsd;
+  cudaGraphSetConditional(hc, ((it < maxiter && rmsd > tol) || it < miniter) ? 1u : 0u);
+}
+
 // ---- conjugate gradients ----------------------------------------------------
 // A x = alpha^-1 x - T x on polarisable ions (T x = field of x).  The step
 // scalars (r.z, p.q) stay on the device; only the rmsd goes to the host.

@@ -751,6 +751,157 @@ static __global__ void __launch_bounds__(256) k_dd_cached64(
 }
 
 // --------------------------------------------------------------------------
+// FP64 pair cache of the dipole operator: for every polarisable ion (row = its
+// slot in polidx) the terms of the undamped dipole field T2(r) mu = B2 r (r.mu)
+// - B1 mu of its polarisable partners within rc, in row order:
+//   cr = (rx, ry, rz, B2), cb1 = B1, cj = j, cn[slot] = count.
+// An SCF or FP64 CG solve applies the operator 10-60 times at fixed positions;
+// reading 44 bytes an entry (mostly from L2) replaces the minimum image, erfc, exp and
+// square root per pair: 8000-ion MgO (900,000 entries) 37 us per application
+// recomputed, 12-15 us cached beside the reciprocal half.
+//
+// k_dd64_build writes the cache and, in the same sweep, E = T2 mu (QQ: + the
+// damped charge field, the static pass merged with the first residual);
+// k_dd64_apply writes E = T2 mu from the cache.  mask0: the reference's condition
+// any(mu_i /= 0) on the row (a zero mu_j adds nothing by itself); else both
+// ions polarisable.  E of other ions is not written.
+template <bool QQ, int K>
+static __global__ void __launch_bounds__(256) k_dd64_build(
+    const double4* __restrict__ s, const double* __restrict__ q, const int* __restrict__ polidx, int npol,
+    const int* __restrict__ nbr, const int* __restrict__ nnb, int cap, const CellC* __restrict__ cell,
+    const ESPair* __restrict__ tab, int ntype, double alpha, double cutsq, int thole, int mask0,
+    const double4* __restrict__ mu, double4* __restrict__ E, double4* __restrict__ cr,
+    double* __restrict__ cb1, int* __restrict__ cj, int* __restrict__ cn) {
+  __shared__ ESPair stab[MDFF_NT * MDFF_NT];
+  __shared__ double cA[9];
+  for (int k = threadIdx.x; k < ntype * ntype; k += blockDim.x) stab[k] = tab[k];
+  if (threadIdx.x < 9) cA[threadIdx.x] = cell->A[threadIdx.x];
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  const int sl = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (sl >= npol) return;
+  const int i = polidx[sl];
+  const double4 si = s[i];
+  const int ti = tag_type(si.w);
+  const double4 mi = mu[i];
+  const bool dip_i = !mask0 || mi.x != 0.0 || mi.y != 0.0 || mi.z != 0.0;
+  const int n = nnb[i];
+  const int* row = nbr + (size_t)i * cap;
+  const size_t base = (size_t)sl * cap;
+  double ex = 0.0, ey = 0.0, ez = 0.0;
+  int m = 0;
+  for (int k0 = 0; k0 < n; k0 += 32) {
+    const int k = k0 + lane;
+    bool keep = false;
+    double rx = 0, ry = 0, rz = 0, B1 = 0, B2 = 0;
+    int j = 0;
+    if (k < n) {
+      j = row[k];
+      const double4 sj = s[j];
+      const bool pp = tag_pol(sj.w);
+      const double qj = QQ ? q[j] : 0.0;
+      if (pp || (QQ && qj != 0.0)) {
+        const double r2 = pair_vec<double>(cA, si, sj, rx, ry, rz);
+        if (r2 <= cutsq) {  // ewald_dir.f90:202
+          const int tj = tag_type(sj.w);
+          const bool i_is_a = half_mask(i, j);
+          const ESPair& P = stab[(i_is_a ? ti : tj) * ntype + (i_is_a ? tj : ti)];
+          Radial<double> g;
+          radial<double, false>(r2, alpha, g);
+          if (QQ && qj != 0.0) {
+            double F1d = 0.0;
+            if (P.ldamp && (i_is_a ? P.ca : P.cb) != 0.0) {  // c = 0 damps nothing
+              double fdm, fdd;
+              if (i_is_a)
+                tt_damp_k<double, K>(P.ba, P.ca, g.d, P.ka, fdm, fdd);
+              else
+                tt_damp_k<double, K>(P.bb, P.cb, g.d, P.kb, fdm, fdd);
+              F1d = 1.0 - fdm;
+            }
+            const double c = qj * g.dm3 * (g.F1 - F1d);
+            ex += c * rx;
+            ey += c * ry;
+            ez += c * rz;
+          }
+          if (pp) {
+            keep = true;
+            double F1 = g.F1, F2 = g.F2;
+            if (thole && P.thole) thole_radial<double>(P, g.d, F1, F2);
+            B1 = F1 * g.dm3;
+            B2 = 3.0 * F2 * g.dm5;
+            if (dip_i) {
+              const double4 mj = mu[j];
+              const double rm = rx * mj.x + ry * mj.y + rz * mj.z;
+              ex += B2 * rx * rm - B1 * mj.x;
+              ey += B2 * ry * rm - B1 * mj.y;
+              ez += B2 * rz * rm - B1 * mj.z;
+            }
+          }
+        }
+      }
+    }
+    const unsigned bal = __ballot_sync(FULL_MASK, keep);
+    if (keep) {
+      const size_t o = base + m + __popc(bal & ((1u << lane) - 1u));
+      cr[o] = make_double4(rx, ry, rz, B2);
+      cb1[o] = B1;
+      cj[o] = j;
+    }
+    m += __popc(bal);
+  }
+  ex = warp_sum(ex);
+  ey = warp_sum(ey);
+  ez = warp_sum(ez);
+  if (lane == 0) {
+    E[i] = make_double4(ex, ey, ez, 0.0);
+    cn[sl] = m;
+  }
+}
+
+static __global__ void __launch_bounds__(256) k_dd64_apply(
+    const double4* __restrict__ mu, const int* __restrict__ polidx, int npol, const double4* __restrict__ cr,
+    const double* __restrict__ cb1, const int* __restrict__ cj, const int* __restrict__ cn, int cap, int mask0,
+    double4* __restrict__ E) {
+  const int lane = threadIdx.x & 31;
+  const int sl = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (sl >= npol) return;
+  const int i = polidx[sl];
+  const double4 mi = mu[i];
+  const bool dip_i = !mask0 || mi.x != 0.0 || mi.y != 0.0 || mi.z != 0.0;
+  const int n = dip_i ? cn[sl] : 0;
+  const size_t base = (size_t)sl * cap;
+  double ex = 0.0, ey = 0.0, ez = 0.0;
+  constexpr int U = 4;
+  for (int k0 = lane; k0 < n; k0 += 32 * U) {
+    double4 r[U], m[U];
+    double b1[U];
+    int j[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int k = k0 + 32 * u;
+      const bool ok = k < n;
+      j[u] = ok ? cj[base + k] : i;
+      r[u] = ok ? cr[base + k] : make_double4(0.0, 0.0, 0.0, 0.0);
+      b1[u] = ok ? cb1[base + k] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) m[u] = mu[j[u]];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (k0 + 32 * u >= n) break;
+      const double rm = r[u].x * m[u].x + r[u].y * m[u].y + r[u].z * m[u].z;
+      ex += r[u].w * r[u].x * rm - b1[u] * m[u].x;
+      ey += r[u].w * r[u].y * rm - b1[u] * m[u].y;
+      ez += r[u].w * r[u].z * rm - b1[u] * m[u].z;
+    }
+  }
+  ex = warp_sum(ex);
+  ey = warp_sum(ey);
+  ez = warp_sum(ez);
+  if (lane == 0) E[i] = make_double4(ex, ey, ez, 0.0);
+}
+
+// --------------------------------------------------------------------------
 // final real-space pass: qq + qd + dd with damping; energy, field, force,
 // (FP32: three blocks per SM, 80 registers, measured 14% faster than two)
 // stress.  Partials per block: [u, tau xx yy zz xy xz yz] -> 7 doubles
