@@ -86,12 +86,13 @@ __device__ __forceinline__ void brho_t(const unsigned char* __restrict__ rec, in
   const int g = lane >> 2, tt = lane & 3;
   const int ng = (nrows + 7) / 8, nz = kz + 1;
   const int pieces = stride / 16, nch = (L.cnt + CH - 1) / CH;
+  // a warp copies whole records, a lane a 16-byte piece of each
   auto fetch = [&](int c) {
-    const int k0 = c * CH, m = (L.cnt - k0 < CH ? L.cnt - k0 : CH) * pieces;
+    const int k0 = c * CH, m = L.cnt - k0 < CH ? L.cnt - k0 : CH;
     unsigned char* o = buf + (size_t)(c & 1) * CH * stride;
-    for (int e = threadIdx.x; e < m; e += blockDim.x) {
-      const int k = e / pieces, pc = e - k * pieces;
-      cp_async16(o + k * stride + pc * 16, rec + (size_t)blist_ion(L, t, k0 + k) * stride + pc * 16);
+    for (int k = warp; k < m; k += nw) {
+      const unsigned char* rp = rec + (size_t)blist_ion(L, t, k0 + k) * stride;
+      for (int pc = lane; pc < pieces; pc += 32) cp_async16(o + k * stride + pc * 16, rp + pc * 16);
     }
     cp_async_commit();
   };
@@ -274,12 +275,14 @@ __device__ __forceinline__ int bfld_t(const unsigned char* __restrict__ rec, int
 #pragma unroll
         for (int d = 0; d < 3; ++d) G[q][d] = H[q][d] = 0.0;
       const int q0 = nr4 * rs / RS, q1 = nr4 * (rs + 1) / RS;
-      // this lane's row of the four, its X and Y one step ahead
-      int4 rn = make_int4(0, 0, 0, 0);
-      double2 Xn[2], Yn[2];
-      auto next = [&](int r4) {
+      // this lane's row of the four: indices two steps ahead, X and Y one
+      auto row_of = [&](int r4) {
         const int r = ra + r4 * 4 + tt;
-        rn = rows[r < nrows ? r : nrows - 1];
+        return rows[r < nrows ? r : nrows - 1];
+      };
+      int4 r1 = row_of(q0), r2 = row_of(q0 + 1);
+      double2 Xn[2], Yn[2];
+      auto next = [&](const int4& rn) {
         const int ye = kx + 1 + (rn.y < 0 ? -rn.y : rn.y);
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
@@ -287,11 +290,13 @@ __device__ __forceinline__ int bfld_t(const unsigned char* __restrict__ rec, int
           Yn[q] = reinterpret_cast<const double2*>(rp[q])[ye];
         }
       };
-      if (q0 < q1) next(q0);
+      next(r1);
       for (int r4 = q0; r4 < q1; ++r4) {
-        const int4 ri = rn;
+        const int4 ri = r1;
         const double2 X[2] = {Xn[0], Xn[1]}, Y[2] = {Yn[0], Yn[1]};
-        if (r4 + 1 < q1) next(r4 + 1);
+        r1 = r2;
+        next(r1);
+        r2 = row_of(r4 + 2);
         double d0[4] = {0, 0, 0, 0}, d1[4] = {0, 0, 0, 0}, d2[4] = {0, 0, 0, 0};
         const double* b = sc + (size_t)r4 * 4 * RL + boff;
 #pragma unroll

@@ -449,10 +449,10 @@ static int rho_dm_attr(int smem) {
   return cudaFuncSetAttribute(k_rho_dm<NT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess;
 }
 // most staged rows of k_field_dm (two blocks per SM up to 9 steps)
-static int field_dm_rc(int ks) { return (ks <= 9 ? 100 : 200) * 1024 / (field_dm_rl(ks) * 8) / 4 * 4; }
+static int field_dm_rc(int ks) { return (ks <= 9 ? 100 : 200) * 1024 / (field_dm_rl(ks) * 8 + 16) / 4 * 4; }
 template <int KS>
 static int field_dm_attr_k() {
-  const int smem = field_dm_rc(KS) * field_dm_rl(KS) * 8;
+  const int smem = field_dm_rc(KS) * (field_dm_rl(KS) * 8 + 16);
   if (cudaFuncSetAttribute(k_field_dm<KS, DM_FIELD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
       cudaFuncSetAttribute(k_field_dm<KS, DM_FORCE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
       cudaFuncSetAttribute(k_field_dm<KS, DM_EFG>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
@@ -849,7 +849,7 @@ static int launch_field_dm_k(mdff_ctx* h, const RecMesh& M, int n, const int* im
   ng = cdiv(M.nrows, rpg);
   const int rc = std::min(rpg, field_dm_rc(KS));
   const dim3 g((unsigned)tiles, (unsigned)ng);
-  const size_t smem = (size_t)rc * field_dm_rl(KS) * 8;
+  const size_t smem = (size_t)rc * (field_dm_rl(KS) * 8 + 16);
   const double2* tab = h->d_tab64;
   const double4* w = h->d_w;
   const double2* rhoA = h->d_rhoA;

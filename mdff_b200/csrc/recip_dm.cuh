@@ -67,8 +67,6 @@ template <int NT, bool HM>
 static __global__ void __launch_bounds__(kDmThreads, 1) k_rho_dm(
     const double2* __restrict__ tab, const double4* __restrict__ w, int natm, const int* __restrict__ imap,
     int nion, int chunk, int ci, RecMesh M, double2* __restrict__ part) {
-  pdl_wait();
-  pdl_trigger();
   extern __shared__ __align__(16) unsigned char dms[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, tt = lane & 3, rg = warp & 7, half = warp >> 3;
@@ -79,24 +77,29 @@ static __global__ void __launch_bounds__(kDmThreads, 1) k_rho_dm(
   double4* sw = reinterpret_cast<double4*>(sp + (size_t)2 * ent * ld);
   const int a0 = blockIdx.y * chunk, a1 = a0 + chunk < nion ? a0 + chunk : nion;
   const int nch = (a1 - a0 + ci - 1) / ci;
-  auto fetch = [&](int c) {
-    double2* o = sp + (size_t)(c & 1) * ent * ld;
-    const int b = a0 + c * ci;
-    for (int e = threadIdx.x; e < ent * ci; e += kDmThreads) {
-      const int en = e / ci, k = e - en * ci;
-      const int sl = b + k < a1 ? b + k : a1 - 1;
-      const int i = imap ? imap[sl] : sl;
+  // a thread copies one ion slot of every (512 / ci)-th entry (the weights are the
+  // last two); its ion index is fetched one chunk ahead
+  const int fk = threadIdx.x & (ci - 1), fe = threadIdx.x / ci, fs = kDmThreads / ci;
+  auto slot_ion = [&](int c) {
+    const int sl = a0 + c * ci + fk < a1 ? a0 + c * ci + fk : a1 - 1;
+    return imap ? imap[sl] : sl;
+  };
+  int inext = slot_ion(0), icur = inext;
+  auto fetch_tab = [&](int c) {
+    const int i = icur = inext;
+    if (c + 1 < nch) inext = slot_ion(c + 1);
+    double2* o = sp + (size_t)(c & 1) * ent * ld + fk;
+    const double2* tb = tab + i;
+    for (int en = fe; en < ent; en += fs) {
       // (entries of n > kz repeat the last one: their columns are not stored)
       const int te = en < nxy ? en : nxy + (n0 + en - nxy < kz ? n0 + en - nxy : kz);
-      dm_cp16(o + en * ld + k, tab + (size_t)te * natm + i);
+      dm_cp16(o + en * ld, tb + (size_t)te * natm);
     }
-    double4* ow = sw + (c & 1) * ci;
-    for (int e = threadIdx.x; e < 2 * ci; e += kDmThreads) {
-      const int k = e >> 1;
-      const int sl = b + k < a1 ? b + k : a1 - 1;
-      const int i = imap ? imap[sl] : sl;
-      dm_cp16(reinterpret_cast<double2*>(ow + k) + (e & 1), reinterpret_cast<const double2*>(w + i) + (e & 1));
-    }
+  };
+  auto fetch_w = [&](int c) {
+    if (fe < 2)
+      dm_cp16(reinterpret_cast<double2*>(sw + (c & 1) * ci + fk) + fe,
+              reinterpret_cast<const double2*>(w + icur) + fe);
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
   const int row = blockIdx.x * kDmRows + rg * 8 + g;
@@ -112,10 +115,17 @@ static __global__ void __launch_bounds__(kDmThreads, 1) k_rho_dm(
       u[s][d] = 0.0;
       if (HM) v[HM ? s : 0][d] = 0.0;
     }
-  fetch(0);
+  // the first phases travel while the weights' kernel finishes (the tables and
+  // the ion map are older than it: every kernel between waits before it lets its
+  // successor start)
+  fetch_tab(0);
+  pdl_wait();
+  pdl_trigger();
+  fetch_w(0);
   for (int c = 0; c < nch; ++c) {
     if (c + 1 < nch) {
-      fetch(c + 1);
+      fetch_tab(c + 1);
+      fetch_w(c + 1);
       asm volatile("cp.async.wait_group 1;" ::: "memory");
     } else {
       asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -244,12 +254,11 @@ static __global__ void __launch_bounds__(kDmFldThreads, KS <= 9 ? 2 : 1) k_field
     const double2* __restrict__ tab, const double4* __restrict__ w, int natm, const int* __restrict__ imap,
     int nion, RecMesh M, const double2* __restrict__ rhoA, int rpg, int rc, double4* __restrict__ Gpart,
     double4* __restrict__ Hpart) {
-  pdl_wait();
-  pdl_trigger();
   constexpr int KN = 2 * KS, RL = field_dm_rl(KS);
   constexpr bool AN = KS <= 9 && MODE == DM_FIELD;  // n (c, s) in registers too
   extern __shared__ __align__(16) unsigned char dms[];
-  double* sc = reinterpret_cast<double*>(dms);
+  int4* srow = reinterpret_cast<int4*>(dms);  // the chunk's rows
+  double* sc = reinterpret_cast<double*>(srow + rc);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, tt = lane & 3;
   const int kx = M.kmax[0], ky = M.kmax[1], kz = M.kmax[2];
@@ -277,8 +286,13 @@ static __global__ void __launch_bounds__(kDmFldThreads, KS <= 9 ? 2 : 1) k_field
       a[q][s] = z;
       if (AN) an[q][AN ? s : 0] = (double)n * z;
     }
-    if (MODE == DM_FORCE) wi[q] = w[ion[q]];
   }
+  // (the phases above are older than the kernel that sums rho', as in k_rho_dm)
+  pdl_wait();
+  pdl_trigger();
+  if (MODE == DM_FORCE)
+#pragma unroll
+    for (int q = 0; q < 2; ++q) wi[q] = w[ion[q]];
   double G[2][3], H[2][3];
 #pragma unroll
   for (int q = 0; q < 2; ++q)
@@ -288,25 +302,27 @@ static __global__ void __launch_bounds__(kDmFldThreads, KS <= 9 ? 2 : 1) k_field
   for (int ra = r0; ra < r1; ra += rc) {
     const int nr = r1 - ra < rc ? r1 - ra : rc, nr4 = (nr + 3) / 4;
     __syncthreads();
+    for (int r = threadIdx.x; r < nr4 * 4; r += kDmFldThreads) srow[r] = M.rows[ra + (r < nr ? r : nr - 1)];
+    __syncthreads();
+#pragma unroll 4
     for (int e = threadIdx.x; e < nr4 * 4 * KN; e += kDmFldThreads) {
       const int rr = e / KN, n = e - rr * KN;
-      double2 rp = make_double2(0.0, 0.0), rm = rp;
-      if (rr < nr && n <= kz) {
-        const int4 ri = M.rows[ra + rr];
-        if (n >= ri.z) rp = rhoA[ri.w + n - ri.z];
-        if (n > 0 && ri.z < 0) rm = rhoA[ri.w - n - ri.z];
-      }
+      const int4 ri = srow[rr];
+      // (a row past the end and an n past kz have zero coefficients)
+      const bool hp = rr < nr && n <= kz && n >= ri.z, hm = rr < nr && n <= kz && n > 0 && ri.z < 0;
+      double2 rp = rhoA[hp ? ri.w + n - ri.z : 0], rm = rhoA[hm ? ri.w - n - ri.z : 0];
+      if (!hp) rp = make_double2(0.0, 0.0);
+      if (!hm) rm = make_double2(0.0, 0.0);
       double2* o = reinterpret_cast<double2*>(sc + (size_t)rr * RL + 4 * n);
       o[0] = make_double2(rp.x + rm.x, rp.y + rm.y);
       o[1] = n ? make_double2(rp.x - rm.x, rp.y - rm.y) : make_double2(0.0, 0.0);
     }
     __syncthreads();
     if (wact) {
-      int4 rn;
+      // this lane's row of the four, X and Y of its ions one step ahead
       double2 Xn[2], Yn[2];
       auto next = [&](int r4) {
-        const int r = ra + r4 * 4 + tt;
-        rn = M.rows[r < M.nrows ? r : M.nrows - 1];
+        const int4 rn = srow[r4 * 4 + tt];
         const int ye = kx + 1 + (rn.y < 0 ? -rn.y : rn.y);
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
@@ -316,7 +332,6 @@ static __global__ void __launch_bounds__(kDmFldThreads, KS <= 9 ? 2 : 1) k_field
       };
       next(0);
       for (int r4 = 0; r4 < nr4; ++r4) {
-        const int4 ri = rn;
         const double2 X[2] = {Xn[0], Xn[1]}, Y[2] = {Yn[0], Yn[1]};
         if (r4 + 1 < nr4) next(r4 + 1);
         double d0[4] = {0, 0, 0, 0}, d1[4] = {0, 0, 0, 0}, d2[4] = {0, 0, 0, 0};
@@ -337,6 +352,7 @@ static __global__ void __launch_bounds__(kDmFldThreads, KS <= 9 ? 2 : 1) k_field
           dmma(d1, n0, n1, b1);
           if (MODE != DM_FIELD) dmma(d2, fn * n0, fn * n1, b0);
         }
+        const int4 ri = srow[r4 * 4 + tt];
         const double fx = (double)ri.x, fy = (double)ri.y;
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
