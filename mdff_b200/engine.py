@@ -16,7 +16,19 @@ from ._abi import MdffError, dptr, iptr
 
 
 def _mat(m):
-    return np.array([[m[a][b] for b in range(3)] for a in range(3)])
+    return np.array(m)
+
+
+# MdffBatchConf as a numpy record: the results of all configurations are read
+# column by column instead of field by field through ctypes
+_CONF = np.dtype([(n, np.float64) for n in ("u_lj", "vir_lj", "u_bmhft", "vir_bmhft", "u_coul", "u_pol",
+                                            "pvirial_coul")]
+                 + [(n, np.float64, (3, 3)) for n in ("tau_nonb", "tau_coul", "tau")]
+                 + [("rmsd", np.float64)]
+                 + [(n, np.int32) for n in ("n_pol_iter", "converged", "catastrophe", "nk")]
+                 + [("alphaES", np.float64), ("cutlongrange", np.float64), ("kES", np.int32, (3,)),
+                    ("pad", np.int32)])
+assert _CONF.itemsize == ctypes.sizeof(_abi.MdffBatchConf)
 
 
 class ForceEngine:
@@ -215,17 +227,10 @@ class BatchEngine:
 
     @staticmethod
     def _conf_dicts(confs):
-        out = []
-        for c in confs:
-            d = {k: getattr(c, k) for k in ("u_lj", "vir_lj", "u_bmhft", "vir_bmhft", "u_coul",
-                                            "u_pol", "pvirial_coul", "rmsd", "n_pol_iter",
-                                            "converged", "catastrophe", "nk", "alphaES",
-                                            "cutlongrange")}
-            d["kES"] = list(c.kES)
-            for k in ("tau_nonb", "tau_coul", "tau"):
-                d[k] = _mat(getattr(c, k))
-            out.append(d)
-        return out
+        a = np.frombuffer(confs, dtype=_CONF).copy()
+        cols = {k: (list(a[k]) if k in ("tau_nonb", "tau_coul", "tau") else a[k].tolist())
+                for k in _CONF.names if k != "pad"}
+        return [dict(zip(cols, v)) for v in zip(*cols.values())]
 
     def engforce(self, rx, ry, rz, allow_status=()):
         n = self.ntot
