@@ -22,6 +22,17 @@
 //   Tang-Toennies b, c of the charge field on a dipole type (damped qd
 //   forces / energy and the damped static field); one charge scale s on all
 //   charges (qq terms scale with s^2, qd terms and the charge field with s).
+//
+// Bound: the dipole solve (to 1e-12, twice the forward's iterations), FP64
+// throughout.  The structure-factor channels are the forward's tensor-core
+// products (brho_t; sigma's weight is a polynomial in nz), the right-hand side's k
+// sums two passes of its field product; the pair loops walk the partner lists
+// with partners fetched ahead, the right-hand side over the CTA's share of the
+// polarisable ions, and form each pair's parameter derivatives once, selected
+// into the gradient by per-type-pair masks.  Measured, 64 boxes of 216-512 ions, all ten
+// parameters of the MgO model: 7.6 -> 3.1 ms (SM time at 2 CTAs: right-hand side's and
+// charge-scale channels 99 -> 46 ms, pair loops 72 -> 47, solve 229 -> 196; the
+// rest from the launch shape: clusters of 2 instead of 8).
 #pragma once
 #include "batch.cuh"
 
@@ -50,16 +61,28 @@ struct AdjArgs {
   FitParam prm[kFitMax];
 };
 
+// One Tang-Toennies role (b, c, order) at distance r: F1d = 1 - f and fd of
+// tt_damp, from f1, fd1 of c = 1 (f = 1 - c (1 - f1), fd = c fd1).  c = 0 damps
+// nothing; its derivatives are formed only where a parameter asks (need).
+template <int K>
+__device__ __forceinline__ void tt_role(double b, double c, double r, int order, bool need, double& F1d,
+                                        double& fd, double& f1, double& fd1) {
+  F1d = fd = fd1 = 0.0;
+  f1 = 1.0;
+  if (c != 0.0) tt_damp_k<double, K>(b, 1.0, r, order, f1, fd1);
+  else if (need) tt_damp<double>(b, 1.0, r, order, f1, fd1);
+  F1d = c * (1.0 - f1);
+  fd = c * fd1;
+}
+
 // d f / d b and d f / d c of tt_damp (f = 1 - c e^{-x} sum_k x^k/k!, fd = c b
-// e^{-x} x^n/n!, x = b r):
+// e^{-x} x^n/n!, x = b r) from f1, fd1 of c = 1:
 //   df/dc = (f - 1)/c ... evaluated without dividing by c:  -e^{-x} S(x)
 //   dfd/dc = b e^{-x} x^n/n!
 //   df/db = r c e^{-x} x^n/n! = (r/b) fd
 //   dfd/db = c e^{-x} x^n/n! (1 + n - x)
-__device__ __forceinline__ void tt_damp_grad(double b, double c, double r, int n, double& dfdb,
-                                             double& dfddb, double& dfdc, double& dfddc) {
-  double f1, fd1;
-  tt_damp<double>(b, 1.0, r, n, f1, fd1);  // c = 1: f1 = 1 - e^{-x}S, fd1 = b e^{-x} x^n/n!
+__device__ __forceinline__ void tt_damp_grad(double b, double c, double r, int n, double f1, double fd1,
+                                             double& dfdb, double& dfddb, double& dfdc, double& dfddc) {
   double x = b * r;
   double en = (b != 0.0) ? fd1 / b : 0.0;  // e^{-x} x^n / n!
   if (b == 0.0) {
@@ -73,343 +96,311 @@ __device__ __forceinline__ void tt_damp_grad(double b, double c, double r, int n
   dfddb = c * en * (1.0 + (double)n - x);
 }
 
-// gradient of one canonical real-space pair (a = "ia", r = r_a - r_b) from
-// the visit of ion `own_a ? a : b`: accumulates this ion's share into g[],
-// and returns d(u_F . F)/d m_own in dm.
 struct PairAdj {
-  const FitParam* prm;
+  double gU, cu, rs;  // rs = 1 / (charge scale)
+  int qs;             // mask of the charge-scale parameters
   int nparam;
-  double qscale, gU, cu;
 };
 
-__device__ __forceinline__ void es_pair_adjoint(const PairAdj& J, const ESPair& P, int ta, int tb,
-                                                double d2, double alpha, const double (&r)[3],
-                                                double qa, double qb, const double (&ma)[3],
-                                                const double (&mb)[3], bool dip_a, bool dip_b,
-                                                int task_qq, int task_qd, int task_dd,
-                                                const double (&wa)[3], const double (&wb)[3],
-                                                const double (&lown)[3], bool own_a,
-                                                double (&dm)[3], double* g) {
+__device__ __forceinline__ double dot3(const double (&a)[3], const double4& b) {
+  return a[0] * b.x + a[1] * b.y + a[2] * b.z;
+}
+__device__ __forceinline__ double dot3(const double4& a, const double4& b) {
+  return a.x * b.x + a.y * b.y + a.z * b.z;
+}
+
+// One real-space pair from the visit of ion i (r = r_i - r_j; the expressions
+// of es_force_ipair, in i's frame; roles by i_is_a).
+//   GRAD = false: dm += d(u_F . F)/dm_i.
+//   GRAD = true:  this visit's share of the parameter gradient (half of the
+//   energy, the force on i, the charge field on i against lambda_i) into g;
+//   hit_i / hit_j: masks of the damping parameters of the field on i / on j.
+template <int K, bool GRAD>
+__device__ __forceinline__ void es_pair_adjoint(const PairAdj& J, const AdjArgs& A, const ESPair& P, bool i_is_a,
+                                                double d2, double alpha, const double (&r)[3], double qi, double qj,
+                                                const double4& mi, const double4& mj, int task_qq, int task_qd,
+                                                int task_dd, const double4& wi, const double4& wj,
+                                                const double4& li, int hit_i, int hit_j, double (&dm)[3],
+                                                double (&g)[kFitMax]) {
   Radial<double> rd;
-  radial<double, true>(d2, alpha, rd);
-  const bool ldamp = P.ldamp != 0;
-  double fa = 1.0, fda = 0.0, fb = 1.0, fdb = 0.0;
-  if (ldamp) {
-    tt_damp<double>(P.ba, P.ca, rd.d, P.ka, fa, fda);
-    tt_damp<double>(P.bb, P.cb, rd.d, P.kb, fb, fdb);
+  radial<double, !GRAD>(d2, alpha, rd);
+  const bool dip_i = mi.x != 0.0 || mi.y != 0.0 || mi.z != 0.0;
+  const bool dip_j = mj.x != 0.0 || mj.y != 0.0 || mj.z != 0.0;
+  const double B0 = rd.dm1 * rd.F0, B1 = rd.F1 * rd.dm3, B2 = 3.0 * rd.F2 * rd.dm5;
+  double C1i = B1, C2i = B2, C1j = B1, C2j = B2;  // B - B_damped for the field on i / on j
+  double bi = 0, ci = 0, bj = 0, cj = 0, f1i = 1, fd1i = 0, f1j = 1, fd1j = 0;
+  int ki = 0, kj = 0;
+  if (P.ldamp) {
+    double F1d, fd;
+    bi = i_is_a ? P.ba : P.bb;
+    ci = i_is_a ? P.ca : P.cb;
+    ki = i_is_a ? P.ka : P.kb;
+    tt_role<K>(bi, ci, rd.d, ki, GRAD && hit_i, F1d, fd, f1i, fd1i);
+    C1i = B1 - F1d * rd.dm3;
+    C2i = B2 - 3.0 * (F1d + (rd.d / 3.0) * fd) * rd.dm5;
+    if (GRAD) {  // (the field on j does not enter dm_i)
+      bj = i_is_a ? P.bb : P.ba;
+      cj = i_is_a ? P.cb : P.ca;
+      kj = i_is_a ? P.kb : P.ka;
+      tt_role<K>(bj, cj, rd.d, kj, hit_j != 0, F1d, fd, f1j, fd1j);
+      C1j = B1 - F1d * rd.dm3;
+      C2j = B2 - 3.0 * (F1d + (rd.d / 3.0) * fd) * rd.dm5;
+    }
   }
-  double F1d = ldamp ? 1.0 - fa : 0.0, F2d = ldamp ? F1d + (rd.d / 3.0) * fda : 0.0;
-  double F1d2 = ldamp ? 1.0 - fb : 0.0, F2d2 = ldamp ? F1d2 + (rd.d / 3.0) * fdb : 0.0;
-  double B0 = rd.dm1 * rd.F0, B1 = rd.F1 * rd.dm3, B2 = 3.0 * rd.F2 * rd.dm5, B3 = 15.0 * rd.F3 * rd.dm7;
-  double B1d = F1d * rd.dm3, B2d = 3.0 * F2d * rd.dm5, B1d2 = F1d2 * rd.dm3, B2d2 = 3.0 * F2d2 * rd.dm5;
-  double rma = r[0] * ma[0] + r[1] * ma[1] + r[2] * ma[2];
-  double rmb = r[0] * mb[0] + r[1] * mb[1] + r[2] * mb[2];
-  double D[3] = {wa[0] - wb[0], wa[1] - wb[1], wa[2] - wb[2]};
-  double Dr = D[0] * r[0] + D[1] * r[1] + D[2] * r[2];
-  double Dma = D[0] * ma[0] + D[1] * ma[1] + D[2] * ma[2];
-  double Dmb = D[0] * mb[0] + D[1] * mb[1] + D[2] * mb[2];
-  const bool dd = task_dd && dip_a && dip_b;
-  const bool qd = task_qd && (dip_a || dip_b);
-  // d(D . f_ab)/dm_own
-  for (int c = 0; c < 3; ++c) dm[c] = 0.0;
-  if (own_a) {
-    if (dd)
-      for (int c = 0; c < 3; ++c)
-        dm[c] += B3 * rmb * Dr * r[c] - B2 * (Dr * mb[c] + rmb * D[c] + Dmb * r[c]);
-    if (qd)
-      for (int c = 0; c < 3; ++c) {
-        dm[c] += qb * (B2 * Dr * r[c] - B1 * D[c]);
-        if (ldamp) dm[c] -= qb * (B2d * Dr * r[c] - B1d * D[c]);
-      }
-  } else {
-    if (dd)
-      for (int c = 0; c < 3; ++c)
-        dm[c] += B3 * rma * Dr * r[c] - B2 * (Dr * ma[c] + Dma * r[c] + rma * D[c]);
-    if (qd)
-      for (int c = 0; c < 3; ++c) {
-        dm[c] -= qa * (B2 * Dr * r[c] - B1 * D[c]);
-        if (ldamp) dm[c] += qa * (B2d2 * Dr * r[c] - B1d2 * D[c]);
-      }
+  const bool qd = task_qd && (dip_i || dip_j);
+  const double rmj = dot3(r, mj);
+  if (!GRAD) {
+    const double4 D = make_double4(wi.x - wj.x, wi.y - wj.y, wi.z - wj.z, 0.0);
+    const double Dr = dot3(r, D), Dmj = dot3(D, mj);
+    double fr = 0.0, fD = 0.0, fm = 0.0;  // coefficients of r, D, m_j
+    if (task_dd && dip_i && dip_j) {
+      const double B3 = 15.0 * rd.F3 * rd.dm7;
+      fr += B3 * rmj * Dr - B2 * Dmj;
+      fm -= B2 * Dr;
+      fD -= B2 * rmj;
+    }
+    if (qd) {
+      fr += qj * C2i * Dr;
+      fD -= qj * C1i;
+    }
+    // u_F . F = -cu D . f
+    dm[0] -= J.cu * (fr * r[0] + fD * D.x + fm * mj.x);
+    dm[1] -= J.cu * (fr * r[1] + fD * D.y + fm * mj.y);
+    dm[2] -= J.cu * (fr * r[2] + fD * D.z + fm * mj.z);
+    return;
   }
-  for (int c = 0; c < 3; ++c) dm[c] *= -J.cu;  // u_F . F = -cu D . f_ab
-  if (!g) return;
-  // this visit's share: force on own = sgn cu f_ab, energy halved (both visits)
-  const double sgn = own_a ? -1.0 : 1.0;
-  const double* wo = own_a ? wa : wb;
-  double wr = wo[0] * r[0] + wo[1] * r[1] + wo[2] * r[2];
-  double wma = wo[0] * ma[0] + wo[1] * ma[1] + wo[2] * ma[2];
-  double wmb = wo[0] * mb[0] + wo[1] * mb[1] + wo[2] * mb[2];
-  double lr = lown[0] * r[0] + lown[1] * r[1] + lown[2] * r[2];
-  for (int p = 0; p < J.nparam; ++p) {
-    const FitParam& fp = J.prm[p];
-    if (fp.kind == FIT_QSCALE) {
-      double s = J.qscale;
-      double val = 0.0;
-      if (task_qq) {
-        // w.f_qq, u_qq scale with s^2; the charge field on own with s
-        double wf_qq = -qa * qb * B1 * wr;
-        val += J.cu * sgn * 2.0 * wf_qq + 0.5 * J.gU * J.cu * 2.0 * qa * qb * B0;
-        double Eown_r = own_a ? qb * (B1 - (ldamp ? B1d : 0.0)) * lr
-                              : -qa * (B1 - (ldamp ? B1d2 : 0.0)) * lr;
-        val += Eown_r;
-      }
-      if (qd) {
-        double wf_qd = -qa * (B2 * wr * rmb - B1 * wmb) + qb * (B2 * wr * rma - B1 * wma);
-        double u_qd = qa * B1 * rmb - qb * B1 * rma;
-        if (ldamp) {
-          wf_qd += -qb * (B2d * wr * rma - B1d * wma) + qa * (B2d2 * wr * rmb - B1d2 * wmb);
-          u_qd += -qa * B1d2 * rmb + qb * B1d * rma;
-        }
-        val += J.cu * sgn * wf_qd + 0.5 * J.gU * J.cu * u_qd;
-      }
-      g[p] += val / s;
-    } else if ((fp.kind == FIT_TTB || fp.kind == FIT_TTC) && ldamp) {
-      // parameter (X = dipole type, Y = charge type): role a if (ta, tb) =
-      // (X, Y) [table (X, X, Y)], role b if (tb, ta) = (X, Y) [table (X, Y, X)]
-      for (int role = 0; role < 2; ++role) {
-        bool hit = role == 0 ? (ta == fp.t1 && tb == fp.t2) : (tb == fp.t1 && ta == fp.t2);
-        if (!hit) continue;
-        double bb = role == 0 ? P.ba : P.bb, cc = role == 0 ? P.ca : P.cb;
-        int kk = role == 0 ? P.ka : P.kb;
-        double dfdb, dfddb, dfdc, dfddc;
-        tt_damp_grad(bb, cc, rd.d, kk, dfdb, dfddb, dfdc, dfddc);
-        double df = fp.kind == FIT_TTB ? dfdb : dfdc;
-        double dfd = fp.kind == FIT_TTB ? dfddb : dfddc;
-        double dB1 = -df * rd.dm3;                              // d(B1d)/dtheta
-        double dB2 = 3.0 * (-df + (rd.d / 3.0) * dfd) * rd.dm5;  // d(B2d)/dtheta
-        double val = 0.0;
-        if (role == 0) {
-          // f_ab += -qb (B2d r rma - B1d ma); u += qb B1d rma; Ea -= qb B1d r
-          if (qd) {
-            double wdf = -qb * (dB2 * wr * rma - dB1 * wma);
-            val += J.cu * sgn * wdf + 0.5 * J.gU * J.cu * qb * dB1 * rma;
-          }
-          if (task_qq && own_a) val += -qb * dB1 * lr;
-        } else {
-          // f_ab += qa (B2d2 r rmb - B1d2 mb); u += -qa B1d2 rmb; Eb += qa B1d2 r
-          if (qd) {
-            double wdf = qa * (dB2 * wr * rmb - dB1 * wmb);
-            val += J.cu * sgn * wdf - 0.5 * J.gU * J.cu * qa * dB1 * rmb;
-          }
-          if (task_qq && !own_a) val += qa * dB1 * lr;
-        }
-        g[p] += val;
-      }
+  const double rmi = dot3(r, mi), wr = dot3(r, wi), lr = dot3(r, li);
+  const double wmi = dot3(wi, mi), wmj = dot3(wi, mj);
+  double vq = 0.0, vb[2] = {0.0, 0.0}, vc[2] = {0.0, 0.0};
+  if (J.qs) {
+    if (task_qq)  // w.f_qq and u_qq scale with s^2; the charge field on i with s
+      vq += 2.0 * J.cu * qi * qj * B1 * wr + J.gU * J.cu * qi * qj * B0 + qj * C1i * lr;
+    if (qd)
+      vq += J.cu * (qi * (C2j * wr * rmj - C1j * wmj) - qj * (C2i * wr * rmi - C1i * wmi)) +
+            0.5 * J.gU * J.cu * (qi * C1j * rmj - qj * C1i * rmi);
+    vq *= J.rs;
+  }
+  if (P.ldamp && hit_i) {
+    double dfdb, dfddb, dfdc, dfddc;
+    tt_damp_grad(bi, ci, rd.d, ki, f1i, fd1i, dfdb, dfddb, dfdc, dfddc);
+    auto val = [&](double df, double dfd) {
+      const double dB1 = -df * rd.dm3, dB2 = 3.0 * (-df + (rd.d / 3.0) * dfd) * rd.dm5;  // of the damped parts
+      double v = 0.0;
+      if (qd) v += J.cu * qj * (dB2 * wr * rmi - dB1 * wmi) + 0.5 * J.gU * J.cu * qj * dB1 * rmi;
+      if (task_qq) v -= qj * dB1 * lr;
+      return v;
+    };
+    vb[0] = val(dfdb, dfddb);
+    vc[0] = val(dfdc, dfddc);
+  }
+  if (P.ldamp && hit_j && qd) {
+    double dfdb, dfddb, dfdc, dfddc;
+    tt_damp_grad(bj, cj, rd.d, kj, f1j, fd1j, dfdb, dfddb, dfdc, dfddc);
+    auto val = [&](double df, double dfd) {
+      const double dB1 = -df * rd.dm3, dB2 = 3.0 * (-df + (rd.d / 3.0) * dfd) * rd.dm5;
+      return -J.cu * qi * (dB2 * wr * rmj - dB1 * wmj) - 0.5 * J.gU * J.cu * qi * dB1 * rmj;
+    };
+    vb[1] = val(dfdb, dfddb);
+    vc[1] = val(dfdc, dfddc);
+  }
+#pragma unroll
+  for (int p = 0; p < kFitMax; ++p) {
+    if (p >= J.nparam) break;
+    const int kind = A.prm[p].kind;
+    if (kind == FIT_QSCALE) {
+      g[p] += vq;
+    } else if (kind == FIT_TTB || kind == FIT_TTC) {
+      if ((hit_i >> p) & 1) g[p] += kind == FIT_TTB ? vb[0] : vc[0];
+      if ((hit_j >> p) & 1) g[p] += kind == FIT_TTB ? vb[1] : vc[1];
     }
   }
 }
 
 // Buckingham / BMH pair parameters from the visit of ion i (r = r_i - r_j):
-// w_i . r dwij/dtheta + 1/2 g_U du/dtheta
-__device__ __forceinline__ void sr_pair_adjoint(const PairAdj& J, const NBPair& P, int lbmhftd,
-                                                int ti, int tj, double rijsq,
-                                                const double (&r)[3], const double (&wi)[3],
-                                                double* g) {
+// w_i . r dwij/dtheta + 1/2 g_U du/dtheta (hit: mask of the pair's parameters)
+__device__ __forceinline__ void sr_pair_adjoint(const PairAdj& J, const AdjArgs& A, const NBPair& P, int lbmhftd,
+                                                int hit, double rijsq, const double (&r)[3], const double4& wi,
+                                                double (&g)[kFitMax]) {
   if (P.A == 0.0) return;  // the reference skips the pair (non_bonded.f90:1153)
-  double d = sqrt(rijsq);
-  double wr = wi[0] * r[0] + wi[1] * r[1] + wi[2] * r[2];
-  double e = exp(-P.B * d);
-  double ir6 = 1.0 / (rijsq * rijsq * rijsq);
+  const double d = sqrt(rijsq), dinv = 1.0 / d;
+  const double wr = dot3(r, wi);
+  const double e = exp(-P.B * d);
+  const double ir2 = dinv * dinv, ir6 = ir2 * ir2 * ir2;
   double f6 = 1.0, fd6 = 0.0;
-  if (lbmhftd) tt_damp<double>(P.BD, 1.0, d, 6, f6, fd6);
-  for (int p = 0; p < J.nparam; ++p) {
-    const FitParam& fp = J.prm[p];
-    if (fp.kind > FIT_C) continue;
-    bool hit = (ti == fp.t1 && tj == fp.t2) || (ti == fp.t2 && tj == fp.t1);
-    if (!hit) continue;
-    double du, dw;
-    if (fp.kind == FIT_A) {
-      du = e;
-      dw = P.B * e / d;
-    } else if (fp.kind == FIT_RHO) {
-      // B = 1/rho: d/drho = -B^2 d/dB
-      double duB = -P.A * d * e, dwB = P.A * e * (1.0 - P.B * d) / d;
-      du = -P.B * P.B * duB;
-      dw = -P.B * P.B * dwB;
-    } else {
-      du = -f6 * ir6;
-      dw = (-6.0 * f6 * ir6 / d + fd6 * ir6) / d;
-    }
-    g[p] += wr * dw + 0.5 * J.gU * du;
+  if (lbmhftd) tt_damp_k<double, 6>(P.BD, 1.0, d, 6, f6, fd6);
+  const double hg = 0.5 * J.gU;
+  const double vA = wr * (P.B * e * dinv) + hg * e;
+  // B = 1/rho: d/drho = -B^2 d/dB
+  const double vR = -P.B * P.B * (wr * (P.A * e * (1.0 - P.B * d) * dinv) - hg * P.A * d * e);
+  const double vC = wr * ((-6.0 * f6 * ir6 * dinv + fd6 * ir6) * dinv) - hg * f6 * ir6;
+#pragma unroll
+  for (int p = 0; p < kFitMax; ++p) {
+    if (p >= J.nparam) break;
+    const int kind = A.prm[p].kind;
+    if ((hit >> p) & 1) g[p] += kind == FIT_A ? vA : kind == FIT_RHO ? vR : vC;
   }
 }
 
 // ---------------------------------------------------------------------------
-// one structure-factor channel over this CTA's k rows (FP64 tables):
-//   W_i(k) = [ (hasq ? q_i : 0) + i (hasv ? k.v_i : 0) ] * (hasw ? k.w_i : 1)
-// v from S.v, w from S.w; out[k] = sum_i W_i(k) e^{i k.r_i} (not A-scaled).
-__device__ void bsf(cgx::cluster_group& cl, const BatchArgs& a, BCtx& X, const BShared& S,
-                    const double4* __restrict__ Sw, bool hasq, bool hasv, bool hasw,
-                    double2* __restrict__ out) {
+// Structure-factor partials of this CTA's ions over all rows (brho_t), visible
+// to the cluster on return:
+//   sum_i [ (has_q ? q_i : 0) + i (has_m ? k.v_i : 0) ] (has_w ? k.w_i : 1) P_i,
+// v from S.v, w from Sw by ion; rot: times i (has_w only).  r: the pass, for the
+// field (bfld) or badj_store of the same partials.
+__device__ __noinline__ void badj_rho(cgx::cluster_group& cl, const BatchArgs& a, BCtx& X, const BShared& S,
+                                      const double4* Sw, bool has_q, bool has_m, bool has_w, bool rot, BRecArgs& r) {
   const BConf& c = *X.c;
-  if (c.nk == 0) return;
-  const int4* rows = a.rows + c.row_off;
-  const int kz = c.kz;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-  cl.sync();
-  int r0 = (int)((long long)c.nrows * X.rank / X.C), r1 = (int)((long long)c.nrows * (X.rank + 1) / X.C);
-  const int ntile = (2 * kz + 1 + kBNZ - 1) / kBNZ;
-  int nitems = (r1 - r0) * ntile;
-  for (int it = warp; it < nitems; it += nwarp) {
-    int row = r0 + it / ntile, tile = it % ntile;
-    int4 ri = rows[row];
-    int nx = ri.x, ny = ri.y;
-    int nz0 = ri.z + tile * kBNZ;
-    if (nz0 > kz) continue;
-    int nzn = min(kBNZ, kz - nz0 + 1);
-    double accR[kBNZ], accI[kBNZ];
-#pragma unroll
-    for (int t = 0; t < kBNZ; ++t) accR[t] = accI[t] = 0.0;
-    for (int i = lane; i < X.n; i += 32) {
-      double2 XY = bphase(a, c, i, nx, ny, 0);
-      double2 Z1 = btab(a, c, c.kx + 1 + c.ky + 1 + 1, i);
-      double2 P = bphase_z(a, c, i, XY, nz0);
-      double qv = hasq ? S.s[i].w : 0.0;
-      double kv = 0.0, v3 = 0.0, kw = 1.0, w3 = 0.0;
-      if (hasv) {
-        double4 u = S.v[i];
-        double3 m = bmvec(c, u.x, u.y, u.z);
-        kv = nx * m.x + ny * m.y + nz0 * m.z;
-        v3 = m.z;
-      }
-      if (hasw) {
-        double4 u = Sw[i];
-        double3 m = bmvec(c, u.x, u.y, u.z);
-        kw = nx * m.x + ny * m.y + nz0 * m.z;
-        w3 = m.z;
-      }
-#pragma unroll
-      for (int t = 0; t < kBNZ; ++t) {
-        double wr = qv * kw, wi = kv * kw;
-        accR[t] += wr * P.x - wi * P.y;
-        accI[t] += wr * P.y + wi * P.x;
-        kv += v3;
-        kw += w3;
-        P = cmul(P, Z1);
-      }
-    }
-#pragma unroll
-    for (int t = 0; t < kBNZ; ++t) {
-      double vr = warp_sum(accR[t]);
-      double vi = warp_sum(accI[t]);
-      if (lane == 0 && t < nzn) {
-        int kl = ri.w + (nz0 - ri.z) + t;
-        out[c.k_off + kl] = make_double2(vr, vi);
-      }
+  r = brec_args(a, X, S, 0, false);
+  r.rot = rot;
+  double4* w = brec_weights(r, S, has_w ? 2 : 1);
+  const BWeights ws{X.c, S.s, S.v, S.v32, r.src.n0, 0, has_q, has_m};
+  __syncthreads();
+  for (int k = threadIdx.x; k < r.src.cnt; k += blockDim.x) {
+    double v[4];
+    ws(k, v);
+    w[k] = make_double4(v[0], v[1], v[2], v[3]);
+    if (has_w) {
+      const double4 u = Sw[r.src.n0 + k];
+      const double3 m = bmvec(c, u.x, u.y, u.z);
+      w[r.src.cnt + k] = make_double4(0.0, m.x, m.y, m.z);
     }
   }
+  __syncthreads();
+  if (has_w) brho<2>(r);
+  else if (has_m) brho<1>(r);
+  else brho<0>(r);
   cl.sync();
 }
-
-// per own ion: out_i = 2 pi B [ sum_k A_k n (k.w_i) Re(X1 P_i*) - sum_k A_k n Re(X2 P_i*) ]
-// (channels X1, X2 not A-scaled; w from Sw)
-__device__ void brecsum(const BatchArgs& a, const BCtx& X, const BShared& S,
-                        const double4* __restrict__ Sw, const double2* __restrict__ X1,
-                        const double2* __restrict__ X2, double4* __restrict__ outv) {
+// the sums of this CTA's share of the rows, by k
+__device__ __noinline__ void badj_store(const BatchArgs& a, const BCtx& X, const BRecArgs& r, double2* __restrict__ out) {
   const BConf& c = *X.c;
-  const int4* rows = a.rows + c.row_off;
-  const int kz = c.kz;
-  int mown = X.i1 - X.i0;
-  int sub = 1;
-  while (sub < 32 && mown * sub * 2 <= (int)blockDim.x) sub *= 2;
-  int slots = blockDim.x / sub;
-  int iters = (mown + slots - 1) / slots;
-  const int half = kBKChunk / 2;  // rho' chunk holds X1 in [0, half), X2 in [half, 2 half)
-  for (int itn = 0; itn < iters; ++itn) {
-    int slot = itn * slots + (int)threadIdx.x / sub;
-    int me = threadIdx.x % sub;
-    bool act = slot < mown;
-    int i = X.i0 + (act ? slot : 0);
-    double H[3] = {0, 0, 0}, K[3] = {0, 0, 0};
-    double4 u = Sw[i];
-    double3 m = bmvec(c, u.x, u.y, u.z);
-    double2 Z1 = btab(a, c, c.kx + 1 + c.ky + 1 + 1, i);
-    int ra = 0;
-    while (ra < c.nrows) {
-      int kbase = rows[ra].w;
-      int rb = ra;
-      while (rb < c.nrows) {
-        int4 rr = rows[rb];
-        if (rr.w + (kz - rr.z + 1) - kbase > half) break;
-        ++rb;
-      }
-      int kend = (rb < c.nrows) ? rows[rb].w : c.nk;
-      __syncthreads();
-      for (int k = threadIdx.x; k < kend - kbase; k += blockDim.x) {
-        size_t gk = (size_t)c.k_off + kbase + k;
-        double A = a.Ak[gk];
-        double2 p1 = __ldcg(X1 + gk), p2 = __ldcg(X2 + gk);
-        S.rho[k] = make_double2(A * p1.x, A * p1.y);
-        S.rho[half + k] = make_double2(A * p2.x, A * p2.y);
-      }
-      __syncthreads();
-      if (act) {
-        for (int r = ra + me; r < rb; r += sub) {
-          int4 ri = rows[r];
-          int nx = ri.x, ny = ri.y, nz_lo = ri.z;
-          double2 XY = bphase(a, c, i, nx, ny, 0);
-          double2 P = bphase_z(a, c, i, XY, nz_lo);
-          double kw = nx * m.x + ny * m.y + nz_lo * m.z;
-          double T0 = 0, Tz = 0, U0 = 0, Uz = 0;
-          int nn = kz - nz_lo + 1;
-          const double2* x1 = S.rho + (ri.w - kbase);
-          const double2* x2 = S.rho + half + (ri.w - kbase);
-          for (int t = 0; t < nn; ++t) {
-            double2 v1 = x1[t], v2 = x2[t];
-            double re1 = v1.x * P.x + v1.y * P.y;  // Re(X1 P*)
-            double re2 = v2.x * P.x + v2.y * P.y;
-            double tt = kw * re1;
-            T0 += tt;
-            Tz += t * tt;
-            U0 += re2;
-            Uz += t * re2;
-            kw += m.z;
-            P = cmul(P, Z1);
-          }
-          H[0] += nx * T0;
-          H[1] += ny * T0;
-          H[2] += nz_lo * T0 + Tz;
-          K[0] += nx * U0;
-          K[1] += ny * U0;
-          K[2] += nz_lo * U0 + Uz;
-        }
-      }
-      ra = rb;
+  const int nz = c.kz + 1;
+  const int r0 = (int)((long long)c.nrows * X.rank / X.C), r1 = (int)((long long)c.nrows * (X.rank + 1) / X.C);
+  for (int e = threadIdx.x; e < (r1 - r0) * nz; e += blockDim.x) {
+    const int row = r0 + e / nz, n = e % nz;
+    const int4 ri = r.rows[row];
+    double2 rp, rm;
+    brho_pm(r.part, r.pld, X.C, (size_t)row * nz + n, nullptr, rp, rm);
+    double2* o = out + c.k_off + ri.w - ri.z;
+    if (n >= ri.z) o[n] = rp;
+    if (n > 0 && ri.z < 0) o[-n] = rm;
+  }
+}
+
+// real-space right-hand side of this CTA's polarisable ions (warp per ion)
+template <int K>
+__device__ __noinline__ void badj_rhs(const BatchArgs& a, const AdjArgs& J, const PairAdj& PJ, const BCtx& X,
+                                      const BShared& S, const double4* Sw) {
+  const BConf& c = *X.c;
+  const int task_qq = (c.flags & BF_QQ) ? 1 : 0, task_qd = (c.flags & BF_QD) ? 1 : 0;
+  const int task_dd = (c.flags & BF_DD) ? 1 : 0;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+  for (int p = X.p0 + warp; p < X.p1; p += nwarp) {
+    const int i = bpl(S.t[p]);
+    const double4 si = S.s[i], mi = S.v[i], wi = Sw[i];
+    const int ti = btyp(S.t[i]);
+    double dm[3] = {0, 0, 0}, g[kFitMax];
+    const unsigned short* row = bnbl(a, X, 0, i);
+    const int nn = __ldcg(bnbn(a, X, 0) + i);
+    int jn = lane < nn ? bnbr(row, lane) : 0;
+    for (int k = lane; k < nn; k += 32) {
+      const int j = jn;
+      if (k + 32 < nn) jn = bnbr(row, k + 32);
+      const double4 sj = S.s[j];
+      double r[3];
+      const double r2 = pair_vec<double>(c.A, si, sj, r[0], r[1], r[2]);
+      if (r2 > c.rc2) continue;
+      const int tj = btyp(S.t[j]);
+      const bool ia = half_mask(i, j);
+      es_pair_adjoint<K, false>(PJ, J, S.es[(ia ? ti : tj) * c.ntype + (ia ? tj : ti)], ia, r2, c.alpha, r, si.w, sj.w,
+                                mi, S.v[j], task_qq, task_qd, task_dd, wi, Sw[j], wi, 0, 0, dm, g);
     }
-    for (int o = 1; o < sub; o <<= 1)
 #pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        H[d] += __shfl_xor_sync(FULL_MASK, H[d], o);
-        K[d] += __shfl_xor_sync(FULL_MASK, K[d], o);
+    for (int d = 0; d < 3; ++d) dm[d] = warp_sum(dm[d]);
+    if (lane == 0) J.rhs[X.off + i] = make_double4(dm[0], dm[1], dm[2], 0.0);
+  }
+}
+
+// pair terms of the parameter gradient (warp per ion of this CTA), added to g.
+// S.es[ti * ntype + tj].thole: bit p, damping parameter p is the field on type ti by
+// charges of type tj; bit 16 + p, short-range parameter p is of the pair.
+template <int K>
+__device__ __noinline__ void badj_pairs(const BatchArgs& a, const AdjArgs& J, const PairAdj& PJ, const BCtx& X,
+                                        const BShared& S, const double4* Sw, bool any_sr, bool any_es,
+                                        double (&gout)[kFitMax]) {
+  const BConf& c = *X.c;
+  const int task_qq = (c.flags & BF_QQ) ? 1 : 0, task_qd = (c.flags & BF_QD) ? 1 : 0;
+  const int task_dd = (c.flags & BF_DD) ? 1 : 0, lbmhftd = (c.flags & BF_BMHFTD) ? 1 : 0;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+  double g[kFitMax];
+#pragma unroll
+  for (int p = 0; p < kFitMax; ++p) g[p] = 0.0;
+  for (int i = X.i0 + warp; i < X.i1; i += nwarp) {
+    const double4 si = S.s[i], mi = S.v[i], wi = Sw[i];
+    const int ti = btyp(S.t[i]);
+    if (any_sr) {
+      const unsigned short* row = bnbl(a, X, 1, i);
+      const int nn = __ldcg(bnbn(a, X, 1) + i);
+      int jn = lane < nn ? bnbr(row, lane) : 0;
+      for (int k = lane; k < nn; k += 32) {
+        const int j = jn;
+        if (k + 32 < nn) jn = bnbr(row, k + 32);
+        const int tp = ti * c.ntype + btyp(S.t[j]), h = (S.es[tp].thole >> 16) & 0xffff;
+        if (!h) continue;
+        double r[3];
+        const double r2 = pair_vec<double>(c.A, si, S.s[j], r[0], r[1], r[2]);
+        const NBPair& P = S.nb[tp];
+        if (r2 < P.rcutsq) sr_pair_adjoint(PJ, J, P, lbmhftd, h, r2, r, wi, g);
       }
-    if (act && me == 0) {
-      double o3[3];
-      for (int d = 0; d < 3; ++d)
-        o3[d] = kTwoPi * (c.B[3 * d] * (H[0] - K[0]) + c.B[3 * d + 1] * (H[1] - K[1]) +
-                          c.B[3 * d + 2] * (H[2] - K[2]));
-      outv[X.off + i] = make_double4(o3[0], o3[1], o3[2], 0.0);
+    }
+    const double4 li = ldcg4(J.lam + X.off + i);
+    const unsigned short* row = bnbl(a, X, 0, i);
+    const int nn = any_es ? __ldcg(bnbn(a, X, 0) + i) : 0;
+    int jn = lane < nn ? bnbr(row, lane) : 0;
+    for (int k = lane; k < nn; k += 32) {
+      const int j = jn;
+      if (k + 32 < nn) jn = bnbr(row, k + 32);
+      const int tj = btyp(S.t[j]);
+      const int hi = S.es[ti * c.ntype + tj].thole & 0xffff, hj = S.es[tj * c.ntype + ti].thole & 0xffff;
+      if (!PJ.qs && !hi && !hj) continue;
+      const double4 sj = S.s[j];
+      double r[3], dm[3];
+      const double r2 = pair_vec<double>(c.A, si, sj, r[0], r[1], r[2]);
+      if (r2 > c.rc2) continue;
+      const bool ia = half_mask(i, j);
+      es_pair_adjoint<K, true>(PJ, J, S.es[(ia ? ti : tj) * c.ntype + (ia ? tj : ti)], ia, r2, c.alpha, r, si.w, sj.w,
+                               mi, S.v[j], task_qq, task_qd, task_dd, wi, wi, li, hi, hj, dm, g);
     }
   }
+#pragma unroll
+  for (int p = 0; p < kFitMax; ++p) gout[p] += g[p];
 }
 
 // ---------------------------------------------------------------------------
 // adjoint of one configuration (the forward of the same positions has run:
-// a.s, a.tab64, a.x (induced dipoles), a.mu (total), a.E (field) are valid)
+// a.s, a.rec, a.x (induced dipoles), a.mu (total), a.E (field) are valid)
 __device__ void bconfig_adjoint(cgx::cluster_group& cl, const BatchArgs& a, const AdjArgs& J, BCtx& X,
                                 const BShared& S, double4* Sw) {
   const BConf& c = *X.c;
   const bool coul = (c.flags & BF_COUL) != 0, polar = (c.flags & BF_POLAR) != 0;
-  const int task_qq = (c.flags & BF_QQ) ? 1 : 0, task_qd = (c.flags & BF_QD) ? 1 : 0;
-  const int task_dd = (c.flags & BF_DD) ? 1 : 0;
+  const int task_qq = (c.flags & BF_QQ) ? 1 : 0;
+  const bool tt4 = (c.flags & BF_TT4) != 0;
   const double cu = c.coul_unit;
   const double gU = J.gE[X.cfg];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
   PairAdj PJ;
-  PJ.prm = J.prm;
   PJ.nparam = J.nparam;
-  PJ.qscale = J.qscale;
   PJ.gU = gU;
   PJ.cu = cu;
+  PJ.rs = 1.0 / J.qscale;
+  PJ.qs = 0;
+  bool any_sr = false, any_es = false;
+  for (int p = 0; p < J.nparam; ++p) {
+    if (J.prm[p].kind <= FIT_C) any_sr = true;
+    if (J.prm[p].kind >= FIT_TTB) any_es = true;
+    if (J.prm[p].kind == FIT_QSCALE) PJ.qs |= 1 << p;
+  }
+  any_sr = any_sr && (c.flags & BF_SR) && (c.flags & BF_BMH);
+  any_es = any_es && coul;
   // ---- load -------------------------------------------------------------
   for (int i = X.i0 + threadIdx.x; i < X.i1; i += blockDim.x) {
     int gi = X.off + i;
@@ -418,6 +409,15 @@ __device__ void bconfig_adjoint(cgx::cluster_group& cl, const BatchArgs& a, cons
   for (int k = threadIdx.x; k < c.ntype * c.ntype; k += blockDim.x) {
     S.nb[k] = a.nbtab[c.nb_off + k];
     S.es[k] = a.estab[c.es_off + k];
+    const int ti = k / c.ntype, tj = k % c.ntype;
+    int h = 0;
+    for (int p = 0; p < J.nparam; ++p) {
+      const FitParam& fp = J.prm[p];
+      const bool ord = ti == fp.t1 && tj == fp.t2, rev = ti == fp.t2 && tj == fp.t1;
+      if ((fp.kind == FIT_TTB || fp.kind == FIT_TTC) && ord) h |= 1 << p;
+      if (fp.kind <= FIT_C && (ord || rev)) h |= 1 << (16 + p);
+    }
+    S.es[k].thole = h;  // (fits have no Thole functions)
   }
   cl.sync();
   for (int i = threadIdx.x; i < X.n; i += blockDim.x) {
@@ -438,55 +438,32 @@ __device__ void bconfig_adjoint(cgx::cluster_group& cl, const BatchArgs& a, cons
   double rmsd = 0.0, tol = 0.0;
   if (coul && polar) {
     // ---- right-hand side: g_U cu R + d(u_F.F)/dmu + u_mu ---------------------
-    for (int i = X.i0 + warp; i < X.i1; i += nwarp) {
-      int gi = X.off + i;
-      double dm[3] = {0, 0, 0};
-      if (a.ipol[gi]) {
-        double4 si = S.s[i];
-        int ti = btyp(S.t[i]);
-        double4 mui = S.v[i], wi4 = Sw[i];
-        const unsigned short* row = bnbl(a, X, 0, i);
-        const int nn = bnbn(a, X, 0)[i];
-        for (int k = lane; k < nn; k += 32) {
-          const int j = bnbr(row, k);
-          double4 sj = S.s[j];
-          double rxd, ryd, rzd;
-          double r2d = min_image_exact(c.A, xsub(si.x, sj.x), xsub(si.y, sj.y), xsub(si.z, sj.z),
-                                       rxd, ryd, rzd);
-          if (r2d > c.rc2) continue;
-          int tj = btyp(S.t[j]);
-          double4 muj = S.v[j], wj4 = Sw[j];
-          bool ia = half_mask(i, j);
-          double sg = ia ? 1.0 : -1.0;
-          double r[3] = {sg * rxd, sg * ryd, sg * rzd};
-          double4 ma4 = ia ? mui : muj, mb4 = ia ? muj : mui, wa4 = ia ? wi4 : wj4, wb4 = ia ? wj4 : wi4;
-          double ma[3] = {ma4.x, ma4.y, ma4.z}, mb[3] = {mb4.x, mb4.y, mb4.z};
-          double wa[3] = {wa4.x, wa4.y, wa4.z}, wb[3] = {wb4.x, wb4.y, wb4.z};
-          double zero[3] = {0, 0, 0}, d3[3];
-          int ta = ia ? ti : tj, tb = ia ? tj : ti;
-          es_pair_adjoint(PJ, S.es[ta * c.ntype + tb], ta, tb, r2d, c.alpha, r, ia ? si.w : sj.w,
-                          ia ? sj.w : si.w, ma, mb, ma4.x != 0.0 || ma4.y != 0.0 || ma4.z != 0.0,
-                          mb4.x != 0.0 || mb4.y != 0.0 || mb4.z != 0.0, task_qq, task_qd, task_dd,
-                          wa, wb, zero, ia, d3, nullptr);
-          for (int d = 0; d < 3; ++d) dm[d] += d3[d];
-        }
+    if (tt4) badj_rhs<4>(a, J, PJ, X, S, Sw);
+    else badj_rhs<0>(a, J, PJ, X, S, Sw);
+    // reciprocal: rho = sum (q + i k.mu) P and i sigma = i sum (k.u)(q + i k.mu) P;
+    // sum_k A n [ (k.w) Re(rho P*) - Re(sigma P*) ] is the dipole force of rho on
+    // the vectors w plus the field sum of i sigma (bfld_get's fm and e)
+    for (int ch = 0; ch < 2 && c.nk > 0; ++ch) {
+      BRecArgs r;
+      badj_rho(cl, a, X, S, Sw, task_qq != 0, true, ch == 1, ch == 1, r);
+      r.wd = BWeights{X.c, S.s, Sw, S.v32, X.i0, 0, false, true};
+      const int RS = ch == 0 ? bfld<true>(r) : bfld<false>(r);
+      for (int i = X.i0 + threadIdx.x; i < X.i1; i += blockDim.x) {
+        double e[3], fm[3];
+        bfld_get(a, c, RS, i - X.i0, ch == 0, e, fm);
+        const double4 o = J.lam[X.off + i];  // lam as scratch
+        J.lam[X.off + i] = ch == 0 ? make_double4(fm[0], fm[1], fm[2], 0.0)
+                                   : make_double4(o.x + e[0], o.y + e[1], o.z + e[2], 0.0);
       }
-      for (int d = 0; d < 3; ++d) dm[d] = warp_sum(dm[d]);
-      if (lane == 0) J.rhs[gi] = make_double4(dm[0], dm[1], dm[2], 0.0);
+      __syncthreads();
     }
-    // reciprocal: rho = sum (q + i k.mu) P and sigma = sum (k.u)(q + i k.mu) P
-    bsf(cl, a, X, S, Sw, task_qq != 0, true, false, J.rq);
-    bsf(cl, a, X, S, Sw, task_qq != 0, true, true, J.sq);
-    __syncthreads();
-    brecsum(a, X, S, Sw, J.rq, J.sq, J.lam);  // lam as scratch
-    __syncthreads();
-    const double scale8 = 2.0 * (2.0 * (kTwoPi / c.omega));
+    cl.sync();  // every CTA's rows of rhs
     double v1[1] = {0.0};
     for (int i = X.i0 + threadIdx.x; i < X.i1; i += blockDim.x) {
       int gi = X.off + i;
       double4 o = make_double4(0, 0, 0, 0);
       if (a.ipol[gi]) {
-        double4 rr = J.rhs[gi], rc = J.lam[gi];
+        double4 rr = ldcg4(J.rhs + gi), rc = c.nk > 0 ? J.lam[gi] : make_double4(0, 0, 0, 0);
         double4 ax = bmat3(a.inv + 9 * (size_t)gi, ldcg4(a.x + gi));
         double4 E = ldcg4(a.E + gi);
         double R[3] = {ax.x - E.x, ax.y - E.y, ax.z - E.z};
@@ -496,9 +473,9 @@ __device__ void bconfig_adjoint(cgx::cluster_group& cl, const BatchArgs& a, cons
           gm[1] = J.gmu[3 * (size_t)gi + 1];
           gm[2] = J.gmu[3 * (size_t)gi + 2];
         }
-        o.x = rr.x + cu * scale8 * rc.x + gU * cu * R[0] + gm[0];
-        o.y = rr.y + cu * scale8 * rc.y + gU * cu * R[1] + gm[1];
-        o.z = rr.z + cu * scale8 * rc.z + gU * cu * R[2] + gm[2];
+        o.x = rr.x + cu * rc.x + gU * cu * R[0] + gm[0];
+        o.y = rr.y + cu * rc.y + gU * cu * R[1] + gm[1];
+        o.z = rr.z + cu * rc.z + gU * cu * R[2] + gm[2];
         v1[0] += o.x * o.x + o.y * o.y + o.z * o.z;
       }
       J.rhs[gi] = o;
@@ -519,60 +496,8 @@ __device__ void bconfig_adjoint(cgx::cluster_group& cl, const BatchArgs& a, cons
     for (int i = X.i0 + threadIdx.x; i < X.i1; i += blockDim.x) J.lam[X.off + i] = make_double4(0, 0, 0, 0);
   }
   // ---- parameter gradient ----------------------------------------------------
-  bool any_sr = false, any_es = false;
-  for (int p = 0; p < J.nparam; ++p) {
-    if (J.prm[p].kind <= FIT_C) any_sr = true;
-    if (J.prm[p].kind >= FIT_TTB) any_es = true;
-  }
-  any_sr = any_sr && (c.flags & BF_SR) && (c.flags & BF_BMH);
-  any_es = any_es && coul;
-  const int lbmhftd = (c.flags & BF_BMHFTD) ? 1 : 0;
-  for (int i = X.i0 + warp; i < X.i1; i += nwarp) {
-    int gi = X.off + i;
-    double4 si = S.s[i];
-    int ti = btyp(S.t[i]);
-    double4 mui = S.v[i], wi4 = Sw[i];
-    double4 li4 = ldcg4(J.lam + gi);
-    double wi[3] = {wi4.x, wi4.y, wi4.z}, li[3] = {li4.x, li4.y, li4.z};
-    if (any_sr) {
-      const unsigned short* row = bnbl(a, X, 1, i);
-      const int nn = bnbn(a, X, 1)[i];
-      for (int k = lane; k < nn; k += 32) {
-        const int j = bnbr(row, k);
-        double4 sj = S.s[j];
-        double r[3];
-        double r2d = min_image_exact(c.A, xsub(si.x, sj.x), xsub(si.y, sj.y), xsub(si.z, sj.z), r[0],
-                                     r[1], r[2]);
-        int tj = btyp(S.t[j]);
-        const NBPair& P = S.nb[ti * c.ntype + tj];
-        if (r2d < P.rcutsq) sr_pair_adjoint(PJ, P, lbmhftd, ti, tj, r2d, r, wi, g);
-      }
-    }
-    const unsigned short* row = bnbl(a, X, 0, i);
-    const int nn = any_es ? bnbn(a, X, 0)[i] : 0;
-    for (int k = lane; k < nn; k += 32) {
-      const int j = bnbr(row, k);
-      double4 sj = S.s[j];
-      double rxd, ryd, rzd;
-      double r2d = min_image_exact(c.A, xsub(si.x, sj.x), xsub(si.y, sj.y), xsub(si.z, sj.z), rxd,
-                                   ryd, rzd);
-      if (r2d > c.rc2) continue;
-      int tj = btyp(S.t[j]);
-      double4 muj = S.v[j], wj4 = Sw[j];
-      bool ia = half_mask(i, j);
-      double sg = ia ? 1.0 : -1.0;
-      double r[3] = {sg * rxd, sg * ryd, sg * rzd};
-      double4 ma4 = ia ? mui : muj, mb4 = ia ? muj : mui, wa4 = ia ? wi4 : wj4, wb4 = ia ? wj4 : wi4;
-      double ma[3] = {ma4.x, ma4.y, ma4.z}, mb[3] = {mb4.x, mb4.y, mb4.z};
-      double wa[3] = {wa4.x, wa4.y, wa4.z}, wb[3] = {wb4.x, wb4.y, wb4.z};
-      double d3[3];
-      int ta = ia ? ti : tj, tb = ia ? tj : ti;
-      es_pair_adjoint(PJ, S.es[ta * c.ntype + tb], ta, tb, r2d, c.alpha, r, ia ? si.w : sj.w,
-                      ia ? sj.w : si.w, ma, mb, ma4.x != 0.0 || ma4.y != 0.0 || ma4.z != 0.0,
-                      mb4.x != 0.0 || mb4.y != 0.0 || mb4.z != 0.0, task_qq, task_qd, task_dd,
-                      wa, wb, li, ia, d3, g);
-    }
-  }
+  if (tt4) badj_pairs<4>(a, J, PJ, X, S, Sw, any_sr, any_es, g);
+  else badj_pairs<0>(a, J, PJ, X, S, Sw, any_sr, any_es, g);
   // per-ion terms: polarisability, self energy of the charges
   const double selfa = c.alpha / sqrt(kPi);
   for (int i = X.i0 + threadIdx.x; i < X.i1; i += blockDim.x) {
@@ -593,18 +518,19 @@ __device__ void bconfig_adjoint(cgx::cluster_group& cl, const BatchArgs& a, cons
     }
   }
   // reciprocal charge-scale terms: rho_lambda, then per k over this CTA's rows
-  bool has_s = false;
-  for (int p = 0; p < J.nparam; ++p) has_s = has_s || J.prm[p].kind == FIT_QSCALE;
-  if (has_s && coul && task_qq && c.nk > 0) {
+  if (PJ.qs && coul && task_qq && c.nk > 0) {
     // channels: rq = rho_q, rm = rho_mu, sq = sigma_q, sm = sigma_mu, rl = rho_lambda
-    bsf(cl, a, X, S, Sw, true, false, false, J.rq);
-    bsf(cl, a, X, S, Sw, false, true, false, J.rm);
-    bsf(cl, a, X, S, Sw, true, false, true, J.sq);
-    bsf(cl, a, X, S, Sw, false, true, true, J.sm);
-    cl.sync();
-    for (int i = threadIdx.x; i < X.n; i += blockDim.x) S.v[i] = ldcg4(J.lam + X.off + i);
+    for (int ch = 0; ch < 5; ++ch) {
+      if (ch == 4) {  // (S.v = mu until here; every CTA's lambda is visible)
+        __syncthreads();
+        for (int i = threadIdx.x; i < X.n; i += blockDim.x) S.v[i] = ldcg4(J.lam + X.off + i);
+        __syncthreads();
+      }
+      BRecArgs r;
+      badj_rho(cl, a, X, S, Sw, ch == 0 || ch == 2, ch != 0 && ch != 2, ch == 2 || ch == 3, false, r);
+      badj_store(a, X, r, ch == 0 ? J.rq : ch == 1 ? J.rm : ch == 2 ? J.sq : ch == 3 ? J.sm : J.rl);
+    }
     __syncthreads();
-    bsf(cl, a, X, S, Sw, false, true, false, J.rl);
     const double fpi_V = 2.0 * (kTwoPi / c.omega), epi_V = 2.0 * fpi_V;
     double acc = 0.0;
     int r0 = (int)((long long)c.nrows * X.rank / X.C), r1 = (int)((long long)c.nrows * (X.rank + 1) / X.C);
@@ -636,10 +562,15 @@ __device__ void bconfig_adjoint(cgx::cluster_group& cl, const BatchArgs& a, cons
   }
 }
 
-__global__ void __launch_bounds__(512) k_batch_adjoint(BatchArgs a, AdjArgs J, int nmax) {
+__global__ void __launch_bounds__(512) k_batch_adjoint(const __grid_constant__ BatchArgs a,
+                                                       const __grid_constant__ AdjArgs J, int nmax) {
   extern __shared__ __align__(16) unsigned char bsm[];
   BShared S = batch_smem(bsm, nmax);
   double4* Sw = reinterpret_cast<double4*>(bsm + batch_smem_extra_offset(nmax));
+  if (a.stage_extra) {
+    S.stage = reinterpret_cast<unsigned char*>(Sw + nmax);
+    S.stage_bytes = a.stage_extra;
+  }
   cgx::cluster_group cl = cgx::this_cluster();
   BCtx X;
   X.rank = (int)cl.block_rank();

@@ -58,7 +58,6 @@ struct mdff_batch {
   double4* d_kvec = nullptr;
   double4 *d_s = nullptr, *d_Estat = nullptr, *d_x = nullptr, *d_r = nullptr, *d_z = nullptr,
           *d_p = nullptr, *d_mu = nullptr, *d_E = nullptr;
-  double2* d_tab64 = nullptr;
   double2* d_apm = nullptr;
   // phase records and the workspaces of the resident CTAs (BatchArgs)
   unsigned char* d_rec = nullptr;
@@ -95,6 +94,7 @@ struct mdff_batch {
   double *d_grad = nullptr, *d_info = nullptr, *d_gin = nullptr;
   long long ktot = 0;
   double ms_adjoint = 0.0;
+  int adj_cluster = 2;  // CTAs per cluster of the adjoint
 };
 
 namespace {
@@ -168,7 +168,6 @@ BatchArgs make_args(mdff_batch* h, const double* d_pos, double* d_force) {
   a.Ak = h->d_Ak;
   a.kvec = h->d_kvec;
   a.s = h->d_s;
-  a.tab64 = h->d_tab64;
   a.apm = h->d_apm;
   a.stage_extra = h->stage_extra;
   a.rec = h->d_rec;
@@ -495,7 +494,7 @@ int create_impl(mdff_batch* h, const mdff_params* psets, int npsets, const mdff_
   std::vector<ESPair> es;
   std::vector<int4> rows;
   std::vector<BoxCost> cost(h->nconf);
-  long long tab_total = 0, rec_total = 0;
+  long long rec_total = 0;
   long long ktot = 0;
   int ntot = 0;
   h->conf.resize(h->nconf);
@@ -620,15 +619,11 @@ int create_impl(mdff_batch* h, const mdff_params* psets, int npsets, const mdff_
       B.kx = P.kES[0];
       B.ky = P.kES[1];
       B.kz = P.kES[2];
-      B.ntab = P.kES[0] + 1 + P.kES[1] + 1 + std::max(P.kES[2], 4) + 1;
-      B.tab_off = tab_total;
-      B.tab_ld = (int)n;
-      // (boxes start on a 128-byte line: a line of one box is never read
-      // while another box's cluster writes it)
-      tab_total += ((long long)B.ntab * n + 15) / 16 * 16;
       const int nz = B.kz + 1, nxy = B.kx + 1 + B.ky + 1;
       B.zo = nxy * 16;
       B.rs = brec_bytes(B.kx, B.ky, B.kz);
+      // (boxes start on a 128-byte line: a line of one box is never read
+      // while another box's cluster writes it)
       B.rec = rec_total;
       rec_total += ((long long)B.rs * n + 127) / 128 * 128;
       B.apm_off = (int)apm.size();
@@ -664,6 +659,10 @@ int create_impl(mdff_batch* h, const mdff_params* psets, int npsets, const mdff_
     int nsm = 148;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
     h->shape = default_shape(cost, h->order, nsm);
+    // an adjoint solves to 1e-12 and has five more structure factors: 64 boxes of
+    // 216-512 ions (avg) 0.72 ms + 3.3 ms / C, forward 0.4 + 1.1 / C
+    for (BoxCost& b : cost) b = BoxCost{1.8 * b.fixed, 3.0 * b.par};
+    h->adj_cluster = default_shape(cost, h->order, nsm).cluster;
   }
   BCK(cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking));
   BCK(cudaEventCreate(&h->ev0));
@@ -692,7 +691,6 @@ int create_impl(mdff_batch* h, const mdff_params* psets, int npsets, const mdff_
   BALLOC(h->d_p, ntot);
   BALLOC(h->d_mu, ntot);
   BALLOC(h->d_E, ntot);
-  BALLOC(h->d_tab64, (size_t)std::max<long long>(tab_total, 1));
   BALLOC(h->d_rec, (size_t)std::max<long long>(rec_total, 1));
   BALLOC(h->d_force, 3 * (size_t)ntot);
   BALLOC(h->d_pack, 3 * (size_t)ntot);
@@ -784,7 +782,7 @@ void destroy_impl(mdff_batch* h) {
   void* bufs[] = {h->d_conf, h->d_order, h->d_queue, h->d_typ, h->d_ipol, h->d_pos, h->d_q,
                   h->d_pol, h->d_inv, h->d_dip, h->d_nb, h->d_es, h->d_rows, h->d_Ak, h->d_kvec,
                   h->d_s, h->d_Estat, h->d_x, h->d_r, h->d_z, h->d_p, h->d_mu, h->d_E,
-                  h->d_tab64, h->d_apm, h->d_rec, h->d_ws, h->d_force, h->d_part, h->d_out, h->d_pack,
+                  h->d_apm, h->d_rec, h->d_ws, h->d_force, h->d_part, h->d_out, h->d_pack,
                   h->d_w, h->d_rhs, h->d_lam, h->d_ch, h->d_grad, h->d_info, h->d_gin};
   for (void* b : bufs)
     if (b) cudaFree(b);
@@ -1055,16 +1053,11 @@ int mdff_gpu_batch_adjoint(mdff_batch_handle h, const double* gE, const double* 
   J.tol_rel = 1e-12;
   J.nparam = h->nparam;
   for (int k = 0; k < kFitMax; ++k) J.prm[k] = (k < h->nparam) ? h->prm[k] : FitParam{-1, 0, 0, 0};
-  // launch: persistent clusters of the forward's block size; the cluster is
-  // widened until the clusters of all configurations cover the SMs twice (a
-  // fitting batch of tens of boxes would otherwise leave most SMs idle)
-  Shape sh = h->shape;
-  {
-    int nsm = 0;
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
-    while (sh.cluster < kBMaxC && (long)h->nconf * sh.cluster < 2L * nsm) sh.cluster *= 2;
-  }
-  size_t smem = batch_smem_extra_offset(h->nmax) + sizeof(double4) * h->nmax;
+  // launch: persistent clusters of the forward's block size, the cluster from
+  // the schedule of the adjoint's own box costs
+  const Shape sh{h->adj_cluster, h->shape.threads};
+  int extra = 0;
+  const size_t smem = smem_with_stage(h, batch_smem_extra_offset(h->nmax) + sizeof(double4) * h->nmax, sh.threads, &extra);
   if (smem > 227 * 1024) {
     h->err = "configurations too large for the adjoint's shared-memory layout";
     return MDFF_ERR_BAD_ARGS;
@@ -1094,7 +1087,7 @@ int mdff_gpu_batch_adjoint(mdff_batch_handle h, const double* gE, const double* 
   }
   cfg.gridDim = dim3(sh.cluster * ncl);
   cfg.stream = h->st;
-  h->stage_extra = 0;  // the adjoint stages in the layout's own buffer
+  h->stage_extra = extra;
   BatchArgs a = make_args(h, h->graph_pos, h->graph_force);
   BCK(cudaMemsetAsync(h->d_queue, 0, sizeof(int), h->st));
   BCK(cudaEventRecord(h->ev0, h->st));

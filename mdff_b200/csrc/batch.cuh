@@ -50,7 +50,6 @@ namespace cgx = cooperative_groups;
 constexpr int kBMaxT = 4;          // types of a batched configuration
 constexpr int kBPart = 16;         // values per CTA partial slot
 constexpr int kBKChunk = 1024;     // double2 of the staging buffer (kBStage bytes)
-constexpr int kBNZ = 8;            // nz per work item of the adjoint's structure factors
 constexpr int kBMaxC = 8;          // largest cluster
 constexpr int kBSlots = 48;        // per-configuration scalar slots
 
@@ -77,9 +76,7 @@ enum {
 struct BConf {
   int off, n, ntype, flags;
   int nk, nrows, row_off, k_off;
-  int kx, ky, kz, ntab;
-  long long tab_off;
-  int tab_ld;            // leading dimension of the tables (= n)
+  int kx, ky, kz;
   int trunc, maxit, npol;
   int nb_off, es_off, pad0, pad1;
   double A[9], B[9], omega;
@@ -113,7 +110,6 @@ struct BatchArgs {
   const double4* kvec;
   const double2* apm;    // (A(+n), A(-n)) by (row, n), per configuration at apm_off
   double4* s;            // [ntot] direct coordinates, w = q
-  double2* tab64;        // phase tables, [entry][ion] per configuration
   unsigned char* rec;    // phase records of every configuration
   // workspace of the resident CTAs (blockIdx.x) and clusters (blockIdx.x / C)
   double4* rpart;        // [CTA][2][rpart_ld] structure-factor partials
@@ -248,25 +244,6 @@ __device__ inline void gather_pol32(const BCtx& X, const int* t, const double4* 
   }
 }
 
-// phase tables of the adjoint's sums
-__device__ __forceinline__ double2 btab(const BatchArgs& a, const BConf& c, int e, int i) {
-  return a.tab64[c.tab_off + (long long)e * c.tab_ld + i];
-}
-// X_nx Y_ny Z_nz of ion i (negative indices by conjugation)
-__device__ __forceinline__ double2 bphase_z(const BatchArgs& a, const BConf& c, int i, double2 XY, int nz) {
-  int az = nz < 0 ? -nz : nz;
-  double2 Z = btab(a, c, c.kx + 1 + c.ky + 1 + az, i);
-  if (nz < 0) Z = cconj(Z);
-  return cmul(XY, Z);
-}
-__device__ __forceinline__ double2 bphase(const BatchArgs& a, const BConf& c, int i, int nx, int ny, int nz) {
-  double2 X = btab(a, c, nx, i);
-  int ay = ny < 0 ? -ny : ny;
-  double2 Y = btab(a, c, c.kx + 1 + ay, i);
-  if (ny < 0) Y = cconj(Y);
-  return bphase_z(a, c, i, cmul(X, Y), nz);
-}
-
 // m = 2 pi B^T mu (so that k.mu = n.m)
 __device__ __forceinline__ double3 bmvec(const BConf& c, double mx, double my, double mz) {
   return make_double3(kTwoPi * (c.B[0] * mx + c.B[3] * my + c.B[6] * mz),
@@ -317,6 +294,7 @@ struct BRecArgs {
   const double4* w;      // weights of src
   unsigned char* buf;    // two buffers of CH records
   int CH;
+  bool rot;              // (brho of kind 2) the sums times i
   double4* out;          // this CTA's partials
   const double4* part;   // rank 0's partials
   size_t pld;
@@ -328,12 +306,12 @@ struct BRecArgs {
   BWeights wd;           // dipole weights of dst
 };
 
-template <int NT, bool HM>
+template <int NT, int HM>
 __device__ __noinline__ void brho_n(const BRecArgs& r) {
   const BConf& c = *r.c;
-  brho_t<NT, HM>(r.rec, c.rs, c.zo, c.kx, c.kz, r.rows, c.nrows, r.src, r.t, r.w, r.buf, r.CH, r.out);
+  brho_t<NT, HM>(r.rec, c.rs, c.zo, c.kx, c.kz, r.rows, c.nrows, r.src, r.t, r.w, r.buf, r.CH, r.out, r.rot);
 }
-template <bool HM>
+template <int HM>
 __device__ __forceinline__ void brho(const BRecArgs& r) {
   switch (r.c->kz / 4) {
     case 0: brho_n<1, HM>(r); break;
@@ -359,17 +337,9 @@ __device__ __forceinline__ int bfld(const BRecArgs& r) {
   }
 }
 
-// Reciprocal pass of one configuration.  mode 0: the weights of all of this
-// CTA's ions with charges and / or the dipoles in S.v; 1 / 2: of its
-// polarisable ions with the vector in S.v / S.v32 by rank.  The field sums are
-// left in this CTA's gpart for all its ions or (dst_pol) its polarisable ones;
-// bfld_get reads them.  With do_str, es[0..6] receives this CTA's share of
-// (u_rec, tau_rec) scaled as k_rec_energy.  Returns the number of row subsets.
-__device__ __noinline__ int brec(cgx::cluster_group& cl, const BatchArgs& a, BCtx& X, const BShared& S, int mode,
-                                 bool has_q, bool has_mu, bool dst_pol, bool muf, bool do_str, double (&es)[7]) {
+// set-up of a pass: ions, workspaces (mode, dst_pol as brec)
+__device__ __forceinline__ BRecArgs brec_args(const BatchArgs& a, BCtx& X, const BShared& S, int mode, bool dst_pol) {
   const BConf& c = *X.c;
-  for (int k = 0; k < 7; ++k) es[k] = 0.0;
-  if (c.nk == 0) return 0;
   BRecArgs r;
   r.c = X.c;
   r.rows = a.rows + c.row_off;
@@ -384,21 +354,44 @@ __device__ __noinline__ int brec(cgx::cluster_group& cl, const BatchArgs& a, BCt
   r.part = a.rpart + ((size_t)(blockIdx.x - X.rank) * 2 + X.rpar) * a.rpart_ld;
   r.out = a.rpart + ((size_t)blockIdx.x * 2 + X.rpar) * a.rpart_ld;
   X.rpar ^= 1;
+  r.rot = false;
   r.C = X.C;
   r.stage = S.stage;
   r.stage_bytes = S.stage_bytes;
   r.gp = a.gpart + (size_t)blockIdx.x * kBSplit * 6 * a.wn;
   r.gld = a.wn;
   r.wd = BWeights{X.c, S.s, S.v, S.v32, r.dst.n0, 0, false, true};
+  return r;
+}
+// room for nw weights per ion (in the staging buffer, else in the field's
+// scratch); the rest of the buffer holds the records in passing
+__device__ __forceinline__ double4* brec_weights(BRecArgs& r, const BShared& S, int nw) {
+  const int bytes = r.src.cnt * 32 * nw;
+  const bool in_stage = bytes <= S.stage_bytes / 3;
+  double4* w = in_stage ? reinterpret_cast<double4*>(S.stage) : reinterpret_cast<double4*>(r.gp);
+  r.buf = S.stage + (in_stage ? (bytes + 127) / 128 * 128 : 0);
+  const int ch = (int)((S.stage + S.stage_bytes - r.buf) / (2 * r.c->rs)) & ~3;
+  r.CH = ch < 32 ? ch : 32;
+  r.w = w;
+  return w;
+}
+
+// Reciprocal pass of one configuration.  mode 0: the weights of all of this
+// CTA's ions with charges and / or the dipoles in S.v; 1 / 2: of its
+// polarisable ions with the vector in S.v / S.v32 by rank.  The field sums are
+// left in this CTA's gpart for all its ions or (dst_pol) its polarisable ones;
+// bfld_get reads them.  With do_str, es[0..6] receives this CTA's share of
+// (u_rec, tau_rec) scaled as k_rec_energy.  Returns the number of row subsets.
+__device__ __noinline__ int brec(cgx::cluster_group& cl, const BatchArgs& a, BCtx& X, const BShared& S, int mode,
+                                 bool has_q, bool has_mu, bool dst_pol, bool muf, bool do_str, double (&es)[7]) {
+  const BConf& c = *X.c;
+  for (int k = 0; k < 7; ++k) es[k] = 0.0;
+  if (c.nk == 0) return 0;
+  BRecArgs r = brec_args(a, X, S, mode, dst_pol);
   {
     // weights once per ion: in the staging buffer, else in the field's scratch
     const BWeights ws{X.c, S.s, S.v, S.v32, r.src.n0, mode, has_q, has_mu};
-    // (the rest of the buffer holds the records in passing)
-    const bool in_stage = r.src.cnt * 32 <= S.stage_bytes / 3;
-    double4* w = in_stage ? reinterpret_cast<double4*>(S.stage) : reinterpret_cast<double4*>(r.gp);
-    r.buf = S.stage + (in_stage ? (r.src.cnt * 32 + 127) / 128 * 128 : 0);
-    const int ch = (int)((S.stage + S.stage_bytes - r.buf) / (2 * c.rs)) & ~3;
-    r.CH = ch < 32 ? ch : 32;
+    double4* w = brec_weights(r, S, 1);
     __syncthreads();
     for (int k = threadIdx.x; k < r.src.cnt; k += blockDim.x) {
       double v[4];
@@ -406,10 +399,9 @@ __device__ __noinline__ int brec(cgx::cluster_group& cl, const BatchArgs& a, BCt
       w[k] = make_double4(v[0], v[1], v[2], v[3]);
     }
     __syncthreads();
-    r.w = w;
   }
-  if (has_mu) brho<true>(r);
-  else brho<false>(r);
+  if (has_mu) brho<1>(r);
+  else brho<0>(r);
   cl.sync();
   if (do_str) {
     // energy and stress of this CTA's share of the rows
@@ -1118,19 +1110,17 @@ __device__ void bconfig(cgx::cluster_group& cl, const BatchArgs& a, BCtx& X, con
     if (coul && c.nk > 0) {
       // e^{2 pi i n s}, s wrapped to [-0.5, 0.5) (k_rec_tables)
       double sv[3] = {sx, sy, sz};
-      int km[3] = {c.kx, c.ky, c.ntab - (c.kx + 1) - (c.ky + 1) - 1};
+      const int km[3] = {c.kx, c.ky, c.kz};
       int e0 = 0;
       for (int d = 0; d < 3; ++d) {
         double w = sv[d] - rint(sv[d]);
         for (int m = 0; m <= km[d]; ++m) {
           double sn, cs;
           sincospi(2.0 * (double)m * w, &sn, &cs);
-          long long o = c.tab_off + (long long)(e0 + m) * c.tab_ld + i;
-          a.tab64[o] = make_double2(cs, sn);
           // (entries of n > kz stay zero)
           unsigned char* rp = a.rec + c.rec + (size_t)i * c.rs;
           if (d < 2) reinterpret_cast<double2*>(rp)[e0 + m] = make_double2(cs, sn);
-          else if (m <= c.kz) reinterpret_cast<double2*>(rp + c.zo)[m] = make_double2(cs, sn);
+          else reinterpret_cast<double2*>(rp + c.zo)[m] = make_double2(cs, sn);
         }
         e0 += km[d] + 1;
       }

@@ -77,11 +77,15 @@ __host__ __device__ inline int brec_bytes(int kx, int ky, int kz) {
 // + n] = (a1, a2).  w: weights (q, m1, m2, m3) of the list entries.  NT: tiles of
 // four n, covering kz + 1.  The records pass through shared memory (buf, two
 // buffers of CH records), every warp reading all of them.
-template <int NT, bool HM>
+// HM: 0 charges only, 1 charges and dipoles, 2 the product with a second vector u
+// (weights (., u1, u2, u3) at w + cnt): sum_i (k.u_i)(q_i + i k.m_i) P_i.  Its row weight
+// is a polynomial in n, alpha + n beta + n^2 gamma; gamma's share goes to U's
+// accumulator with n^2 (c_n, s_n) as operand.  rot: the sums times i.
+template <int NT, int HM>
 __device__ __forceinline__ void brho_t(const unsigned char* __restrict__ rec, int stride, int zoff, int kx,
                                        int kz, const int4* __restrict__ rows, int nrows, const BList& L,
                                        const int* t, const double4* w, unsigned char* buf, int CH,
-                                       double4* __restrict__ out) {
+                                       double4* __restrict__ out, bool rot = false) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int g = lane >> 2, tt = lane & 3;
   const int ng = (nrows + 7) / 8, nz = kz + 1;
@@ -136,6 +140,25 @@ __device__ __forceinline__ void brho_t(const unsigned char* __restrict__ rec, in
           double2 wa = wp[0], wb = wp[1];
           if (!ok) wa.x = wa.y = wb.x = wb.y = 0.0;
           const double2 P = cmul(X, Y);
+          if (HM == 2) {
+            const double2* up = wp + 2 * (size_t)L.cnt;
+            double2 ua = up[0], ub = up[1];
+            if (!ok) ua.y = ub.x = ub.y = 0.0;
+            const double km = fx * wa.y + fy * wb.x, ku = fx * ua.y + fy * ub.x;
+            const double a0 = ku * wa.x, a1 = ku * km, b0 = wa.x * ub.y, b1 = km * ub.y + ku * wb.y, g1 = wb.y * ub.y;
+            const double Ur = a0 * P.x - a1 * P.y, Ui = a0 * P.y + a1 * P.x;
+            const double Vr = b0 * P.x - b1 * P.y, Vi = b0 * P.y + b1 * P.x;
+            const double Gr = -g1 * P.y, Gi = g1 * P.x;
+#pragma unroll
+            for (int s = 0; s < NT; ++s) {
+              const double b = reinterpret_cast<const double*>(rp + zoff)[8 * s + g];
+              const double fn = (double)(4 * s + (g >> 1));
+              dmma(u[s], Ur, Ui, b);
+              dmma(v[HM ? s : 0], Vr, Vi, b);
+              dmma(u[s], Gr, Gi, fn * fn * b);
+            }
+            continue;
+          }
           double Ur = wa.x * P.x, Ui = wa.x * P.y;
           if (HM) {
             const double km = fx * wa.y + fy * wb.x;
@@ -169,6 +192,7 @@ __device__ __forceinline__ void brho_t(const unsigned char* __restrict__ rec, in
           o.z += fn * V[0];
           o.w += fn * V[2];
         }
+        if (HM == 2 && rot) o = make_double4(-o.y, o.x, -o.w, o.z);
         out[(size_t)row * nz + n] = o;
       }
     }
