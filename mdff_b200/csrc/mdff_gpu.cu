@@ -459,6 +459,15 @@ static int field_dm_attr_k() {
     return 1;
   return 0;
 }
+#define FIELD_TC_SWITCH(kf, F) \
+  switch (kf) {                \
+    case 16: F(16) break;      \
+    case 24: F(24) break;      \
+    case 32: F(32) break;      \
+    case 40: F(40) break;      \
+    case 48: F(48) break;      \
+    default: F(64) break;      \
+  }
 #define FIELD_DM_SWITCH(KSV, CALL)  \
   switch (KSV) {                    \
     case 3: CALL(3); break;         \
@@ -590,20 +599,22 @@ static int build_mesh(mdff_ctx* h) {
     const char* env = std::getenv("MDFF_FIELD_TC");
     int kf = field_tc_kf(h->p.kES[2]);
     h->field_tc = kf > 0 && nrows > 0 && !(env && env[0] == '0') &&
-                  field_tc_smem(kf, h->p.kES[1]) <= 227 * 1024;
+                  field_tc_smem(kf <= 32 ? 32 : 64, h->p.kES[1]) <= 227 * 1024;
     cudaFree(h->d_fb);
     h->d_fb = nullptr;
     if (h->field_tc) {
       // B tiles for the smaller row tile (with dipole forces): hi + lo per tile
       DALLOC(h->d_fb, (size_t)cdiv(nrows, field_tc_rpt(true)) * 2 * 128 * kf);
       int smem = (int)field_tc_smem(kf, h->p.kES[1]);
-      if (kf == 32) {
-        CK(cudaFuncSetAttribute(k_rec_field_tc<true, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        CK(cudaFuncSetAttribute(k_rec_field_tc<false, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-      } else {
-        CK(cudaFuncSetAttribute(k_rec_field_tc<true, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        CK(cudaFuncSetAttribute(k_rec_field_tc<false, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-      }
+      cudaError_t e = cudaSuccess;
+#define FTA(KF)                                                                                                     \
+  {                                                                                                                 \
+    e = cudaFuncSetAttribute(k_rec_field_tc<true, KF>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);          \
+    if (!e) e = cudaFuncSetAttribute(k_rec_field_tc<false, KF>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); \
+  }
+      FIELD_TC_SWITCH(kf, FTA)
+#undef FTA
+      CK(e);
     }
   }
   DALLOC(h->d_rhoA, std::max(nk, 1));
@@ -905,9 +916,20 @@ static int launch_field_tc_k(mdff_ctx* h, const RecMesh& M, int n, bool muf, int
   int ntile = cdiv(M.nrows, rpt);
   int ion_tiles = cdiv(nion, 128);
   int nalloc = (int)h->rchunk.size() - 1;
-  int ng = std::max(1, std::min({(2 * (h->nsm > 0 ? h->nsm : 148)) / std::max(ion_tiles, 1), ntile, nalloc}));
-  int tpg = cdiv(ntile, ng);
-  ng = cdiv(ntile, tpg);
+  // groups of row tiles: one CTA per SM, waves x (start-up of about two tiles + the
+  // group's tiles) shortest
+  const int nsm = h->nsm > 0 ? h->nsm : 148;
+  int tpg = ntile;
+  long best = 0;
+  for (int g = 1; g <= std::min(ntile, nalloc); ++g) {
+    const int t = cdiv(ntile, g);
+    const long cost = (long)cdiv((long)ion_tiles * cdiv(ntile, t), nsm) * (2 + t);
+    if (g == 1 || cost < best) {
+      best = cost;
+      tpg = t;
+    }
+  }
+  const int ng = cdiv(ntile, tpg);
   dim3 g((unsigned)ion_tiles, (unsigned)ng);
   size_t smem = field_tc_smem(KF, M.kmax[1]);
   size_t bsmem = (size_t)kBtRows * (2 * M.kmax[2] + 1) * sizeof(double2);
@@ -933,8 +955,11 @@ static int launch_field_tc_k(mdff_ctx* h, const RecMesh& M, int n, bool muf, int
 
 static int launch_field_tc(mdff_ctx* h, const RecMesh& M, int n, bool muf, int npart, const int* imap,
                            int nion, double2* rho_out) {
-  if (field_tc_kf(M.kmax[2]) == 32) return launch_field_tc_k<32>(h, M, n, muf, npart, imap, nion, rho_out);
-  return launch_field_tc_k<64>(h, M, n, muf, npart, imap, nion, rho_out);
+  int ng = 0;
+#define FTK(KF) ng = launch_field_tc_k<KF>(h, M, n, muf, npart, imap, nion, rho_out);
+  FIELD_TC_SWITCH(field_tc_kf(M.kmax[2]), FTK)
+#undef FTK
+  return ng;
 }
 
 // reciprocal pass: E += rec field (+ the self / surface field sf, when on);

@@ -232,10 +232,16 @@ static __global__ void __launch_bounds__(128) k_rec_rho(const typename cplx<R>::
 static __device__ __forceinline__ double2 rho_prime(const double2* __restrict__ part, int nchunk,
                                                     const double* __restrict__ Ak, int nk, int k) {
   double r = 0.0, im = 0.0;
-  for (int c = 0; c < nchunk; ++c) {
-    double2 v = part[(size_t)c * nk + k];
-    r += v.x;
-    im += v.y;
+  for (int c0 = 0; c0 < nchunk; c0 += 8) {  // (eight loads in flight)
+    double2 v[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+      v[c] = c0 + c < nchunk ? part[(size_t)(c0 + c) * nk + k] : make_double2(0.0, 0.0);
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      r += v[c].x;
+      im += v[c].y;
+    }
   }
   double A = Ak[k];
   return make_double2(A * r, A * im);

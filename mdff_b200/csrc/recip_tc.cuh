@@ -598,16 +598,28 @@ namespace mdff {
 // B tiles are built once per pass (k_rec_field_btiles, which also sums the
 // structure-factor chunks when no energy is needed).  The ions are all of them
 // or the subset imap (the polarisable ions, where the dipole solve's operator
-// needs its field).  CTA = 128 ions x a
-// group of row tiles (128 columns each), 256 threads: the next B tile is copied
-// in (cp.async) while the tensor core multiplies the current one into one half
-// of a double-buffered tensor-memory accumulator and the threads reduce the
-// previous one from the other half.
-constexpr int kFieldTcThreads = 256;
+// needs its field).  CTA = 128 ions x a group of row tiles (128 columns each),
+// one CTA per SM: 16 warps reduce a tile, one thread issues the products of the
+// next into the other half of a double-buffered tensor-memory accumulator,
+// one thread bulk-copies the B tile after that; mbarriers only, no CTA-wide
+// barrier in the loop.  The ions' features and phases are formed before the
+// wait for the predecessor (the B tiles), which they do not depend on.
+//
+// Bound: per tile the products (3 K / 8 of 128 x 128 x 8, about 1000 cycles at K =
+// 40) and the reduction (8 rows x 16 FP32 operations a thread, about 700 issue cycles a
+// scheduler) run side by side; what is left is start-up and the wave.  Two CTAs
+// of 256 threads with barriers between copy, product and reduction and K = 32 or
+// 64 took, in an MD step: the operator's field of 4000 dipoles on 572 rows (kz 16)
+// 34 us, now 14; with dipole forces, 8000 ions, 65 -> 32; 13700 ions on 1050 rows
+// (kz 20) 97 -> 46.
+constexpr int kFieldTcRed = 512;                    // reducing threads: 128 ions x 4 column chunks
+constexpr int kFieldTcThreads = kFieldTcRed + 64;   // + the MMA warp and the copy warp
 
-// features per ion (K), 32 or 64 (0: kz too large for this kernel)
+// features per ion (K): 2 (kz + 1) rounded up to an instantiated multiple of
+// the MMA's 8 (0: kz too large for this kernel)
 __host__ __device__ constexpr int field_tc_kf(int kz) {
-  return 2 * (kz + 1) <= 32 ? 32 : (2 * (kz + 1) <= 64 ? 64 : 0);
+  const int f = 2 * (kz + 1);
+  return f <= 16 ? 16 : f <= 24 ? 24 : f <= 32 ? 32 : f <= 40 ? 40 : f <= 48 ? 48 : f <= 64 ? 64 : 0;
 }
 // rows per 128-column tile
 __host__ __device__ constexpr int field_tc_rpt(bool has_h) { return has_h ? 16 : 32; }
@@ -625,7 +637,7 @@ __host__ __device__ constexpr size_t field_tc_smem(int KF, int ky) {
 // from the structure-factor chunk partials in chunk order (rho_prime, the same
 // sums as k_rec_sum), which saves that pass when no energy is needed; rho_out
 // (optional) receives those rho' values.
-constexpr int kBtRows = 4;
+constexpr int kBtRows = 2;
 
 template <bool HAS_H, int KF>
 static __global__ void __launch_bounds__(128) k_rec_field_btiles(RecMesh M, const double2* __restrict__ rhoA,
@@ -692,14 +704,12 @@ static __global__ void __launch_bounds__(128) k_rec_field_btiles(RecMesh M, cons
 }
 
 template <bool HAS_H, int KF>
-static __global__ void __launch_bounds__(kFieldTcThreads) k_rec_field_tc(
+static __global__ void __launch_bounds__(kFieldTcThreads, 1) k_rec_field_tc(
     const float2* __restrict__ tab, const float4* __restrict__ w, int natm, const int* __restrict__ imap,
     int nion, RecMesh M,
     const uint32_t* __restrict__ fb, int tiles_per_group, double4* __restrict__ Gpart,
     double4* __restrict__ Hpart, int* __restrict__ err) {
-  pdl_wait();
-  pdl_trigger();
-  constexpr int NT = kFieldTcThreads;
+  constexpr int NT = kFieldTcRed;
   constexpr int CPR = HAS_H ? 8 : 4;     // columns per mesh row (6 used with H)
   constexpr int RPT = 128 / CPR;         // mesh rows per tile
   constexpr int RPC = 32 / CPR;          // mesh rows per 32-column chunk
@@ -707,9 +717,12 @@ static __global__ void __launch_bounds__(kFieldTcThreads) k_rec_field_tc(
   constexpr uint32_t LBO = (128 / 8) * 128, SBO = 128;
   extern __shared__ unsigned char smraw[];
   unsigned char* sm = (unsigned char*)(((uintptr_t)smraw + 1023) & ~(uintptr_t)1023);
-  __shared__ __align__(8) uint64_t mbar[2];
+  // bfull[b]: B tile landed in buffer b; mdone[b]: its products are complete
+  // (buffer b free, accumulator half b ready); dfree[b]: every warp has read that half
+  __shared__ __align__(8) uint64_t bfull[2], mdone[2], dfree[2];
   __shared__ uint32_t tslot;
-  __shared__ int abort_flag;
+  __shared__ int abort_flag, issued_sh;
+  const volatile int* abort_v = &abort_flag;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int kx = M.kmax[0], ky = M.kmax[1], kz = M.kmax[2];
   const int nzc = kz + 1;
@@ -718,6 +731,7 @@ static __global__ void __launch_bounds__(kFieldTcThreads) k_rec_field_tc(
     uint32_t dyn;
     asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
     if (dyn < field_tc_smem(KF, ky) || field_tc_kf(kz) != KF) {
+      pdl_wait();
       if (tid == 0) atomicExch(err, 2);
       return;
     }
@@ -725,70 +739,69 @@ static __global__ void __launch_bounds__(kFieldTcThreads) k_rec_field_tc(
   const int ntile = (M.nrows + RPT - 1) / RPT;
   const int tbeg = blockIdx.y * tiles_per_group;
   const int tend = min(tbeg + tiles_per_group, ntile);
+  const int T = tend - tbeg;
   const int i0 = blockIdx.x * 128;
+  if (tid == 0) {
+    abort_flag = 0;
+    issued_sh = 0;
+    for (int b = 0; b < 2; ++b) {
+      tc::mbar_init_n(tc::smem_u32(&bfull[b]), 1);
+      tc::mbar_init_n(tc::smem_u32(&mdone[b]), 1);
+      tc::mbar_init_n(tc::smem_u32(&dfree[b]), NT / 32);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;");
+  }
+  unsigned char* Ahi = sm;
+  unsigned char* Alo = sm + TILE;
+  auto Bbuf = [&](int b) { return sm + 2 * TILE + b * 2 * TILE; };
+  float2* Ys = reinterpret_cast<float2*>(sm + 6 * TILE);  // [ky + 1][128]
+  // the ion of tile slot s (imap: a subset of the ions), -1 past the ions
+  auto ion_of = [&](int s) { return s < nion ? (imap ? imap[s] : s) : -1; };
+  // per-thread sums: ion m = 32 (warp & 3) + lane, column chunk warp >> 2
+  const int q = warp & 3, hh = (warp >> 2) & 3;
+  const int m = q * 32 + lane, ion = ion_of(i0 + m);
+  const bool ion_ok = ion >= 0;
+  const int ionc = ion_ok ? ion : 0;
+  if (warp < NT / 32) {
+    // A: the features of ion m, 4 at a time, fc = hh, hh + 4, ..
+#pragma unroll
+    for (int fq = 0; fq < (KF / 4 + 3) / 4; ++fq) {
+      const int fc = hh + 4 * fq;
+      if (fc >= KF / 4) break;
+      uint32_t hi[4], lo[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int f = fc * 4 + u;
+        float x = 0.f;
+        if (ion_ok && f < 2 * nzc) {
+          const float2 Z = tab[(zoff + (f < nzc ? f : f - nzc)) * natm + ion];
+          x = f < nzc ? Z.x : Z.y;
+        }
+        tc::tf32_split(x, hi[u], lo[u]);
+      }
+      const uint32_t o = tc::canon(m, fc * 4, 128);
+      *reinterpret_cast<uint4*>(Ahi + o) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+      *reinterpret_cast<uint4*>(Alo + o) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    }
+    // the reduction's Y_ny phases of the CTA's ions (zero past the ions)
+#pragma unroll 4
+    for (int a = hh; a <= ky; a += 4)
+      Ys[a * 128 + m] = ion_ok ? tab[(size_t)(kx + 1 + a) * natm + ion] : make_float2(0.f, 0.f);
+  }
+  pdl_wait();
+  pdl_trigger();
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      tc::smem_u32(&tslot)),
                  "r"(256));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
-  if (tid == 0) {
-    abort_flag = 0;
-    tc::mbar_init(tc::smem_u32(&mbar[0]));
-    tc::mbar_init(tc::smem_u32(&mbar[1]));
-    asm volatile("fence.mbarrier_init.release.cluster;");
-  }
+  tc::fence_async_smem();
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem = tslot;
-  unsigned char* Ahi = sm;
-  unsigned char* Alo = sm + TILE;
-  auto Bbuf = [&](int b) { return sm + 2 * TILE + b * 2 * TILE; };
-  float2* Ys = reinterpret_cast<float2*>(sm + 6 * TILE);  // [ky + 1][128]
-  const int T = tend - tbeg;
-  // B tile t (hi | lo, 2 TILE bytes) -> buffer b, 16-byte copies
-  auto load_b = [&](int t, int b) {
-    const uint4* src = reinterpret_cast<const uint4*>(fb) + (size_t)t * (2 * TILE / 16);
-    uint32_t dst = tc::smem_u32(Bbuf(b));
-    for (int e = tid; e < 2 * TILE / 16; e += NT) cp_async16(dst + e * 16, src + e, 16);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  if (T > 0) load_b(tbeg, 0);
-  // the ion of tile slot s (imap: a subset of the ions), -1 past the ions
-  auto ion_of = [&](int s) { return s < nion ? (imap ? imap[s] : s) : -1; };
-
-  // A: ion features, items (ion m, 4 features) with m = it % 128
-  for (int it = tid; it < 128 * (KF / 4); it += NT) {
-    int m = it & 127, fc = it >> 7;
-    int i = ion_of(i0 + m);
-    uint32_t hi[4], lo[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      int f = fc * 4 + u;
-      float x = 0.f;
-      if (i >= 0 && f < 2 * nzc) {
-        float2 Z = tab[(zoff + (f < nzc ? f : f - nzc)) * natm + i];
-        x = f < nzc ? Z.x : Z.y;
-      }
-      tc::tf32_split(x, hi[u], lo[u]);
-    }
-    uint32_t o = tc::canon(m, fc * 4, 128);
-    *reinterpret_cast<uint4*>(Ahi + o) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-    *reinterpret_cast<uint4*>(Alo + o) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-  }
-  // the epilogue's Y_ny phases of the CTA's ions (zero past the ions); made
-  // visible by the barrier before the first products
-  for (int e = tid; e < (ky + 1) * 128; e += NT) {
-    const int a = e >> 7, i = ion_of(i0 + (e & 127));
-    Ys[e] = i >= 0 ? tab[(size_t)(kx + 1 + a) * natm + i] : make_float2(0.f, 0.f);
-  }
-  // per-thread sums: ion m = 32 (warp & 3) + lane, column chunks (warp >> 2) and +2
-  const int q = warp & 3, hh = warp >> 2;
-  const int m = q * 32 + lane, ion = ion_of(i0 + m);
-  const bool ion_ok = ion >= 0;
-  const int ionc = ion_ok ? ion : 0;
-  const float4 wi = ion_ok ? w[ion] : make_float4(0.f, 0.f, 0.f, 0.f);
+  const float4 wi = HAS_H && ion_ok ? w[ion] : make_float4(0.f, 0.f, 0.f, 0.f);
   double G[3] = {0.0, 0.0, 0.0}, H[3] = {0.0, 0.0, 0.0};
   // The rows a thread visits come in non-decreasing nx.  With conj(P) =
   // conj(X_nx) conj(Y'_ny) (Y' = Y, conjugated for ny < 0) and Q = conj(Y') T,
@@ -800,8 +813,9 @@ static __global__ void __launch_bounds__(kFieldTcThreads) k_rec_field_tc(
   //   H += (nx (m1 nx Re(cX W0) + m2 Re(cX W1) + m3 Re(cX V0)),
   //         m1 nx Re(cX W1) + m2 Re(cX W2) + m3 Re(cX V1),
   //         m1 nx Re(cX V0) + m2 Re(cX V1) + m3 Re(cX U0)).
+  // (X of nx + 1 is fetched when nx is applied)
   int gnx = -1;
-  float2 xval = make_float2(0.f, 0.f);
+  float2 xval = make_float2(0.f, 0.f), xnext = xval;
   float2 W0{}, W1{}, V0{}, W2{}, V1{}, U0{};
   auto flush = [&]() {
     if (gnx >= 0) {
@@ -821,116 +835,119 @@ static __global__ void __launch_bounds__(kFieldTcThreads) k_rec_field_tc(
     }
     W0 = W1 = V0 = W2 = V1 = U0 = make_float2(0.f, 0.f);
   };
-  auto epilogue = [&](int t, int b) {
-#pragma unroll
-    for (int cc = 0; cc < 2; ++cc) {
-      int ch = hh + 2 * cc;
-      // the chunk's rows and this ion's Y_ny (shared) first
-      int nxr[RPC], nyr[RPC];
-      float okr[RPC];
-      bool rok[RPC];
-      float2 Y[RPC];
-#pragma unroll
-      for (int jj = 0; jj < RPC; ++jj) {
-        int row = t * RPT + ch * RPC + jj;
-        bool ok = row < M.nrows;
-        int4 ri = M.rows[ok ? row : 0];
-        nxr[jj] = ri.x;
-        nyr[jj] = ri.y;
-        rok[jj] = ok;
-        okr[jj] = (ok && ion_ok) ? 1.f : 0.f;
-        int ay = ri.y < 0 ? -ri.y : ri.y;
-        Y[jj] = Ys[ay * 128 + m];
+  const uint32_t idesc = tc::idesc_tf32(128, 128);
+  if (warp < NT / 32) {
+    // ---- reduction ---------------------------------------------------------
+    // this warp's RPC rows of a tile, one record per lane, a tile ahead
+    auto rows_of = [&](int t) {
+      const int row = t * RPT + hh * RPC + (lane & (RPC - 1));
+      const int4 r = M.rows[row < M.nrows ? row : M.nrows - 1];  // (past the mesh: zero columns)
+      return make_int2(r.x, r.y);
+    };
+    int2 rn = rows_of(tbeg);
+    for (int k = 0; k < T; ++k) {
+      const int b = k & 1;
+      const int2 rc = rn;
+      if (k + 1 < T) rn = rows_of(tbeg + k + 1);
+      if (!__all_sync(0xffffffffu, tc::mbar_wait_ab(tc::smem_u32(&mdone[b]), (k >> 1) & 1, tc::kWaitLimit, abort_v))) {
+        abort_flag = 1;
+        break;
       }
+      tc::fence_after_sync();
       float v[32];
-      tc::tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * 128 + ch * 32), v);
+      tc::tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * 128 + hh * 32), v);
+      tc::fence_before_sync();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(tc::smem_u32(&dfree[b]));
 #pragma unroll
       for (int jj = 0; jj < RPC; ++jj) {
-        if (rok[jj] && nxr[jj] != gnx) {
+        const int nx = __shfl_sync(0xffffffffu, rc.x, jj), ny = __shfl_sync(0xffffffffu, rc.y, jj);
+        if (nx != gnx) {
           flush();
-          gnx = nxr[jj];
-          xval = tab[(size_t)gnx * natm + ionc];
+          xval = gnx >= 0 && nx == gnx + 1 ? xnext : tab[(size_t)nx * natm + ionc];
+          gnx = nx;
+          xnext = tab[(size_t)(nx < kx ? nx + 1 : nx) * natm + ionc];
         }
-        const int ny = nyr[jj];
         const float fy = (float)ny;
-        const float yr = okr[jj] * Y[jj].x, yi = okr[jj] * (ny < 0 ? -Y[jj].y : Y[jj].y);
+        const float2 Y = Ys[(ny < 0 ? -ny : ny) * 128 + m];
+        const float yr = Y.x, yi = ny < 0 ? -Y.y : Y.y;
         const float* d = v + jj * CPR;
         const float qr = yr * d[0] + yi * d[1], qi = yr * d[1] - yi * d[0];
-        const float vr = yr * d[2] + yi * d[3], vi = yr * d[3] - yi * d[2];
         W0.x += qr;
         W0.y += qi;
         W1.x += fy * qr;
         W1.y += fy * qi;
-        V0.x += vr;
-        V0.y += vi;
         if (HAS_H) {
+          const float vr = yr * d[2] + yi * d[3], vi = yr * d[3] - yi * d[2];
+          V0.x += vr;
+          V0.y += vi;
           W2.x += fy * fy * qr;
           W2.y += fy * fy * qi;
           V1.x += fy * vr;
           V1.y += fy * vi;
           U0.x += yr * d[4] + yi * d[5];
           U0.y += yr * d[5] - yi * d[4];
+        } else {
+          V0.x += yr * d[2] + yi * d[3];
+          V0.y += yr * d[3] - yi * d[2];
         }
       }
     }
-  };
-
-  const uint32_t idesc = tc::idesc_tf32(128, 128);
-  int issued = 0, done = 0;  // tiles multiplied / tiles whose MMA completion was seen
-  for (int k = 0; k < T; ++k) {
-    const int b = k & 1;
-    if (k >= 1) {
-      // tile k - 1 multiplied: B buffer (k + 1) & 1 is free, its D is ready
-      if (tid == 0 && !tc::mbar_wait(tc::smem_u32(&mbar[(k - 1) & 1]), ((k - 1) >> 1) & 1, tc::kWaitLimit))
+  } else if (warp == NT / 32 + 1) {
+    // ---- copies: B tile (hi | lo, 2 TILE bytes) tbeg + k into buffer k & 1 once
+    // the products of tile k - 2 are complete
+    if (lane == 0) {
+      int copied = 0;
+      for (int k = 0; k < T; ++k) {
+        const int b = k & 1;
+        if (k >= 2 && !tc::mbar_wait_ab(tc::smem_u32(&mdone[b]), ((k - 2) >> 1) & 1, tc::kWaitLimit, abort_v)) {
+          abort_flag = 1;
+          break;
+        }
+        const uint32_t fbar = tc::smem_u32(&bfull[b]);
+        tc::mbar_expect_tx(fbar, 2 * TILE);
+        tc::bulk_g2s(tc::smem_u32(Bbuf(b)), reinterpret_cast<const unsigned char*>(fb) + (size_t)(tbeg + k) * 2 * TILE,
+                     2 * TILE, fbar);
+        copied = k + 1;
+      }
+      // no copy may still be landing when the CTA leaves (after an abort):
+      // wait (bounded) for the last tile copied into each buffer
+      for (int b = 0; b < 2 && b < copied; ++b) {
+        const int last = b + 2 * ((copied - 1 - b) / 2);
+        if (!tc::mbar_wait(tc::smem_u32(&bfull[b]), (last >> 1) & 1, tc::kWaitLimit)) abort_flag = 1;
+      }
+    }
+  } else if (lane == 0) {
+    // ---- MMA issue: split TF32 products of tile k into accumulator half k & 1
+    int issued = 0;
+    const uint32_t aH = tc::smem_u32(Ahi), aL = tc::smem_u32(Alo);
+    for (int k = 0; k < T; ++k) {
+      const int b = k & 1;
+      if (!tc::mbar_wait_ab(tc::smem_u32(&bfull[b]), (k >> 1) & 1, tc::kWaitLimit, abort_v) ||
+          (k >= 2 && !tc::mbar_wait_ab(tc::smem_u32(&dfree[b]), ((k - 2) >> 1) & 1, tc::kWaitLimit, abort_v))) {
         abort_flag = 1;
-      __syncthreads();
-      if (abort_flag) break;
-      done = k;
-    }
-    if (k + 1 < T) {
-      load_b(tbeg + k + 1, (k + 1) & 1);
-      asm volatile("cp.async.wait_group 1;" ::: "memory");
-    } else {
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
-    }
-    tc::fence_async_smem();
-    __syncthreads();
-    if (tid == 0) {
+        break;
+      }
       tc::fence_after_sync();
-      const uint32_t aH = tc::smem_u32(Ahi), aL = tc::smem_u32(Alo);
       const uint32_t bH = tc::smem_u32(Bbuf(b)), bL = bH + TILE;
       const uint32_t d = tmem + (uint32_t)(b * 128);
 #pragma unroll
       for (int s = 0; s < KF / 8; ++s) {
-        uint32_t o = (uint32_t)s * 2 * LBO;
-        uint64_t dAH = tc::smem_desc(aH + o, LBO, SBO), dAL = tc::smem_desc(aL + o, LBO, SBO);
-        uint64_t dBH = tc::smem_desc(bH + o, LBO, SBO), dBL = tc::smem_desc(bL + o, LBO, SBO);
+        const uint32_t o = (uint32_t)s * 2 * LBO;
+        const uint64_t dAH = tc::smem_desc(aH + o, LBO, SBO), dAL = tc::smem_desc(aL + o, LBO, SBO);
+        const uint64_t dBH = tc::smem_desc(bH + o, LBO, SBO), dBL = tc::smem_desc(bL + o, LBO, SBO);
         tc::mma_tf32(d, dAH, dBH, idesc, s > 0 ? 1u : 0u);
         tc::mma_tf32(d, dAH, dBL, idesc, 1u);
         tc::mma_tf32(d, dAL, dBH, idesc, 1u);
       }
-      tc::mma_commit(tc::smem_u32(&mbar[b]));
+      tc::mma_commit(tc::smem_u32(&mdone[b]));
+      issued = k + 1;
     }
-    issued = k + 1;
-    if (k >= 1) {
-      tc::fence_after_sync();
-      epilogue(tbeg + k - 1, (k - 1) & 1);
-    }
-    tc::fence_before_sync();
-  }
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
-  if (!abort_flag && issued > done) {
-    if (tid == 0 && !tc::mbar_wait(tc::smem_u32(&mbar[(issued - 1) & 1]), ((issued - 1) >> 1) & 1, tc::kWaitLimit))
+    // every issued product is complete before its operands and tensor memory
+    // go (also after an abort)
+    if (issued > 0 && !tc::mbar_wait(tc::smem_u32(&mdone[(issued - 1) & 1]), ((issued - 1) >> 1) & 1, tc::kWaitLimit))
       abort_flag = 1;
-    __syncthreads();
-    if (!abort_flag) {
-      tc::fence_after_sync();
-      epilogue(tbeg + issued - 1, (issued - 1) & 1);
-      done = issued;
-    }
-  } else if (abort_flag && issued > done && tid == 0) {
-    // stopped early: let the last issued MMA finish before freeing its memory
-    tc::mbar_wait(tc::smem_u32(&mbar[(issued - 1) & 1]), ((issued - 1) >> 1) & 1, tc::kWaitLimit);
+    issued_sh = issued;
   }
   tc::fence_before_sync();
   __syncthreads();
@@ -938,28 +955,28 @@ static __global__ void __launch_bounds__(kFieldTcThreads) k_rec_field_tc(
     tc::fence_after_sync();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256));
   }
-  if (abort_flag) {
+  if (abort_flag || issued_sh != T) {
     if (tid == 0) atomicExch(err, 1);
     return;
   }
   flush();
-  // combine the two column halves of each ion (A is free: every MMA is done)
+  // combine the four column chunks of each ion (the operands are free: every MMA
+  // is done)
   double* red = reinterpret_cast<double*>(sm);
-  if (hh == 1) {
-    red[m * 6 + 0] = G[0];
-    red[m * 6 + 1] = G[1];
-    red[m * 6 + 2] = G[2];
-    red[m * 6 + 3] = H[0];
-    red[m * 6 + 4] = H[1];
-    red[m * 6 + 5] = H[2];
+  constexpr int NC = HAS_H ? 6 : 3;
+  if (warp < NT / 32 && hh > 0) {
+#pragma unroll
+    for (int d = 0; d < NC; ++d) red[((hh - 1) * 6 + d) * 128 + m] = d < 3 ? G[d % 3] : H[d % 3];
   }
   __syncthreads();
-  if (hh == 0 && ion_ok) {
-    Gpart[(size_t)blockIdx.y * natm + ion] =
-        make_double4(G[0] + red[m * 6 + 0], G[1] + red[m * 6 + 1], G[2] + red[m * 6 + 2], 0.0);
-    if (HAS_H)
-      Hpart[(size_t)blockIdx.y * natm + ion] =
-          make_double4(H[0] + red[m * 6 + 3], H[1] + red[m * 6 + 4], H[2] + red[m * 6 + 5], 0.0);
+  if (warp < 4 && ion_ok) {
+#pragma unroll
+    for (int d = 0; d < NC; ++d) {
+      double& x = d < 3 ? G[d % 3] : H[d % 3];
+      for (int c = 0; c < 3; ++c) x += red[(c * 6 + d) * 128 + m];
+    }
+    Gpart[(size_t)blockIdx.y * natm + ion] = make_double4(G[0], G[1], G[2], 0.0);
+    if (HAS_H) Hpart[(size_t)blockIdx.y * natm + ion] = make_double4(H[0], H[1], H[2], 0.0);
   }
 }
 
