@@ -1154,6 +1154,16 @@ static int dd64_field(mdff_ctx* h, cudaStream_t st, const double4* mu, bool mask
 // induced pass / the CG operator.  E = T mu.
 // weights_ready: d_w32 / d_mu32 already hold the FP32 operands of mu (written
 // by the CG direction kernels)
+// the FP32 pair cache's field of d_mu32 at the polarisable ions into d_Edd, on
+// the side stream
+static int dd32_part(mdff_ctx* h) {
+  const int np = h->d_polidx ? (int)h->polidx.size() : h->natm;
+  k_dd_cached_part<<<cdiv((long)np * 32, 256), 256, 0, h->st_rs>>>(h->d_mu32, h->d_ddr, h->d_ddb1, h->d_ddj, h->d_ddn,
+                                                                   h->L.cap, h->d_polidx, np, h->d_Edd);
+  LAUNCH_CHECK();
+  return MDFF_OK;
+}
+
 static int field_of_mu(mdff_ctx* h, const double4* mu, int dd_mask, bool fp32, double4* E,
                        bool weights_ready = false, bool cached64 = false) {
   int n = h->natm;
@@ -1198,9 +1208,7 @@ static int field_of_mu(mdff_ctx* h, const double4* mu, int dd_mask, bool fp32, d
   if (dd_side) {
     if ((s = fork_to(h, h->st_rs))) return s;
     h->rs_open = true;
-    k_dd_cached_part<<<nb, 256, 0, h->st_rs>>>(h->d_mu32, h->d_ddr, h->d_ddb1, h->d_ddj, h->d_ddn,
-                                                h->L.cap, n, h->d_Edd);
-    LAUNCH_CHECK();
+    if ((s = dd32_part(h))) return s;
   }
   s = rec_pass(h, fp32, mu, 0, 1, 0, E, nullptr, sf, h->d_mu32, fused ? &nch : nullptr, weights_ready, true);
   if (s) return s;
@@ -1722,6 +1730,7 @@ __global__ void k_cg_plan(double* __restrict__ sc, double* __restrict__ plan, in
     sc[7] = maxit;
     plan[2] = outer + 1.0;
     plan[3] = trust ? 1.0 : 0.0;
+    sc[3] = sc[0];  // r.z (k_cg_step)
   }
   cudaGraphSetConditional(hc, stop ? 0u : 1u);
 }
@@ -1735,13 +1744,63 @@ __global__ void k_setd2(double* __restrict__ a, double va, double* __restrict__ 
   }
 }
 
+// second set of block partials
+static double* upol_part(mdff_ctx* h) { return h->d_part + h->part_cap / 2; }
+
 // one inner CG iteration: p -> T p -> q = A p; x, r, z updated; p <- z + beta p
 static bool rho_acc_enabled(const mdff_ctx* h);
+
+// The graph's iterations defer the sum of the operator's parts to the vector
+// kernels (k_cg_q ..) where these are in place: the pair cache on the side
+// stream (FP32) or of the FP64 engine, field partials of a tensor-core kernel or, FP32,
+// of any.  Else the operator is formed as a field and five more kernels follow.
+static bool cg_fused(const mdff_ctx* h, bool fp32) {
+  if (!h->nk || !h->d_polidx || h->prof) return false;
+  return fp32 ? h->dd_cache_ok && h->overlap && h->d_Edd : h->d_c64r && field_dm_ks(h->p.kES[2]);
+}
+// FP64 weights written with the CG directions
+static double4* cg_w64(const mdff_ctx* h, bool fp32) { return !fp32 && cg_fused(h, false) ? h->d_w : nullptr; }
 
 static int cg_iteration(mdff_ctx* h, bool fp32, int in_graph, cudaGraphConditionalHandle hc) {
   int n = h->natm, nb = cdiv(n, 256), s;
   PolDev P = poldev(h);
   double* sc = h->d_scal + S_CG;
+  if (in_graph && cg_fused(h, fp32)) {
+    const int np = (int)h->polidx.size(), most = 2 * (h->nsm > 0 ? h->nsm : 148);
+    const bool acc = rho_acc_enabled(h);
+    double4* E = fp32 ? h->d_Edd : h->d_Tp;
+    if (h->p.lsurf && (s = moments(h, h->d_pv, 0, h->d_scal + S_MOM2))) return s;
+    if (fp32) {
+      if ((s = fork_to(h, h->st_rs))) return s;
+      h->rs_open = true;
+      if ((s = dd32_part(h))) return s;
+    } else {
+      cudaStream_t rs;
+      if ((s = rs_fork(h, &rs))) return s;
+      if ((s = dd64_field(h, rs, h->d_pv, false, false, E))) return s;
+    }
+    int nch = 0;
+    const SelfField sf = self_field(h, h->d_pv, h->d_scal + S_MOM2);
+    h->rec_mode = acc ? REC_NEED_RHOA : REC_PLAIN;
+    s = rec_pass(h, fp32, h->d_pv, 0, 1, 0, E, nullptr, sf, fp32 ? h->d_mu32 : nullptr, &nch, true, true);
+    h->rec_mode = REC_PLAIN;
+    if (s) return s;
+    // (block partials of p.q and of r.z, |r|^2: neither kernel overwrites what it reads)
+    double *pq = h->d_part, *rz = upol_part(h);
+    const int nq = std::min(cdiv((long)np * 4, 256), most);
+    const int nu = std::min(cdiv((long)std::max(np, acc ? h->nk : 0), 256), most);
+    k_cg_q<<<nq, 256, 0, h->st>>>(h->d_G, nch, n, h->d_polidx, np, h->d_cell, 2.0 * (2.0 * (kTwoPi / h->omega)), sf, E,
+                                  h->d_pv, P, h->d_qv, pq);
+    LAUNCH_CHECK();
+    PDL_CHECK(pdl_launch(k_cg_step, dim3(nu), dim3(256), 0, h->st, sc, (const double*)pq, nq, P,
+                         (const int*)h->d_polidx, np, (const double4*)h->d_pv, (const double4*)h->d_qv, h->d_mu_ind,
+                         h->d_r, h->d_z, rz, acc ? h->d_rho_acc : (double2*)nullptr, (const double2*)h->d_rhoA, h->nk));
+    PDL_CHECK(pdl_launch(k_cg_next, dim3(std::min(cdiv(np, 256), most)), dim3(256), 0, h->st, sc, (const double*)rz, nu,
+                         h->npol, (const int*)h->d_polidx, np, (const double4*)h->d_z, h->d_pv,
+                         (const CellC*)h->d_cell, fp32 ? h->d_w32 : (float4*)nullptr, h->d_mu32, slotw(h),
+                         cg_w64(h, fp32), hc));
+    return MDFF_OK;
+  }
   // with the accumulated structure factor the operator's rho'(p) stays in
   // rhoA for the update, which adds al rho'(p)
   const bool acc = rho_acc_enabled(h);
@@ -1777,7 +1836,6 @@ static bool scf_device_loop(const mdff_ctx* h) {
 
 // one SCF iteration from the second on (pim.cuh); u_pol's partials go to the
 // upper half of d_part
-static double* upol_part(mdff_ctx* h) { return h->d_part + h->part_cap / 2; }
 static int scf_iteration(mdff_ctx* h, cudaGraphConditionalHandle hc) {
   const int n = h->natm, np = (int)h->polidx.size(), nb = cdiv(n, 256);
   int s;
@@ -1962,7 +2020,7 @@ static int cg_residual(mdff_ctx* h, bool fp32) {
   PolDev P = poldev(h);
   if ((s = field_of_mu(h, h->d_mu_ind, 1, false, h->d_Tp, false, fp32))) return s;
   PDL_CHECK(pdl_launch(k_cg_init, dim3(nb), dim3(256), 0, h->st, h->d_Estat, h->d_Tp, h->d_mu_ind, P, n, h->d_r, h->d_z, h->d_pv, h->d_part,
-                                   h->d_cell, fp32 ? h->d_w32 : nullptr, h->d_mu32, slotw(h)));
+                                   h->d_cell, fp32 ? h->d_w32 : nullptr, h->d_mu32, slotw(h), cg_w64(h, fp32)));
   return reduce_into(h, nb, 2, h->d_scal + S_CG);
 }
 
@@ -2034,7 +2092,7 @@ static int merged_residual(mdff_ctx* h, bool fp32) {
   h->rho_acc_ok = acc;
   PDL_CHECK(pdl_launch(k_cg_init, dim3(nb), dim3(256), 0, h->st, (const double4*)nullptr, (const double4*)E,
                        (const double4*)h->d_mu_ind, P, n, h->d_r, h->d_z, h->d_pv, h->d_part,
-                       (const CellC*)h->d_cell, fp32 ? h->d_w32 : (float4*)nullptr, h->d_mu32, slotw(h)));
+                       (const CellC*)h->d_cell, fp32 ? h->d_w32 : (float4*)nullptr, h->d_mu32, slotw(h), cg_w64(h, fp32)));
   return reduce_into(h, nb, 2, h->d_scal + S_CG);
 }
 
@@ -2763,6 +2821,8 @@ static int create_impl(mdff_ctx* h, const mdff_params* pin, const double* cellA)
   h->part_cap = (size_t)std::max(cdiv((long)n * 32, 256), cdiv(n, 256)) * 16 + 64;
   // kO_v4_1 Gram row: kKoHist + 2 dot products per block
   h->part_cap = std::max(h->part_cap, (size_t)cdiv(n, 256) * (kKoHist + 2));
+  // (either half holds two sums of 2 x SM blocks)
+  h->part_cap = std::max(h->part_cap, (size_t)8 * std::max(h->nsm, 148));
   DALLOC(h->d_part, h->part_cap);
   DALLOC(h->d_part2, h->part_cap);
   DALLOC(h->d_scal, S_NSCAL);

@@ -283,11 +283,20 @@ __device__ __forceinline__ void cg_dir_weights(const CellC* __restrict__ cell, d
   sw.put(i, wv);
 }
 
+// FP64 operator: w = (0, m)
+__device__ __forceinline__ void cg_dir_weights64(const CellC* __restrict__ cell, double4 u, int i,
+                                                 double4* __restrict__ w) {
+  const double* B = cell->B;
+  w[i] = make_double4(0.0, kTwoPi * (B[0] * u.x + B[3] * u.y + B[6] * u.z),
+                      kTwoPi * (B[1] * u.x + B[4] * u.y + B[7] * u.z),
+                      kTwoPi * (B[2] * u.x + B[5] * u.y + B[8] * u.z));
+}
+
 __global__ void k_cg_init(const double4* __restrict__ b, const double4* __restrict__ Tx,
                           const double4* __restrict__ x, PolDev P, int natm, double4* __restrict__ r,
                           double4* __restrict__ z, double4* __restrict__ p, double* __restrict__ part,
                           const CellC* __restrict__ cell, float4* __restrict__ w32,
-                          float4* __restrict__ mu32, SlotW sw) {
+                          float4* __restrict__ mu32, SlotW sw, double4* __restrict__ w64) {
   pdl_wait();
   pdl_trigger();
   __shared__ double red[2 * 32];
@@ -310,6 +319,7 @@ __global__ void k_cg_init(const double4* __restrict__ b, const double4* __restri
     z[i] = zi;
     p[i] = zi;
     if (w32) cg_dir_weights(cell, zi, i, w32, mu32, sw);
+    if (w64) cg_dir_weights64(cell, zi, i, w64);
     v[0] = ri.x * zi.x + ri.y * zi.y + ri.z * zi.z;
   }
   block_sum<2>(v, red);
@@ -404,6 +414,178 @@ __global__ void k_cg_dir(const double* __restrict__ rz_p, const double* __restri
     p[i] = pn;
     if (w32) cg_dir_weights(cell, pn, i, w32, mu32, sw);
   }
+}
+
+// ---------------------------------------------------------------------------
+// The three vector kernels of a CG iteration whose operator's parts are deferred
+// to it (field partials per row group, real-space field in Edd), over the
+// polarisable ions (polidx):
+//   k_cg_q     T p = real + reciprocal + self (+ surface), q = alpha^-1 p - T p, p.q
+//   k_cg_step  al; x, r, z updated (and the accumulated rho'); r.z, |r|^2
+//   k_cg_next  beta; p <- z + beta p with the next operator's weights; the step
+//              scalars and the loop's condition
+// Each kernel sums its predecessor's block partials itself (every block the same
+// order): a sum of a few hundred numbers costs a block about 1 us, a launch of its
+// own 4 us.  Scalars are read and written by different kernels: sc[3] is r.z for
+// k_cg_step (whose block 0 moves it to sc[0]), sc[0] is r.z for k_cg_next (whose block
+// 0 leaves the new one in sc[3]).  An iteration of 8000 MgO ions had ten kernels, 66 us,
+// of which 23 us were these and their reductions; now six.
+template <int NV>
+__device__ __forceinline__ void block_partials(const double* __restrict__ part, int nblk, double (&v)[NV],
+                                               double* red, double* out) {
+#pragma unroll
+  for (int k = 0; k < NV; ++k) v[k] = 0.0;
+  for (int b = threadIdx.x; b < nblk; b += blockDim.x)
+#pragma unroll
+    for (int k = 0; k < NV; ++k) v[k] += part[(size_t)b * NV + k];
+  block_sum<NV>(v, red);
+  if (threadIdx.x == 0)
+#pragma unroll
+    for (int k = 0; k < NV; ++k) out[k] = v[k];
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < NV; ++k) v[k] = out[k];
+}
+
+// four threads per ion split the field partials, as k_rec_field_sum
+__global__ void __launch_bounds__(256) k_cg_q(const double4* __restrict__ Gpart, int nchunk, int natm,
+                                              const int* __restrict__ polidx, int npol,
+                                              const CellC* __restrict__ cell, double scale, SelfField sf,
+                                              const double4* __restrict__ Edd, const double4* __restrict__ p, PolDev P,
+                                              double4* __restrict__ qv, double* __restrict__ part) {
+  pdl_trigger();  // (a plain launch: everything before it is complete)
+  __shared__ double red[32];
+  double v[1] = {0.0};
+  const int sub = threadIdx.x & 3;
+  for (int s0 = blockIdx.x * (blockDim.x / 4); s0 < npol; s0 += gridDim.x * (blockDim.x / 4)) {
+    const int sl = s0 + (threadIdx.x >> 2);
+    const bool ok = sl < npol;
+    const int i = polidx[ok ? sl : npol - 1];
+    double g[3] = {0.0, 0.0, 0.0};
+    for (int c = sub; c < nchunk; c += 4) {
+      const double4 u = Gpart[(size_t)c * natm + i];
+      g[0] += u.x;
+      g[1] += u.y;
+      g[2] += u.z;
+    }
+    const double4 pi = p[i], o = Edd[i];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      g[a] += __shfl_xor_sync(FULL_MASK, g[a], 1);
+      g[a] += __shfl_xor_sync(FULL_MASK, g[a], 2);
+    }
+    if (!ok || sub != 0) continue;
+    const double* B = cell->B;
+    const double4 ap = matvec3(P.invpol + 9 * (size_t)i, pi);
+    const double pp[3] = {pi.x, pi.y, pi.z}, oo[3] = {o.x, o.y, o.z}, aa[3] = {ap.x, ap.y, ap.z};
+    double q[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const double er = -kTwoPi * (B[3 * a] * g[0] + B[3 * a + 1] * g[1] + B[3 * a + 2] * g[2]) * scale;
+      double self = 2.0 * sf.selfa2 * pp[a];
+      if (sf.lsurf) self -= (sf.mom[a] + sf.mom[3 + a]) * sf.fpi_3V;
+      q[a] = aa[a] - (oo[a] + er + self);
+      v[0] += pp[a] * q[a];
+    }
+    qv[i] = make_double4(q[0], q[1], q[2], 0.0);
+  }
+  block_sum<1>(v, red);
+  if (threadIdx.x == 0) part[blockIdx.x] = v[0];
+}
+
+__global__ void __launch_bounds__(256) k_cg_step(double* __restrict__ sc, const double* __restrict__ pq_part, int npq,
+                                                 PolDev P, const int* __restrict__ polidx, int npol,
+                                                 const double4* __restrict__ p, const double4* __restrict__ qv,
+                                                 double4* __restrict__ x, double4* __restrict__ r,
+                                                 double4* __restrict__ z, double* __restrict__ part,
+                                                 double2* __restrict__ acc, const double2* __restrict__ rhoA, int nk) {
+  __shared__ double red[2 * 32], bc[2];
+  const int t0 = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+  // what k_cg_q does not write is read before the wait for it
+  const int i0 = polidx[t0 < npol ? t0 : npol - 1];
+  const double4 x0 = x[i0], r0 = r[i0], p0 = p[i0];
+  double a0[9];
+#pragma unroll
+  for (int c = 0; c < 9; ++c) a0[c] = P.pol[9 * (size_t)i0 + c];
+  const double rz = sc[3];
+  pdl_wait();
+  pdl_trigger();
+  const double4 q0 = qv[i0];
+  double pq[1], v[2] = {0.0, 0.0};
+  block_partials<1>(pq_part, npq, pq, red, bc);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    sc[0] = rz;
+    sc[2] = pq[0];
+  }
+  const double al = (pq[0] != 0.0) ? rz / pq[0] : 0.0;
+  auto step = [&](int i, double4 xi, double4 ri, const double4& pi, const double4& qi, const double* a) {
+    xi.x += al * pi.x;
+    xi.y += al * pi.y;
+    xi.z += al * pi.z;
+    ri.x -= al * qi.x;
+    ri.y -= al * qi.y;
+    ri.z -= al * qi.z;
+    const double4 zi = matvec3(a, ri);
+    x[i] = xi;
+    r[i] = ri;
+    z[i] = zi;
+    v[0] += ri.x * zi.x + ri.y * zi.y + ri.z * zi.z;
+    const double rr[3] = {ri.x, ri.y, ri.z};
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+      if (a[4 * c] != 0.0) v[1] += rr[c] * rr[c];
+  };
+  if (t0 < npol) step(i0, x0, r0, p0, q0, a0);
+  for (int sl = t0 + nt; sl < npol; sl += nt) {
+    const int i = polidx[sl];
+    step(i, x[i], r[i], p[i], qv[i], P.pol + 9 * (size_t)i);
+  }
+  if (acc)  // (k_cg_update)
+    for (int k = t0; k < nk; k += nt) {
+      const double2 a = acc[k], d = rhoA[k];
+      acc[k] = make_double2(a.x + al * d.x, a.y + al * d.y);
+    }
+  block_sum<2>(v, red);
+  if (threadIdx.x == 0) {
+    part[(size_t)blockIdx.x * 2] = v[0];
+    part[(size_t)blockIdx.x * 2 + 1] = v[1];
+  }
+}
+
+__global__ void __launch_bounds__(256) k_cg_next(double* __restrict__ sc, const double* __restrict__ rz_part, int nrz,
+                                                 int npol_r, const int* __restrict__ polidx, int npol,
+                                                 const double4* __restrict__ z, double4* __restrict__ p,
+                                                 const CellC* __restrict__ cell, float4* __restrict__ w32,
+                                                 float4* __restrict__ mu32, SlotW sw, double4* __restrict__ w64,
+                                                 cudaGraphConditionalHandle hc) {
+  __shared__ double red[2 * 32], bc[2];
+  const int t0 = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+  // (as k_cg_step: only z and the partials are its)
+  const int i0 = polidx[t0 < npol ? t0 : npol - 1];
+  const double4 p0 = p[i0];
+  pdl_wait();
+  pdl_trigger();
+  const double4 z0 = z[i0];
+  double v[2];
+  block_partials<2>(rz_part, nrz, v, red, bc);
+  const double rz = sc[0];
+  const double be = (rz != 0.0) ? v[0] / rz : 0.0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    sc[3] = v[0];
+    sc[4] = v[1];
+    const double it = sc[6] + 1.0, rm = sqrt(v[1] / (double)npol_r);
+    sc[6] = it;
+    sc[8] = rm;
+    cudaGraphSetConditional(hc, (rm > sc[5] && it < sc[7]) ? 1u : 0u);
+  }
+  auto next = [&](int i, const double4& pi, const double4& zi) {
+    const double4 pn = make_double4(zi.x + be * pi.x, zi.y + be * pi.y, zi.z + be * pi.z, 0.0);
+    p[i] = pn;
+    if (w32) cg_dir_weights(cell, pn, i, w32, mu32, sw);
+    if (w64) cg_dir_weights64(cell, pn, i, w64);
+  };
+  if (t0 < npol) next(i0, p0, z0);
+  for (int sl = t0 + nt; sl < npol; sl += nt) next(polidx[sl], p[polidx[sl]], z[polidx[sl]]);
 }
 
 __global__ void k_copy1(double* __restrict__ dst, const double* __restrict__ src) {

@@ -688,16 +688,17 @@ __device__ __forceinline__ void dd_cached_row(const typename vec4t<R>::T* __rest
   }
 }
 
-// the cached dipole field of every row as a warp-summed double4 (0 for rows
-// without partners), for the CG operator to add in its final kernel: it runs
+// the cached dipole field of every polarisable ion's row as a warp-summed
+// double4, for the CG operator to add in its final kernel: it runs
 // on a side stream beside the reciprocal pass of the same operator
 static __global__ void __launch_bounds__(256) k_dd_cached_part(
     const float4* __restrict__ mu, const float4* __restrict__ cr, const float* __restrict__ cb1,
-    const int* __restrict__ cj, const int* __restrict__ cn, int cap, int natm,
-    double4* __restrict__ Edd) {
+    const int* __restrict__ cj, const int* __restrict__ cn, int cap, const int* __restrict__ polidx,
+    int npol, double4* __restrict__ Edd) {
   int lane = threadIdx.x & 31;
-  int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (i >= natm) return;
+  const int sl = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (sl >= npol) return;
+  const int i = polidx ? polidx[sl] : sl;
   int n = cn[i];
   float ex = 0.f, ey = 0.f, ez = 0.f;
   dd_cached_row<float>(mu, cr, cb1, cj, (size_t)i * cap, n, lane, ex, ey, ez);
