@@ -1113,16 +1113,12 @@ static int build_tables(mdff_ctx* h) {
   if (h->nk == 0) return MDFF_OK;
   int n = h->natm;
   int kzt = std::max(h->p.kES[2], 4);
-  PDL_CHECK(pdl_launch(k_rec_tables<double>, dim3(cdiv(n, 128)), dim3(128), 0, h->st, h->d_s, n, h->p.kES[0], h->p.kES[1], kzt, h->d_tab64));
-  if (h->p.precision == MDFF_PREC_MIXED) {
-    PDL_CHECK(pdl_launch(k_rec_tables<float>, dim3(cdiv(n, 128)), dim3(128), 0, h->st, h->d_s, n, h->p.kES[0], h->p.kES[1], kzt, h->d_tab32));
-    // the same tables blocked by K block for the tensor-core structure
-    // factor of the dipole solve
-    if (h->rho_tc && h->lpolar)
-      PDL_CHECK(pdl_launch(k_rec_rho_timg, dim3((unsigned)h->tc_nkb), dim3(256), 0, h->st, (const float2*)h->d_tab32, n,
-                           (const int*)h->d_polidx, rho_tc_nion(h), h->p.kES[0], h->p.kES[1], h->p.kES[2],
-                           h->d_rho_timg));
-  }
+  const bool mixed = h->p.precision == MDFF_PREC_MIXED, img = mixed && h->rho_tc && h->lpolar;
+  const int nt = h->p.kES[0] + h->p.kES[1] + kzt + 3;
+  PDL_CHECK(pdl_launch(k_rec_tables, dim3((unsigned)cdiv(n, 128), (unsigned)cdiv(nt, kTabEntries)), dim3(128), 0, h->st,
+                       (const double4*)h->d_s, n, h->p.kES[0], h->p.kES[1], h->p.kES[2], kzt, h->d_tab64,
+                       mixed ? h->d_tab32 : (float2*)nullptr, img ? h->d_rho_timg : (float2*)nullptr,
+                       (const int*)h->d_polslot, (int)(kStageRow / sizeof(float2))));
   return MDFF_OK;
 }
 

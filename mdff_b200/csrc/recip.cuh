@@ -51,29 +51,41 @@ struct RecMesh {
   const double4* kvec;   // [nk] (kx, ky, kz, kcoe)
 };
 
-// per-ion phase tables: [n][natm], X: n = 0..kx, Y: 0..ky, Z: 0..max(kz, 4).
+// per-ion phase tables: [n][natm], X: n = 0..kx, Y: 0..ky, Z: 0..kzt (max(kz, 4)).
 // s is wrapped to [-0.5, 0.5) first: e^{2 pi i n s} is periodic in s.
-template <typename R>
-static __global__ void k_rec_tables(const double4* __restrict__ s, int natm, int kx, int ky, int kz,
-                             typename cplx<R>::T* __restrict__ tab) {
+// tab32 (mixed): the same values rounded.  img (mixed, dipoles): those of the ions
+// with a slot (slot[i] >= 0), n <= kz, blocked by 32 slots for the tensor-core structure
+// factor: block b holds the rows X_0..X_kx, Y_0..Y_ky, Z_0..Z_kz of slots 32 b .. 32 b +
+// 31, rw float2 per row (entries of no slot stay zero), so that one bulk copy
+// stages a block.
+// grid (ions / 128, entry groups): the sines of an ion are independent; one thread
+// per ion and a kernel per precision and for the blocks took 27 + 38 + 15 us in a step of
+// 8000 ions, kmax 16 (408,000 sines), this kernel 14 us beside the
+// short-range pass (2.2 us alone for 1728 ions, kmax 10; was 5.4).
+constexpr int kTabEntries = 4;  // entries per thread
+static __global__ void __launch_bounds__(128) k_rec_tables(const double4* __restrict__ s, int natm, int kx, int ky,
+                                                           int kz, int kzt, double2* __restrict__ tab,
+                                                           float2* __restrict__ tab32, float2* __restrict__ img,
+                                                           const int* __restrict__ slot, int rw) {
   pdl_wait();
   pdl_trigger();
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= natm) return;
-  double sv[3] = {s[i].x, s[i].y, s[i].z};
-  int km[3] = {kx, ky, kz};
-  int off = 0;
-  for (int a = 0; a < 3; ++a) {
-    double w = sv[a] - rint(sv[a]);
-    for (int n = 0; n <= km[a]; ++n) {
-      double sn, cs;
-      sincospi(2.0 * (double)n * w, &sn, &cs);
-      typename cplx<R>::T v;
-      v.x = (R)cs;
-      v.y = (R)sn;
-      tab[(size_t)(off + n) * natm + i] = v;
+  const double4 si = s[i];
+  const int sl = img ? slot[i] : -1, nx = kx + 1, nxy = nx + ky + 1, nt = nxy + kzt + 1, tr = nxy + kz + 1;
+  const int e0 = blockIdx.y * kTabEntries, e1 = min(e0 + kTabEntries, nt);
+  for (int e = e0; e < e1; ++e) {
+    const int n = e < nx ? e : e < nxy ? e - nx : e - nxy;
+    const double sv = e < nx ? si.x : e < nxy ? si.y : si.z;
+    const double w = sv - rint(sv);
+    double sn, cs;
+    sincospi(2.0 * (double)n * w, &sn, &cs);
+    tab[(size_t)e * natm + i] = make_double2(cs, sn);
+    if (tab32) {
+      const float2 v = make_float2((float)cs, (float)sn);
+      tab32[(size_t)e * natm + i] = v;
+      if (sl >= 0 && e < tr) img[((size_t)(sl >> 5) * tr + e) * rw + (sl & 31)] = v;
     }
-    off += km[a] + 1;
   }
 }
 

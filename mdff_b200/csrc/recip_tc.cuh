@@ -225,29 +225,6 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t
 }
 }  // namespace tc
 
-// The phase tables of the structure factor blocked by K block, once per call
-// (positions fixed): block kb holds the rows X_0..X_kx, Y_0..Y_ky, Z_0..Z_kz
-// of ion slots 32 kb .. 32 kb + 31 (slot s is ion imap[s], or s without a
-// map; zero past nion slots), each row 32 complex values
-// and 16 bytes of padding (kStageRow bytes: the bank-spread row stride of the
-// staging buffers), so that one bulk copy stages a K block.
-// grid = K blocks, 256 threads.
-static __global__ void __launch_bounds__(256) k_rec_rho_timg(const float2* __restrict__ tab, int natm,
-                                                             const int* __restrict__ imap, int nion, int kx,
-                                                             int ky, int kz, float2* __restrict__ img) {
-  pdl_wait();
-  pdl_trigger();
-  constexpr int RW = kStageRow / (int)sizeof(float2);  // row width in float2 (32 ions + padding)
-  const int TR = kx + ky + kz + 3;
-  float2* blk = img + (size_t)blockIdx.x * TR * RW;
-  for (int e = threadIdx.x; e < TR * RW; e += blockDim.x) {
-    const int t = e / RW, j = e % RW;
-    const int sl = blockIdx.x * kRhoTcKB + j;
-    const int i = (j < kRhoTcKB && sl < nion) ? (imap ? imap[sl] : sl) : -1;
-    blk[e] = i >= 0 ? tab[(size_t)t * natm + i] : make_float2(0.f, 0.f);
-  }
-}
-
 // structure factor of the dipoles on the tensor cores.  grid = (row tiles of
 // 64 mesh rows, ion chunks of a multiple of 32 ions), one CTA per SM;
 // part[chunk][k] = this chunk's rho(k).  The K dimension runs over ion slots
