@@ -282,7 +282,7 @@ size_t smem_with_stage(mdff_batch* h, size_t base, int threads, int* extra) {
 int prepare_shape(mdff_batch* h, Shape sh, int* nclusters) {
   size_t smem = smem_with_stage(h, batch_smem_bytes(h->nmax), sh.threads, &h->stage_extra);
   void (*fn)(BatchArgs, int) = h->mixed ? k_batch<true> : k_batch<false>;
-  BCK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  BCK(allow_smem((const void*)fn, smem));
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1062,7 +1062,7 @@ int mdff_gpu_batch_adjoint(mdff_batch_handle h, const double* gE, const double* 
     h->err = "configurations too large for the adjoint's shared-memory layout";
     return MDFF_ERR_BAD_ARGS;
   }
-  BCK(cudaFuncSetAttribute(k_batch_adjoint, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  BCK(allow_smem((const void*)k_batch_adjoint, smem));
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;

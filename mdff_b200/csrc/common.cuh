@@ -279,4 +279,19 @@ struct SlotW {
   }
 };
 
+// Dynamic shared memory up to the device's limit for a kernel that needs `need` bytes.  The
+// attribute belongs to the function, not to a handle: set to one handle's
+// size it would make the launches of another with a larger mesh or box fail.
+inline cudaError_t allow_smem(const void* fn, size_t need) {
+  int dev = 0, most = 0;
+  cudaFuncAttributes a;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (!e) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (!e) e = cudaFuncGetAttributes(&a, fn);
+  if (e) return e;
+  most -= (int)a.sharedSizeBytes;
+  if (need > (size_t)most) return cudaErrorInvalidValue;
+  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+}
+
 }  // namespace mdff

@@ -444,18 +444,18 @@ static void rho_dm_shape(const mdff_ctx* h, int nion, int* chunk, int* nchunk) {
 }
 template <int NT>
 static int rho_dm_attr(int smem) {
-  if (cudaFuncSetAttribute(k_rho_dm<NT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+  if (allow_smem((const void*)k_rho_dm<NT, true>, smem) != cudaSuccess)
     return 1;
-  return cudaFuncSetAttribute(k_rho_dm<NT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess;
+  return allow_smem((const void*)k_rho_dm<NT, false>, smem) != cudaSuccess;
 }
 // most staged rows of k_field_dm (two blocks per SM up to 9 steps)
 static int field_dm_rc(int ks) { return (ks <= 9 ? 100 : 200) * 1024 / (field_dm_rl(ks) * 8 + 16) / 4 * 4; }
 template <int KS>
 static int field_dm_attr_k() {
   const int smem = field_dm_rc(KS) * (field_dm_rl(KS) * 8 + 16);
-  if (cudaFuncSetAttribute(k_field_dm<KS, DM_FIELD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
-      cudaFuncSetAttribute(k_field_dm<KS, DM_FORCE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
-      cudaFuncSetAttribute(k_field_dm<KS, DM_EFG>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+  if (allow_smem((const void*)k_field_dm<KS, DM_FIELD>, smem) != cudaSuccess ||
+      allow_smem((const void*)k_field_dm<KS, DM_FORCE>, smem) != cudaSuccess ||
+      allow_smem((const void*)k_field_dm<KS, DM_EFG>, smem) != cudaSuccess)
     return 1;
   return 0;
 }
@@ -593,8 +593,7 @@ static int build_mesh(mdff_ctx* h) {
     }
   }
   if (h->rho_tc)
-    CK(cudaFuncSetAttribute(k_rec_rho_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)rho_tc_smem(h->p.kES[0], h->p.kES[1], h->p.kES[2])));
+    CK(allow_smem((const void*)k_rec_rho_tc, rho_tc_smem(h->p.kES[0], h->p.kES[1], h->p.kES[2])));
   {
     const char* env = std::getenv("MDFF_FIELD_TC");
     int kf = field_tc_kf(h->p.kES[2]);
@@ -607,10 +606,10 @@ static int build_mesh(mdff_ctx* h) {
       DALLOC(h->d_fb, (size_t)cdiv(nrows, field_tc_rpt(true)) * 2 * 128 * kf);
       int smem = (int)field_tc_smem(kf, h->p.kES[1]);
       cudaError_t e = cudaSuccess;
-#define FTA(KF)                                                                                                     \
-  {                                                                                                                 \
-    e = cudaFuncSetAttribute(k_rec_field_tc<true, KF>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);          \
-    if (!e) e = cudaFuncSetAttribute(k_rec_field_tc<false, KF>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); \
+#define FTA(KF)                                                      \
+  {                                                                  \
+    e = allow_smem((const void*)k_rec_field_tc<true, KF>, smem);     \
+    if (!e) e = allow_smem((const void*)k_rec_field_tc<false, KF>, smem); \
   }
       FIELD_TC_SWITCH(kf, FTA)
 #undef FTA
