@@ -709,6 +709,15 @@ static int upload_cell(mdff_ctx* h) {
 // ---------------------------------------------------------------------------
 // device passes
 
+// warps per block of k_build_rows<true> (a bitmap of the ions each, 100 KB in all so
+// that two blocks share an SM), 0: too many ions (262144) for a bitmap per warp
+static size_t list_map_bytes(int n) { return (size_t)cdiv(n, 32) * sizeof(unsigned); }
+static int list_map_warps(int n) {
+  int w = 8;
+  while (w > 1 && list_map_bytes(n) * w > 100 * 1024) w /= 2;
+  return list_map_bytes(n) <= 32 * 1024 ? w : 0;
+}
+
 static int list_update(mdff_ctx* h) {
   int n = h->natm;
   int pr = prof_begin(h, KC_LIST, 0);
@@ -723,14 +732,21 @@ static int list_update(mdff_ctx* h) {
   }
   PDL_CHECK(pdl_launch(k_cell_count, dim3(cdiv(n, 256)), dim3(256), 0, h->st, h->d_s, n, h->L));
   PDL_CHECK(pdl_launch(k_cell_scan, dim3(1), dim3(1024), 0, h->st, h->L, h->ncell));
-  PDL_CHECK(pdl_launch(k_cell_scatter, dim3(cdiv(n, 256)), dim3(256), 0, h->st, n, h->L));
+  PDL_CHECK(pdl_launch(k_cell_scatter, dim3(cdiv(n, 256)), dim3(256), 0, h->st, (const double4*)h->d_s, n, h->L));
   // grid-stride build and sort: a step without a rebuild launches a few
   // blocks per SM that read the flag and leave
   int nsm = h->nsm > 0 ? h->nsm : 148;
-  PDL_CHECK(pdl_launch(k_build_rows, dim3(std::min(cdiv((long)n * 32, 256), 8 * nsm)), dim3(256), 0, h->st, h->d_s, n, h->d_cell, h->L));
-  int P = 1;
-  while (P < h->L.cap) P <<= 1;
-  PDL_CHECK(pdl_launch(k_sort_rows, dim3(std::min(n, 8 * nsm)), dim3(256), P * sizeof(int), h->st, h->L, n));
+  const int wpb = list_map_warps(n);
+  if (wpb) {
+    PDL_CHECK(pdl_launch(k_build_rows<true>, dim3(std::min(cdiv(n, wpb), 64 / wpb * nsm)), dim3(32 * wpb),
+                         list_map_bytes(n) * wpb, h->st, (const double4*)h->d_s, n, (const CellC*)h->d_cell, h->L));
+  } else {
+    PDL_CHECK(pdl_launch(k_build_rows<false>, dim3(std::min(cdiv((long)n * 32, 256), 8 * nsm)), dim3(256), 0, h->st,
+                         (const double4*)h->d_s, n, (const CellC*)h->d_cell, h->L));
+    int P = 1;
+    while (P < h->L.cap) P <<= 1;
+    PDL_CHECK(pdl_launch(k_sort_rows, dim3(std::min(n, 8 * nsm)), dim3(256), P * sizeof(int), h->st, h->L, n));
+  }
   PDL_CHECK(pdl_launch(k_build_done, dim3(cdiv(n, 256)), dim3(256), 0, h->st, h->d_s, n, h->L));
   PDL_CHECK(pdl_launch(k_build_clear, dim3(1), dim3(256), 0, h->st, h->L, h->ncell));
   prof_end(h, pr);
@@ -2761,7 +2777,9 @@ static int create_impl(mdff_ctx* h, const mdff_params* pin, const double* cellA)
   DALLOC(h->L.flags, 4);
   DALLOC(h->L.sref, n);
   DALLOC(h->L.cell_of, n);
-  DALLOC(h->L.cell_atoms, n);
+  DALLOC(h->L.cell_pos, n);
+  if (const int wpb = list_map_warps(n))
+    CK(allow_smem((const void*)k_build_rows<true>, list_map_bytes(n) * wpb));
   DALLOC(h->d_disp_part, cdiv(n, 256));
   CK(cudaMallocHost((void**)&h->h_flags, sizeof(int) * 4));
   lattice(h, cellA);
@@ -3220,7 +3238,7 @@ void mdff_gpu_destroy(mdff_handle h) {
   void* ptrs[] = {h->d_cell, h->d_pos, h->d_s, h->d_itype, h->d_ipolar, h->d_q, h->d_qzero,
                   h->d_dipia, h->d_pol, h->d_invpol, h->d_nbtab, h->d_estab, h->L.nbr, h->L.nnb,
                   h->L.flags, h->L.sref, h->L.cell_of, h->L.cell_count, h->L.cell_start,
-                  h->L.cell_fill, h->L.cell_atoms, h->d_disp_part, h->d_rows, h->d_Ak, h->d_kvec,
+                  h->L.cell_fill, h->L.cell_pos, h->d_disp_part, h->d_rows, h->d_Ak, h->d_kvec,
                   h->d_rchunk, h->d_tab64, h->d_tab32, h->d_w, h->d_w32, h->d_rho_part, h->d_rhoA, h->d_str,
                   h->d_G, h->d_H, h->d_Estat, h->d_Eind, h->d_Efield, h->d_mu_ind, h->d_mu_tot,
                   h->d_hist, h->d_E, h->d_r, h->d_z, h->d_pv, h->d_qv, h->d_Tp, h->d_mu32, h->d_force,
