@@ -168,14 +168,15 @@ __device__ __forceinline__ void sr_pair_lj(const NBPair& P, int trunc, R rijsq, 
 // MODE bit 0: BMH / BMHFTD (+ wall), bit 1: n-m LJ.  One instantiation per
 // mode keeps the accumulators of the absent potential out of the registers.
 template <typename R, int MODE>
-static __global__ void __launch_bounds__(256, MODE == 3 ? 2 : 4) k_shortrange(
+static __global__ void __launch_bounds__(256, MODE == 3 ? 2 : 3) k_shortrange(
     const double4* __restrict__ s, const int* __restrict__ itype, const int* __restrict__ nbr,
     const int* __restrict__ nnb, int cap, int natm, const CellC* __restrict__ cell,
     const NBPair* __restrict__ tab, int ntype, int lbmhftd, int trunc,
     double* __restrict__ force /* SoA [3][natm] */, double* __restrict__ part) {
   constexpr bool do_bmh = (MODE & 1) != 0, do_lj = (MODE & 2) != 0;
   __shared__ NBPair stab[MDFF_NT * MDFF_NT];
-  __shared__ double red[kSRPart * 8];
+  __shared__ double red[kSRPart * 8], cA[9];
+  if (threadIdx.x < 9) cA[threadIdx.x] = cell->A[threadIdx.x];
   for (int k = threadIdx.x; k < ntype * ntype; k += blockDim.x) stab[k] = tab[k];
   __syncthreads();
   int lane = threadIdx.x & 31;
@@ -189,12 +190,14 @@ static __global__ void __launch_bounds__(256, MODE == 3 ? 2 : 4) k_shortrange(
     int ti = itype[i];
     int n = nnb[i];
     const int* row = nbr + (size_t)i * cap;
+    int jn = lane < n ? row[lane] : 0;
     for (int k = lane; k < n; k += 32) {
-      int j = row[k];
+      const int j = jn;
+      if (k + 32 < n) jn = row[k + 32];
       double4 sj = s[j];
       int tj = tag_type(sj.w);
       double rxd, ryd, rzd;
-      double r2d = min_image_exact(cell->A, xsub(si.x, sj.x), xsub(si.y, sj.y), xsub(si.z, sj.z),
+      double r2d = min_image_exact(cA, xsub(si.x, sj.x), xsub(si.y, sj.y), xsub(si.z, sj.z),
                                    rxd, ryd, rzd);
       const NBPair& P = stab[ti * ntype + tj];
       if (r2d >= P.rcutsq) continue;  // non_bonded.f90:1154 strict <
@@ -208,14 +211,13 @@ static __global__ void __launch_bounds__(256, MODE == 3 ? 2 : 4) k_shortrange(
         fb[0] += (double)fx;
         fb[1] += (double)fy;
         fb[2] += (double)fz;
-        acc[0] += 0.5 * (double)u;
-        acc[1] += 0.5 * (double)(rx * fx + ry * fy + rz * fz);
-        acc[4] += (double)(rx * fx);  // 0.5*(r_a f_b + r_b f_a) on the diagonal = r_a f_a
+        acc[0] += (double)u;
+        acc[4] += (double)(rx * fx);  // 0.5*(r_a f_b + r_b f_a) = r_a f_b: f is along r
         acc[5] += (double)(ry * fy);
         acc[6] += (double)(rz * fz);
-        acc[7] += 0.5 * (double)(rx * fy + ry * fx);
-        acc[8] += 0.5 * (double)(rx * fz + rz * fx);
-        acc[9] += 0.5 * (double)(ry * fz + rz * fy);
+        acc[7] += (double)(rx * fy);
+        acc[8] += (double)(rx * fz);
+        acc[9] += (double)(ry * fz);
       }
       if (do_lj) {
         R e, wij;
@@ -224,16 +226,20 @@ static __global__ void __launch_bounds__(256, MODE == 3 ? 2 : 4) k_shortrange(
         fl[0] += (double)fx;
         fl[1] += (double)fy;
         fl[2] += (double)fz;
-        acc[2] += 0.5 * (double)e;
-        acc[3] += 0.5 * (double)(wij * rijsq);
+        acc[2] += (double)e;
         acc[10] += (double)(rx * fx);
         acc[11] += (double)(ry * fy);
         acc[12] += (double)(rz * fz);
-        acc[13] += 0.5 * (double)(rx * fy + ry * fx);
-        acc[14] += 0.5 * (double)(rx * fz + rz * fx);
-        acc[15] += 0.5 * (double)(ry * fz + rz * fy);
+        acc[13] += (double)(rx * fy);
+        acc[14] += (double)(rx * fz);
+        acc[15] += (double)(ry * fz);
       }
     }
+    // every pair is visited from both sides; the virial is the trace
+    acc[0] *= 0.5;
+    acc[2] *= 0.5;
+    acc[1] = 0.5 * (acc[4] + acc[5] + acc[6]);
+    acc[3] = 0.5 * (acc[10] + acc[11] + acc[12]);
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
       fb[a] = warp_sum(fb[a]);
@@ -1068,8 +1074,10 @@ static __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 2) k_es_force
     R la[kESPart];
 #pragma unroll
     for (int k = 0; k < kESPart; ++k) la[k] = R(0);
+    int jn = lane < n ? row[lane] : 0;
     for (int k = lane; k < n; k += 32) {
-      const int j = row[k];
+      const int j = jn;
+      if (k + 32 < n) jn = row[k + 32];
       const double4 sj = s[j];
       R r[3];
       const R r2 = pvec<R>(cA, A32, si, sj, r);
