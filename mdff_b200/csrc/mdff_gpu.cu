@@ -54,7 +54,12 @@ enum {
   S_CGP = 64,    // CG plan of the graph: 64 rmsd of the FP64 residual, 65 stop,
                  // 66 outer iterations, 67 recurrence trusted
   S_SCF = 68,    // 2: iterations and rmsd of the SCF loop on the device
-  S_NSCAL = 72
+  S_NSCAL = 72,
+  // beside the scalars, so that one copy brings all a call's host needs
+  S_CATA = 72,   // 4 ints: d_cata
+  S_FLAGS = 74,  // 4 ints: the list's flags
+  S_EKIN = 76,   // kinetic energy of the last MD step
+  S_NALL = 77
 };
 
 // FP32 CG: the recurrence residual drifts from the true one by about the FP32
@@ -212,6 +217,7 @@ struct mdff_ctx {
   int* d_lwfc = nullptr;
   double4* d_mu_wfc = nullptr;
   double* d_pack = nullptr;      // [natm][3] staging for mu/ef output
+  double* h_stage = nullptr;     // pinned: positions [3][natm], outputs [9 natm] (host arrays of a call)
   double* d_ekin_part = nullptr;
   // stats
   mdff_stats stats{};
@@ -418,6 +424,42 @@ __global__ void k_vv_kick(double* __restrict__ vel, const double* __restrict__ f
   }
   block_sum<1>(e, red);
   if (threadIdx.x == 0) part[blockIdx.x] = e[0];
+}
+// k_vv_kick of one step, then k_vv_kick_drift of the next (the same operations)
+__global__ void k_vv_step(double* __restrict__ pos, double* __restrict__ vel, const double* __restrict__ f,
+                          const double* __restrict__ invm, int natm, double dt, double* __restrict__ part) {
+  pdl_wait();
+  pdl_trigger();
+  __shared__ double red[32];
+  double e[1] = {0.0};
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < natm) {
+    const double im = invm[i];
+    for (int a = 0; a < 3; ++a) {
+      size_t k = (size_t)a * natm + i;
+      double v = vel[k] + 0.5 * dt * f[k] * im;
+      e[0] += 0.5 * v * v / im;
+      v = v + 0.5 * dt * f[k] * im;
+      vel[k] = v;
+      pos[k] += dt * v;
+    }
+  }
+  block_sum<1>(e, red);
+  if (threadIdx.x == 0) part[blockIdx.x] = e[0];
+}
+
+// results of a call into mapped pinned host memory: force [3][natm], then mu
+// and E as [natm][3] (absent ones skipped)
+__global__ void k_outputs(const double* __restrict__ force, const double4* __restrict__ mu,
+                          const double4* __restrict__ E, int natm, double* __restrict__ out) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, n3 = 3 * natm;
+  if (t < n3) {
+    out[t] = force[t];
+  } else if (t < 3 * n3) {
+    const int e = (t - n3) % n3;
+    const double4* v = t < 2 * n3 ? mu : E;
+    if (v) out[t] = reinterpret_cast<const double*>(v + e / 3)[e % 3];
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -2272,7 +2314,8 @@ static int ef_front(mdff_ctx* h, bool fp32) {
   PDL_CHECK(pdl_launch(k_kardir, dim3(cdiv(n, 256)), dim3(256), 0, h->st, h->d_pos, n, h->d_cell, h->d_itype,
                        h->d_ipolar, h->d_q, h->d_s));
   if ((s = list_update(h))) return s;
-  CK(cudaMemsetAsync(h->d_scal, 0, sizeof(double) * S_NSCAL, h->st));
+  // (and the per-call flags: [0] catastrophe, [1] a tensor-core wait gave up, [2] Wannier count)
+  CK(cudaMemsetAsync(h->d_scal, 0, sizeof(double) * S_NSCAL + 3 * sizeof(int), h->st));
   int nbw = cdiv((long)n * 32, 256);
   if (h->lsr) {
     int do_bmh = (h->p.lbmhft || h->p.lbmhftd) ? 1 : 0;
@@ -2296,8 +2339,6 @@ static int ef_front(mdff_ctx* h, bool fp32) {
     k_reduce_partials<<<kSRPart, 256, 0, ss>>>(h->d_part2, nbw, kSRPart, h->d_scal + S_SR);
     LAUNCH_CHECK();
   }
-  // per-call flags: [0] catastrophe, [1] a tensor-core wait gave up, [2] Wannier count
-  CK(cudaMemsetAsync(h->d_cata, 0, 3 * sizeof(int), h->st));
   if (h->p.lcoulomb) {
     if ((s = build_tables(h))) return s;
     CK(cudaMemsetAsync(h->d_mu_ind, 0, sizeof(double4) * n, h->st));
@@ -2380,9 +2421,7 @@ static int ef_back(mdff_ctx* h, bool fp32) {
     if (s) return s;
   }
   if ((s = rs_join(h))) return s;
-  CK(cudaMemcpyAsync(h->h_scal, h->d_scal, sizeof(double) * S_NSCAL, cudaMemcpyDeviceToHost, h->st));
-  CK(cudaMemcpyAsync(h->h_flags, h->L.flags, sizeof(int) * 4, cudaMemcpyDeviceToHost, h->st));
-  CK(cudaMemcpyAsync(h->h_cata, h->d_cata, 3 * sizeof(int), cudaMemcpyDeviceToHost, h->st));
+  CK(cudaMemcpyAsync(h->h_scal, h->d_scal, sizeof(double) * S_NALL, cudaMemcpyDeviceToHost, h->st));
   return MDFF_OK;
 }
 
@@ -2774,14 +2813,18 @@ static int create_impl(mdff_ctx* h, const mdff_params* pin, const double* cellA)
   h->L.rskinsq = h->rskin_build * h->rskin_build;
   h->L.skindiff = p.skindiff;
   DALLOC(h->L.nnb, n);
-  DALLOC(h->L.flags, 4);
+  DALLOC(h->d_scal, S_NALL);
+  h->d_cata = (int*)(h->d_scal + S_CATA);
+  h->L.flags = (int*)(h->d_scal + S_FLAGS);
   DALLOC(h->L.sref, n);
   DALLOC(h->L.cell_of, n);
   DALLOC(h->L.cell_pos, n);
   if (const int wpb = list_map_warps(n))
     CK(allow_smem((const void*)k_build_rows<true>, list_map_bytes(n) * wpb));
   DALLOC(h->d_disp_part, cdiv(n, 256));
-  CK(cudaMallocHost((void**)&h->h_flags, sizeof(int) * 4));
+  CK(cudaMallocHost((void**)&h->h_scal, sizeof(double) * S_NALL));
+  h->h_cata = (int*)(h->h_scal + S_CATA);
+  h->h_flags = (int*)(h->h_scal + S_FLAGS);
   lattice(h, cellA);
   double dens = n / h->omega;
   double est = 4.0 / 3.0 * kPi * h->rskin_build * h->rskin_build * h->rskin_build * dens * 1.4 + 64;
@@ -2838,8 +2881,6 @@ static int create_impl(mdff_ctx* h, const mdff_params* pin, const double* cellA)
   h->part_cap = std::max(h->part_cap, (size_t)8 * std::max(h->nsm, 148));
   DALLOC(h->d_part, h->part_cap);
   DALLOC(h->d_part2, h->part_cap);
-  DALLOC(h->d_scal, S_NSCAL);
-  DALLOC(h->d_cata, 4);  // [0] catastrophe, [1] a tensor-core wait gave up, [2] Wannier count
   k_seti<<<1, 32, 0, h->st>>>(h->d_cata + 3, -1);  // [3] default operand-wait limit
   LAUNCH_CHECK();
   for (int it = 0; it < p.ntype; ++it)
@@ -2854,8 +2895,6 @@ static int create_impl(mdff_ctx* h, const mdff_params* pin, const double* cellA)
     }
   }
   DALLOC(h->d_ekin_part, cdiv(n, 256));
-  CK(cudaMallocHost((void**)&h->h_scal, sizeof(double) * S_NSCAL));
-  CK(cudaMallocHost((void**)&h->h_cata, 3 * sizeof(int)));
   CK(cudaStreamSynchronize(h->st));
   return MDFF_OK;
 }
@@ -2887,8 +2926,48 @@ int mdff_gpu_set_cell(mdff_handle h, const double cell_A[9]) {
   return MDFF_OK;
 }
 
+// Host arrays of a call pass through one pinned buffer up to this many ions (25
+// MB): one copy of the positions instead of three from pageable memory (10 us
+// each), one kernel that writes every result across the bus instead of five copies and
+// two packing kernels with a synchronisation between (1728 ions: 30 + 110 us, now
+// about 5 + 15).
+constexpr int kHostStage = 262144;
+static bool host_stage(mdff_ctx* h) {
+  if (h->natm > kHostStage) return false;
+  if (!h->h_stage && cudaMallocHost((void**)&h->h_stage, sizeof(double) * 12 * (size_t)h->natm) != cudaSuccess) {
+    cudaGetLastError();
+    h->h_stage = nullptr;
+  }
+  return h->h_stage != nullptr;
+}
+static int positions_to_device(mdff_ctx* h, const double* rx, const double* ry, const double* rz) {
+  const size_t n = h->natm;
+  const double* r[3] = {rx, ry, rz};
+  if (host_stage(h)) {
+    for (int a = 0; a < 3; ++a) memcpy(h->h_stage + a * n, r[a], sizeof(double) * n);
+    CK(cudaMemcpyAsync(h->d_pos, h->h_stage, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, h->st));
+    return MDFF_OK;
+  }
+  for (int a = 0; a < 3; ++a)
+    CK(cudaMemcpyAsync(h->d_pos + a * n, r[a], sizeof(double) * n, cudaMemcpyHostToDevice, h->st));
+  return MDFF_OK;
+}
+
 static int outputs_to_host(mdff_ctx* h, mdff_result* out) {
   int n = h->natm;
+  if (host_stage(h)) {
+    double* o = h->h_stage + 3 * (size_t)n;
+    k_outputs<<<cdiv(9L * n, 256), 256, 0, h->st>>>(h->d_force, out->mu ? h->d_mu_tot : nullptr,
+                                                    out->ef ? h->d_E : nullptr, n, o);
+    LAUNCH_CHECK();
+    CK(cudaStreamSynchronize(h->st));
+    memcpy(out->fx, o, sizeof(double) * n);
+    memcpy(out->fy, o + n, sizeof(double) * n);
+    memcpy(out->fz, o + 2 * (size_t)n, sizeof(double) * n);
+    if (out->mu) memcpy(out->mu, o + 3 * (size_t)n, sizeof(double) * 3 * n);
+    if (out->ef) memcpy(out->ef, o + 6 * (size_t)n, sizeof(double) * 3 * n);
+    return MDFF_OK;
+  }
   CK(cudaMemcpyAsync(out->fx, h->d_force, sizeof(double) * n, cudaMemcpyDeviceToHost, h->st));
   CK(cudaMemcpyAsync(out->fy, h->d_force + n, sizeof(double) * n, cudaMemcpyDeviceToHost, h->st));
   CK(cudaMemcpyAsync(out->fz, h->d_force + 2 * (size_t)n, sizeof(double) * n, cudaMemcpyDeviceToHost, h->st));
@@ -2912,13 +2991,11 @@ int mdff_gpu_engforce(mdff_handle h, const double* rx, const double* ry, const d
                       int itime, mdff_result* out) {
   if (!h || !rx || !ry || !rz || !out || !out->fx || !out->fy || !out->fz) return MDFF_ERR_BAD_ARGS;
   CK(cudaSetDevice(h->device));
-  int n = h->natm;
   h->md_valid = false;
   call_begin(h);
-  CK(cudaMemcpyAsync(h->d_pos, rx, sizeof(double) * n, cudaMemcpyHostToDevice, h->st));
-  CK(cudaMemcpyAsync(h->d_pos + n, ry, sizeof(double) * n, cudaMemcpyHostToDevice, h->st));
-  CK(cudaMemcpyAsync(h->d_pos + 2 * (size_t)n, rz, sizeof(double) * n, cudaMemcpyHostToDevice, h->st));
-  int s = engforce_retry(h, itime);
+  int s = positions_to_device(h, rx, ry, rz);
+  if (s) return s;
+  s = engforce_retry(h, itime);
   if (s != MDFF_OK && s != MDFF_ERR_CATASTROPHE && s != MDFF_ERR_NOT_CONVERGED) return s;
   fill_scalars(h, out);
   int s2 = outputs_to_host(h, out);
@@ -3074,22 +3151,40 @@ int mdff_gpu_md_nve(mdff_handle h, double* d_pos, double* d_vel, const double* d
     if (s) return s;
   }
   h->md_valid = false;
+  // The second kick of a step is one kernel with the first kick and the drift of
+  // the next; its kinetic energy comes to the host with the scalars of the next
+  // step's forces, so that a step has one synchronisation.
+  const int nb = cdiv(n, 256);
+  double* d_ek = h->d_scal + S_EKIN;
   for (int step = 0; step < nsteps; ++step) {
-    PDL_CHECK(pdl_launch(k_vv_kick_drift, dim3(cdiv(n, 256)), dim3(256), 0, h->st, h->d_pos, d_vel, h->d_force, d_invmass, n, dt));
+    if (step == 0) {
+      PDL_CHECK(pdl_launch(k_vv_kick_drift, dim3(nb), dim3(256), 0, h->st, h->d_pos, d_vel, h->d_force, d_invmass, n, dt));
+    } else {
+      PDL_CHECK(pdl_launch(k_vv_step, dim3(nb), dim3(256), 0, h->st, h->d_pos, d_vel, (const double*)h->d_force,
+                           d_invmass, n, dt, h->d_ekin_part));
+      PDL_CHECK(pdl_launch(k_reduce_partials, dim3(1), dim3(256), 0, h->st, (const double*)h->d_ekin_part, nb, 1, d_ek));
+    }
+    h->launches_call += step ? 2 : 1;
     s = engforce_retry(h, itime0 + step + 1);
+    if (ekin_pot && step > 0) {
+      if (s) {  // (the call may not have read the scalars)
+        double ek;
+        const int e = read_scal(h, S_EKIN, &ek);
+        if (e) return e;
+      }
+      ekin_pot[2 * (step - 1)] = h->h_scal[S_EKIN];
+    }
     if (s) return s;
-    int nb = cdiv(n, 256);
-    PDL_CHECK(pdl_launch(k_vv_kick, dim3(nb), dim3(256), 0, h->st, d_vel, h->d_force, d_invmass, n, dt, h->d_ekin_part));
-    k_reduce_partials<<<1, 256, 0, h->st>>>(h->d_ekin_part, nb, 1, h->d_scal + S_NSCAL - 1);
-    LAUNCH_CHECK();
-    h->launches_call += 3;
     if (ekin_pot) {
       fill_scalars(h, &r);
-      double ek;
-      if ((s = read_scal(h, S_NSCAL - 1, &ek))) return s;
-      ekin_pot[2 * step] = ek;
       ekin_pot[2 * step + 1] = r.u_lj + r.u_bmhft + r.u_coul;
     }
+  }
+  if (nsteps > 0) {
+    PDL_CHECK(pdl_launch(k_vv_kick, dim3(nb), dim3(256), 0, h->st, d_vel, h->d_force, d_invmass, n, dt, h->d_ekin_part));
+    PDL_CHECK(pdl_launch(k_reduce_partials, dim3(1), dim3(256), 0, h->st, (const double*)h->d_ekin_part, nb, 1, d_ek));
+    h->launches_call += 2;
+    if (ekin_pot && (s = read_scal(h, S_EKIN, &ekin_pot[2 * (nsteps - 1)]))) return s;
   }
   CK(cudaMemcpyAsync(d_pos, h->d_pos, sizeof(double) * 3 * n, cudaMemcpyDeviceToDevice, h->st));
   call_end(h);
@@ -3237,12 +3332,12 @@ void mdff_gpu_destroy(mdff_handle h) {
   if (h->st) cudaStreamSynchronize(h->st);
   void* ptrs[] = {h->d_cell, h->d_pos, h->d_s, h->d_itype, h->d_ipolar, h->d_q, h->d_qzero,
                   h->d_dipia, h->d_pol, h->d_invpol, h->d_nbtab, h->d_estab, h->L.nbr, h->L.nnb,
-                  h->L.flags, h->L.sref, h->L.cell_of, h->L.cell_count, h->L.cell_start,
+                  h->L.sref, h->L.cell_of, h->L.cell_count, h->L.cell_start,
                   h->L.cell_fill, h->L.cell_pos, h->d_disp_part, h->d_rows, h->d_Ak, h->d_kvec,
                   h->d_rchunk, h->d_tab64, h->d_tab32, h->d_w, h->d_w32, h->d_rho_part, h->d_rhoA, h->d_str,
                   h->d_G, h->d_H, h->d_Estat, h->d_Eind, h->d_Efield, h->d_mu_ind, h->d_mu_tot,
                   h->d_hist, h->d_E, h->d_r, h->d_z, h->d_pv, h->d_qv, h->d_Tp, h->d_mu32, h->d_force,
-                  h->d_part, h->d_scal, h->d_cata, h->d_pack, h->d_ekin_part, h->d_ddr,
+                  h->d_part, h->d_scal, h->d_pack, h->d_ekin_part, h->d_ddr,
                   h->d_ddb1, h->d_ddj, h->d_ddn, h->d_efg, h->d_fb, h->d_ko_f, h->d_ko_dmu,
                   h->d_ko_g, h->d_ko_muprev, h->d_ko_fdir, h->d_Fh, h->d_muh, h->d_ko_x, h->d_part2,
                   h->d_lwfc, h->d_mu_wfc, h->d_qm32, h->d_Edd, h->d_fsr, h->d_hist_save,
@@ -3254,8 +3349,7 @@ void mdff_gpu_destroy(mdff_handle h) {
   if (h->cg_exec) cudaGraphExecDestroy(h->cg_exec);
   if (h->cg_graph) cudaGraphDestroy(h->cg_graph);
   if (h->h_scal) cudaFreeHost(h->h_scal);
-  if (h->h_flags) cudaFreeHost(h->h_flags);
-  if (h->h_cata) cudaFreeHost(h->h_cata);
+  if (h->h_stage) cudaFreeHost(h->h_stage);
   if (h->h_ko) cudaFreeHost(h->h_ko);
   if (h->ev_fork) cudaEventDestroy(h->ev_fork);
   if (h->ev_join_sr) cudaEventDestroy(h->ev_join_sr);
