@@ -141,7 +141,7 @@ struct mdff_ctx {
   int n_rho_chunks = 0;
   // FP64 structure factor on the tensor cores (k_rho_dm): ions a staged buffer
   // holds (0: the mesh does not fit), n tiles per pass and passes; most ion chunks
-  int dm_ci = 0, dm_nt = 0, dm_groups = 0;
+  int dm_ci[2] = {0, 0}, dm_nt[2] = {0, 0}, dm_groups[2] = {0, 0};  // [1] with dipoles, [0] charges alone
   int nsm = 0;  // SMs of the device
   // FP32 structure factor of the CG operator on the tensor cores
   // (k_rec_rho_tc): ion chunk size and count; off when the mesh does not
@@ -478,18 +478,31 @@ static void lattice(mdff_ctx* h, const double* Ain) {
 
 // ions per chunk of k_rho_dm over nion ions, and the chunks: one block per SM
 // over (row blocks x chunks x n passes), at least 16 ions a chunk
-static void rho_dm_shape(const mdff_ctx* h, int nion, int* chunk, int* nchunk) {
-  const int per = cdiv((int)h->rows.size(), kDmRows) * std::max(h->dm_groups, 1);
+static void rho_dm_shape(const mdff_ctx* h, int nion, bool hm, int* chunk, int* nchunk) {
+  const int per = cdiv((int)h->rows.size(), kDmRows) * std::max(h->dm_groups[hm], 1);
   const int want = std::max(1, (h->nsm > 0 ? h->nsm : 148) / std::max(per, 1));
   *chunk = std::max(16, cdiv(cdiv(nion, want), 8) * 8);
   *nchunk = cdiv(nion, *chunk);
 }
-template <int NT>
-static int rho_dm_attr(int smem) {
-  if (allow_smem((const void*)k_rho_dm<NT, true>, smem) != cudaSuccess)
-    return 1;
-  return allow_smem((const void*)k_rho_dm<NT, false>, smem) != cudaSuccess;
-}
+#define RHO_DM_SWITCH(NTV, CALL) \
+  switch (NTV) {                 \
+    case 1: CALL(1); break;      \
+    case 2: CALL(2); break;      \
+    case 3: CALL(3); break;      \
+    case 4: CALL(4); break;      \
+    default: CALL(5); break;     \
+  }
+#define RHO_DM_SWITCH0(NTV, CALL) \
+  switch (NTV) {                  \
+    case 1: CALL(1); break;       \
+    case 2: CALL(2); break;       \
+    case 3: CALL(3); break;       \
+    case 4: CALL(4); break;       \
+    case 5: CALL(5); break;       \
+    case 6: CALL(6); break;       \
+    case 7: CALL(7); break;       \
+    default: CALL(8); break;      \
+  }
 // most staged rows of k_field_dm (two blocks per SM up to 9 steps)
 static int field_dm_rc(int ks) { return (ks <= 9 ? 100 : 200) * 1024 / (field_dm_rl(ks) * 8 + 16) / 4 * 4; }
 template <int KS>
@@ -578,9 +591,17 @@ static int build_mesh(mdff_ctx* h) {
   DALLOC(h->d_kvec, std::max(nk, 1));
   DALLOC(h->d_rchunk, h->rchunk.size());
   h->n_rho_chunks = cdiv(h->natm, kRhoChunk);
-  h->dm_ci = nrows > 0 ? rho_dm_ci(h->p.kES[0], h->p.kES[1], h->p.kES[2]) : 0;
-  h->dm_nt = rho_dm_nt(h->p.kES[2]);
-  h->dm_groups = rho_dm_groups(h->p.kES[2]);
+  for (int hm = 1; hm >= 0; --hm) {
+    // (charges alone: not at the price of smaller stagings)
+    int nt = rho_dm_nt(h->p.kES[2], hm), ci = rho_dm_ci(h->p.kES[0], h->p.kES[1], nt);
+    if (!hm && ci < h->dm_ci[1]) {
+      nt = h->dm_nt[1];
+      ci = h->dm_ci[1];
+    }
+    h->dm_nt[hm] = nt;
+    h->dm_ci[hm] = nrows > 0 ? ci : 0;
+    h->dm_groups[hm] = cdiv(h->p.kES[2] / 4 + 1, nt);
+  }
   {
     // tensor-core structure factor: one CTA per SM over (row tiles x ion chunks)
     const char* env = std::getenv("MDFF_REC_TC");
@@ -610,19 +631,23 @@ static int build_mesh(mdff_ctx* h) {
       CK(cudaMemcpy(h->d_polslot, slot.data(), sizeof(int) * h->natm, cudaMemcpyHostToDevice));
     }
   }
-  int dm_chunks = 0, dm_len = 0;
-  rho_dm_shape(h, h->natm, &dm_len, &dm_chunks);
+  int dm_chunks = 0, dm_len = 0, dm_chunks0 = 0;
+  rho_dm_shape(h, h->natm, true, &dm_len, &dm_chunks);
+  rho_dm_shape(h, h->natm, false, &dm_len, &dm_chunks0);
+  dm_chunks = std::max(dm_chunks, dm_chunks0);
   DALLOC(h->d_rho_part, (size_t)std::max({h->n_rho_chunks, h->n_tc_chunks, dm_chunks}) * std::max(nk, 1));
-  if (h->dm_ci) {
-    const int smem = (int)rho_dm_smem(h->p.kES[0], h->p.kES[1], h->p.kES[2], h->dm_ci);
+  if (h->dm_ci[1]) {
     int e = 0;
-    switch (h->dm_nt) {
-      case 1: e = rho_dm_attr<1>(smem); break;
-      case 2: e = rho_dm_attr<2>(smem); break;
-      case 3: e = rho_dm_attr<3>(smem); break;
-      case 4: e = rho_dm_attr<4>(smem); break;
-      default: e = rho_dm_attr<5>(smem); break;
+#define RDA(NT) e = allow_smem((const void*)k_rho_dm<NT, HM>, rho_dm_smem(h->p.kES[0], h->p.kES[1], NT, h->dm_ci[HM]))
+    {
+      constexpr bool HM = true;
+      RHO_DM_SWITCH(h->dm_nt[1], RDA)
     }
+    if (!e) {
+      constexpr bool HM = false;
+      RHO_DM_SWITCH0(h->dm_nt[0], RDA)
+    }
+#undef RDA
     if (e) {
       h->err = "shared memory of k_rho_dm";
       return MDFF_ERR_CUDA;
@@ -866,31 +891,26 @@ static SlotW slotw(const mdff_ctx* h) {
 // FP64 structure factor of the weights d_w over the ions of imap (nion of them;
 // nullptr: all) into d_rho_part; returns the number of partial chunks.  Launch
 // errors surface at the caller's LAUNCH_CHECK.
-template <int NT>
-static void launch_rho_dm_n(mdff_ctx* h, dim3 g, size_t smem, const RecMesh& M, int n, const int* imap, int nion,
-                            int chunk, int has_mu) {
-  const double2* tab = h->d_tab64;
-  const double4* w = h->d_w;
-  if (has_mu)
-    (void)pdl_launch(k_rho_dm<NT, true>, g, dim3(kDmThreads), smem, h->st, tab, w, n, imap, nion, chunk, h->dm_ci, M,
-                     h->d_rho_part);
-  else
-    (void)pdl_launch(k_rho_dm<NT, false>, g, dim3(kDmThreads), smem, h->st, tab, w, n, imap, nion, chunk, h->dm_ci, M,
-                     h->d_rho_part);
-}
 static int launch_rho64(mdff_ctx* h, const RecMesh& M, int n, const int* imap, int nion, int has_q, int has_mu) {
-  if (h->dm_ci) {
+  const int hm = has_mu ? 1 : 0;
+  if (h->dm_ci[1]) {
     int chunk, nchunk;
-    rho_dm_shape(h, nion, &chunk, &nchunk);
-    const dim3 g((unsigned)cdiv(M.nrows, kDmRows), (unsigned)nchunk, (unsigned)h->dm_groups);
-    const size_t smem = rho_dm_smem(M.kmax[0], M.kmax[1], M.kmax[2], h->dm_ci);
-    switch (h->dm_nt) {
-      case 1: launch_rho_dm_n<1>(h, g, smem, M, n, imap, nion, chunk, has_mu); break;
-      case 2: launch_rho_dm_n<2>(h, g, smem, M, n, imap, nion, chunk, has_mu); break;
-      case 3: launch_rho_dm_n<3>(h, g, smem, M, n, imap, nion, chunk, has_mu); break;
-      case 4: launch_rho_dm_n<4>(h, g, smem, M, n, imap, nion, chunk, has_mu); break;
-      default: launch_rho_dm_n<5>(h, g, smem, M, n, imap, nion, chunk, has_mu); break;
+    rho_dm_shape(h, nion, hm, &chunk, &nchunk);
+    const dim3 g((unsigned)cdiv(M.nrows, kDmRows), (unsigned)nchunk, (unsigned)h->dm_groups[hm]);
+    const size_t smem = rho_dm_smem(M.kmax[0], M.kmax[1], h->dm_nt[hm], h->dm_ci[hm]);
+    const double2* tab = h->d_tab64;
+    const double4* w = h->d_w;
+#define RDL(NT)                                                                                                     \
+  (void)pdl_launch(k_rho_dm<NT, HM>, g, dim3(kDmThreads), smem, h->st, tab, w, n, imap, nion, chunk, h->dm_ci[HM], M, \
+                   h->d_rho_part)
+    if (hm) {
+      constexpr bool HM = true;
+      RHO_DM_SWITCH(h->dm_nt[1], RDL)
+    } else {
+      constexpr bool HM = false;
+      RHO_DM_SWITCH0(h->dm_nt[0], RDL)
     }
+#undef RDL
     return nchunk;
   }
   // a mesh too large for the staging buffers: the phase recurrence over all ions
@@ -1882,7 +1902,7 @@ static int cg_iteration(mdff_ctx* h, bool fp32, int in_graph, cudaGraphCondition
 // iteration).  Otherwise solve_scf's host loop runs them.
 static bool scf_device_loop(const mdff_ctx* h) {
   return h->p.lcoulomb && h->lpolar && h->p.solver == MDFF_SOLVER_SCF && h->p.precision == MDFF_PREC_FP64 &&
-         h->p.algo_moment_from_pola == MDFF_ALGO_SCF && !h->p.lsurf && h->nk > 0 && h->dm_ci &&
+         h->p.algo_moment_from_pola == MDFF_ALGO_SCF && !h->p.lsurf && h->nk > 0 && h->dm_ci[1] &&
          field_dm_ks(h->p.kES[2]) && h->d_c64r && !h->prof &&
          (h->p.max_scf_pol_iter > 0 || h->p.min_scf_pol_iter > 0);
 }
