@@ -381,7 +381,7 @@ __device__ __forceinline__ double4* brec_weights(BRecArgs& r, const BShared& S, 
 // polarisable ions with the vector in S.v / S.v32 by rank.  The field sums are
 // left in this CTA's gpart for all its ions or (dst_pol) its polarisable ones;
 // bfld_get reads them.  With do_str, es[0..6] receives this CTA's share of
-// (u_rec, tau_rec) scaled as k_rec_energy.  Returns the number of row subsets.
+// (u_rec, tau_rec) scaled as in k_rec_field_sum.  Returns the number of row subsets.
 __device__ __noinline__ int brec(cgx::cluster_group& cl, const BatchArgs& a, BCtx& X, const BShared& S, int mode,
                                  bool has_q, bool has_mu, bool dst_pol, bool muf, bool do_str, double (&es)[7]) {
   const BConf& c = *X.c;

@@ -137,7 +137,7 @@ struct mdff_ctx {
   double2* d_rho_acc = nullptr;
   bool rho_acc_ok = false;
   int rec_mode = 0;
-  double* d_str = nullptr;
+  double* d_epart = nullptr;  // block sums of the reciprocal energy terms
   int n_rho_chunks = 0;
   // FP64 structure factor on the tensor cores (k_rho_dm): ions a staged buffer
   // holds (0: the mesh does not fit), n tiles per pass and passes; most ion chunks
@@ -582,7 +582,7 @@ static int build_mesh(mdff_ctx* h) {
   cudaFree(h->d_rchunk);
   cudaFree(h->d_rho_part);
   cudaFree(h->d_rhoA);
-  cudaFree(h->d_str);
+  cudaFree(h->d_epart);
   cudaFree(h->d_G);
   cudaFree(h->d_H);
   h->d_rows = nullptr;
@@ -687,7 +687,7 @@ static int build_mesh(mdff_ctx* h) {
   cudaFree(h->d_rho_acc);
   h->d_rho_acc = nullptr;
   DALLOC(h->d_rho_acc, std::max(nk, 1));
-  DALLOC(h->d_str, std::max(nk, 1));
+  DALLOC(h->d_epart, (size_t)7 * cdiv(std::max(nk, 1), 32));
   DALLOC(h->d_G, (size_t)(h->rchunk.size() - 1) * h->natm);
   DALLOC(h->d_H, (size_t)(h->rchunk.size() - 1) * h->natm);
   CK(cudaMemcpyAsync(h->d_rows, h->rows.data(), sizeof(int4) * nrows, cudaMemcpyHostToDevice, h->st));
@@ -958,14 +958,19 @@ static int launch_field_dm(mdff_ctx* h, const RecMesh& M, int n, const int* imap
   return ng;
 }
 
-// rho over the chunk partials (A_k scaled) into rhoA, A |rho|^2 into str
-static int rho_sum(mdff_ctx* h, const RecMesh& M, int nparts, double2* acc) {
-  if (nparts > 8)
-    PDL_CHECK(pdl_launch(k_rec_sum8, dim3(cdiv(h->nk, 32)), dim3(256), 0, h->st, (const double2*)h->d_rho_part, nparts,
-                         M, h->d_rhoA, h->d_str, acc));
-  else
-    PDL_CHECK(pdl_launch(k_rec_sum, dim3(cdiv(h->nk, 256)), dim3(256), 0, h->st, (const double2*)h->d_rho_part, nparts,
-                         M, h->d_rhoA, h->d_str, acc));
+// rho over the chunk partials (A_k scaled) into rhoA; energy: the blocks' energy
+// terms too (*nep of them)
+static int rho_sum(mdff_ctx* h, const RecMesh& M, int nparts, double2* acc, bool energy, int* nep) {
+  double* ep = energy ? h->d_epart : nullptr;
+  if (nparts > 8) {
+    *nep = cdiv(h->nk, 32);
+    PDL_CHECK(pdl_launch(k_rec_sum8, dim3(*nep), dim3(256), 0, h->st, (const double2*)h->d_rho_part, nparts, M,
+                         h->d_rhoA, ep, acc));
+  } else {
+    *nep = cdiv(h->nk, 256);
+    PDL_CHECK(pdl_launch(k_rec_sum, dim3(*nep), dim3(256), 0, h->st, (const double2*)h->d_rho_part, nparts, M,
+                         h->d_rhoA, ep, acc));
+  }
   return MDFF_OK;
 }
 
@@ -1077,7 +1082,7 @@ static int rec_pass_t(mdff_ctx* h, const typename cplx<R>::T* tab, const double4
   double ops_rho = (has_q && has_mu) ? 20.0 : (has_mu ? 16.0 : 11.0);
   double ops_fld = (forces && has_mu) ? 32.0 : (forces ? 17.0 : 20.0);
   int pr = prof_begin(h, KC_RHO, (double)h->nk * n * ops_rho);
-  int nparts = 0;
+  int nparts = 0, nep = 0;
   const int mode = h->rec_mode;
   // the tensor-core TF32 structure factor serves the FP32 CG operator (dipoles
   // alone, no forces), whose error the FP64 residual refinement removes; every
@@ -1085,7 +1090,8 @@ static int rec_pass_t(mdff_ctx* h, const typename cplx<R>::T* tab, const double4
   // solve's accumulated rho' instead (REC_FROM_ACC).
   if (mode == REC_FROM_ACC) {
     PDL_CHECK(pdl_launch(k_rec_acc_finish, dim3(cdiv(h->nk, 256)), dim3(256), 0, h->st,
-                         (const double2*)h->d_rho_acc, M, h->d_rhoA, h->d_str));
+                         (const double2*)h->d_rho_acc, M, h->d_rhoA, h->d_epart));
+    nep = cdiv(h->nk, 256);
   } else if (F32 && h->rho_tc && pol_dipoles && !has_q && has_mu && !forces) {
     nparts = h->n_tc_chunks;
     launch_rho_tc(h, M, n);
@@ -1109,13 +1115,10 @@ static int rec_pass_t(mdff_ctx* h, const typename cplx<R>::T* tab, const double4
     // (REC_SAVE_ACC: this rho' starts the solve's accumulation; REC_NEED_RHOA:
     // the CG step after this operator adds it, which the tensor-core B-tile
     // builder writes while it sums the partials)
-    int e = rho_sum(h, M, nparts, mode == REC_SAVE_ACC ? h->d_rho_acc : (double2*)nullptr);
+    int e = rho_sum(h, M, nparts, mode == REC_SAVE_ACC ? h->d_rho_acc : (double2*)nullptr, e_out != nullptr, &nep);
     if (e) return e;
   } else {
     npart = nparts;
-  }
-  if (e_out) {
-    PDL_CHECK(pdl_launch(k_rec_energy, dim3(1), dim3(1024), 0, h->st, h->d_str, M, tpi_V, h->omega, 1, e_out));
   }
   int nch = (int)h->rchunk.size() - 1;
   // a pass without forces feeds the dipole solvers, which read its field at
@@ -1153,9 +1156,10 @@ static int rec_pass_t(mdff_ctx* h, const typename cplx<R>::T* tab, const double4
     *defer_nch = nch;
     return MDFF_OK;
   }
-  k_rec_field_sum<<<cdiv((long)n * 4, 256), 256, 0, h->st>>>(h->d_G, h->d_H, nch, n, h->d_cell, h->d_q,
+  k_rec_field_sum<<<cdiv((long)n * 4, 256) + (e_out ? 1 : 0), 256, 0, h->st>>>(h->d_G, h->d_H, nch, n, h->d_cell, h->d_q,
                                                    2.0 * fpi_V, muf ? 1 : 0, forces, h->coul_unit, E,
-                                                   h->d_force, sf, field_pol ? h->d_ipolar : nullptr);
+                                                   h->d_force, sf, field_pol ? h->d_ipolar : nullptr, h->d_epart,
+                                                   nep, tpi_V, h->omega, e_out);
   LAUNCH_CHECK();
   return MDFF_OK;
 }
@@ -3253,7 +3257,8 @@ int mdff_gpu_efg(mdff_handle h, double* efg) {
     LAUNCH_CHECK();
     const int nparts = launch_rho64(h, M, n, nullptr, n, has_q, has_mu);
     LAUNCH_CHECK();
-    int e = rho_sum(h, M, nparts, nullptr);
+    int nep;
+    int e = rho_sum(h, M, nparts, nullptr, false, &nep);
     if (e) return e;
     const double scale = 2.0 * (2.0 * (kTwoPi / h->omega));
     if (field_dm_ks(M.kmax[2])) {
@@ -3354,7 +3359,7 @@ void mdff_gpu_destroy(mdff_handle h) {
                   h->d_dipia, h->d_pol, h->d_invpol, h->d_nbtab, h->d_estab, h->L.nbr, h->L.nnb,
                   h->L.sref, h->L.cell_of, h->L.cell_count, h->L.cell_start,
                   h->L.cell_fill, h->L.cell_pos, h->d_disp_part, h->d_rows, h->d_Ak, h->d_kvec,
-                  h->d_rchunk, h->d_tab64, h->d_tab32, h->d_w, h->d_w32, h->d_rho_part, h->d_rhoA, h->d_str,
+                  h->d_rchunk, h->d_tab64, h->d_tab32, h->d_w, h->d_w32, h->d_rho_part, h->d_rhoA, h->d_epart,
                   h->d_G, h->d_H, h->d_Estat, h->d_Eind, h->d_Efield, h->d_mu_ind, h->d_mu_tot,
                   h->d_hist, h->d_E, h->d_r, h->d_z, h->d_pv, h->d_qv, h->d_Tp, h->d_mu32, h->d_force,
                   h->d_part, h->d_scal, h->d_pack, h->d_ekin_part, h->d_ddr,

@@ -10,8 +10,9 @@
 //
 //   k_rec_rho   : rho(k) = sum_i (q_i + i k.mu_i) e^{i k.r_i}   (ewald_rec.f90:118-148)
 //                 block = (row, nz tile) x ion chunk; fixed-order partials.
-//   k_rec_sum   : rho over chunks; rho' = A_k rho; str = A_k |rho|^2 (:173)
-//   k_rec_energy: u_rec and the stress (:255-263, 300-358), one block, fixed order
+//   k_rec_sum   : rho over chunks; rho' = A_k rho; with energy its blocks' sums of
+//                 A_k |rho|^2 (:173) for u_rec and the stress (:255-263, 300-358), which
+//                 k_rec_field_sum adds up in fixed order
 //   k_rec_field : per ion sum over k of recarg / recarg2 (:181-250), ion-major,
 //                 rho' of the block's k chunk staged in shared memory
 //   k_rec_field_sum : chunk sum, E = -2 pi B G, F = q E + 2 pi B H, scaled
@@ -259,67 +260,66 @@ static __device__ __forceinline__ double2 rho_prime(const double2* __restrict__ 
   return make_double2(A * r, A * im);
 }
 
-// rho = sum over chunks; rhoA = A_k rho; str = A_k |rho|^2 (acc: also a
-// copy of rhoA, the start of the dipole solve's accumulated rho')
-static __global__ void k_rec_sum(const double2* __restrict__ part, int nchunk, RecMesh M,
-                          double2* __restrict__ rhoA, double* __restrict__ str,
+// the terms s = A_k |rho|^2 of u_rec and of tau xx yy zz xy xz yz.  The sums over the
+// blocks that form rho' cost them nothing; a kernel of its own (one block over all
+// k) stood 15 us between rho' and the field in a force pass of 18,000 k.
+__device__ __forceinline__ void rec_energy_terms(double s, double4 kv, double (&v)[7]) {
+  v[0] = s;
+  v[1] = (1.0 - kv.w * kv.x * kv.x) * s;
+  v[2] = (1.0 - kv.w * kv.y * kv.y) * s;
+  v[3] = (1.0 - kv.w * kv.z * kv.z) * s;
+  v[4] = -(kv.w * kv.x * kv.y * s);
+  v[5] = -(kv.w * kv.x * kv.z * s);
+  v[6] = -(kv.w * kv.y * kv.z * s);
+}
+
+// rho = sum over chunks; rhoA = A_k rho (acc: also a copy of rhoA, the start of the
+// dipole solve's accumulated rho'; epart: this block's energy terms)
+static __global__ void __launch_bounds__(256) k_rec_sum(const double2* __restrict__ part, int nchunk, RecMesh M,
+                          double2* __restrict__ rhoA, double* __restrict__ epart,
                           double2* __restrict__ acc = nullptr) {
   pdl_wait();
   pdl_trigger();
+  __shared__ double red[7 * 8];
   int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= M.nk) return;
-  double r = 0.0, im = 0.0;
-  for (int c = 0; c < nchunk; ++c) {
-    double2 v = part[(size_t)c * M.nk + k];
-    r += v.x;
-    im += v.y;
-  }
-  double A = M.Ak[k];
-  rhoA[k] = make_double2(A * r, A * im);
-  str[k] = (r * r + im * im) * A;
-  if (acc) acc[k] = make_double2(A * r, A * im);
-}
-
-// rhoA and str of the force pass from the dipole solve's accumulated rho'
-// (rho' of the charges and the first guess, plus alpha_k rho'(p_k) of every
-// CG step: the structure factor is linear in the dipoles); str = |rho'|^2 / A_k
-static __global__ void k_rec_acc_finish(const double2* __restrict__ acc, RecMesh M,
-                                        double2* __restrict__ rhoA, double* __restrict__ str) {
-  pdl_wait();
-  pdl_trigger();
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= M.nk) return;
-  const double2 a = acc[k];
-  rhoA[k] = a;
-  str[k] = (a.x * a.x + a.y * a.y) / M.Ak[k];
-}
-
-// u_rec (x2 x tpi_V) and tau_rec (x2, symmetric, x tpi_V/omega): out[0..6] =
-// u, tau xx yy zz xy xz yz.  One block.
-static __global__ void k_rec_energy(const double* __restrict__ str, RecMesh M, double tpi_V,
-                             double omega, int do_stress, double* __restrict__ out) {
-  pdl_wait();
-  pdl_trigger();
-  __shared__ double red[7 * 32];
-  double v[7] = {0, 0, 0, 0, 0, 0, 0};
-  for (int k = threadIdx.x; k < M.nk; k += blockDim.x) {
-    double s = str[k];
-    double4 kv = M.kvec[k];
-    v[0] += s;
-    if (do_stress) {
-      v[1] += (1.0 - kv.w * kv.x * kv.x) * s;
-      v[2] += (1.0 - kv.w * kv.y * kv.y) * s;
-      v[3] += (1.0 - kv.w * kv.z * kv.z) * s;
-      v[4] -= kv.w * kv.x * kv.y * s;
-      v[5] -= kv.w * kv.x * kv.z * s;
-      v[6] -= kv.w * kv.y * kv.z * s;
+  double ev[7] = {0, 0, 0, 0, 0, 0, 0};
+  if (k < M.nk) {
+    double r = 0.0, im = 0.0;
+    for (int c = 0; c < nchunk; ++c) {
+      double2 v = part[(size_t)c * M.nk + k];
+      r += v.x;
+      im += v.y;
     }
+    double A = M.Ak[k];
+    rhoA[k] = make_double2(A * r, A * im);
+    if (acc) acc[k] = make_double2(A * r, A * im);
+    if (epart) rec_energy_terms((r * r + im * im) * A, M.kvec[k], ev);
   }
-  block_sum<7>(v, red);
-  if (threadIdx.x == 0) {
-    out[0] = v[0] * 2.0 * tpi_V;
-    for (int a = 1; a < 7; ++a) out[a] = v[a] * 2.0 * tpi_V / omega;
+  if (!epart) return;
+  block_sum<7>(ev, red);
+  if (threadIdx.x == 0)
+    for (int a = 0; a < 7; ++a) epart[(size_t)blockIdx.x * 7 + a] = ev[a];
+}
+
+// rhoA and the energy terms of the force pass from the dipole solve's accumulated
+// rho' (rho' of the charges and the first guess, plus alpha_k rho'(p_k) of every CG
+// step: the structure factor is linear in the dipoles); A |rho|^2 = |rho'|^2 / A
+static __global__ void __launch_bounds__(256) k_rec_acc_finish(const double2* __restrict__ acc, RecMesh M,
+                                                               double2* __restrict__ rhoA,
+                                                               double* __restrict__ epart) {
+  pdl_wait();
+  pdl_trigger();
+  __shared__ double red[7 * 8];
+  int k = blockIdx.x * blockDim.x + threadIdx.x;
+  double ev[7] = {0, 0, 0, 0, 0, 0, 0};
+  if (k < M.nk) {
+    const double2 a = acc[k];
+    rhoA[k] = a;
+    rec_energy_terms((a.x * a.x + a.y * a.y) / M.Ak[k], M.kvec[k], ev);
   }
+  block_sum<7>(ev, red);
+  if (threadIdx.x == 0)
+    for (int a = 0; a < 7; ++a) epart[(size_t)blockIdx.x * 7 + a] = ev[a];
 }
 
 // field / force partials.  grid.x = ion blocks (128), grid.y = k chunks
@@ -483,7 +483,24 @@ static __global__ void k_rec_field_sum(const double4* __restrict__ Gpart, const 
                                 const double* __restrict__ q, double scale /* 2 fpi_V */,
                                 int has_mu_force, int do_forces, double coul_unit,
                                 double4* __restrict__ E, double* __restrict__ force,
-                                SelfField sf, const int* __restrict__ ipolar) {
+                                SelfField sf, const int* __restrict__ ipolar,
+                                const double* __restrict__ epart, int nep, double tpi_V, double omega,
+                                double* __restrict__ e_out) {
+  if (e_out && blockIdx.x == gridDim.x - 1) {
+    // (a block of its own) u_rec (x2 x tpi_V) and tau_rec (x2, symmetric, x tpi_V /
+    // omega): u, tau xx yy zz xy xz yz from the block sums of the energy terms
+    __shared__ double red[7 * 8];
+    double v[7] = {0, 0, 0, 0, 0, 0, 0};
+    for (int b = threadIdx.x; b < nep; b += blockDim.x)
+#pragma unroll
+      for (int a = 0; a < 7; ++a) v[a] += epart[(size_t)b * 7 + a];
+    block_sum<7>(v, red);
+    if (threadIdx.x == 0) {
+      e_out[0] = v[0] * 2.0 * tpi_V;
+      for (int a = 1; a < 7; ++a) e_out[a] = v[a] * 2.0 * tpi_V / omega;
+    }
+    return;
+  }
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   int i = t >> 2, sub = t & 3;
   double g[3] = {0, 0, 0}, h[3] = {0, 0, 0};

@@ -201,7 +201,7 @@ static __global__ void __launch_bounds__(kDmThreads, 1) k_rho_dm(
 // rho over the chunks (as k_rec_sum): 32 k x 8 chunk subsets per block, the
 // subsets added in order; up to a few tens of chunks
 static __global__ void __launch_bounds__(256) k_rec_sum8(const double2* __restrict__ part, int nchunk, RecMesh M,
-                                                         double2* __restrict__ rhoA, double* __restrict__ str,
+                                                         double2* __restrict__ rhoA, double* __restrict__ epart,
                                                          double2* __restrict__ acc) {
   pdl_wait();
   pdl_trigger();
@@ -217,17 +217,25 @@ static __global__ void __launch_bounds__(256) k_rec_sum8(const double2* __restri
     }
   sh[ly][lx] = make_double2(r, im);
   __syncthreads();
-  if (ly != 0 || k >= M.nk) return;
+  if (ly != 0) return;
 #pragma unroll
   for (int y = 1; y < 8; ++y) {
     r += sh[y][lx].x;
     im += sh[y][lx].y;
   }
-  const double A = M.Ak[k];
-  const double2 ra = make_double2(A * r, A * im);
-  rhoA[k] = ra;
-  str[k] = (r * r + im * im) * A;
-  if (acc) acc[k] = ra;
+  double ev[7] = {0, 0, 0, 0, 0, 0, 0};
+  if (k < M.nk) {
+    const double A = M.Ak[k];
+    const double2 ra = make_double2(A * r, A * im);
+    rhoA[k] = ra;
+    if (acc) acc[k] = ra;
+    if (epart) rec_energy_terms((r * r + im * im) * A, M.kvec[k], ev);
+  }
+  if (!epart) return;
+#pragma unroll
+  for (int a = 0; a < 7; ++a) ev[a] = warp_sum(ev[a]);
+  if (lx == 0)
+    for (int a = 0; a < 7; ++a) epart[(size_t)blockIdx.x * 7 + a] = ev[a];
 }
 
 // ---------------------------------------------------------------------------
