@@ -59,7 +59,8 @@ enum {
   S_CATA = 72,   // 4 ints: d_cata
   S_FLAGS = 74,  // 4 ints: the list's flags
   S_EKIN = 76,   // kinetic energy of the last MD step
-  S_NALL = 77
+  S_TICK = 77,   // int: block ticket of k_scf_tail
+  S_NALL = 78
 };
 
 // FP32 CG: the recurrence residual drifts from the true one by about the FP32
@@ -1911,28 +1912,22 @@ static bool scf_device_loop(const mdff_ctx* h) {
          (h->p.max_scf_pol_iter > 0 || h->p.min_scf_pol_iter > 0);
 }
 
-// one SCF iteration from the second on (pim.cuh); u_pol's partials go to the
-// upper half of d_part
+// one SCF iteration from the second on (pim.cuh); the iterate is in d_pv
 static int scf_iteration(mdff_ctx* h, cudaGraphConditionalHandle hc) {
-  const int n = h->natm, np = (int)h->polidx.size(), nb = cdiv(n, 256);
+  const int n = h->natm, np = (int)h->polidx.size();
   int s;
   PolDev P = poldev(h);
-  PDL_CHECK(pdl_launch(k_scf_step, dim3(nb), dim3(256), 0, h->st, (const double4*)h->d_Estat,
-                       (const double4*)h->d_Eind, P, n, (const CellC*)h->d_cell, h->d_mu_ind, h->d_w, upol_part(h)));
   cudaStream_t rs;
   if ((s = rs_fork(h, &rs))) return s;
-  if ((s = dd64_field(h, rs, h->d_mu_ind, true, false, h->d_Eind))) return s;
+  if ((s = dd64_field(h, rs, h->d_pv, true, false, h->d_Eind))) return s;
   int nch = 0;
-  SelfField sf = self_field(h, h->d_mu_ind, h->d_scal + S_MOM2);
-  if ((s = rec_pass(h, false, h->d_mu_ind, 0, 1, 0, h->d_Eind, nullptr, sf, nullptr, &nch, true, true))) return s;
-  const int nbf = cdiv((long)np * 4, 256);
-  k_scf_field<<<nbf, 256, 0, h->st>>>(h->d_G, nch, n, h->d_polidx, np, h->d_cell,
-                                      2.0 * (2.0 * (kTwoPi / h->omega)), sf.selfa2, h->d_mu_ind, h->d_Estat, P,
-                                      h->d_Eind, h->d_part);
+  const SelfField sf = self_field(h, h->d_pv, h->d_scal + S_MOM2);
+  if ((s = rec_pass(h, false, h->d_pv, 0, 1, 0, h->d_Eind, nullptr, sf, nullptr, &nch, true, true))) return s;
+  k_scf_tail<<<cdiv((long)np * 4, 256), 256, 0, h->st>>>(
+      h->d_G, nch, n, h->d_polidx, np, h->d_cell, 2.0 * (2.0 * (kTwoPi / h->omega)), sf.selfa2, h->d_Estat, P, h->d_pv,
+      h->d_mu_ind, h->d_Eind, h->d_w, h->d_part, (int*)(h->d_scal + S_TICK), h->npol, h->p.conv_tol_ind,
+      h->p.min_scf_pol_iter, h->p.max_scf_pol_iter, h->d_scal + S_SCF, h->d_scal + S_UPOL, hc);
   LAUNCH_CHECK();
-  PDL_CHECK(pdl_launch(k_scf_check, dim3(1), dim3(256), 0, h->st, (const double*)h->d_part, nbf,
-                       (const double*)nullptr, h->npol, h->p.conv_tol_ind, h->p.min_scf_pol_iter,
-                       h->p.max_scf_pol_iter, h->d_scal + S_SCF, hc));
   return MDFF_OK;
 }
 
@@ -1951,11 +1946,11 @@ static int add_solver_loop(mdff_ctx* h, cudaGraph_t g, const cudaGraphNode_t* de
   double maxit = (double)(h->p.cg_max_iter > 0 ? h->p.cg_max_iter : 200);
   int f32 = fp32 ? 1 : 0;
   void* cargs[] = {&sc, &plan, &npol, &tol, &maxit, &f32, &hc};
-  const double *nopart = nullptr, *r2 = h->d_scal + S_RMS;
-  int zero = 0, mn = h->p.min_scf_pol_iter, mx = h->p.max_scf_pol_iter;
+  const double* r2 = h->d_scal + S_RMS;
+  int mn = h->p.min_scf_pol_iter, mx = h->p.max_scf_pol_iter;
   double stol = h->p.conv_tol_ind;
   double* ssc = h->d_scal + S_SCF;
-  void* sargs[] = {&nopart, &zero, &r2, &npol, &stol, &mn, &mx, &ssc, &hc};
+  void* sargs[] = {&r2, &npol, &stol, &mn, &mx, &ssc, &hc};
   cudaKernelNodeParams kp = {};
   kp.func = cg ? (void*)k_cg_plan : (void*)k_scf_check;
   kp.gridDim = dim3(1);
@@ -2022,19 +2017,22 @@ static int scf_first(mdff_ctx* h, int itime, bool fp32) {
   } else if ((s = aspc_predict(h, itime))) {
     return s;
   }
-  PDL_CHECK(pdl_launch(k_upol_part, dim3(nb), dim3(256), 0, h->st, (const double4*)h->d_mu_ind, P, n, upol_part(h)));
+  PDL_CHECK(pdl_launch(k_upol_part, dim3(nb), dim3(256), 0, h->st, (const double4*)h->d_mu_ind, P, n, h->d_part));
+  if ((s = reduce_into(h, nb, 1, h->d_scal + S_UPOL))) return s;
   if ((s = field_of_mu(h, h->d_mu_ind, 0, fp32, h->d_Eind))) return s;
   k_add4<<<nb, 256, 0, h->st>>>(h->d_Estat, h->d_Eind, n, h->d_Efield);
   LAUNCH_CHECK();
   if (ismd && (s = aspc_correct(h, itime))) return s;
   k_rmsd_part<<<nb, 256, 0, h->st>>>(h->d_mu_ind, h->d_Efield, P, n, h->d_part);
   LAUNCH_CHECK();
-  return reduce_into(h, nb, 1, h->d_scal + S_RMS);
+  if ((s = reduce_into(h, nb, 1, h->d_scal + S_RMS))) return s;
+  // the second iteration's dipoles
+  PDL_CHECK(pdl_launch(k_scf_step, dim3(nb), dim3(256), 0, h->st, (const double4*)h->d_Estat,
+                       (const double4*)h->d_Eind, P, n, (const CellC*)h->d_cell, h->d_pv, h->d_w));
+  return MDFF_OK;
 }
-// after the loop: u_pol of the last iteration's dipoles, the ASPC history
+// after the loop: the ASPC history
 static int scf_epilogue(mdff_ctx* h) {
-  PDL_CHECK(pdl_launch(k_reduce_partials, dim3(1), dim3(256), 0, h->st, (const double*)upol_part(h),
-                       cdiv(h->natm, 256), 1, h->d_scal + S_UPOL));
   CK(cudaMemcpyAsync(h->d_hist, h->d_mu_ind, sizeof(double4) * h->natm, cudaMemcpyDeviceToDevice, h->st));
   return MDFF_OK;
 }

@@ -162,48 +162,54 @@ __global__ void k_self_surf_field(const double4* __restrict__ mu, int natm, doub
 }
 
 // ---- SCF iterations on the device -------------------------------------------
-// From the second on, an SCF iteration (moment_from_pola.f90:340-460) is
-//   k_scf_step: mu = alpha (E_stat + E_ind), the reciprocal weights of mu, u_pol
-//   the dipole field: cached real-space part (side stream), rho, field sums
-//   k_scf_field: E_ind = real + reciprocal + self, and the rmsd partials
-//   k_scf_check: rmsd, count, and the WHILE condition of the graph that runs
-// them, so that a solve needs no host round trip per iteration (14 launches, two
-// fills, a copy and a synchronisation before).
+// From the second on, an SCF iteration (moment_from_pola.f90:340-460) is the dipole
+// field of the iterate mun (cached real-space part on the side stream, rho, field
+// sums) and
+//   k_scf_tail: mu = mun, E_ind = real + reciprocal + self, the residual and u_pol;
+//   the next iterate mun = alpha (E_stat + E_ind) and its reciprocal weights; the last
+//   block to finish adds the partials in fixed order and sets rmsd, count, u_pol and
+//   the WHILE condition of the graph that runs the iterations,
+// so that a solve needs no host round trip per iteration.  An iterate formed after
+// the last iteration is not used.  At 216 ions an iteration is a chain of launch
+// latencies: with step, field sum and check as three kernels XX us, now YY.
 
+// mun = alpha (E_stat + E_ind) and its weights, for the first iteration of the loop
+__device__ __forceinline__ void scf_iterate(const double* al, const double (&E)[3], const CellC* __restrict__ cell,
+                                            int i, double4* __restrict__ mun, double4* __restrict__ w) {
+  double m[3];
+#pragma unroll
+  for (int x = 0; x < 3; ++x) m[x] = ((al[3 * x] * E[0]) + al[3 * x + 1] * E[1]) + al[3 * x + 2] * E[2];
+  mun[i] = make_double4(m[0], m[1], m[2], 0.0);
+  const double* B = cell->B;
+  w[i] = make_double4(0.0, kTwoPi * (B[0] * m[0] + B[3] * m[1] + B[6] * m[2]),
+                      kTwoPi * (B[1] * m[0] + B[4] * m[1] + B[7] * m[2]),
+                      kTwoPi * (B[2] * m[0] + B[5] * m[1] + B[8] * m[2]));
+}
 __global__ void k_scf_step(const double4* __restrict__ Estat, const double4* __restrict__ Eind, PolDev P,
-                           int natm, const CellC* __restrict__ cell, double4* __restrict__ mu,
-                           double4* __restrict__ w, double* __restrict__ part) {
+                           int natm, const CellC* __restrict__ cell, double4* __restrict__ mun,
+                           double4* __restrict__ w) {
   pdl_wait();
   pdl_trigger();
-  __shared__ double red[32];
-  double v[1] = {0.0};
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < natm && P.ipolar[i]) {
-    const double4 a = Estat[i], b = Eind[i];
-    const double E[3] = {a.x + b.x, a.y + b.y, a.z + b.z};
-    const double* al = P.pol + 9 * (size_t)i;
-    const double* iv = P.invpol + 9 * (size_t)i;
-    double m[3];
-    for (int x = 0; x < 3; ++x) m[x] = ((al[3 * x] * E[0]) + al[3 * x + 1] * E[1]) + al[3 * x + 2] * E[2];
-    mu[i] = make_double4(m[0], m[1], m[2], 0.0);
-    const double* B = cell->B;
-    w[i] = make_double4(0.0, kTwoPi * (B[0] * m[0] + B[3] * m[1] + B[6] * m[2]),
-                        kTwoPi * (B[1] * m[0] + B[4] * m[1] + B[7] * m[2]),
-                        kTwoPi * (B[2] * m[0] + B[5] * m[1] + B[8] * m[2]));
-    for (int x = 0; x < 3; ++x)
-      for (int y = 0; y < 3; ++y) v[0] += m[x] * iv[3 * x + y] * m[y];
-  }
-  block_sum<1>(v, red);
-  if (threadIdx.x == 0) part[blockIdx.x] = v[0];
+  if (i >= natm || !P.ipolar[i]) return;
+  const double4 a = Estat[i], b = Eind[i];
+  const double E[3] = {a.x + b.x, a.y + b.y, a.z + b.z};
+  scf_iterate(P.pol + 9 * (size_t)i, E, cell, i, mun, w);
 }
 
 // four threads per polarisable ion split the field partials, as k_rec_field_sum
-__global__ void k_scf_field(const double4* __restrict__ Gpart, int nchunk, int natm, const int* __restrict__ polidx,
-                            int npol, const CellC* __restrict__ cell, double scale, double selfa2,
-                            const double4* __restrict__ mu, const double4* __restrict__ Estat, PolDev P,
-                            double4* __restrict__ Eind, double* __restrict__ part) {
-  __shared__ double red[32];
-  double v[1] = {0.0};
+__global__ void __launch_bounds__(256) k_scf_tail(const double4* __restrict__ Gpart, int nchunk, int natm,
+                                                  const int* __restrict__ polidx, int npol,
+                                                  const CellC* __restrict__ cell, double scale, double selfa2,
+                                                  const double4* __restrict__ Estat, PolDev P,
+                                                  double4* __restrict__ mun, double4* __restrict__ mu,
+                                                  double4* __restrict__ Eind, double4* __restrict__ w,
+                                                  double* __restrict__ part, int* __restrict__ ticket, int npol_r, double tol,
+                                                  int miniter, int maxiter, double* __restrict__ sc,
+                                                  double* __restrict__ upol, cudaGraphConditionalHandle hc) {
+  __shared__ double red[2 * 32];
+  __shared__ int last;
+  double v[2] = {0.0, 0.0};
   const int t = blockIdx.x * blockDim.x + threadIdx.x, sl = t >> 2, sub = t & 3;
   double g[3] = {0.0, 0.0, 0.0};
   int i = 0;
@@ -223,43 +229,62 @@ __global__ void k_scf_field(const double4* __restrict__ Gpart, int nchunk, int n
   }
   if (sl < npol && sub == 0) {
     const double* B = cell->B;
-    const double4 m = mu[i], o = Eind[i], st = Estat[i];
+    const double4 m = mun[i], o = Eind[i], st = Estat[i];
     const double mm[3] = {m.x, m.y, m.z}, oo[3] = {o.x, o.y, o.z}, ss[3] = {st.x, st.y, st.z};
     const double* al = P.pol + 9 * (size_t)i;
-    double e[3];
+    const double* iv = P.invpol + 9 * (size_t)i;
+    double e[3], E[3];
+#pragma unroll
     for (int a = 0; a < 3; ++a) {
       const double er = -kTwoPi * (B[3 * a] * g[0] + B[3 * a + 1] * g[1] + B[3 * a + 2] * g[2]) * scale;
       e[a] = oo[a] + er + 2.0 * selfa2 * mm[a];
+      E[a] = ss[a] + e[a];
       if (al[4 * a] != 0.0) {  // get_rmsd_mu (:998-1027)
-        const double d = mm[a] / al[4 * a] - (ss[a] + e[a]);
+        const double d = mm[a] / al[4 * a] - E[a];
         v[0] += d * d;
       }
+#pragma unroll
+      for (int b = 0; b < 3; ++b) v[1] += mm[a] * iv[3 * a + b] * mm[b];
     }
+    mu[i] = m;
     Eind[i] = make_double4(e[0], e[1], e[2], 0.0);
+    scf_iterate(al, E, cell, i, mun, w);
   }
-  block_sum<1>(v, red);
-  if (threadIdx.x == 0) part[blockIdx.x] = v[0];
-}
-
-// sc[0] = iterations, sc[1] = rmsd; r2 (head of the graph): the residual sum of
-// the first iteration, else the partials of k_scf_field.  The condition is the
-// host loop's.
-__global__ void k_scf_check(const double* __restrict__ part, int nblk, const double* __restrict__ r2, int npol,
-                            double tol, int miniter, int maxiter, double* __restrict__ sc,
-                            cudaGraphConditionalHandle hc) {
-  pdl_wait();
-  pdl_trigger();
-  __shared__ double red[32];
-  double v[1] = {0.0};
-  if (!r2)
-    for (int b = threadIdx.x; b < nblk; b += blockDim.x) v[0] += part[b];
-  block_sum<1>(v, red);
+  block_sum<2>(v, red);
+  if (threadIdx.x == 0) {
+    part[(size_t)blockIdx.x * 2] = v[0];
+    part[(size_t)blockIdx.x * 2 + 1] = v[1];
+    __threadfence();
+    last = atomicAdd(ticket, 1) == (int)gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  v[0] = v[1] = 0.0;
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) {
+    v[0] += __ldcg(part + (size_t)b * 2);
+    v[1] += __ldcg(part + (size_t)b * 2 + 1);
+  }
+  block_sum<2>(v, red);
   if (threadIdx.x != 0) return;
-  const double rmsd = sqrt((r2 ? *r2 : v[0]) / (double)npol);
-  const int it = r2 ? 1 : (int)sc[0] + 1;
+  *ticket = 0;
+  const double rmsd = sqrt(v[0] / (double)npol_r);
+  const int it = (int)sc[0] + 1;
   sc[0] = (double)it;
   sc[1] = rmsd;
+  *upol = v[1];
   cudaGraphSetConditional(hc, ((it < maxiter && rmsd > tol) || it < miniter) ? 1u : 0u);
+}
+
+// head of the loop: sc[0] = iterations, sc[1] = rmsd from the residual sum r2 of
+// the first iteration.  The condition is the host loop's.
+__global__ void k_scf_check(const double* __restrict__ r2, int npol, double tol, int miniter, int maxiter,
+                            double* __restrict__ sc, cudaGraphConditionalHandle hc) {
+  if (threadIdx.x != 0) return;
+  const double rmsd = sqrt(*r2 / (double)npol);
+  sc[0] = 1.0;
+  sc[1] = rmsd;
+  cudaGraphSetConditional(hc, ((1 < maxiter && rmsd > tol) || 1 < miniter) ? 1u : 0u);
 }
 
 // ---- conjugate gradients ----------------------------------------------------
