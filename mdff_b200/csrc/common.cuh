@@ -279,6 +279,11 @@ struct SlotW {
   }
 };
 
+// A solver's loop body holds several iterations; the kernels of those after the one
+// that finished leave at once (stop: flag set by its last kernel, nullptr outside
+// a loop).  Kernels two or more after that one read it before their pdl_wait.
+__device__ __forceinline__ bool loop_stopped(const int* stop) { return stop && __ldcg(stop) != 0; }
+
 // Dynamic shared memory up to the device's limit for a kernel that needs `need` bytes.  The
 // attribute belongs to the function, not to a handle: set to one handle's
 // size it would make the launches of another with a larger mesh or box fail.

@@ -59,7 +59,7 @@ enum {
   S_CATA = 72,   // 4 ints: d_cata
   S_FLAGS = 74,  // 4 ints: the list's flags
   S_EKIN = 76,   // kinetic energy of the last MD step
-  S_TICK = 77,   // int: block ticket of k_scf_tail
+  S_TICK = 77,   // 2 ints: block ticket of k_scf_tail, stop flag of the solver's loop
   S_NALL = 78
 };
 
@@ -217,6 +217,7 @@ struct mdff_ctx {
   bool lwannier = false;
   int* d_lwfc = nullptr;
   double4* d_mu_wfc = nullptr;
+  const int* loop_stop = nullptr;  // stop flag for the kernels of a loop body being captured
   double* d_pack = nullptr;      // [natm][3] staging for mu/ef output
   double* h_stage = nullptr;     // pinned: positions [3][natm], outputs [9 natm] (host arrays of a call)
   double* d_ekin_part = nullptr;
@@ -903,7 +904,7 @@ static int launch_rho64(mdff_ctx* h, const RecMesh& M, int n, const int* imap, i
     const double4* w = h->d_w;
 #define RDL(NT)                                                                                                     \
   (void)pdl_launch(k_rho_dm<NT, HM>, g, dim3(kDmThreads), smem, h->st, tab, w, n, imap, nion, chunk, h->dm_ci[HM], M, \
-                   h->d_rho_part)
+                   h->d_rho_part, h->loop_stop)
     if (hm) {
       constexpr bool HM = true;
       RHO_DM_SWITCH(h->dm_nt[1], RDL)
@@ -944,7 +945,7 @@ static int launch_field_dm_k(mdff_ctx* h, const RecMesh& M, int n, const int* im
   const double2* rhoA = h->d_rhoA;
 #define FDL(MODE)                                                                                             \
   (void)pdl_launch(k_field_dm<KS, MODE>, g, dim3(kDmFldThreads), smem, h->st, tab, w, n, imap, nion, M, rhoA, \
-                   rpg, rc, h->d_G, h->d_H)
+                   rpg, rc, h->d_G, h->d_H, h->loop_stop)
   if (mode == DM_FORCE) FDL(DM_FORCE);
   else if (mode == DM_EFG) FDL(DM_EFG);
   else FDL(DM_FIELD);
@@ -966,11 +967,11 @@ static int rho_sum(mdff_ctx* h, const RecMesh& M, int nparts, double2* acc, bool
   if (nparts > 8) {
     *nep = cdiv(h->nk, 32);
     PDL_CHECK(pdl_launch(k_rec_sum8, dim3(*nep), dim3(256), 0, h->st, (const double2*)h->d_rho_part, nparts, M,
-                         h->d_rhoA, ep, acc));
+                         h->d_rhoA, ep, acc, h->loop_stop));
   } else {
     *nep = cdiv(h->nk, 256);
     PDL_CHECK(pdl_launch(k_rec_sum, dim3(*nep), dim3(256), 0, h->st, (const double2*)h->d_rho_part, nparts, M,
-                         h->d_rhoA, ep, acc));
+                         h->d_rhoA, ep, acc, h->loop_stop));
   }
   return MDFF_OK;
 }
@@ -986,7 +987,7 @@ static void launch_rho_tc(mdff_ctx* h, const RecMesh& M, int n) {
   (void)n;
   (void)pdl_launch(k_rec_rho_tc, g, dim3(kRhoTcThreads), smem, h->st, (const float2*)h->d_rho_timg,
                    (const float4*)h->d_w32s, rho_tc_nion(h), h->tc_chunk, M,
-                   h->d_rho_part, h->d_cata + 1, (const int*)(h->d_cata + 3));
+                   h->d_rho_part, h->d_cata + 1, (const int*)(h->d_cata + 3), h->loop_stop);
 }
 
 // FP32 field / force partials on the tensor cores into d_G / d_H (B tiles
@@ -1025,13 +1026,15 @@ static int launch_field_tc_k(mdff_ctx* h, const RecMesh& M, int n, bool muf, int
   const uint32_t* fb = h->d_fb;
   h->launches++;  // two launches here; the caller's LAUNCH_CHECK counts one
   if (muf) {
-    (void)pdl_launch(k_rec_field_btiles<true, KF>, gb, dim3(128), bsmem, h->st, M, rhoA, rpart, npart, h->d_fb, rho_out);
+    (void)pdl_launch(k_rec_field_btiles<true, KF>, gb, dim3(128), bsmem, h->st, M, rhoA, rpart, npart, h->d_fb, rho_out,
+                     h->loop_stop);
     (void)pdl_launch(k_rec_field_tc<true, KF>, g, dim3(kFieldTcThreads), smem, h->st, tab, w, n, imap, nion,
-                     M, fb, tpg, h->d_G, h->d_H, err);
+                     M, fb, tpg, h->d_G, h->d_H, err, h->loop_stop);
   } else {
-    (void)pdl_launch(k_rec_field_btiles<false, KF>, gb, dim3(128), bsmem, h->st, M, rhoA, rpart, npart, h->d_fb, rho_out);
+    (void)pdl_launch(k_rec_field_btiles<false, KF>, gb, dim3(128), bsmem, h->st, M, rhoA, rpart, npart, h->d_fb, rho_out,
+                     h->loop_stop);
     (void)pdl_launch(k_rec_field_tc<false, KF>, g, dim3(kFieldTcThreads), smem, h->st, tab, w, n, imap, nion,
-                     M, fb, tpg, h->d_G, h->d_H, err);
+                     M, fb, tpg, h->d_G, h->d_H, err, h->loop_stop);
   }
   return ng;
 }
@@ -1222,7 +1225,7 @@ static int dd64_field(mdff_ctx* h, cudaStream_t st, const double4* mu, bool mask
     h->dd64_ok = true;
   } else {
     k_dd64_apply<<<nb, 256, 0, st>>>(mu, h->d_polidx, np, h->d_c64r, h->d_c64b, h->d_c64j, h->d_c64n, h->L.cap,
-                                     mask0 ? 1 : 0, E);
+                                     mask0 ? 1 : 0, E, h->loop_stop);
   }
   LAUNCH_CHECK();
   return MDFF_OK;
@@ -1237,7 +1240,8 @@ static int dd64_field(mdff_ctx* h, cudaStream_t st, const double4* mu, bool mask
 static int dd32_part(mdff_ctx* h) {
   const int np = h->d_polidx ? (int)h->polidx.size() : h->natm;
   k_dd_cached_part<<<cdiv((long)np * 32, 256), 256, 0, h->st_rs>>>(h->d_mu32, h->d_ddr, h->d_ddb1, h->d_ddj, h->d_ddn,
-                                                                   h->L.cap, h->d_polidx, np, h->d_Edd);
+                                                                   h->L.cap, h->d_polidx, np, h->d_Edd,
+                                                                   h->loop_stop);
   LAUNCH_CHECK();
   return MDFF_OK;
 }
@@ -1795,8 +1799,9 @@ __global__ void k_cg_inner_check(double* __restrict__ sc, int npol, int in_graph
 // trusted), taken on the device so that the graph follows the residual
 // without a host round trip; sets the WHILE condition of the inner loop
 __global__ void k_cg_plan(double* __restrict__ sc, double* __restrict__ plan, int npol, double tol,
-                          double maxit, int fp32, cudaGraphConditionalHandle hc) {
+                          double maxit, int fp32, int* __restrict__ stopf, cudaGraphConditionalHandle hc) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
+  *stopf = 0;
   const double rmsd = sqrt(sc[1] / (double)npol);
   const double outer = plan[2];
   plan[0] = rmsd;
@@ -1821,6 +1826,10 @@ __global__ void k_setd2(double* __restrict__ a, double va, double* __restrict__ 
     *b = vb;
   }
 }
+
+// stop flag of the solver's loop, and its iterations per pass
+static int* loop_flag(const mdff_ctx* h) { return (int*)(h->d_scal + S_TICK) + 1; }
+constexpr int kLoopUnroll = 4;
 
 // second set of block partials
 static double* upol_part(mdff_ctx* h) { return h->d_part + h->part_cap / 2; }
@@ -1872,11 +1881,12 @@ static int cg_iteration(mdff_ctx* h, bool fp32, int in_graph, cudaGraphCondition
     LAUNCH_CHECK();
     PDL_CHECK(pdl_launch(k_cg_step, dim3(nu), dim3(256), 0, h->st, sc, (const double*)pq, nq, P,
                          (const int*)h->d_polidx, np, (const double4*)h->d_pv, (const double4*)h->d_qv, h->d_mu_ind,
-                         h->d_r, h->d_z, rz, acc ? h->d_rho_acc : (double2*)nullptr, (const double2*)h->d_rhoA, h->nk));
+                         h->d_r, h->d_z, rz, acc ? h->d_rho_acc : (double2*)nullptr, (const double2*)h->d_rhoA, h->nk,
+                         h->loop_stop));
     PDL_CHECK(pdl_launch(k_cg_next, dim3(std::min(cdiv(np, 256), most)), dim3(256), 0, h->st, sc, (const double*)rz, nu,
                          h->npol, (const int*)h->d_polidx, np, (const double4*)h->d_z, h->d_pv,
                          (const CellC*)h->d_cell, fp32 ? h->d_w32 : (float4*)nullptr, h->d_mu32, slotw(h),
-                         cg_w64(h, fp32), hc));
+                         cg_w64(h, fp32), loop_flag(h), hc));
     return MDFF_OK;
   }
   // with the accumulated structure factor the operator's rho'(p) stays in
@@ -1926,7 +1936,7 @@ static int scf_iteration(mdff_ctx* h, cudaGraphConditionalHandle hc) {
   k_scf_tail<<<cdiv((long)np * 4, 256), 256, 0, h->st>>>(
       h->d_G, nch, n, h->d_polidx, np, h->d_cell, 2.0 * (2.0 * (kTwoPi / h->omega)), sf.selfa2, h->d_Estat, P, h->d_pv,
       h->d_mu_ind, h->d_Eind, h->d_w, h->d_part, (int*)(h->d_scal + S_TICK), h->npol, h->p.conv_tol_ind,
-      h->p.min_scf_pol_iter, h->p.max_scf_pol_iter, h->d_scal + S_SCF, h->d_scal + S_UPOL, hc);
+      h->p.min_scf_pol_iter, h->p.max_scf_pol_iter, h->d_scal + S_SCF, h->d_scal + S_UPOL, loop_flag(h), hc);
   LAUNCH_CHECK();
   return MDFF_OK;
 }
@@ -1945,12 +1955,13 @@ static int add_solver_loop(mdff_ctx* h, cudaGraph_t g, const cudaGraphNode_t* de
   double tol = h->p.cg_tol > 0 ? h->p.cg_tol : h->p.conv_tol_ind;
   double maxit = (double)(h->p.cg_max_iter > 0 ? h->p.cg_max_iter : 200);
   int f32 = fp32 ? 1 : 0;
-  void* cargs[] = {&sc, &plan, &npol, &tol, &maxit, &f32, &hc};
+  int* stopf = loop_flag(h);
+  void* cargs[] = {&sc, &plan, &npol, &tol, &maxit, &f32, &stopf, &hc};
   const double* r2 = h->d_scal + S_RMS;
   int mn = h->p.min_scf_pol_iter, mx = h->p.max_scf_pol_iter;
   double stol = h->p.conv_tol_ind;
   double* ssc = h->d_scal + S_SCF;
-  void* sargs[] = {&r2, &npol, &stol, &mn, &mx, &ssc, &hc};
+  void* sargs[] = {&r2, &npol, &stol, &mn, &mx, &ssc, &stopf, &hc};
   cudaKernelNodeParams kp = {};
   kp.func = cg ? (void*)k_cg_plan : (void*)k_scf_check;
   kp.gridDim = dim3(1);
@@ -1971,12 +1982,18 @@ static int add_solver_loop(mdff_ctx* h, cudaGraph_t g, const cudaGraphNode_t* de
   int launches0 = h->launches;
   CK(cudaStreamBeginCaptureToGraph(h->st, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
                                    cudaStreamCaptureModeThreadLocal));
-  int s = cg ? cg_iteration(h, fp32, 1, hc) : scf_iteration(h, hc);
+  // several iterations per pass of the loop (a pass has about 5 us of its own), when
+  // their last kernels know the stop flag
+  const int unroll = !cg || cg_fused(h, fp32) ? kLoopUnroll : 1;
+  h->loop_stop = unroll > 1 ? stopf : nullptr;
+  int s = MDFF_OK;
+  for (int u = 0; u < unroll && !s; ++u) s = cg ? cg_iteration(h, fp32, 1, hc) : scf_iteration(h, hc);
+  h->loop_stop = nullptr;
   cudaGraph_t captured;
   cudaError_t e = cudaStreamEndCapture(h->st, &captured);
   h->prof = prof;
   h->call_overlap = ovl;
-  *body_launches = h->launches - launches0;
+  *body_launches = (h->launches - launches0) / unroll;  // of an iteration
   h->launches = launches0;
   if (s) return s;
   if (e != cudaSuccess) {

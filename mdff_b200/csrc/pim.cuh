@@ -171,7 +171,8 @@ __global__ void k_self_surf_field(const double4* __restrict__ mu, int natm, doub
 //   the WHILE condition of the graph that runs the iterations,
 // so that a solve needs no host round trip per iteration.  An iterate formed after
 // the last iteration is not used.  At 216 ions an iteration is a chain of launch
-// latencies: with step, field sum and check as three kernels XX us, now YY.
+// latencies: with step, field sum and check as three kernels 24 us, as one 20.5, with
+// four iterations per pass of the loop (a pass has about 5 us of its own) 18.
 
 // mun = alpha (E_stat + E_ind) and its weights, for the first iteration of the loop
 __device__ __forceinline__ void scf_iterate(const double* al, const double (&E)[3], const CellC* __restrict__ cell,
@@ -206,7 +207,9 @@ __global__ void __launch_bounds__(256) k_scf_tail(const double4* __restrict__ Gp
                                                   double4* __restrict__ Eind, double4* __restrict__ w,
                                                   double* __restrict__ part, int* __restrict__ ticket, int npol_r, double tol,
                                                   int miniter, int maxiter, double* __restrict__ sc,
-                                                  double* __restrict__ upol, cudaGraphConditionalHandle hc) {
+                                                  double* __restrict__ upol, int* __restrict__ stop,
+                                                  cudaGraphConditionalHandle hc) {
+  if (loop_stopped(stop)) return;
   __shared__ double red[2 * 32];
   __shared__ int last;
   double v[2] = {0.0, 0.0};
@@ -273,14 +276,17 @@ __global__ void __launch_bounds__(256) k_scf_tail(const double4* __restrict__ Gp
   sc[0] = (double)it;
   sc[1] = rmsd;
   *upol = v[1];
-  cudaGraphSetConditional(hc, ((it < maxiter && rmsd > tol) || it < miniter) ? 1u : 0u);
+  const bool more = (it < maxiter && rmsd > tol) || it < miniter;
+  if (!more) *stop = 1;
+  cudaGraphSetConditional(hc, more ? 1u : 0u);
 }
 
 // head of the loop: sc[0] = iterations, sc[1] = rmsd from the residual sum r2 of
 // the first iteration.  The condition is the host loop's.
 __global__ void k_scf_check(const double* __restrict__ r2, int npol, double tol, int miniter, int maxiter,
-                            double* __restrict__ sc, cudaGraphConditionalHandle hc) {
+                            double* __restrict__ sc, int* __restrict__ stop, cudaGraphConditionalHandle hc) {
   if (threadIdx.x != 0) return;
+  *stop = 0;
   const double rmsd = sqrt(*r2 / (double)npol);
   sc[0] = 1.0;
   sc[1] = rmsd;
@@ -523,7 +529,9 @@ __global__ void __launch_bounds__(256) k_cg_step(double* __restrict__ sc, const 
                                                  const double4* __restrict__ p, const double4* __restrict__ qv,
                                                  double4* __restrict__ x, double4* __restrict__ r,
                                                  double4* __restrict__ z, double* __restrict__ part,
-                                                 double2* __restrict__ acc, const double2* __restrict__ rhoA, int nk) {
+                                                 double2* __restrict__ acc, const double2* __restrict__ rhoA, int nk,
+                                                 const int* __restrict__ stop) {
+  const bool stopped = loop_stopped(stop);
   __shared__ double red[2 * 32], bc[2];
   const int t0 = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
   // what k_cg_q does not write is read before the wait for it
@@ -535,6 +543,7 @@ __global__ void __launch_bounds__(256) k_cg_step(double* __restrict__ sc, const 
   const double rz = sc[3];
   pdl_wait();
   pdl_trigger();
+  if (stopped) return;
   const double4 q0 = qv[i0];
   double pq[1], v[2] = {0.0, 0.0};
   block_partials<1>(pq_part, npq, pq, red, bc);
@@ -582,7 +591,8 @@ __global__ void __launch_bounds__(256) k_cg_next(double* __restrict__ sc, const 
                                                  const double4* __restrict__ z, double4* __restrict__ p,
                                                  const CellC* __restrict__ cell, float4* __restrict__ w32,
                                                  float4* __restrict__ mu32, SlotW sw, double4* __restrict__ w64,
-                                                 cudaGraphConditionalHandle hc) {
+                                                 int* __restrict__ stop, cudaGraphConditionalHandle hc) {
+  const bool stopped = loop_stopped(stop);
   __shared__ double red[2 * 32], bc[2];
   const int t0 = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
   // (as k_cg_step: only z and the partials are its)
@@ -590,6 +600,7 @@ __global__ void __launch_bounds__(256) k_cg_next(double* __restrict__ sc, const 
   const double4 p0 = p[i0];
   pdl_wait();
   pdl_trigger();
+  if (stopped) return;
   const double4 z0 = z[i0];
   double v[2];
   block_partials<2>(rz_part, nrz, v, red, bc);
@@ -601,7 +612,9 @@ __global__ void __launch_bounds__(256) k_cg_next(double* __restrict__ sc, const 
     const double it = sc[6] + 1.0, rm = sqrt(v[1] / (double)npol_r);
     sc[6] = it;
     sc[8] = rm;
-    cudaGraphSetConditional(hc, (rm > sc[5] && it < sc[7]) ? 1u : 0u);
+    const bool more = rm > sc[5] && it < sc[7];
+    if (!more) *stop = 1;
+    cudaGraphSetConditional(hc, more ? 1u : 0u);
   }
   auto next = [&](int i, const double4& pi, const double4& zi) {
     const double4 pn = make_double4(zi.x + be * pi.x, zi.y + be * pi.y, zi.z + be * pi.z, 0.0);

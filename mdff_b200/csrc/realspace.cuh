@@ -700,7 +700,8 @@ __device__ __forceinline__ void dd_cached_row(const typename vec4t<R>::T* __rest
 static __global__ void __launch_bounds__(256) k_dd_cached_part(
     const float4* __restrict__ mu, const float4* __restrict__ cr, const float* __restrict__ cb1,
     const int* __restrict__ cj, const int* __restrict__ cn, int cap, const int* __restrict__ polidx,
-    int npol, double4* __restrict__ Edd) {
+    int npol, double4* __restrict__ Edd, const int* __restrict__ stop) {
+  if (loop_stopped(stop)) return;
   int lane = threadIdx.x & 31;
   const int sl = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (sl >= npol) return;
@@ -868,7 +869,8 @@ static __global__ void __launch_bounds__(256) k_dd64_build(
 static __global__ void __launch_bounds__(256) k_dd64_apply(
     const double4* __restrict__ mu, const int* __restrict__ polidx, int npol, const double4* __restrict__ cr,
     const double* __restrict__ cb1, const int* __restrict__ cj, const int* __restrict__ cn, int cap, int mask0,
-    double4* __restrict__ E) {
+    double4* __restrict__ E, const int* __restrict__ stop) {
+  if (loop_stopped(stop)) return;
   const int lane = threadIdx.x & 31;
   const int sl = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (sl >= npol) return;

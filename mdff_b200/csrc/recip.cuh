@@ -277,9 +277,11 @@ __device__ __forceinline__ void rec_energy_terms(double s, double4 kv, double (&
 // dipole solve's accumulated rho'; epart: this block's energy terms)
 static __global__ void __launch_bounds__(256) k_rec_sum(const double2* __restrict__ part, int nchunk, RecMesh M,
                           double2* __restrict__ rhoA, double* __restrict__ epart,
-                          double2* __restrict__ acc = nullptr) {
+                          double2* __restrict__ acc, const int* __restrict__ stop) {
+  const bool stopped = loop_stopped(stop);
   pdl_wait();
   pdl_trigger();
+  if (stopped) return;
   __shared__ double red[7 * 8];
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   double ev[7] = {0, 0, 0, 0, 0, 0, 0};

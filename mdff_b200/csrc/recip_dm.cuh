@@ -65,7 +65,7 @@ inline int rho_dm_ci(int kx, int ky, int nt) {
 template <int NT, bool HM>
 static __global__ void __launch_bounds__(kDmThreads, 1) k_rho_dm(
     const double2* __restrict__ tab, const double4* __restrict__ w, int natm, const int* __restrict__ imap,
-    int nion, int chunk, int ci, RecMesh M, double2* __restrict__ part) {
+    int nion, int chunk, int ci, RecMesh M, double2* __restrict__ part, const int* __restrict__ stop) {
   extern __shared__ __align__(16) unsigned char dms[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, tt = lane & 3, rg = warp & 7, half = warp >> 3;
@@ -121,6 +121,10 @@ static __global__ void __launch_bounds__(kDmThreads, 1) k_rho_dm(
   pdl_wait();
   pdl_trigger();
   fetch_w(0);
+  if (loop_stopped(stop)) {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    return;
+  }
   for (int c = 0; c < nch; ++c) {
     if (c + 1 < nch) {
       fetch_tab(c + 1);
@@ -202,9 +206,11 @@ static __global__ void __launch_bounds__(kDmThreads, 1) k_rho_dm(
 // subsets added in order; up to a few tens of chunks
 static __global__ void __launch_bounds__(256) k_rec_sum8(const double2* __restrict__ part, int nchunk, RecMesh M,
                                                          double2* __restrict__ rhoA, double* __restrict__ epart,
-                                                         double2* __restrict__ acc) {
+                                                         double2* __restrict__ acc, const int* __restrict__ stop) {
+  const bool stopped = loop_stopped(stop);
   pdl_wait();
   pdl_trigger();
+  if (stopped) return;
   __shared__ double2 sh[8][32];
   const int lx = threadIdx.x & 31, ly = threadIdx.x >> 5;
   const int k = blockIdx.x * 32 + lx;
@@ -260,8 +266,9 @@ template <int KS, int MODE>
 static __global__ void __launch_bounds__(kDmFldThreads, KS <= 9 ? 2 : 1) k_field_dm(
     const double2* __restrict__ tab, const double4* __restrict__ w, int natm, const int* __restrict__ imap,
     int nion, RecMesh M, const double2* __restrict__ rhoA, int rpg, int rc, double4* __restrict__ Gpart,
-    double4* __restrict__ Hpart) {
+    double4* __restrict__ Hpart, const int* __restrict__ stop) {
   constexpr int KN = 2 * KS, RL = field_dm_rl(KS);
+  const bool stopped = loop_stopped(stop);
   constexpr bool AN = KS <= 9 && MODE == DM_FIELD;  // n (c, s) in registers too
   extern __shared__ __align__(16) unsigned char dms[];
   int4* srow = reinterpret_cast<int4*>(dms);  // the chunk's rows
@@ -297,6 +304,7 @@ static __global__ void __launch_bounds__(kDmFldThreads, KS <= 9 ? 2 : 1) k_field
   // (the phases above are older than the kernel that sums rho', as in k_rho_dm)
   pdl_wait();
   pdl_trigger();
+  if (stopped) return;
   if (MODE == DM_FORCE)
 #pragma unroll
     for (int q = 0; q < 2; ++q) wi[q] = w[ion[q]];

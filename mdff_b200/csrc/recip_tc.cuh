@@ -242,9 +242,8 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t
 // up to two ahead of the products.
 static __global__ void __launch_bounds__(kRhoTcThreads, 1) k_rec_rho_tc(
     const float2* __restrict__ timg, const float4* __restrict__ ws, int nion, int chunk, RecMesh M,
-    double2* __restrict__ part, int* __restrict__ err, const int* __restrict__ wait_cfg) {
-  pdl_wait();
-  pdl_trigger();
+    double2* __restrict__ part, int* __restrict__ err, const int* __restrict__ wait_cfg,
+    const int* __restrict__ stop) {
   constexpr int NG = kRhoTcGen, RPT = kRhoTcRows, KB = kRhoTcKB, KC = KB / 4, NS = kRhoTcStg;
   static_assert(RPT * KC == NG, "A items: one (row, 4 ions) per generating thread");
   extern __shared__ unsigned char smraw[];
@@ -265,6 +264,7 @@ static __global__ void __launch_bounds__(kRhoTcThreads, 1) k_rec_rho_tc(
     uint32_t dyn;
     asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
     if (dyn < rho_tc_smem(kx, ky, kz) || Nr > 256) {
+      pdl_wait();
       if (tid == 0) atomicExch(err, 2);
       return;
     }
@@ -307,10 +307,18 @@ static __global__ void __launch_bounds__(kRhoTcThreads, 1) k_rec_rho_tc(
       *reinterpret_cast<uint4*>(S + tc::canon((sp & 1) * Nr + c, kc * 4, NB2)) = make_uint4(0u, 0u, 0u, 0u);
     }
   }
+  // (up to here nothing of an earlier kernel is read)
+  pdl_wait();
+  pdl_trigger();
+  const bool stopped = loop_stopped(stop);
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem = tslot;
+  if (stopped) {
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols));
+    return;
+  }
 
   const int r0 = blockIdx.x * RPT;
   const int a0 = blockIdx.y * chunk;
@@ -620,9 +628,12 @@ template <bool HAS_H, int KF>
 static __global__ void __launch_bounds__(128) k_rec_field_btiles(RecMesh M, const double2* __restrict__ rhoA,
                                                                  const double2* __restrict__ part, int npart,
                                                                  uint32_t* __restrict__ fb,
-                                                                 double2* __restrict__ rho_out) {
+                                                                 double2* __restrict__ rho_out,
+                                                                 const int* __restrict__ stop) {
+  const bool stopped = loop_stopped(stop);
   pdl_wait();
   pdl_trigger();
+  if (stopped) return;
   constexpr int CPR = HAS_H ? 8 : 4, RPT = 128 / CPR;
   constexpr int TILE = 128 * KF * 4;
   const int kz = M.kmax[2], nzc = kz + 1, nzs = 2 * kz + 1;
@@ -685,7 +696,8 @@ static __global__ void __launch_bounds__(kFieldTcThreads, 1) k_rec_field_tc(
     const float2* __restrict__ tab, const float4* __restrict__ w, int natm, const int* __restrict__ imap,
     int nion, RecMesh M,
     const uint32_t* __restrict__ fb, int tiles_per_group, double4* __restrict__ Gpart,
-    double4* __restrict__ Hpart, int* __restrict__ err) {
+    double4* __restrict__ Hpart, int* __restrict__ err, const int* __restrict__ stop) {
+  const bool stopped = loop_stopped(stop);
   constexpr int NT = kFieldTcRed;
   constexpr int CPR = HAS_H ? 8 : 4;     // columns per mesh row (6 used with H)
   constexpr int RPT = 128 / CPR;         // mesh rows per tile
@@ -767,6 +779,7 @@ static __global__ void __launch_bounds__(kFieldTcThreads, 1) k_rec_field_tc(
   }
   pdl_wait();
   pdl_trigger();
+  if (stopped) return;
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      tc::smem_u32(&tslot)),
