@@ -216,14 +216,19 @@ __global__ void __launch_bounds__(256) k_scf_tail(const double4* __restrict__ Gp
   const int t = blockIdx.x * blockDim.x + threadIdx.x, sl = t >> 2, sub = t & 3;
   double g[3] = {0.0, 0.0, 0.0};
   int i = 0;
+  double4 m, o, st;
+  double al[9], iv[9];
   if (sl < npol) {
     i = polidx[sl];
-    for (int c = sub; c < nchunk; c += 4) {
-      const double4 u = Gpart[(size_t)c * natm + i];
-      g[0] += u.x;
-      g[1] += u.y;
-      g[2] += u.z;
+    m = mun[i];
+    o = Eind[i];
+    st = Estat[i];
+#pragma unroll
+    for (int a = 0; a < 9; ++a) {
+      al[a] = P.pol[9 * (size_t)i + a];
+      iv[a] = P.invpol[9 * (size_t)i + a];
     }
+    chunk_sum4(Gpart, nchunk, natm, i, sub, g);
   }
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
@@ -232,10 +237,7 @@ __global__ void __launch_bounds__(256) k_scf_tail(const double4* __restrict__ Gp
   }
   if (sl < npol && sub == 0) {
     const double* B = cell->B;
-    const double4 m = mun[i], o = Eind[i], st = Estat[i];
     const double mm[3] = {m.x, m.y, m.z}, oo[3] = {o.x, o.y, o.z}, ss[3] = {st.x, st.y, st.z};
-    const double* al = P.pol + 9 * (size_t)i;
-    const double* iv = P.invpol + 9 * (size_t)i;
     double e[3], E[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
@@ -493,13 +495,8 @@ __global__ void __launch_bounds__(256) k_cg_q(const double4* __restrict__ Gpart,
     const bool ok = sl < npol;
     const int i = polidx[ok ? sl : npol - 1];
     double g[3] = {0.0, 0.0, 0.0};
-    for (int c = sub; c < nchunk; c += 4) {
-      const double4 u = Gpart[(size_t)c * natm + i];
-      g[0] += u.x;
-      g[1] += u.y;
-      g[2] += u.z;
-    }
     const double4 pi = p[i], o = Edd[i];
+    chunk_sum4(Gpart, nchunk, natm, i, sub, g);
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
       g[a] += __shfl_xor_sync(FULL_MASK, g[a], 1);

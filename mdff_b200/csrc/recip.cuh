@@ -43,6 +43,24 @@ struct SelfField {
   const double* mom;
 };
 
+// chunk sums of the field partials of ion i: this thread's chunks sub, sub + 4, ..
+// (four threads per ion), four loads in flight
+__device__ __forceinline__ void chunk_sum4(const double4* __restrict__ part, int nchunk, int natm, int i, int sub,
+                                           double (&g)[3]) {
+  for (int c0 = sub; c0 < nchunk; c0 += 16) {
+    double4 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      v[u] = c0 + 4 * u < nchunk ? part[(size_t)(c0 + 4 * u) * natm + i] : make_double4(0.0, 0.0, 0.0, 0.0);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      g[0] += v[u].x;
+      g[1] += v[u].y;
+      g[2] += v[u].z;
+    }
+  }
+}
+
 struct RecMesh {
   int kmax[3];
   int nrows;
@@ -507,18 +525,8 @@ static __global__ void k_rec_field_sum(const double4* __restrict__ Gpart, const 
   int i = t >> 2, sub = t & 3;
   double g[3] = {0, 0, 0}, h[3] = {0, 0, 0};
   if (i < natm) {
-    for (int c = sub; c < nchunk; c += 4) {
-      double4 v = Gpart[(size_t)c * natm + i];
-      g[0] += v.x;
-      g[1] += v.y;
-      g[2] += v.z;
-      if (has_mu_force) {
-        double4 u = Hpart[(size_t)c * natm + i];
-        h[0] += u.x;
-        h[1] += u.y;
-        h[2] += u.z;
-      }
-    }
+    chunk_sum4(Gpart, nchunk, natm, i, sub, g);
+    if (has_mu_force) chunk_sum4(Hpart, nchunk, natm, i, sub, h);
   }
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
