@@ -75,6 +75,7 @@ struct mdff_batch {
   int ws_ctas = 0, ws_clusters = 0;  // CTAs and clusters the workspaces are sized for
   double *d_force = nullptr, *d_part = nullptr, *d_out = nullptr, *d_pack = nullptr;
   double* h_out = nullptr;
+  double* h_stage = nullptr;  // pinned: positions [3][ntot], outputs [9 ntot] (host arrays of a call)
   // launch
   Shape shape{2, 512};
   cudaGraph_t graph = nullptr;
@@ -362,13 +363,19 @@ int build_graph(mdff_batch* h, const double* d_pos, double* d_force) {
   return MDFF_OK;
 }
 
-int run(mdff_batch* h, const double* d_pos, double* d_force) {
+// (outs: the call's results into pinned host memory too, mu and E when asked for)
+int run(mdff_batch* h, const double* d_pos, double* d_force, double* outs = nullptr, bool mu = false, bool ef = false) {
   int s;
   if (!h->exec || h->graph_pos != d_pos || h->graph_force != d_force)
     if ((s = build_graph(h, d_pos, d_force))) return s;
   BCK(cudaEventRecord(h->ev0, h->st));
   BCK(cudaGraphLaunch(h->exec, h->st));
   BCK(cudaEventRecord(h->ev1, h->st));
+  if (outs) {
+    k_outputs<<<(int)((9L * h->ntot + 255) / 256), 256, 0, h->st>>>(h->d_force, mu ? h->d_mu : nullptr,
+                                                                  ef ? h->d_E : nullptr, h->ntot, outs);
+    BCK(cudaGetLastError());
+  }
   BCK(cudaMemcpyAsync(h->h_out, h->d_out, sizeof(double) * kBSlots * h->nconf,
                       cudaMemcpyDeviceToHost, h->st));
   BCK(cudaStreamSynchronize(h->st));
@@ -787,6 +794,7 @@ void destroy_impl(mdff_batch* h) {
   for (void* b : bufs)
     if (b) cudaFree(b);
   if (h->h_out) cudaFreeHost(h->h_out);
+  if (h->h_stage) cudaFreeHost(h->h_stage);
   if (h->ev0) cudaEventDestroy(h->ev0);
   if (h->ev1) cudaEventDestroy(h->ev1);
   if (h->st) cudaStreamDestroy(h->st);
@@ -837,6 +845,26 @@ int mdff_gpu_batch_engforce(mdff_batch_handle h, const double* rx, const double*
   if (!h || !rx || !ry || !rz || !fx || !fy || !fz) return MDFF_ERR_BAD_ARGS;
   BCK(cudaSetDevice(h->device));
   size_t nb = sizeof(double) * h->ntot;
+  if (h->ntot <= kHostStage && !h->h_stage && cudaMallocHost((void**)&h->h_stage, 12 * nb) != cudaSuccess) {
+    cudaGetLastError();
+    h->h_stage = nullptr;
+  }
+  if (h->h_stage) {
+    const size_t n = h->ntot;
+    double* o = h->h_stage + 3 * n;
+    memcpy(h->h_stage, rx, nb);
+    memcpy(h->h_stage + n, ry, nb);
+    memcpy(h->h_stage + 2 * n, rz, nb);
+    BCK(cudaMemcpyAsync(h->d_pos, h->h_stage, 3 * nb, cudaMemcpyHostToDevice, h->st));
+    const int s = run(h, h->d_pos, h->d_force, o, mu != nullptr, ef != nullptr);
+    if (s) return s;
+    memcpy(fx, o, nb);
+    memcpy(fy, o + n, nb);
+    memcpy(fz, o + 2 * n, nb);
+    if (mu) memcpy(mu, o + 3 * n, 3 * nb);
+    if (ef) memcpy(ef, o + 6 * n, 3 * nb);
+    return finish(h, conf);
+  }
   BCK(cudaMemcpyAsync(h->d_pos, rx, nb, cudaMemcpyHostToDevice, h->st));
   BCK(cudaMemcpyAsync(h->d_pos + h->ntot, ry, nb, cudaMemcpyHostToDevice, h->st));
   BCK(cudaMemcpyAsync(h->d_pos + 2 * (size_t)h->ntot, rz, nb, cudaMemcpyHostToDevice, h->st));

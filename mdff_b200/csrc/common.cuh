@@ -279,6 +279,26 @@ struct SlotW {
   }
 };
 
+// Host arrays of a call pass through one pinned buffer up to this many ions (25
+// MB): one copy of the positions instead of three from pageable memory (10 us
+// each), one kernel that writes every result across the bus instead of five copies and
+// two packing kernels with a synchronisation between (1728 ions: 30 + 110 us, now
+// about 5 + 15).
+constexpr int kHostStage = 262144;
+// results of a call into mapped pinned host memory: force [3][natm], then mu
+// and E as [natm][3] (absent ones skipped)
+static __global__ void k_outputs(const double* __restrict__ force, const double4* __restrict__ mu,
+                          const double4* __restrict__ E, int natm, double* __restrict__ out) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, n3 = 3 * natm;
+  if (t < n3) {
+    out[t] = force[t];
+  } else if (t < 3 * n3) {
+    const int e = (t - n3) % n3;
+    const double4* v = t < 2 * n3 ? mu : E;
+    if (v) out[t] = reinterpret_cast<const double*>(v + e / 3)[e % 3];
+  }
+}
+
 // A solver's loop body holds several iterations; the kernels of those after the one
 // that finished leave at once (stop: flag set by its last kernel, nullptr outside
 // a loop).  Kernels two or more after that one read it before their pdl_wait.

@@ -450,20 +450,6 @@ __global__ void k_vv_step(double* __restrict__ pos, double* __restrict__ vel, co
   if (threadIdx.x == 0) part[blockIdx.x] = e[0];
 }
 
-// results of a call into mapped pinned host memory: force [3][natm], then mu
-// and E as [natm][3] (absent ones skipped)
-__global__ void k_outputs(const double* __restrict__ force, const double4* __restrict__ mu,
-                          const double4* __restrict__ E, int natm, double* __restrict__ out) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x, n3 = 3 * natm;
-  if (t < n3) {
-    out[t] = force[t];
-  } else if (t < 3 * n3) {
-    const int e = (t - n3) % n3;
-    const double4* v = t < 2 * n3 ? mu : E;
-    if (v) out[t] = reinterpret_cast<const double*>(v + e / 3)[e % 3];
-  }
-}
-
 // ---------------------------------------------------------------------------
 // set-up (host): the reference's *_init routines
 
@@ -2965,12 +2951,6 @@ int mdff_gpu_set_cell(mdff_handle h, const double cell_A[9]) {
   return MDFF_OK;
 }
 
-// Host arrays of a call pass through one pinned buffer up to this many ions (25
-// MB): one copy of the positions instead of three from pageable memory (10 us
-// each), one kernel that writes every result across the bus instead of five copies and
-// two packing kernels with a synchronisation between (1728 ions: 30 + 110 us, now
-// about 5 + 15).
-constexpr int kHostStage = 262144;
 static bool host_stage(mdff_ctx* h) {
   if (h->natm > kHostStage) return false;
   if (!h->h_stage && cudaMallocHost((void**)&h->h_stage, sizeof(double) * 12 * (size_t)h->natm) != cudaSuccess) {

@@ -9,7 +9,8 @@
 // Likewise k.mu = n . m with m = 2 pi B^T mu, and sum_k k f(k) = 2 pi B sum_k n f(k).
 //
 //   k_rec_rho   : rho(k) = sum_i (q_i + i k.mu_i) e^{i k.r_i}   (ewald_rec.f90:118-148)
-//                 block = (row, nz tile) x ion chunk; fixed-order partials.
+//                 block = (row, nz tile) x ion chunk; fixed-order partials; serves the
+//                 meshes whose tables do not fit the tensor-core kernel (recip_dm.cuh)
 //   k_rec_sum   : rho over chunks; rho' = A_k rho; with energy its blocks' sums of
 //                 A_k |rho|^2 (:173) for u_rec and the stress (:255-263, 300-358), which
 //                 k_rec_field_sum adds up in fixed order

@@ -17,12 +17,12 @@
 //
 // Both are bound by the FP64 pipe (18.5e12 multiply-adds a second).  Measured on
 // one B200 (cold caches, in isolation): 8000-ion MgO, kmax 16 (17,968 k), the
-// 4000 dipoles of an operator application: structure factor 132 -> 41 us (the
-// recurrence ran over all ions; 15.5 us at the pipe's rate), field 81 -> 37 us.
+// 4000 dipoles of an operator application: structure factor 132 -> 39 us (the
+// recurrence ran over all ions; 15.5 us at the pipe's rate), field 81 -> 39 us.
 // 13,700-ion NaCl, kmax 20 (34,460 k), charges, where the FP32 recurrence ran
-// in the mixed engine: 272 -> 163 us.  Whole calls: 8000-ion MgO, FP64 SCF from
-// scratch (43 iterations) 12.1 -> 7.1 ms; 5100-ion silica, FP64 CG and field
-// gradients 1.99 -> 1.34 ms (the gradient's reciprocal part 405 -> 18 us).
+// in the mixed engine: 272 -> 108 us.  Whole calls: 8000-ion MgO, FP64 SCF from
+// scratch (43 iterations) 12.1 -> 7.1 ms with these kernels alone; 5100-ion silica, FP64 CG
+// and field gradients 1.99 -> 1.34 ms (the gradient's reciprocal part 405 -> 18 us).
 #pragma once
 #include "dmma.cuh"
 #include "recip.cuh"
