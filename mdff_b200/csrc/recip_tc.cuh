@@ -590,12 +590,14 @@ namespace mdff {
 // barrier in the loop.  The ions' features and phases are formed before the
 // wait for the predecessor (the B tiles), which they do not depend on.
 //
-// Bound: per tile the products (3 K / 8 of 128 x 128 x 8, about 1000 cycles at K =
-// 40) and the reduction (8 rows x 16 FP32 operations a thread, about 700 issue cycles a
-// scheduler) run side by side; what is left is start-up and the wave.  Two CTAs
+// Bound: per tile the products (3 K / 8 of 128 x 128 x 8, about 1200 cycles at K =
+// 48) and the reduction (8 rows a warp, about 350 instructions, 1400 issue cycles a
+// scheduler) run side by side at half of their rates each, 2700 cycles a tile (13700
+// ions; a third B buffer, indices and phases read before the wait, or fewer waves of
+// CTAs change nothing).  Two CTAs
 // of 256 threads with barriers between copy, product and reduction and K = 32 or
-// 64 took, in an MD step: the operator's field of 4000 dipoles on 572 rows (kz 16)
-// 34 us, now 14; with dipole forces, 8000 ions, 65 -> 32; 13700 ions on 1050 rows
+// 64 took, in an MD step: the operator's field of 4000 dipoles on 545 rows (kz 16)
+// 34 us, now 14; with dipole forces, 8000 ions, 65 -> 32; 13700 ions on 841 rows
 // (kz 20) 97 -> 46.
 constexpr int kFieldTcRed = 512;                    // reducing threads: 128 ions x 4 column chunks
 constexpr int kFieldTcThreads = kFieldTcRed + 64;   // + the MMA warp and the copy warp
