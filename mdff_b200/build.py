@@ -9,7 +9,7 @@ CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "libmdff_gpu.so")
 SOURCES = ["mdff_gpu.cu", "mdff_noalloc.cu", "batch.cu"]
 HEADERS = ["common.cuh", "nlist.cuh", "realspace.cuh", "recip.cuh", "recip_dm.cuh", "recip_tc.cuh", "pim.cuh", "ko.cuh", "dmma.cuh", "batch_rec.cuh", "batch.cuh", "adjoint.cuh",
-           "setup.h"]
+           "setup.h", "shapes.h"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

@@ -140,6 +140,7 @@ struct mdff_ctx {
   int rec_mode = 0;
   double* d_epart = nullptr;  // block sums of the reciprocal energy terms
   int n_rho_chunks = 0;
+  int rho_part_chunks = 0;  // chunks that d_rho_part holds
   // FP64 structure factor on the tensor cores (k_rho_dm): ions a staged buffer
   // holds (0: the mesh does not fit), n tiles per pass and passes; most ion chunks
   int dm_ci[2] = {0, 0}, dm_nt[2] = {0, 0}, dm_groups[2] = {0, 0};  // [1] with dipoles, [0] charges alone
@@ -464,13 +465,9 @@ static void lattice(mdff_ctx* h, const double* Ain) {
   h->omega = L.omega;
 }
 
-// ions per chunk of k_rho_dm over nion ions, and the chunks: one block per SM
-// over (row blocks x chunks x n passes), at least 16 ions a chunk
-static void rho_dm_shape(const mdff_ctx* h, int nion, bool hm, int* chunk, int* nchunk) {
-  const int per = cdiv((int)h->rows.size(), kDmRows) * std::max(h->dm_groups[hm], 1);
-  const int want = std::max(1, (h->nsm > 0 ? h->nsm : 148) / std::max(per, 1));
-  *chunk = std::max(16, cdiv(cdiv(nion, want), 8) * 8);
-  *nchunk = cdiv(nion, *chunk);
+// ion chunks wanted of k_rho_dm on this mesh, with and without dipoles
+static int rho_dm_want_of(const mdff_ctx* h, bool hm) {
+  return rho_dm_want(h->nsm, (int)h->rows.size(), h->dm_groups[hm]);
 }
 #define RHO_DM_SWITCH(NTV, CALL) \
   switch (NTV) {                 \
@@ -619,11 +616,10 @@ static int build_mesh(mdff_ctx* h) {
       CK(cudaMemcpy(h->d_polslot, slot.data(), sizeof(int) * h->natm, cudaMemcpyHostToDevice));
     }
   }
-  int dm_chunks = 0, dm_len = 0, dm_chunks0 = 0;
-  rho_dm_shape(h, h->natm, true, &dm_len, &dm_chunks);
-  rho_dm_shape(h, h->natm, false, &dm_len, &dm_chunks0);
-  dm_chunks = std::max(dm_chunks, dm_chunks0);
-  DALLOC(h->d_rho_part, (size_t)std::max({h->n_rho_chunks, h->n_tc_chunks, dm_chunks}) * std::max(nk, 1));
+  // k_rho_dm runs over all ions or the polarisable ones
+  h->rho_part_chunks = std::max({h->n_rho_chunks, h->n_tc_chunks, rho_dm_most(h->natm, rho_dm_want_of(h, true)),
+                                 rho_dm_most(h->natm, rho_dm_want_of(h, false))});
+  DALLOC(h->d_rho_part, (size_t)h->rho_part_chunks * std::max(nk, 1));
   if (h->dm_ci[1]) {
     int e = 0;
 #define RDA(NT) e = allow_smem((const void*)k_rho_dm<NT, HM>, rho_dm_smem(h->p.kES[0], h->p.kES[1], NT, h->dm_ci[HM]))
@@ -877,13 +873,18 @@ static SlotW slotw(const mdff_ctx* h) {
 }
 
 // FP64 structure factor of the weights d_w over the ions of imap (nion of them;
-// nullptr: all) into d_rho_part; returns the number of partial chunks.  Launch
+// nullptr: all) into d_rho_part; *nparts: the number of partial chunks.  Launch
 // errors surface at the caller's LAUNCH_CHECK.
-static int launch_rho64(mdff_ctx* h, const RecMesh& M, int n, const int* imap, int nion, int has_q, int has_mu) {
+static int launch_rho64(mdff_ctx* h, const RecMesh& M, int n, const int* imap, int nion, int has_q, int has_mu,
+                        int* nparts) {
   const int hm = has_mu ? 1 : 0;
   if (h->dm_ci[1]) {
     int chunk, nchunk;
-    rho_dm_shape(h, nion, hm, &chunk, &nchunk);
+    rho_dm_split(nion, rho_dm_want_of(h, hm), &chunk, &nchunk);
+    if (nchunk > h->rho_part_chunks) {
+      h->err = "structure-factor partials: more chunks than allocated";
+      return MDFF_ERR_CUDA;
+    }
     const dim3 g((unsigned)cdiv(M.nrows, kDmRows), (unsigned)nchunk, (unsigned)h->dm_groups[hm]);
     const size_t smem = rho_dm_smem(M.kmax[0], M.kmax[1], h->dm_nt[hm], h->dm_ci[hm]);
     const double2* tab = h->d_tab64;
@@ -899,7 +900,8 @@ static int launch_rho64(mdff_ctx* h, const RecMesh& M, int n, const int* imap, i
       RHO_DM_SWITCH0(h->dm_nt[0], RDL)
     }
 #undef RDL
-    return nchunk;
+    *nparts = nchunk;
+    return MDFF_OK;
   }
   // a mesh too large for the staging buffers: the phase recurrence over all ions
   const int ntiles = cdiv(2 * M.kmax[2] + 1, kRhoNzt);
@@ -911,7 +913,8 @@ static int launch_rho64(mdff_ctx* h, const RecMesh& M, int n, const int* imap, i
     (void)pdl_launch(k_rec_rho<double, true, false, kRhoNzt>, g, dim3(kRhoThreads), 0, h->st, tab, h->d_w, n, kRhoChunk, M, ntiles, h->d_rho_part);
   else
     (void)pdl_launch(k_rec_rho<double, false, true, kRhoNzt>, g, dim3(kRhoThreads), 0, h->st, tab, h->d_w, n, kRhoChunk, M, ntiles, h->d_rho_part);
-  return h->n_rho_chunks;
+  *nparts = h->n_rho_chunks;
+  return MDFF_OK;
 }
 
 // FP64 field (mode DM_*) of rhoA at the ions of imap into d_G / d_H on the tensor
@@ -1090,7 +1093,9 @@ static int rec_pass_t(mdff_ctx* h, const typename cplx<R>::T* tab, const double4
     if (F32 && weights_ready)  // (the CG direction kernels write FP32 weights only)
       PDL_CHECK(pdl_launch(k_rec_weights, dim3(cdiv(n, 256)), dim3(256), 0, h->st, h->d_q, mu, n, h->d_cell, has_q,
                            has_mu, h->d_w, (float4*)nullptr, (float4*)nullptr, SlotW()));
-    nparts = launch_rho64(h, M, n, pol ? h->d_polidx : nullptr, pol ? (int)h->polidx.size() : n, has_q, has_mu);
+    const int e = launch_rho64(h, M, n, pol ? h->d_polidx : nullptr, pol ? (int)h->polidx.size() : n, has_q, has_mu,
+                               &nparts);
+    if (e) return e;
   }
   LAUNCH_CHECK();
   prof_end(h, pr);
@@ -3250,10 +3255,10 @@ int mdff_gpu_efg(mdff_handle h, double* efg) {
     int has_q = h->task_qq ? 1 : 0, has_mu = (h->task_qd || h->task_dd) ? 1 : 0;
     k_rec_weights<<<cdiv(n, 256), 256, 0, h->st>>>(h->d_q, h->d_mu_tot, n, h->d_cell, has_q, has_mu, h->d_w, nullptr, nullptr);
     LAUNCH_CHECK();
-    const int nparts = launch_rho64(h, M, n, nullptr, n, has_q, has_mu);
+    int nparts, nep, e;
+    if ((e = launch_rho64(h, M, n, nullptr, n, has_q, has_mu, &nparts))) return e;
     LAUNCH_CHECK();
-    int nep;
-    int e = rho_sum(h, M, nparts, nullptr, false, &nep);
+    e = rho_sum(h, M, nparts, nullptr, false, &nep);
     if (e) return e;
     const double scale = 2.0 * (2.0 * (kTwoPi / h->omega));
     if (field_dm_ks(M.kmax[2])) {

@@ -26,38 +26,17 @@
 #pragma once
 #include "dmma.cuh"
 #include "recip.cuh"
+#include "shapes.h"
 
 namespace mdff {
 
 constexpr int kDmThreads = 512;    // k_rho_dm: 8 groups of 8 rows x 2 ion halves
-constexpr int kDmRows = 64;        // mesh rows per block
 constexpr int kDmFldThreads = 256; // k_field_dm: 8 warps of 16 ions
 constexpr int kDmFldIons = 128;
 
 __device__ __forceinline__ void dm_cp16(void* smem, const void* g) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(g)
                : "memory");
-}
-
-// n tiles (of four n) per pass over the ions, and passes: as many as their
-// accumulators allow (registers: 8 a tile, 16 with dipoles).  Charges alone have
-// one product per tile for the same loads of the ions' phases: 13700 ions, kz 20, two
-// passes of three tiles 141 us, one of six 108 us.
-inline int rho_dm_nt(int kz, bool hm) {
-  const int most = hm ? 5 : 8, tiles = kz / 4 + 1, groups = (tiles + most - 1) / most;
-  return (tiles + groups - 1) / groups;
-}
-// shared memory of k_rho_dm staging ci ions a buffer, and the largest ci (32, 16
-// or 8) whose two buffers fit half an SM (0: the mesh does not fit)
-inline size_t rho_dm_smem(int kx, int ky, int nt, int ci) {
-  const size_t ent = (size_t)(kx + 1 + ky + 1 + 4 * nt);
-  const size_t b = 2 * (ent * (ci + 4) * 16 + (size_t)ci * 32), red = 8 * 32 * 8 * 8;
-  return b > red ? b : red;
-}
-inline int rho_dm_ci(int kx, int ky, int nt) {
-  for (int ci = 32; ci >= 8; ci /= 2)
-    if (rho_dm_smem(kx, ky, nt, ci) <= (ci > 8 ? 110 * 1024 : 227 * 1024)) return ci;
-  return 0;
 }
 
 // Structure-factor partials: grid (row blocks, ion chunks, n passes).  imap: the
