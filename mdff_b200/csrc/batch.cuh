@@ -363,15 +363,13 @@ __device__ __forceinline__ BRecArgs brec_args(const BatchArgs& a, BCtx& X, const
   r.wd = BWeights{X.c, S.s, S.v, S.v32, r.dst.n0, 0, false, true};
   return r;
 }
-// room for nw weights per ion (in the staging buffer, else in the field's
-// scratch); the rest of the buffer holds the records in passing
+// room for nw weights per ion, the rest of the staging buffer for the records in
+// passing (brec_staging)
 __device__ __forceinline__ double4* brec_weights(BRecArgs& r, const BShared& S, int nw) {
-  const int bytes = r.src.cnt * 32 * nw;
-  const bool in_stage = bytes <= S.stage_bytes / 3;
-  double4* w = in_stage ? reinterpret_cast<double4*>(S.stage) : reinterpret_cast<double4*>(r.gp);
-  r.buf = S.stage + (in_stage ? (bytes + 127) / 128 * 128 : 0);
-  const int ch = (int)((S.stage + S.stage_bytes - r.buf) / (2 * r.c->rs)) & ~3;
-  r.CH = ch < 32 ? ch : 32;
+  const BStaging st = brec_staging(S.stage_bytes, r.src.cnt, nw, r.c->rs);
+  double4* w = st.weights ? reinterpret_cast<double4*>(S.stage) : reinterpret_cast<double4*>(r.gp);
+  r.buf = S.stage + st.weights;
+  r.CH = st.ch;
   r.w = w;
   return w;
 }

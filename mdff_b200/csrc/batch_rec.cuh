@@ -31,10 +31,10 @@
 #include "dmma.cuh"
 #include "realspace.cuh"
 #include "recip.cuh"
+#include "shapes.h"
 
 namespace mdff {
 
-constexpr int kBStage = 16384;  // least bytes of the shared staging buffer
 constexpr int kBSplit = 8;      // most row subsets of the field's ion blocks
 
 // words of an ion: type (4 bits), polarisable flag (1), its rank among the
@@ -62,15 +62,6 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
-// bytes of an ion's phase record: X, Y, then (c, s) of n = 0..kz padded with
-// zeros to whole tiles of brho (4 n) and steps of bfld (2 n, at least 3 steps);
-// 32 mod 128, so that the lanes of a fragment load hit distinct banks
-__host__ __device__ inline int brec_bytes(int kx, int ky, int kz) {
-  const int z1 = (kz / 4 + 1) * 64, z2 = (kz / 2 < 2 ? 3 : kz / 2 + 1) * 32;
-  const int b = (kx + 1 + ky + 1) * 16 + (z1 > z2 ? z1 : z2);
-  return (b + 95) / 128 * 128 + 32;
 }
 
 // Partial structure factor of this CTA's ions over all rows: out[row * (kz + 1)

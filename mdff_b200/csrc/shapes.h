@@ -4,6 +4,12 @@
 #include <algorithm>
 #include <cstddef>
 
+#ifdef __CUDACC__
+#define MDFF_HD __host__ __device__
+#else
+#define MDFF_HD
+#endif
+
 namespace mdff {
 
 inline int ceil_div(long a, long b) { return (int)((a + b - 1) / b); }
@@ -48,5 +54,37 @@ inline void rho_dm_split(int nion, int want, int* chunk, int* nchunk) {
 // most chunks of any subset of natm ions: a chunk holds at least nion / want ions
 // and at least 16
 inline int rho_dm_most(int natm, int want) { return std::min(want, ceil_div(natm, 16)); }
+
+// ---------------------------------------------------------------------------
+// reciprocal sums of the batched engine (brho_t, bfld_t)
+
+constexpr int kBStage = 16384;  // least bytes of the shared staging buffer
+
+// bytes of an ion's phase record: X, Y, then (c, s) of n = 0..kz padded with
+// zeros to whole tiles of brho (4 n) and steps of bfld (2 n, at least 3 steps);
+// 32 mod 128, so that the lanes of a fragment load hit distinct banks
+MDFF_HD inline int brec_bytes(int kx, int ky, int kz) {
+  const int z1 = (kz / 4 + 1) * 64, z2 = (kz / 2 < 2 ? 3 : kz / 2 + 1) * 32;
+  const int b = (kx + 1 + ky + 1) * 16 + (z1 > z2 ? z1 : z2);
+  return (b + 95) / 128 * 128 + 32;
+}
+
+// The staging buffer of brho_t: the weights (nw of 32 bytes for each of cnt ions) lie in
+// its first `weights` bytes when they take at most a third of it and leave two buffers
+// of four records of rs bytes (a step takes four ions), else in the field's scratch (weights
+// = 0); ch: records per buffer, at most 32, fewer than four only where the whole
+// buffer has no room for eight records (kx + ky above 110 in the least buffer).
+struct BStaging {
+  int weights, ch;
+};
+MDFF_HD inline BStaging brec_staging(int stage_bytes, int cnt, int nw, int rs) {
+  const int bytes = (cnt * 32 * nw + 127) / 128 * 128;
+  const bool in_stage = cnt * 32 * nw <= stage_bytes / 3 && (stage_bytes - bytes) / (2 * rs) >= 4;
+  BStaging s;
+  s.weights = in_stage ? bytes : 0;
+  const int ch = (stage_bytes - s.weights) / (2 * rs);
+  s.ch = ch >= 32 ? 32 : ch >= 4 ? ch / 4 * 4 : ch;
+  return s;
+}
 
 }  // namespace mdff

@@ -42,6 +42,26 @@ int dm_overruns(int nsm, int kmax, int natm_lo, int natm_hi) {
   }
   return bad;
 }
+// stagings of the batched engine's structure factor over the meshes that a batch
+// takes (kx, ky <= 64, kz <= 12), 0-2048 ions, one or two weights an ion, for one
+// buffer size: records that do not fit, none at all, or fewer than four although eight fit
+int batch_staging_faults(int stage, int* least) {
+  int bad = 0;
+  *least = 1 << 30;
+  for (int kxy = 0; kxy <= 128; ++kxy)
+    for (int kz = 0; kz <= 12; ++kz) {
+      const int rs = brec_bytes(kxy / 2, kxy - kxy / 2, kz);
+      for (int cnt = 0; cnt <= 2048; cnt += cnt < 64 ? 1 : 13)
+        for (int nw = 1; nw <= 2; ++nw) {
+          const BStaging s = brec_staging(stage, cnt, nw, rs);
+          bad += s.ch < 1 || s.ch > 32 || s.weights + 2 * s.ch * rs > stage || s.weights % 128 != 0;
+          bad += s.weights && s.weights < cnt * 32 * nw;
+          bad += s.ch >= 4 ? s.ch % 4 != 0 : stage >= 8 * rs;
+          if (s.ch < *least) *least = s.ch;
+        }
+    }
+  return bad;
+}
 }
 """
 
@@ -73,3 +93,10 @@ def test_structure_factor_chunks_fit_their_buffer(shapes, kmax, nsm):
     assert shapes.dm_overruns(nsm, kmax, 1, 6000) == 0
     assert shapes.dm_overruns(nsm, kmax, 13600, 13800) == 0
     assert shapes.dm_overruns(nsm, kmax, 100000, 100050) == 0
+
+
+@pytest.mark.parametrize("stage", [16384] + list(range(20480, 40960 + 1, 1280)))
+def test_batch_staging_holds_records(shapes, stage):
+    least = ctypes.c_int()
+    assert shapes.batch_staging_faults(stage, ctypes.byref(least)) == 0
+    assert least.value >= 3
