@@ -59,8 +59,9 @@ enum {
   S_CATA = 72,   // 4 ints: d_cata
   S_FLAGS = 74,  // 4 ints: the list's flags
   S_EKIN = 76,   // kinetic energy of the last MD step
-  S_TICK = 77,   // 2 ints: block ticket of k_scf_tail, stop flag of the solver's loop
-  S_NALL = 78
+  S_TICK = 77,   // 3 ints: block ticket of k_scf_tail, stop flag of the solver's loop and
+                 // its copy of this CG iteration
+  S_NALL = 79
 };
 
 // FP32 CG: the recurrence residual drifts from the true one by about the FP32
@@ -1873,11 +1874,11 @@ static int cg_iteration(mdff_ctx* h, bool fp32, int in_graph, cudaGraphCondition
     PDL_CHECK(pdl_launch(k_cg_step, dim3(nu), dim3(256), 0, h->st, sc, (const double*)pq, nq, P,
                          (const int*)h->d_polidx, np, (const double4*)h->d_pv, (const double4*)h->d_qv, h->d_mu_ind,
                          h->d_r, h->d_z, rz, acc ? h->d_rho_acc : (double2*)nullptr, (const double2*)h->d_rhoA, h->nk,
-                         h->loop_stop));
+                         h->loop_stop, loop_flag(h) + 1));
     PDL_CHECK(pdl_launch(k_cg_next, dim3(std::min(cdiv(np, 256), most)), dim3(256), 0, h->st, sc, (const double*)rz, nu,
                          h->npol, (const int*)h->d_polidx, np, (const double4*)h->d_z, h->d_pv,
                          (const CellC*)h->d_cell, fp32 ? h->d_w32 : (float4*)nullptr, h->d_mu32, slotw(h),
-                         cg_w64(h, fp32), loop_flag(h), hc));
+                         cg_w64(h, fp32), (const int*)(loop_flag(h) + 1), loop_flag(h), hc));
     return MDFF_OK;
   }
   // with the accumulated structure factor the operator's rho'(p) stays in

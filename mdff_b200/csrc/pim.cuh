@@ -461,7 +461,9 @@ __global__ void k_cg_dir(const double* __restrict__ rz_p, const double* __restri
 // order): a sum of a few hundred numbers costs a block about 1 us, a launch of its
 // own 4 us.  Scalars are read and written by different kernels: sc[3] is r.z for
 // k_cg_step (whose block 0 moves it to sc[0]), sc[0] is r.z for k_cg_next (whose block
-// 0 leaves the new one in sc[3]).  An iteration of 8000 MgO ions had ten kernels, 66 us,
+// 0 leaves the new one in sc[3]).  So is the stop flag: k_cg_next sets it and cannot leave
+// by it (a block that starts late would see this launch's own), it leaves by
+// the copy that this iteration's k_cg_step took.  An iteration of 8000 MgO ions had ten kernels, 66 us,
 // of which 23 us were these and their reductions; now six.
 template <int NV>
 __device__ __forceinline__ void block_partials(const double* __restrict__ part, int nblk, double (&v)[NV],
@@ -527,7 +529,7 @@ __global__ void __launch_bounds__(256) k_cg_step(double* __restrict__ sc, const 
                                                  double4* __restrict__ x, double4* __restrict__ r,
                                                  double4* __restrict__ z, double* __restrict__ part,
                                                  double2* __restrict__ acc, const double2* __restrict__ rhoA, int nk,
-                                                 const int* __restrict__ stop) {
+                                                 const int* __restrict__ stop, int* __restrict__ stop_copy) {
   const bool stopped = loop_stopped(stop);
   __shared__ double red[2 * 32], bc[2];
   const int t0 = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
@@ -540,6 +542,7 @@ __global__ void __launch_bounds__(256) k_cg_step(double* __restrict__ sc, const 
   const double rz = sc[3];
   pdl_wait();
   pdl_trigger();
+  if (blockIdx.x == 0 && threadIdx.x == 0) *stop_copy = stopped ? 1 : 0;
   if (stopped) return;
   const double4 q0 = qv[i0];
   double pq[1], v[2] = {0.0, 0.0};
@@ -588,16 +591,16 @@ __global__ void __launch_bounds__(256) k_cg_next(double* __restrict__ sc, const 
                                                  const double4* __restrict__ z, double4* __restrict__ p,
                                                  const CellC* __restrict__ cell, float4* __restrict__ w32,
                                                  float4* __restrict__ mu32, SlotW sw, double4* __restrict__ w64,
-                                                 int* __restrict__ stop, cudaGraphConditionalHandle hc) {
-  const bool stopped = loop_stopped(stop);
+                                                 const int* __restrict__ stop_copy, int* __restrict__ stop,
+                                                 cudaGraphConditionalHandle hc) {
   __shared__ double red[2 * 32], bc[2];
   const int t0 = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
-  // (as k_cg_step: only z and the partials are its)
+  // (as k_cg_step: only z, the partials and the flag's copy are its)
   const int i0 = polidx[t0 < npol ? t0 : npol - 1];
   const double4 p0 = p[i0];
   pdl_wait();
   pdl_trigger();
-  if (stopped) return;
+  if (loop_stopped(stop_copy)) return;
   const double4 z0 = z[i0];
   double v[2];
   block_partials<2>(rz_part, nrz, v, red, bc);
