@@ -220,7 +220,7 @@ int ensure_workspace(mdff_batch* h, int ncl, int cluster) {
   size_t mfree = 0, mtot = 0;
   BCK(cudaMemGetInfo(&mfree, &mtot));
   size_t cap = h->npol_max * h->npol_max;
-  cap = std::min(cap, std::min(mtot / 8, mfree / 2) / (entry * nl));
+  cap = std::min(cap, pair_cache_room(mfree, mtot) / (entry * nl));
   for (int pass = 0; pass < 2; ++pass) {
     size_t o = 0;
     auto take = [&](size_t bytes) {

@@ -311,10 +311,24 @@ static void prof_collect(mdff_ctx* h) {
 
 static inline int cdiv(long a, long b) { return (int)((a + b - 1) / b); }
 
+// the FP64 pair cache is optional: it gives way to what is not
+static void drop_pair_cache(mdff_ctx* h) {
+  if (!h->d_c64r) return;
+  cudaFree(h->d_c64r);  // (waits for the device)
+  h->d_c64r = nullptr;
+  h->dd64_ok = false;
+  h->gen++;  // the graphs hold its address
+}
+
 template <typename T>
 static int dalloc(mdff_ctx* h, T** p, size_t n) {
   if (n == 0) n = 1;
   cudaError_t e = cudaMalloc((void**)p, n * sizeof(T));
+  if (e != cudaSuccess && h->d_c64r) {
+    cudaGetLastError();
+    drop_pair_cache(h);
+    e = cudaMalloc((void**)p, n * sizeof(T));
+  }
   if (e != cudaSuccess) {
     h->err = std::string("cudaMalloc: ") + cudaGetErrorString(e);
     return MDFF_ERR_NOMEM;
@@ -711,6 +725,7 @@ static int setup_list_cells(mdff_ctx* h) {
 static int alloc_list(mdff_ctx* h, int cap) {
   cap = ((cap + 31) / 32) * 32;
   h->gen++;
+  drop_pair_cache(h);
   cudaFree(h->L.nbr);
   h->L.nbr = nullptr;
   DALLOC(h->L.nbr, (size_t)h->natm * cap);
@@ -729,22 +744,28 @@ static int alloc_list(mdff_ctx* h, int cap) {
     if (!h->d_ddn) DALLOC(h->d_ddn, h->natm);
     if (!h->d_Edd) DALLOC(h->d_Edd, h->natm);
   }
-  if (h->d_c64r) cudaFree(h->d_c64r);
-  h->d_c64r = nullptr;
-  h->dd64_ok = false;
-  if (h->p.precision == MDFF_PREC_FP64 && h->lpolar && !h->polidx.empty()) {
-    // one allocation, 44 bytes an entry; optional: without room the field
-    // kernels recompute the pairs
-    const size_t ent = h->polidx.size() * (size_t)cap;
-    if (!h->d_c64n) DALLOC(h->d_c64n, h->polidx.size());
-    if (ent <= ((size_t)1 << 30) && cudaMalloc((void**)&h->d_c64r, ent * 44) != cudaSuccess) {
-      cudaGetLastError();
-      h->d_c64r = nullptr;
-    }
-    h->d_c64b = (double*)(h->d_c64r + ent);
-    h->d_c64j = (int*)(h->d_c64b + ent);
-  }
   h->stats.list_capacity = cap * h->natm;
+  return MDFF_OK;
+}
+
+// FP64 pair cache for the list's capacity, after everything that is not optional:
+// without room (pair_cache_fits) the field kernels recompute the pairs.  One
+// allocation, 44 bytes an entry.
+static int alloc_pair_cache(mdff_ctx* h) {
+  if (h->p.precision != MDFF_PREC_FP64 || !h->lpolar || h->polidx.empty()) return MDFF_OK;
+  if (!h->d_c64n) DALLOC(h->d_c64n, h->polidx.size());
+  drop_pair_cache(h);
+  const size_t ent = h->polidx.size() * (size_t)h->L.cap;
+  size_t mfree = 0, mtot = 0;
+  CK(cudaMemGetInfo(&mfree, &mtot));
+  if (!pair_cache_fits(ent * 44, mfree, mtot)) return MDFF_OK;
+  if (cudaMalloc((void**)&h->d_c64r, ent * 44) != cudaSuccess) {
+    cudaGetLastError();
+    h->d_c64r = nullptr;
+    return MDFF_OK;
+  }
+  h->d_c64b = (double*)(h->d_c64r + ent);
+  h->d_c64j = (int*)(h->d_c64b + ent);
   return MDFF_OK;
 }
 
@@ -2655,6 +2676,7 @@ static int engforce_retry(mdff_ctx* h, int itime) {
     int need = h->h_flags[2];
     int cap = (int)(need * 1.25) + 32;
     int e = alloc_list(h, cap);
+    if (!e) e = alloc_pair_cache(h);
     if (e) return e;
     k_seti<<<1, 32, 0, h->st>>>(&h->L.flags[1], 0);
     h->have_list = false;
@@ -2926,6 +2948,7 @@ static int create_impl(mdff_ctx* h, const mdff_params* pin, const double* cellA)
     }
   }
   DALLOC(h->d_ekin_part, cdiv(n, 256));
+  if ((s = alloc_pair_cache(h))) return s;
   CK(cudaStreamSynchronize(h->st));
   return MDFF_OK;
 }
@@ -3132,6 +3155,7 @@ int mdff_gpu_verlet_half_list(mdff_handle h, int which, const double* rx, const 
     CK(cudaStreamSynchronize(h->st));
     if (!h->h_flags[1]) break;
     if ((s = alloc_list(h, (int)(h->h_flags[2] * 1.25) + 32))) return s;
+    if ((s = alloc_pair_cache(h))) return s;
     k_seti<<<1, 32, 0, h->st>>>(&h->L.flags[1], 0);
   }
   if (h->h_flags[1]) return MDFF_ERR_LIST_OVERFLOW;

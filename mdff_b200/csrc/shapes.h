@@ -56,6 +56,13 @@ inline void rho_dm_split(int nion, int want, int* chunk, int* nchunk) {
 inline int rho_dm_most(int natm, int want) { return std::min(want, ceil_div(natm, 16)); }
 
 // ---------------------------------------------------------------------------
+// Optional caches of pair terms: an eighth of the device's memory at most and half
+// of what is free, so that later allocations, other handles and the caller's own
+// tensors find room.
+inline size_t pair_cache_room(size_t mfree, size_t mtotal) { return std::min(mtotal / 8, mfree / 2); }
+inline bool pair_cache_fits(size_t bytes, size_t mfree, size_t mtotal) { return bytes <= pair_cache_room(mfree, mtotal); }
+
+// ---------------------------------------------------------------------------
 // reciprocal sums of the batched engine (brho_t, bfld_t)
 
 constexpr int kBStage = 16384;  // least bytes of the shared staging buffer

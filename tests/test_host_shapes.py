@@ -42,6 +42,9 @@ int dm_overruns(int nsm, int kmax, int natm_lo, int natm_hi) {
   }
   return bad;
 }
+int cache_fits(double gb, double free_gb, double total_gb) {
+  return pair_cache_fits((size_t)(gb * 1e9), (size_t)(free_gb * 1e9), (size_t)(total_gb * 1e9));
+}
 // stagings of the batched engine's structure factor over the meshes that a batch
 // takes (kx, ky <= 64, kz <= 12), 0-2048 ions, one or two weights an ion, for one
 // buffer size: records that do not fit, none at all, or fewer than four although eight fit
@@ -100,3 +103,10 @@ def test_batch_staging_holds_records(shapes, stage):
     least = ctypes.c_int()
     assert shapes.batch_staging_faults(stage, ctypes.byref(least)) == 0
     assert least.value >= 3
+
+
+@pytest.mark.parametrize("gb,free,total,fits", [(0.09, 180, 190, 1), (20, 180, 190, 1), (47, 180, 190, 0),
+                                                (20, 30, 190, 0), (0.09, 0.15, 190, 0), (0.0, 0.0, 190, 1)])
+def test_pair_cache_leaves_room(shapes, gb, free, total, fits):
+    d = ctypes.c_double
+    assert shapes.cache_fits(d(gb), d(free), d(total)) == fits
