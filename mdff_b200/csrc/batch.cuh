@@ -461,7 +461,8 @@ __device__ __forceinline__ void bfld_get(const BatchArgs& a, const BConf& c, int
 // the box, half of which lie outside the half-box cutoff and nearly all
 // outside a 4-6 A short-range cutoff.  The test is FP32 on coordinates wrapped
 // to [-0.5, 0.5); the margin covers its rounding, and a pair whose image is
-// ambiguous at that precision is always kept.
+// ambiguous at that precision is always kept, as is one whose distance is not a
+// number (the pair loops carry it into the results).
 __device__ __forceinline__ unsigned short* bnbl(const BatchArgs& a, const BCtx& X, int which, int i) {
   return a.nbl + (((size_t)X.slot * 2 + which) * a.wn + i) * a.wn;
 }
@@ -506,8 +507,8 @@ __device__ __noinline__ void blists(const BatchArgs& a, const BCtx& X, const BSh
         const float z = A[6] * dx + A[7] * dy + A[8] * dz;
         const float r2 = x * x + y * y + z * z;
         const bool edge = fmaxf(fabsf(dx), fmaxf(fabsf(dy), fabsf(dz))) > 0.49999f;
-        kl = coul && (r2 <= l2 || edge);
-        ksr = sr && (r2 <= s2 || edge);
+        kl = coul && (!(r2 > l2) || edge);
+        ksr = sr && (!(r2 > s2) || edge);
       }
       const unsigned bl = __ballot_sync(FULL_MASK, kl), bs = __ballot_sync(FULL_MASK, ksr);
       const unsigned lt = (1u << lane) - 1u;
