@@ -817,23 +817,25 @@ __device__ __noinline__ void bshort(const BatchArgs& a, const BCtx& X, const BSh
 }
 
 // final real-space pass (k_es_force) on this CTA's ions; mu in S.v (FP64).  K,
-// THOLE as k_es_force; a lane sums its visits in R (about sixteen), as there.
+// THOLE as k_es_force.  The pair's vector and the cutoff decision are the exact FP64
+// ones and the lane sums FP64 in both engines: the mixed one evaluates the pair's terms in
+// FP32 and nothing else.
 template <typename R, int K, bool THOLE>
 __device__ __noinline__ void bforce_n(const BatchArgs& a, const BCtx& X, const BShared& S, double (&acc)[kESPart]) {
   const BConf& c = *X.c;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
   const int task_qq = (c.flags & BF_QQ) ? 1 : 0, task_qd = (c.flags & BF_QD) ? 1 : 0;
   const int task_dd = (c.flags & BF_DD) ? 1 : 0;
-  for (int k = 0; k < kESPart; ++k) acc[k] = 0.0;
+  double la[kESPart];
+#pragma unroll
+  for (int k = 0; k < kESPart; ++k) la[k] = 0.0;
   for (int i = X.i0 + warp; i < X.i1; i += nwarp) {
     const double4 si = S.s[i];
     const int ti = btyp(S.t[i]);
     const double4 mui = S.v[i];
     const R qi = (R)si.w, mi[3] = {(R)mui.x, (R)mui.y, (R)mui.z};
     const bool dip_i = mui.x != 0.0 || mui.y != 0.0 || mui.z != 0.0;
-    R e[3] = {0, 0, 0}, f[3] = {0, 0, 0}, la[kESPart];
-#pragma unroll
-    for (int k = 0; k < kESPart; ++k) la[k] = R(0);
+    double e[3] = {0, 0, 0}, f[3] = {0, 0, 0};
     const unsigned short* row = bnbl(a, X, 0, i);
     const int nn = bnbn(a, X, 0)[i];
     int jn = lane < nn ? bnbr(row, lane) : 0;
@@ -841,9 +843,10 @@ __device__ __noinline__ void bforce_n(const BatchArgs& a, const BCtx& X, const B
       const int j = jn;
       if (k + 32 < nn) jn = bnbr(row, k + 32);
       const double4 sj = S.s[j];
-      R r[3];
-      const R r2 = pair_vec<R>(c.A, si, sj, r[0], r[1], r[2]);
-      if (r2 > (R)c.rc2) continue;
+      double rd[3];
+      const double r2 = pair_vec<double>(c.A, si, sj, rd[0], rd[1], rd[2]);
+      if (r2 > c.rc2) continue;
+      const R r[3] = {(R)rd[0], (R)rd[1], (R)rd[2]};
       const int tj = btyp(S.t[j]);
       const double4 muj = S.v[j];
       const bool i_is_a = half_mask(i, j);
@@ -852,37 +855,36 @@ __device__ __noinline__ void bforce_n(const BatchArgs& a, const BCtx& X, const B
       const bool dip_j = muj.x != 0.0 || muj.y != 0.0 || muj.z != 0.0;
       R u, fi[3], Ei[3];
       // the single engine's pair (i's frame)
-      es_force_ipair<R, K, THOLE>(P, i_is_a, P.ldamp != 0, r2, (R)c.alpha, r, qi, (R)sj.w, mi, mj, dip_i, dip_j,
+      es_force_ipair<R, K, THOLE>(P, i_is_a, P.ldamp != 0, (R)r2, (R)c.alpha, r, qi, (R)sj.w, mi, mj, dip_i, dip_j,
                                   task_qq, task_qd, task_dd, u, fi, Ei);
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
-        f[d] += fi[d];
-        e[d] += Ei[d];
+        f[d] += (double)fi[d];
+        e[d] += (double)Ei[d];
       }
-      la[0] += u;
-      la[1] += r[0] * fi[0];
-      la[2] += r[1] * fi[1];
-      la[3] += r[2] * fi[2];
-      la[4] += r[0] * fi[1] + r[1] * fi[0];
-      la[5] += r[0] * fi[2] + r[2] * fi[0];
-      la[6] += r[1] * fi[2] + r[2] * fi[1];
+      la[0] += 0.5 * (double)u;
+      la[1] += (double)(r[0] * fi[0]);
+      la[2] += (double)(r[1] * fi[1]);
+      la[3] += (double)(r[2] * fi[2]);
+      la[4] += 0.5 * (double)(r[0] * fi[1] + r[1] * fi[0]);
+      la[5] += 0.5 * (double)(r[0] * fi[2] + r[2] * fi[0]);
+      la[6] += 0.5 * (double)(r[1] * fi[2] + r[2] * fi[1]);
     }
 #pragma unroll
-    for (int k = 0; k < kESPart; ++k) acc[k] += (k >= 1 && k < 4 ? 1.0 : 0.5) * (double)la[k];
-    double ed[3], fd[3];
-#pragma unroll
     for (int d = 0; d < 3; ++d) {
-      ed[d] = warp_sum((double)e[d]);
-      fd[d] = warp_sum((double)f[d]);
+      e[d] = warp_sum(e[d]);
+      f[d] = warp_sum(f[d]);
     }
     if (lane == 0) {
       int gi = X.off + i;
-      a.E[gi] = make_double4(ed[0], ed[1], ed[2], 0.0);
-      a.force[gi] += fd[0] * c.coul_unit;
-      a.force[a.ntot + gi] += fd[1] * c.coul_unit;
-      a.force[2 * (size_t)a.ntot + gi] += fd[2] * c.coul_unit;
+      a.E[gi] = make_double4(e[0], e[1], e[2], 0.0);
+      a.force[gi] += f[0] * c.coul_unit;
+      a.force[a.ntot + gi] += f[1] * c.coul_unit;
+      a.force[2 * (size_t)a.ntot + gi] += f[2] * c.coul_unit;
     }
   }
+#pragma unroll
+  for (int k = 0; k < kESPart; ++k) acc[k] = la[k];
 }
 template <typename R>
 __device__ __forceinline__ void bforce(const BatchArgs& a, const BCtx& X, const BShared& S, double (&acc)[kESPart]) {
