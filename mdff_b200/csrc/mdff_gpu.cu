@@ -930,11 +930,11 @@ static int launch_rho64(mdff_ctx* h, const RecMesh& M, int n, const int* imap, i
   const dim3 g((unsigned)(M.nrows * ntiles), (unsigned)h->n_rho_chunks);
   const double2* tab = h->d_tab64;
   if (has_q && has_mu)
-    (void)pdl_launch(k_rec_rho<double, true, true, kRhoNzt>, g, dim3(kRhoThreads), 0, h->st, tab, h->d_w, n, kRhoChunk, M, ntiles, h->d_rho_part);
+    (void)pdl_launch(k_rec_rho<double, true, true, kRhoNzt>, g, dim3(kRhoThreads), 0, h->st, tab, h->d_w, n, kRhoChunk, M, ntiles, h->d_rho_part, h->loop_stop);
   else if (has_q)
-    (void)pdl_launch(k_rec_rho<double, true, false, kRhoNzt>, g, dim3(kRhoThreads), 0, h->st, tab, h->d_w, n, kRhoChunk, M, ntiles, h->d_rho_part);
+    (void)pdl_launch(k_rec_rho<double, true, false, kRhoNzt>, g, dim3(kRhoThreads), 0, h->st, tab, h->d_w, n, kRhoChunk, M, ntiles, h->d_rho_part, h->loop_stop);
   else
-    (void)pdl_launch(k_rec_rho<double, false, true, kRhoNzt>, g, dim3(kRhoThreads), 0, h->st, tab, h->d_w, n, kRhoChunk, M, ntiles, h->d_rho_part);
+    (void)pdl_launch(k_rec_rho<double, false, true, kRhoNzt>, g, dim3(kRhoThreads), 0, h->st, tab, h->d_w, n, kRhoChunk, M, ntiles, h->d_rho_part, h->loop_stop);
   *nparts = h->n_rho_chunks;
   return MDFF_OK;
 }
@@ -1089,7 +1089,7 @@ static int rec_pass_t(mdff_ctx* h, const typename cplx<R>::T* tab, const double4
   // (the FP32 CG direction kernels and the SCF step write their weights themselves)
   if (!weights_ready) {
     PDL_CHECK(pdl_launch(k_rec_weights, dim3(cdiv(n, 256)), dim3(256), 0, h->st, h->d_q, mu, n, h->d_cell, has_q, has_mu, h->d_w,
-                         F32 ? h->d_w32 : nullptr, mu32, slotw(h)));
+                         F32 ? h->d_w32 : nullptr, mu32, slotw(h), h->loop_stop));
   }
   // algorithmic op counts per (k, ion) term (add = mul = 1, FMA = 2,
   // sin/cos/exp/sqrt = 1): structure factor k.r 5 + sin,cos 2 + q part 4 +
@@ -1114,7 +1114,7 @@ static int rec_pass_t(mdff_ctx* h, const typename cplx<R>::T* tab, const double4
     const bool pol = pol_dipoles && !has_q && has_mu && h->d_polidx;
     if (F32 && weights_ready)  // (the CG direction kernels write FP32 weights only)
       PDL_CHECK(pdl_launch(k_rec_weights, dim3(cdiv(n, 256)), dim3(256), 0, h->st, h->d_q, mu, n, h->d_cell, has_q,
-                           has_mu, h->d_w, (float4*)nullptr, (float4*)nullptr, SlotW()));
+                           has_mu, h->d_w, (float4*)nullptr, (float4*)nullptr, SlotW(), h->loop_stop));
     const int e = launch_rho64(h, M, n, pol ? h->d_polidx : nullptr, pol ? (int)h->polidx.size() : n, has_q, has_mu,
                                &nparts);
     if (e) return e;
@@ -1156,9 +1156,9 @@ static int rec_pass_t(mdff_ctx* h, const typename cplx<R>::T* tab, const double4
   } else if constexpr (std::is_same<R, float>::value) {
     dim3 gx((unsigned)cdiv(n, 2 * kFieldThreads), (unsigned)nch);
     if (muf)
-      (void)pdl_launch(k_rec_field_x2<true>, dim3(gx), dim3(kFieldThreads), smem, h->st, tab, h->d_w32, n, M, h->d_rchunk, h->d_rhoA, h->d_rho_part, npart, h->d_G, h->d_H);
+      (void)pdl_launch(k_rec_field_x2<true>, dim3(gx), dim3(kFieldThreads), smem, h->st, tab, h->d_w32, n, M, h->d_rchunk, h->d_rhoA, h->d_rho_part, npart, h->d_G, h->d_H, h->loop_stop);
     else
-      (void)pdl_launch(k_rec_field_x2<false>, dim3(gx), dim3(kFieldThreads), smem, h->st, tab, h->d_w32, n, M, h->d_rchunk, h->d_rhoA, h->d_rho_part, npart, h->d_G, h->d_H);
+      (void)pdl_launch(k_rec_field_x2<false>, dim3(gx), dim3(kFieldThreads), smem, h->st, tab, h->d_w32, n, M, h->d_rchunk, h->d_rhoA, h->d_rho_part, npart, h->d_G, h->d_H, h->loop_stop);
   } else if (muf)
     (void)pdl_launch(k_rec_field<R, true>, dim3(gf), dim3(kFieldThreads), smem, h->st, tab, h->d_w, n, imap, nion, M, h->d_rchunk, h->d_rhoA, h->d_rho_part, npart, h->d_G, h->d_H);
   else
@@ -1996,7 +1996,8 @@ static int add_solver_loop(mdff_ctx* h, cudaGraph_t g, const cudaGraphNode_t* de
   CK(cudaStreamBeginCaptureToGraph(h->st, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
                                    cudaStreamCaptureModeThreadLocal));
   // several iterations per pass of the loop (a pass has about 5 us of its own), when
-  // their last kernels know the stop flag
+  // their kernels know the stop flag (of an iteration after the last, the dipole sum of
+  // the surface term and the vector kernel of q run, 3 us each)
   const int unroll = !cg || cg_fused(h, fp32) ? kLoopUnroll : 1;
   h->loop_stop = unroll > 1 ? stopf : nullptr;
   int s = MDFF_OK;

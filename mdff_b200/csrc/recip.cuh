@@ -113,9 +113,11 @@ static __global__ void __launch_bounds__(128) k_rec_tables(const double4* __rest
 static __global__ void k_rec_weights(const double* __restrict__ q, const double4* __restrict__ mu,
                               int natm, const CellC* __restrict__ cell, int has_q, int has_mu,
                               double4* __restrict__ w, float4* __restrict__ w32,
-                              float4* __restrict__ mu32, SlotW sw = SlotW()) {
+                              float4* __restrict__ mu32, SlotW sw = SlotW(),
+                              const int* __restrict__ stop = nullptr) {
   pdl_wait();
   pdl_trigger();
+  if (loop_stopped(stop)) return;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= natm) return;
   const double* B = cell->B;
@@ -189,9 +191,10 @@ template <typename R, bool HAS_Q, bool HAS_MU, int NZT>
 static __global__ void __launch_bounds__(128) k_rec_rho(const typename cplx<R>::T* __restrict__ tab,
                                                  const double4* __restrict__ w, int natm,
                                                  int chunk, RecMesh M, int ntiles,
-                                                 double2* __restrict__ part) {
+                                                 double2* __restrict__ part, const int* __restrict__ stop) {
   pdl_wait();
   pdl_trigger();
+  if (loop_stopped(stop)) return;
   typedef typename cplx<R>::T C;
   __shared__ double red[2 * NZT][4];
   int row = blockIdx.x / ntiles, tile = blockIdx.x % ntiles;
@@ -678,9 +681,11 @@ static __global__ void __launch_bounds__(128) k_rec_field_x2(const float2* __res
                                                       const double2* __restrict__ rhoA,
                                                       const double2* __restrict__ part, int npart,
                                                       double4* __restrict__ Gpart,
-                                                      double4* __restrict__ Hpart) {
+                                                      double4* __restrict__ Hpart,
+                                                      const int* __restrict__ stop) {
   pdl_wait();
   pdl_trigger();
+  if (loop_stopped(stop)) return;
   extern __shared__ unsigned char shraw[];
   float2* sh = reinterpret_cast<float2*>(shraw);
   int r0 = rchunk[blockIdx.y], r1 = rchunk[blockIdx.y + 1];

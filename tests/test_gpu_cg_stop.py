@@ -3,7 +3,7 @@
 The iterations after the one that ended the solve leave the dipoles, the counters and
 the scalars alone: with a cap of 1..9 iterations the graph's loop gives the dipoles
 of the launch-by-launch loop (per-kernel profiling), which runs no iteration too
-many.  The same iterations of the same FP64 operator in other summation orders: 1e-9; mixed,
+many.  kz 34 and rows of 600 ny take the recurrence kernels.  The same iterations of the same FP64 operator in other summation orders: 1e-9; mixed,
 FP32 sums in other orders: 1e-5 of the dipoles."""
 import pytest
 
@@ -17,10 +17,11 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("precision", [_abi.PREC_FP64, _abi.PREC_MIXED])
-@pytest.mark.parametrize("cap", [1, 2, 3, 4, 5, 8, 9])
-def test_iteration_caps(cap, precision):
+@pytest.mark.parametrize("cap,mesh", [(c, (7, 7, 7)) for c in (1, 2, 3, 4, 5, 8, 9)]
+                         + [(c, m) for c in (3, 5) for m in ((2, 2, 34), (0, 600, 1))])
+def test_iteration_caps(cap, mesh, precision):
     s = systems.random_ionic((20, 30, 20), L=13.0, seed=18, q=(-1.5, 2.0, -1.5), pol=(1.1, 0.0, 1.1),
-                             calc=_abi.CALC_OTHER)
+                             kES=mesh, calc=_abi.CALC_OTHER)
     p = params_copy(s.params)
     p.solver, p.precision, p.cg_max_iter = _abi.SOLVER_CG, precision, cap
     p.fail_on_nonconvergence = 0
