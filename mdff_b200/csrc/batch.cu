@@ -198,13 +198,8 @@ BatchArgs make_args(mdff_batch* h, const double* d_pos, double* d_force) {
   return a;
 }
 
-// Workspaces for `ncl` resident clusters of `cluster` CTAs: grown (never
-// shrunk) when a launch shape has more of them; the graph, which holds their
-// addresses, is rebuilt then.  The pair cache takes at most an eighth of the
-// device memory; boxes whose pairs do not fit recompute them.
-int ensure_workspace(mdff_batch* h, int ncl, int cluster) {
-  const int ctas = ncl * cluster;
-  if (ctas <= h->ws_ctas && ncl <= h->ws_clusters) return MDFF_OK;
+// gives the workspaces back; the graph, which holds their addresses, goes too
+int drop_workspace(mdff_batch* h) {
   BCK(cudaStreamSynchronize(h->st));
   if (h->exec) {
     cudaGraphExecDestroy(h->exec);
@@ -212,8 +207,20 @@ int ensure_workspace(mdff_batch* h, int ncl, int cluster) {
   }
   if (h->d_ws) cudaFree(h->d_ws);
   h->d_ws = nullptr;
-  const size_t nc = std::max(ctas, h->ws_ctas), nl = std::max(ncl, h->ws_clusters), wn = h->nmax;
   h->ws_ctas = h->ws_clusters = 0;
+  h->ccap = 0;
+  return MDFF_OK;
+}
+
+// Workspaces for `ncl` resident clusters of `cluster` CTAs: those of the default shape
+// are part of creation, later ones grow when a launch shape (or the adjoint's) has
+// more clusters; a change of the shape in use gives them back first.  The pair
+// cache is optional (pair_cache_room); boxes whose pairs do not fit recompute them.
+int ensure_workspace(mdff_batch* h, int ncl, int cluster) {
+  const int ctas = ncl * cluster;
+  if (ctas <= h->ws_ctas && ncl <= h->ws_clusters) return MDFF_OK;
+  const size_t nc = std::max(ctas, h->ws_ctas), nl = std::max(ncl, h->ws_clusters), wn = h->nmax;
+  if (int s = drop_workspace(h)) return s;
   // one allocation, carved up; nothing of it is read before it is written
   const size_t entry = sizeof(double4) + sizeof(double) + sizeof(unsigned short) +
                        (h->mixed ? sizeof(float4) + sizeof(float) : 0);
@@ -280,6 +287,17 @@ size_t smem_with_stage(mdff_batch* h, size_t base, int threads, int* extra) {
   return *extra ? o + *extra : base;
 }
 
+// workspaces for *ncl clusters, for fewer where the partner lists (4 n^2 bytes a
+// cluster) of that many find no room
+int ensure_clusters(mdff_batch* h, int cluster, int* ncl) {
+  int s;
+  while ((s = ensure_workspace(h, *ncl, cluster)) == MDFF_ERR_NOMEM && *ncl > 1) {
+    *ncl = (*ncl + 1) / 2;
+    h->err.clear();
+  }
+  return s;
+}
+
 int prepare_shape(mdff_batch* h, Shape sh, int* nclusters) {
   size_t smem = smem_with_stage(h, batch_smem_bytes(h->nmax), sh.threads, &h->stage_extra);
   void (*fn)(BatchArgs, int) = h->mixed ? k_batch<true> : k_batch<false>;
@@ -302,7 +320,7 @@ int prepare_shape(mdff_batch* h, Shape sh, int* nclusters) {
     return MDFF_ERR_CUDA;
   }
   *nclusters = std::min(ncl, h->nconf);
-  return ensure_workspace(h, *nclusters, sh.cluster);
+  return ensure_clusters(h, sh.cluster, nclusters);
 }
 
 int launch_batch(mdff_batch* h, const BatchArgs& a, Shape sh, int ncl, cudaStream_t st) {
@@ -708,6 +726,13 @@ int create_impl(mdff_batch* h, const mdff_params* psets, int npsets, const mdff_
     h->err = "configurations too large for the shared-memory layout";
     return MDFF_ERR_BAD_ARGS;
   }
+  {
+    // the memory of the default shape (another one may yet be set: only its lack is an error here)
+    int ncl = 0;
+    if (prepare_shape(h, h->shape, &ncl) == MDFF_ERR_NOMEM) return MDFF_ERR_NOMEM;
+    h->err.clear();
+    cudaGetLastError();
+  }
   BCK(cudaStreamSynchronize(h->st));
   return MDFF_OK;
 }
@@ -924,7 +949,9 @@ int mdff_gpu_batch_tune(mdff_batch_handle h, int* cluster, int* threads, double*
     }
   }
   h->shape = bs;
-  int s = build_graph(h, pos, force);
+  // (sized for every shape tried: a pair cache shared among more clusters)
+  int s = drop_workspace(h);
+  if (!s) s = build_graph(h, pos, force);
   if (s) return s;
   if (cluster) *cluster = bs.cluster;
   if (threads) *threads = bs.threads;
@@ -940,12 +967,10 @@ int mdff_gpu_batch_set_shape(mdff_batch_handle h, int cluster, int threads) {
     h->err = "shape must be cluster 1/2/4/8 x threads 256/512";
     return MDFF_ERR_BAD_ARGS;
   }
+  if (cluster == h->shape.cluster && threads == h->shape.threads) return MDFF_OK;
+  BCK(cudaSetDevice(h->device));
   h->shape = Shape{cluster, threads};
-  if (h->exec) {
-    cudaGraphExecDestroy(h->exec);
-    h->exec = nullptr;
-  }
-  return MDFF_OK;
+  return drop_workspace(h);
 }
 
 int mdff_gpu_batch_info(mdff_batch_handle h, int* ntot, int* nconf, int* cluster, int* threads,
@@ -1110,7 +1135,7 @@ int mdff_gpu_batch_adjoint(mdff_batch_handle h, const double* gE, const double* 
   }
   ncl = std::min(ncl, h->nconf);
   {
-    int s = ensure_workspace(h, ncl, sh.cluster);
+    int s = ensure_clusters(h, sh.cluster, &ncl);
     if (s) return s;
   }
   cfg.gridDim = dim3(sh.cluster * ncl);
