@@ -278,12 +278,11 @@ int ensure_workspace(mdff_batch* h, int ncl, int cluster) {
 // Shared memory of one CTA: `base` bytes of layout plus a larger staging buffer
 // where it costs no resident CTA (512 threads of 128 registers fill an SM, 256
 // half of it).
-size_t smem_with_stage(mdff_batch* h, size_t base, int threads, int* extra) {
+size_t smem_with_stage(size_t base, int threads, int* extra) {
   const size_t room = threads >= 512 ? 227 * 1024 : 113 * 1024;
   const size_t o = (base + 15) & ~(size_t)15;
   *extra = 0;
   if (o + 20 * 1024 <= room) *extra = (int)(std::min<size_t>(room - o, 40 * 1024) & ~(size_t)127);
-  (void)h;
   return *extra ? o + *extra : base;
 }
 
@@ -299,7 +298,7 @@ int ensure_clusters(mdff_batch* h, int cluster, int* ncl) {
 }
 
 int prepare_shape(mdff_batch* h, Shape sh, int* nclusters) {
-  size_t smem = smem_with_stage(h, batch_smem_bytes(h->nmax), sh.threads, &h->stage_extra);
+  size_t smem = smem_with_stage(batch_smem_bytes(h->nmax), sh.threads, &h->stage_extra);
   void (*fn)(BatchArgs, int) = h->mixed ? k_batch<true> : k_batch<false>;
   BCK(allow_smem((const void*)fn, smem));
   cudaLaunchConfig_t cfg = {};
@@ -335,7 +334,7 @@ int launch_batch(mdff_batch* h, const BatchArgs& a, Shape sh, int ncl, cudaStrea
   cfg.numAttrs = 1;
   cfg.blockDim = dim3(sh.threads);
   int extra = 0;
-  cfg.dynamicSmemBytes = smem_with_stage(h, batch_smem_bytes(h->nmax), sh.threads, &extra);
+  cfg.dynamicSmemBytes = smem_with_stage(batch_smem_bytes(h->nmax), sh.threads, &extra);
   cfg.stream = st;
   cfg.gridDim = dim3(sh.cluster * ncl);
   BCK(cudaLaunchKernelEx(&cfg, fn, a, h->nmax));
@@ -346,7 +345,7 @@ int launch_batch(mdff_batch* h, const BatchArgs& a, Shape sh, int ncl, cudaStrea
 int enqueue(mdff_batch* h, const double* d_pos, double* d_force, Shape sh, int ncl, cudaStream_t st) {
   BCK(cudaMemsetAsync(h->d_queue, 0, sizeof(int), st));
   BCK(cudaMemsetAsync(h->d_out, 0, sizeof(double) * kBSlots * h->nconf, st));
-  smem_with_stage(h, batch_smem_bytes(h->nmax), sh.threads, &h->stage_extra);
+  smem_with_stage(batch_smem_bytes(h->nmax), sh.threads, &h->stage_extra);
   return launch_batch(h, make_args(h, d_pos, d_force), sh, ncl, st);
 }
 
@@ -1110,7 +1109,7 @@ int mdff_gpu_batch_adjoint(mdff_batch_handle h, const double* gE, const double* 
   // the schedule of the adjoint's own box costs
   const Shape sh{h->adj_cluster, h->shape.threads};
   int extra = 0;
-  const size_t smem = smem_with_stage(h, batch_smem_extra_offset(h->nmax) + sizeof(double4) * h->nmax, sh.threads, &extra);
+  const size_t smem = smem_with_stage(batch_smem_extra_offset(h->nmax) + sizeof(double4) * h->nmax, sh.threads, &extra);
   if (smem > 227 * 1024) {
     h->err = "configurations too large for the adjoint's shared-memory layout";
     return MDFF_ERR_BAD_ARGS;

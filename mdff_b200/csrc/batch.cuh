@@ -49,7 +49,6 @@ namespace cgx = cooperative_groups;
 
 constexpr int kBMaxT = 4;          // types of a batched configuration
 constexpr int kBPart = 16;         // values per CTA partial slot
-constexpr int kBKChunk = 1024;     // double2 of the staging buffer (kBStage bytes)
 constexpr int kBMaxC = 8;          // largest cluster
 constexpr int kBSlots = 48;        // per-configuration scalar slots
 
@@ -141,7 +140,6 @@ struct BShared {
   double4* v;      // [nmax] vector operand (FP64)
   float4* v32;     // [nmax] vector operand (FP32)
   int* t;          // [nmax]
-  double2* rho;    // [kBKChunk]
   NBPair* nb;      // [kBMaxT^2]
   ESPair* es;      // [kBMaxT^2]
   double* red;     // [kBPart * 32]
@@ -154,7 +152,7 @@ struct BShared {
 __host__ __device__ inline size_t batch_smem_bytes(int nmax) {
   size_t b = 0;
   b += sizeof(double4) * nmax * 2;
-  b += sizeof(double2) * kBKChunk;
+  b += kBStage;
   b += sizeof(float4) * nmax;
   b += sizeof(NBPair) * kBMaxT * kBMaxT;
   b += sizeof(ESPair) * kBMaxT * kBMaxT;
@@ -174,7 +172,7 @@ __device__ inline BShared batch_smem(unsigned char* base, int nmax) {
   size_t o = 0;
   S.s = reinterpret_cast<double4*>(base + o); o += sizeof(double4) * nmax;
   S.v = reinterpret_cast<double4*>(base + o); o += sizeof(double4) * nmax;
-  S.rho = reinterpret_cast<double2*>(base + o); o += sizeof(double2) * kBKChunk;
+  S.stage = base + o; o += kBStage;
   S.v32 = reinterpret_cast<float4*>(base + o); o += sizeof(float4) * nmax;
   S.nb = reinterpret_cast<NBPair*>(base + o); o += sizeof(NBPair) * kBMaxT * kBMaxT;
   S.es = reinterpret_cast<ESPair*>(base + o); o += sizeof(ESPair) * kBMaxT * kBMaxT;
@@ -182,8 +180,7 @@ __device__ inline BShared batch_smem(unsigned char* base, int nmax) {
   S.res = reinterpret_cast<double*>(base + o); o += sizeof(double) * kBPart;
   S.t = reinterpret_cast<int*>(base + o); o += sizeof(int) * nmax;
   S.cfg = reinterpret_cast<int*>(base + o);
-  S.stage = reinterpret_cast<unsigned char*>(S.rho);
-  S.stage_bytes = kBKChunk * (int)sizeof(double2);
+  S.stage_bytes = kBStage;
   return S;
 }
 

@@ -930,11 +930,11 @@ static int launch_rho64(mdff_ctx* h, const RecMesh& M, int n, const int* imap, i
   const dim3 g((unsigned)(M.nrows * ntiles), (unsigned)h->n_rho_chunks);
   const double2* tab = h->d_tab64;
   if (has_q && has_mu)
-    (void)pdl_launch(k_rec_rho<double, true, true, kRhoNzt>, g, dim3(kRhoThreads), 0, h->st, tab, h->d_w, n, kRhoChunk, M, ntiles, h->d_rho_part, h->loop_stop);
+    (void)pdl_launch(k_rec_rho<true, true, kRhoNzt>, g, dim3(kRhoThreads), 0, h->st, tab, h->d_w, n, kRhoChunk, M, ntiles, h->d_rho_part, h->loop_stop);
   else if (has_q)
-    (void)pdl_launch(k_rec_rho<double, true, false, kRhoNzt>, g, dim3(kRhoThreads), 0, h->st, tab, h->d_w, n, kRhoChunk, M, ntiles, h->d_rho_part, h->loop_stop);
+    (void)pdl_launch(k_rec_rho<true, false, kRhoNzt>, g, dim3(kRhoThreads), 0, h->st, tab, h->d_w, n, kRhoChunk, M, ntiles, h->d_rho_part, h->loop_stop);
   else
-    (void)pdl_launch(k_rec_rho<double, false, true, kRhoNzt>, g, dim3(kRhoThreads), 0, h->st, tab, h->d_w, n, kRhoChunk, M, ntiles, h->d_rho_part, h->loop_stop);
+    (void)pdl_launch(k_rec_rho<false, true, kRhoNzt>, g, dim3(kRhoThreads), 0, h->st, tab, h->d_w, n, kRhoChunk, M, ntiles, h->d_rho_part, h->loop_stop);
   *nparts = h->n_rho_chunks;
   return MDFF_OK;
 }
@@ -1156,20 +1156,21 @@ static int rec_pass_t(mdff_ctx* h, const typename cplx<R>::T* tab, const double4
   } else if constexpr (std::is_same<R, float>::value) {
     dim3 gx((unsigned)cdiv(n, 2 * kFieldThreads), (unsigned)nch);
     if (muf)
-      (void)pdl_launch(k_rec_field_x2<true>, dim3(gx), dim3(kFieldThreads), smem, h->st, tab, h->d_w32, n, M, h->d_rchunk, h->d_rhoA, h->d_rho_part, npart, h->d_G, h->d_H, h->loop_stop);
+      (void)pdl_launch(k_rec_field_x2<true>, dim3(gx), dim3(kFieldThreads), smem, h->st, tab, h->d_w32, n, M, h->d_rchunk, h->d_rhoA, h->d_G, h->d_H, h->loop_stop);
     else
-      (void)pdl_launch(k_rec_field_x2<false>, dim3(gx), dim3(kFieldThreads), smem, h->st, tab, h->d_w32, n, M, h->d_rchunk, h->d_rhoA, h->d_rho_part, npart, h->d_G, h->d_H, h->loop_stop);
+      (void)pdl_launch(k_rec_field_x2<false>, dim3(gx), dim3(kFieldThreads), smem, h->st, tab, h->d_w32, n, M, h->d_rchunk, h->d_rhoA, h->d_G, h->d_H, h->loop_stop);
   } else if (muf)
-    (void)pdl_launch(k_rec_field<R, true>, dim3(gf), dim3(kFieldThreads), smem, h->st, tab, h->d_w, n, imap, nion, M, h->d_rchunk, h->d_rhoA, h->d_rho_part, npart, h->d_G, h->d_H);
+    (void)pdl_launch(k_rec_field<true>, dim3(gf), dim3(kFieldThreads), smem, h->st, tab, h->d_w, n, imap, nion, M, h->d_rchunk, h->d_rhoA, h->d_G, h->d_H);
   else
-    PDL_CHECK(pdl_launch(k_rec_field<R, false>, dim3(gf), dim3(kFieldThreads), smem, h->st, tab, h->d_w, n, imap, nion, M, h->d_rchunk, h->d_rhoA, h->d_rho_part, npart, h->d_G, h->d_H));
+    PDL_CHECK(pdl_launch(k_rec_field<false>, dim3(gf), dim3(kFieldThreads), smem, h->st, tab, h->d_w, n, imap, nion, M, h->d_rchunk, h->d_rhoA, h->d_G, h->d_H));
   prof_end(h, pr);
   double fpi_V = 2.0 * tpi_V;
   // the real-space half of this pass (side stream) adds into the same E / forces
   int e = rs_join(h);
   if (e) return e;
   if (defer_nch) {
-    // the caller's kernel sums the field partials (k_dd_cached_rec)
+    // the caller's kernel sums the field partials (k_cg_q, k_scf_tail; k_dd_cached_rec
+    // where the operator is formed as a field)
     *defer_nch = nch;
     return MDFF_OK;
   }
@@ -2529,14 +2530,14 @@ static int run_engforce(mdff_ctx* h, int itime) {
 }
 
 // ---------------------------------------------------------------------------
-// Whole-step graph.  In the steady state of an MD run with the CG solver (the
-// list built, the ASPC order ramp past, no per-kernel profiling) one
-// engforce is the same ~130 launches every step; they are replayed as one
-// CUDA graph: ef_front + the CG prologue and first FP64 residual (captured),
-// k_cg_plan, the CG inner WHILE node, the CG epilogue + ef_back (captured).
-// The host then reads the scalars once.  A solve that needs another outer
-// iteration (rare: the trusted-recurrence test failed) continues with the CG
-// graph and repeats ef_back; a list overflow redoes the call without the
+// Whole-step graph.  Once the list is built and the ASPC order ramp past (no
+// per-kernel profiling), one engforce is the same launches every call, with the CG solver,
+// with the SCF iterations that run on the device (scf_device_loop) or without
+// dipoles; they are replayed as one CUDA graph: ef_front + the solver's start and
+// first residual (captured), the head kernel and WHILE node of its loop, its epilogue +
+// ef_back (captured).  The host then reads the scalars once.  A CG solve that needs
+// another outer iteration (the trusted-recurrence test failed) continues with
+// the loop's own graph and repeats ef_back; a list overflow redoes the call without the
 // graph after growing the list.
 
 static bool step_graph_usable(const mdff_ctx* h, int itime) {

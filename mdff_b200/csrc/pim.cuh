@@ -626,10 +626,6 @@ __global__ void __launch_bounds__(256) k_cg_next(double* __restrict__ sc, const 
   for (int sl = t0 + nt; sl < npol; sl += nt) next(polidx[sl], p[polidx[sl]], z[polidx[sl]]);
 }
 
-__global__ void k_copy1(double* __restrict__ dst, const double* __restrict__ src) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) *dst = *src;
-}
-
 // moment_from_WFc (moment_from_pola.f90:632-807), warp per ion over its
 // (full, ascending) neighbour row: every ion of a type with lwfc >= 0 sums
 // r_j - r_i (minimum image, the reference's two-rounding arithmetic) over

@@ -185,17 +185,15 @@ __device__ __forceinline__ typename cplx<R>::T phase_z(const typename cplx<R>::T
 // rho partials.  grid.x = nrows * ntiles, grid.y = ion chunks; block 128.
 // part[chunk][k] (double2).  Each thread keeps NZT accumulators (one per nz
 // of the tile) over its ions; the phase advances by one complex multiply per
-// nz and is re-anchored on the exact table every 4 nz (FP32 drift bound).
-// Warp partial sums in R, block and chunk sums in FP64, fixed order.
-template <typename R, bool HAS_Q, bool HAS_MU, int NZT>
-static __global__ void __launch_bounds__(128) k_rec_rho(const typename cplx<R>::T* __restrict__ tab,
+// nz.  FP64, sums in fixed order.
+template <bool HAS_Q, bool HAS_MU, int NZT>
+static __global__ void __launch_bounds__(128) k_rec_rho(const double2* __restrict__ tab,
                                                  const double4* __restrict__ w, int natm,
                                                  int chunk, RecMesh M, int ntiles,
                                                  double2* __restrict__ part, const int* __restrict__ stop) {
   pdl_wait();
   pdl_trigger();
   if (loop_stopped(stop)) return;
-  typedef typename cplx<R>::T C;
   __shared__ double red[2 * NZT][4];
   int row = blockIdx.x / ntiles, tile = blockIdx.x % ntiles;
   int4 ri = M.rows[row];
@@ -207,28 +205,21 @@ static __global__ void __launch_bounds__(128) k_rec_rho(const typename cplx<R>::
   if (nzn > NZT) nzn = NZT;
   int a0 = blockIdx.y * chunk, a1 = a0 + chunk;
   if (a1 > natm) a1 = natm;
-  R accR[NZT], accI[NZT];
+  double accR[NZT], accI[NZT];
 #pragma unroll
-  for (int t = 0; t < NZT; ++t) accR[t] = accI[t] = R(0);
+  for (int t = 0; t < NZT; ++t) accR[t] = accI[t] = 0.0;
   const int kx = M.kmax[0], ky = M.kmax[1];
   const size_t zoff = (size_t)(kx + 1 + ky + 1);
   for (int i = a0 + threadIdx.x; i < a1; i += blockDim.x) {
-    C XY = phase_xyz<R>(tab, natm, i, nx, ny, 0, kx, ky);
-    C Z1 = tab[(zoff + 1) * natm + i];
+    double2 XY = phase_xyz<double>(tab, natm, i, nx, ny, 0, kx, ky);
+    double2 Z1 = tab[(zoff + 1) * natm + i];
     double4 wi = w[i];
-    R q = (R)wi.x;
-    R m3 = (R)wi.w;
-    R km = (R)(nx * wi.y + ny * wi.z + nz0 * wi.w);
-    C P;
+    double q = wi.x;
+    double m3 = wi.w;
+    double km = nx * wi.y + ny * wi.z + nz0 * wi.w;
+    double2 P = phase_z<double>(tab, natm, i, XY, nz0, kx, ky);
 #pragma unroll
     for (int t = 0; t < NZT; ++t) {
-      if ((t & 3) == 0 && (t == 0 || sizeof(R) == 4)) {
-        // anchor on the table; slots beyond the row's end only compute
-        // values that are never stored, so clamp their index into the table
-        int nz = nz0 + t;
-        nz = nz > kz ? kz : nz;
-        P = phase_z<R>(tab, natm, i, XY, nz, kx, ky);
-      }
       if (HAS_Q) {
         accR[t] += q * P.x;
         accI[t] += q * P.y;
@@ -238,18 +229,17 @@ static __global__ void __launch_bounds__(128) k_rec_rho(const typename cplx<R>::
         accI[t] += km * P.x;
         km += m3;
       }
-      if (t + 1 < NZT && ((t + 1) & 3) != 0) P = cmul(P, Z1);
-      else if (t + 1 < NZT && sizeof(R) == 8) P = cmul(P, Z1);
+      if (t + 1 < NZT) P = cmul(P, Z1);
     }
   }
   int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
 #pragma unroll
   for (int t = 0; t < NZT; ++t) {
-    R vr = warp_sum(accR[t]);
-    R vi = warp_sum(accI[t]);
+    double vr = warp_sum(accR[t]);
+    double vi = warp_sum(accI[t]);
     if (lane == 0) {
-      red[2 * t][wp] = (double)vr;
-      red[2 * t + 1][wp] = (double)vi;
+      red[2 * t][wp] = vr;
+      red[2 * t + 1][wp] = vi;
     }
   }
   __syncthreads();
@@ -349,30 +339,22 @@ static __global__ void __launch_bounds__(256) k_rec_acc_finish(const double2* __
 // field / force partials.  grid.x = ion blocks (128), grid.y = k chunks
 // (row ranges rc[c]..rc[c+1]); dynamic smem = rho' of the chunk.
 // G accumulates sum_k n recarg, H accumulates sum_k n (k.mu) recarg2.
-template <typename R, bool HAS_MU_FORCE>
-static __global__ void __launch_bounds__(128) k_rec_field(const typename cplx<R>::T* __restrict__ tab,
+template <bool HAS_MU_FORCE>
+static __global__ void __launch_bounds__(128) k_rec_field(const double2* __restrict__ tab,
                                                    const double4* __restrict__ w, int natm,
                                                    const int* __restrict__ imap, int nion,
                                                    RecMesh M, const int* __restrict__ rchunk,
                                                    const double2* __restrict__ rhoA,
-                                                   const double2* __restrict__ part, int npart,
                                                    double4* __restrict__ Gpart,
                                                    double4* __restrict__ Hpart) {
   pdl_wait();
   pdl_trigger();
-  typedef typename cplx<R>::T C;
   extern __shared__ unsigned char shraw[];
-  C* sh = reinterpret_cast<C*>(shraw);
+  double2* sh = reinterpret_cast<double2*>(shraw);
   int r0 = rchunk[blockIdx.y], r1 = rchunk[blockIdx.y + 1];
   int k0 = M.rows[r0].w;
   int k1 = (r1 < M.nrows) ? M.rows[r1].w : M.nk;
-  for (int k = k0 + threadIdx.x; k < k1; k += blockDim.x) {
-    double2 v = npart ? rho_prime(part, npart, M.Ak, M.nk, k) : rhoA[k];
-    C c;
-    c.x = (R)v.x;
-    c.y = (R)v.y;
-    sh[k - k0] = c;
-  }
+  for (int k = k0 + threadIdx.x; k < k1; k += blockDim.x) sh[k - k0] = rhoA[k];
   __syncthreads();
   // thread slot -> ion (imap: the ions whose field is wanted, else all)
   const int sl = blockIdx.x * blockDim.x + threadIdx.x;
@@ -380,55 +362,53 @@ static __global__ void __launch_bounds__(128) k_rec_field(const typename cplx<R>
   const int i = imap ? imap[sl] : sl;
   const int kx = M.kmax[0], ky = M.kmax[1], kz = M.kmax[2];
   double4 wi = w[i];
-  R m3 = (R)wi.w;
-  C Z1 = tab[(size_t)(kx + 1 + ky + 1 + 1) * natm + i];
+  double m3 = wi.w;
+  double2 Z1 = tab[(size_t)(kx + 1 + ky + 1 + 1) * natm + i];
   double G[3] = {0, 0, 0}, H[3] = {0, 0, 0};
   for (int r = r0; r < r1; ++r) {
     int4 ri = M.rows[r];
     int nx = ri.x, ny = ri.y, nz_lo = ri.z;
-    C XY = phase_xyz<R>(tab, natm, i, nx, ny, 0, kx, ky);
+    double2 XY = phase_xyz<double>(tab, natm, i, nx, ny, 0, kx, ky);
     // sums over the row, nz measured from the row start: Sz = sum t recarg
-    R S0 = R(0), Sz = R(0), T0 = R(0), Tz = R(0);
-    R km = (R)(nx * wi.y + ny * wi.z + nz_lo * wi.w);
-    const C* rr = sh + (ri.w - k0);
+    double S0 = 0.0, Sz = 0.0, T0 = 0.0, Tz = 0.0;
+    double km = nx * wi.y + ny * wi.z + nz_lo * wi.w;
+    const double2* rr = sh + (ri.w - k0);
     int nn = kz - nz_lo + 1;
-    C P = phase_z<R>(tab, natm, i, XY, nz_lo, kx, ky);
+    double2 P = phase_z<double>(tab, natm, i, XY, nz_lo, kx, ky);
     int t0 = 0;
-    R tf = R(0);  // t0 as R, advanced by 4 (no int->float conversion per term)
-    for (; t0 + 4 <= nn; t0 += 4, tf += R(4)) {
-      if (sizeof(R) == 4 && t0 > 0) P = phase_z<R>(tab, natm, i, XY, nz_lo + t0, kx, ky);
-      R a[4], b[4];
+    double tf = 0.0;  // t0, advanced by 4 (no conversion per term)
+    for (; t0 + 4 <= nn; t0 += 4, tf += 4.0) {
+      double a[4], b[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        C rho = rr[t0 + u];
+        double2 rho = rr[t0 + u];
         a[u] = rho.y * P.x - rho.x * P.y;
-        if (HAS_MU_FORCE) b[u] = (km + R(u) * m3) * (rho.x * P.x + rho.y * P.y);
-        if (u < 3 || sizeof(R) == 8) P = cmul(P, Z1);
+        if (HAS_MU_FORCE) b[u] = (km + (double)u * m3) * (rho.x * P.x + rho.y * P.y);
+        P = cmul(P, Z1);
       }
       // sum_u a_u and sum_u u a_u of the group (u = 0..3)
-      R sa = (a[0] + a[1]) + (a[2] + a[3]);
-      R sb = a[1] + R(2) * a[2] + R(3) * a[3];
+      double sa = (a[0] + a[1]) + (a[2] + a[3]);
+      double sb = a[1] + 2.0 * a[2] + 3.0 * a[3];
       S0 += sa;
       Sz += tf * sa + sb;
       if (HAS_MU_FORCE) {
-        R ta = (b[0] + b[1]) + (b[2] + b[3]);
-        R tb = b[1] + R(2) * b[2] + R(3) * b[3];
+        double ta = (b[0] + b[1]) + (b[2] + b[3]);
+        double tb = b[1] + 2.0 * b[2] + 3.0 * b[3];
         T0 += ta;
         Tz += tf * ta + tb;
-        km += R(4) * m3;
+        km += 4.0 * m3;
       }
     }
     if (t0 < nn) {
-      if (sizeof(R) == 4 && t0 > 0) P = phase_z<R>(tab, natm, i, XY, nz_lo + t0, kx, ky);
       for (int t = t0; t < nn; ++t) {
-        C rho = rr[t];
-        R recarg = rho.y * P.x - rho.x * P.y;
-        R tt_ = (R)t;
+        double2 rho = rr[t];
+        double recarg = rho.y * P.x - rho.x * P.y;
+        double tt_ = (double)t;
         S0 += recarg;
         Sz += tt_ * recarg;
         if (HAS_MU_FORCE) {
-          R recarg2 = rho.x * P.x + rho.y * P.y;
-          R tt = km * recarg2;
+          double recarg2 = rho.x * P.x + rho.y * P.y;
+          double tt = km * recarg2;
           T0 += tt;
           Tz += tt_ * tt;
           km += m3;
@@ -436,13 +416,13 @@ static __global__ void __launch_bounds__(128) k_rec_field(const typename cplx<R>
         P = cmul(P, Z1);
       }
     }
-    G[0] += (double)nx * (double)S0;
-    G[1] += (double)ny * (double)S0;
-    G[2] += (double)nz_lo * (double)S0 + (double)Sz;
+    G[0] += (double)nx * S0;
+    G[1] += (double)ny * S0;
+    G[2] += (double)nz_lo * S0 + Sz;
     if (HAS_MU_FORCE) {
-      H[0] += (double)nx * (double)T0;
-      H[1] += (double)ny * (double)T0;
-      H[2] += (double)nz_lo * (double)T0 + (double)Tz;
+      H[0] += (double)nx * T0;
+      H[1] += (double)ny * T0;
+      H[2] += (double)nz_lo * T0 + Tz;
     }
   }
   Gpart[(size_t)blockIdx.y * natm + i] = make_double4(G[0], G[1], G[2], 0.0);
@@ -679,7 +659,6 @@ static __global__ void __launch_bounds__(128) k_rec_field_x2(const float2* __res
                                                       const float4* __restrict__ w, int natm,
                                                       RecMesh M, const int* __restrict__ rchunk,
                                                       const double2* __restrict__ rhoA,
-                                                      const double2* __restrict__ part, int npart,
                                                       double4* __restrict__ Gpart,
                                                       double4* __restrict__ Hpart,
                                                       const int* __restrict__ stop) {
@@ -692,7 +671,7 @@ static __global__ void __launch_bounds__(128) k_rec_field_x2(const float2* __res
   int k0 = M.rows[r0].w;
   int k1 = (r1 < M.nrows) ? M.rows[r1].w : M.nk;
   for (int k = k0 + threadIdx.x; k < k1; k += blockDim.x) {
-    double2 v = npart ? rho_prime(part, npart, M.Ak, M.nk, k) : rhoA[k];
+    const double2 v = rhoA[k];
     sh[k - k0] = make_float2((float)v.x, (float)v.y);
   }
   __syncthreads();

@@ -37,13 +37,7 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
 
-// FP32 -> TF32 bit pattern, round to nearest (ties away), low 13 bits zero
-__device__ __forceinline__ uint32_t tf32_rna(float x) {
-  uint32_t r;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-  return r;
-}
-
+// FP32 -> TF32 bit pattern, round to nearest (ties away), low 13 bits zero;
 // x = hi + lo with hi, lo TF32 (|x - hi - lo| <= 2^-22 |x|)
 __device__ __forceinline__ uint32_t tf32_round(uint32_t b) { return (b + 0x1000u) & 0xFFFFE000u; }
 __device__ __forceinline__ void tf32_split(float x, uint32_t& hi, uint32_t& lo) {
@@ -85,10 +79,6 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, long li
     if (ok) return true;
   }
   return false;
-}
-
-__device__ __forceinline__ void mbar_init(uint32_t bar) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar));
 }
 
 __device__ __forceinline__ void mma_tf32(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc,
@@ -181,10 +171,6 @@ __host__ __device__ constexpr size_t rho_tc_smem(int kx, int ky, int kz) {
 // the mesh fits one MMA's N and one CTA's shared memory
 inline bool rho_tc_fits(int kx, int ky, int kz) {
   return rho_tc_nr(kz) <= 256 && rho_tc_smem(kx, ky, kz) <= 227 * 1024;
-}
-
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, int bytes) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
 
 namespace tc {
