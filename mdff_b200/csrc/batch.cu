@@ -456,7 +456,8 @@ int finish(mdff_batch* h, mdff_batch_conf* conf) {
 // fixed part is the chain of barriers and latencies of a dipole solve (it does not shrink
 // with the cluster), par the pair loops (~ n^2) and the reciprocal sums (~ n nk).
 // Constants from 200 boxes of 64-200 and 10 of 100-900 ions (MgO type) over
-// C = 1..8; boxes without polarisation make one pass instead of a solve.
+// C = 1..8; boxes without polarisation make one pass instead of a solve (64, 216 and
+// 1000 NaCl ions, C = 1: 0.11, 0.28, 1.9 ms; C = 8: 0.08, 0.11, 0.32).
 struct BoxCost {
   double fixed, par;
 };
@@ -469,7 +470,9 @@ BoxCost box_cost(int n, int nk, int npol) {
 // nsm / C clusters (one CTA of 512 threads per SM).  Many boxes want C = 1 or 2
 // (256 boxes of 64-1000 ions, mixed: C = 1 8.0, 2 4.9, 4 6.7 ms; 200 of 64-200:
 // 1.3, 1.6, 2.7), few boxes large clusters (24 boxes of 64-300, FP64: C = 2
-// 1.04, 4 0.77, 8 0.69 ms).
+// 1.04, 4 0.77, 8 0.69 ms).  nsm / C is an upper bound: 33 clusters of 4 and 15 of 8 are
+// resident on 148 SMs, so that 16 equal small boxes get C = 8 and take two rounds
+// (64 MgO ions 0.80 ms, C = 4 0.38); the autotuner finds these.
 Shape default_shape(const std::vector<BoxCost>& cost, const std::vector<int>& order, int nsm) {
   Shape best{2, 512};
   double tbest = 1e300;
@@ -725,13 +728,6 @@ int create_impl(mdff_batch* h, const mdff_params* psets, int npsets, const mdff_
     h->err = "configurations too large for the shared-memory layout";
     return MDFF_ERR_BAD_ARGS;
   }
-  {
-    // the memory of the default shape (another one may yet be set: only its lack is an error here)
-    int ncl = 0;
-    if (prepare_shape(h, h->shape, &ncl) == MDFF_ERR_NOMEM) return MDFF_ERR_NOMEM;
-    h->err.clear();
-    cudaGetLastError();
-  }
   BCK(cudaStreamSynchronize(h->st));
   return MDFF_OK;
 }
@@ -835,6 +831,19 @@ int mdff_gpu_batch_create(const mdff_params* psets, int npsets, const mdff_batch
   *out = nullptr;
   mdff_batch* h = new mdff_batch();
   int s = create_impl(h, psets, npsets, desc);
+  if (!s) {
+    // the memory of the default shape (another one may yet be set: only its lack is an
+    // error here), taken when create_impl has given its host tables back: among them,
+    // the heap did not keep their pages for the next creation (host set-up of 256
+    // boxes 14 -> 31 ms)
+    int ncl = 0;
+    if (prepare_shape(h, h->shape, &ncl) == MDFF_ERR_NOMEM) {
+      s = MDFF_ERR_NOMEM;
+    } else {
+      h->err.clear();
+      cudaGetLastError();
+    }
+  }
   if (s) {
     g_berr = h->err;
     destroy_impl(h);
